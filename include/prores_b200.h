@@ -330,8 +330,8 @@ int prores_job_kernel_times(const void *job, int is_encode, const char **names, 
  * an output. None of these changes any decoded sample or encoded byte;
  * rivet_prores_b200.autotune times them on the device at hand. */
 typedef struct prores_tuning {
-    /* Rate-control costing runs a lane per slice component when the batch
-     * has at least this many components per SM, else a warp per component. */
+    /* Kept for callers that set it: rate-control costing runs a warp per
+     * slice component at every batch size, so the value steers nothing. */
     int32_t cost_lane_items_per_sm;
     /* Entropy decoder: warps per block (1-16), resident blocks per SM (0 =
      * as many as fit), and slice components a lane takes per grab of the

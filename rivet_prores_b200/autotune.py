@@ -2,10 +2,9 @@
 
 The shapes are the fields of `Tuning` (prores_tuning in the C ABI):
 
-* `cost_lane_items_per_sm`: the batch size (slice components per SM) from
-  which rate-control costing runs a lane per slice component rather than a
-  warp per component. Lanes need many components to fill the GPU; warps
-  finish a small batch sooner.
+* `cost_lane_items_per_sm`: not searched. Rate-control costing runs a warp
+  per slice component at every batch size, so the value steers nothing; the
+  evidence holds the encode's time by batch size.
 * `decode_fused`, `decode_slot_positions`: whether the per-slice decode
   runs as one kernel, and how many coefficient positions (so how many
   slices) one of its CTAs holds in shared memory at once.
@@ -169,7 +168,6 @@ def tune(device: int = 0, quick: bool = False, store: bool = True, frames: Optio
     say = log or (lambda s: None)
     ctx = context(device)
     tuning = ctx.tuning
-    sms = torch.cuda.get_device_properties(device).multi_processor_count
     cfg = Config(Profile.Hq)
     n_big = 8 if quick else 16
     frames = frames or workloads.uhd_422_hq(n_big, config=9, unique=4)
@@ -177,21 +175,15 @@ def tune(device: int = 0, quick: bool = False, store: bool = True, frames: Optio
     reps = 3 if quick else 5
     evidence: dict = {}
 
-    # Costing: lanes against warps by batch size.
-    sizes = [1, 4, n_big] if quick else [1, 2, 4, 8, 16]
-    points = []
+    # The encode by batch size (no shape of it is searched).
+    sizes = [1, n_big] if quick else [1, 4, 16]
+    evidence["cost"] = []
     for n in sizes:
         job = EncodeJob(frames[:n], cfg, device=device)
-        t = {}
-        for mode, items in (("lane", 0), ("warp", 1 << 30)):
-            ctx.set_tuning(type(tuning)(**{**asdict(tuning), "cost_lane_items_per_sm": items}))
-            t[mode] = _time(lambda: job.launch(stream), stream, reps)
-        slices = n * slices_in(frames[0])
-        points.append((slices, t["lane"], t["warp"]))
-        say(f"encode {n} frames: lane {t['lane']:.3f} ms, warp {t['warp']:.3f} ms")
+        ms = _time(lambda: job.launch(stream), stream, reps)
+        evidence["cost"].append({"slices": n * slices_in(frames[0]), "ms": round(ms, 4)})
+        say(f"encode {n} frames: {ms:.3f} ms")
         job.close()
-    tuning = type(tuning)(**{**asdict(tuning), "cost_lane_items_per_sm": lane_threshold(points, sms)})
-    evidence["cost"] = [{"slices": s, "lane_ms": round(a, 4), "warp_ms": round(b, 4)} for s, a, b in points]
 
     # Entropy decoder shapes.
     enc = EncodeJob(frames, cfg, device=device)

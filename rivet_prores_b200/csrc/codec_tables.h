@@ -69,6 +69,21 @@ PR_HD uint32_t cb_len(Codebook cb, uint32_t n32) {
     return cb.q + 1u + eg_len(n - threshold, cb.e);
 }
 
+// cb_len for symbols below 2^30, in 32-bit arithmetic.
+PR_HD uint32_t bit_len32(uint32_t v) {
+#if defined(__CUDA_ARCH__)
+    return 32u - (uint32_t)__clz((int)v);
+#else
+    return v ? 32u - (uint32_t)__builtin_clz(v) : 0u;
+#endif
+}
+PR_HD uint32_t cb_len32(Codebook cb, uint32_t n) {
+    const uint32_t threshold = cb.eg ? 0u : (uint32_t)(cb.q + 1) << cb.r;
+    if (n < threshold) return (n >> cb.r) + 1u + cb.r;
+    const uint32_t k = cb.eg ? cb.r : cb.e;
+    return (cb.eg ? 0u : cb.q + 1u) + 2u * bit_len32(n - threshold + (1u << k)) - k - 1u;
+}
+
 // The codeword for symbol n as its significant bits (the leading zeros are
 // implied by the length): Rice part `1` + r bits, or the exp-Golomb value
 // n - threshold + 2^e after q + 1 zeros.

@@ -365,31 +365,6 @@ struct LenTables {
     }
 };
 
-// The DC part of the bit count (src/encode.rs:383-395): EG5 of the first,
-// then Table 9 by |previous difference|, the sign flipped after a negative
-// one.
-template <class Get>
-__device__ __forceinline__ uint32_t dc_bits_of(Get get, uint32_t n_blocks, float inv0) {
-    uint32_t bits = 0;
-    int32_t prev_dc = 0, prev_diff = 3;
-    for (uint32_t i = 0; i < n_blocks; i++) {
-        const int32_t q = quantise1(get(i), inv0, 0.5f);
-        if (i == 0) {
-            bits += cb_len(kFirstDcBook, signed_to_symbol(q));
-        } else {
-            const int32_t diff = (int32_t)((uint32_t)q - (uint32_t)prev_dc);
-            bits += cb_len(dc_book(prev_diff), signed_to_symbol(prev_diff < 0 ? -diff : diff));
-            prev_diff = diff;
-        }
-        prev_dc = q;
-    }
-    return bits;
-}
-
-__device__ __forceinline__ uint32_t dc_bits(const float *f, uint32_t n_blocks, float inv0) {
-    return dc_bits_of([&](uint32_t i) { return __ldg(f + i); }, n_blocks, inv0);
-}
-
 // One AC position of a lane's walk: x = F inv, m = floor(|x| + 0.42)
 // (src/dsp/scalar.rs:19-39) as an integer; only a non-zero coefficient is
 // coded (its run from the last one, its level, both by context).
@@ -433,43 +408,8 @@ __device__ __forceinline__ bool chunk_is_zero(const float *cmax, const CompQuant
     return __ldg(cmax + j) < __ldg(q.chunk + j);
 }
 
-// Walks a component's AC positions (n_blocks onwards) in order, position by
-// position, skipping the chunks that quantise to zero; `emit` gets every
-// position's coefficient and inverse weight.
-template <class Emit>
-__device__ __forceinline__ void ac_walk_dense(const float *f, const float *cmax, uint32_t n_blocks,
-                                              const CompQuant &q, Emit emit) {
-    const uint32_t total = 64u * n_blocks;
-    const uint32_t shift = 31u - __clz(n_blocks);
-    for (uint32_t c0 = n_blocks & ~31u; c0 < total; c0 += 32) {
-        if (chunk_is_zero(cmax, q, c0 >> 5)) continue;
-        if (n_blocks >= 4) {
-            for (uint32_t p0 = max(c0, n_blocks); p0 < c0 + 32u; p0 += 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(f + p0));
-                const float iv = __ldg(q.inv + (p0 >> shift));
-                emit(v.x, iv, p0);
-                emit(v.y, iv, p0 + 1);
-                emit(v.z, iv, p0 + 2);
-                emit(v.w, iv, p0 + 3);
-            }
-        } else {
-            // Two blocks: positions 0 and 1 are the DCs; p and p + 1 share
-            // scan position p / 2.
-            for (uint32_t p0 = c0; p0 < c0 + 32u; p0 += 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(f + p0));
-                const float ia = __ldg(q.inv + (p0 >> 1)), ib = __ldg(q.inv + (p0 >> 1) + 1);
-                if (p0 > 0) {
-                    emit(v.x, ia, p0);
-                    emit(v.y, ia, p0 + 1);
-                }
-                emit(v.z, ib, p0 + 2);
-                emit(v.w, ib, p0 + 3);
-            }
-        }
-    }
-}
-
-// The same walk over candidates only: a chunk's candidate mask takes one
+// Walks the candidates of a component's AC positions (n_blocks onwards) in
+// order: chunks that quantise to zero are skipped, a chunk's candidate mask takes one
 // compare per coefficient against the non-zero bound of its position (so
 // it holds every non-zero, and each candidate is re-quantised exactly),
 // and the lane then visits the candidates alone. Suited to heavy per-code
@@ -504,172 +444,74 @@ __device__ __forceinline__ void ac_walk_sparse(const float *f, const float *cmax
     }
 }
 
-// The AC part of a lane's bit count at one position: the position is
-// quantised and its code length (run by the previous run's context, level
-// by the previous level's, a sign bit) taken from the length tables
-// whether or not it is a non-zero, and kept only if it is. Lanes that count
-// different components so stay in step, with no branch per position; only
-// a run or level past the tables (32 and above) takes a branch.
-struct AcCount {
-    uint32_t bits = 0, pos = 0, run_ctx = 4, level_ctx = 1;
+// Code lengths by context for the warps that count bits: of run symbols
+// below 63, and of level symbols below 127 with the sign bit added. The last
+// column stands for every symbol past those (kLongCode: no two lengths of
+// the rest add up to it).
+constexpr uint32_t kRunLens = 64, kLevelLens = 128, kLongCode = 128;
+struct CountTables {
+    // Both indices are context x kRow + symbol; a row is 33 words, so that
+    // neighbouring contexts lie in different banks.
+    static constexpr uint32_t kRow = 132;
+    uint8_t run[16][kRow];
+    uint8_t level[9][kRow];
+    __device__ void fill() {
+        for (uint32_t i = threadIdx.x; i < 16 * kRunLens; i += blockDim.x) {
+            const uint32_t c = i / kRunLens, n = i % kRunLens;
+            run[c][n] = (uint8_t)(n + 1u < kRunLens ? cb_len32(run_book(c), n) : kLongCode);
+        }
+        for (uint32_t i = threadIdx.x; i < 9 * kLevelLens; i += blockDim.x) {
+            const uint32_t c = i / kLevelLens, n = i % kLevelLens;
+            level[c][n] = (uint8_t)(n + 1u < kLevelLens ? cb_len32(level_book(c), n) + 1u : kLongCode);
+        }
+    }
 };
 
-__device__ __forceinline__ void count_position(AcCount &c, float f, float inv, uint32_t p, const LenTables &t) {
-    const int32_t m = magnitude(__fmul_rn(f, inv), kAcRounding);
-    const bool nz = m >= 1;
-    const uint32_t run = p - c.pos;
-    const uint32_t level = (uint32_t)m - 1u;
-    uint32_t add = (uint32_t)t.run[c.run_ctx][min(run, 31u)] + (uint32_t)t.level[c.level_ctx][min(level, 31u)] + 1u;
-    if (nz && (run | level) >= 32u)
-        add = cb_len(run_book(c.run_ctx), run) + cb_len(level_book(c.level_ctx), level) + 1u;
-    if (nz) {
-        c.bits += add;
-        c.run_ctx = min(run, 15u);
-        c.level_ctx = min(level, 8u);
-        c.pos = p + 1u;
+// A warp's non-zeros on their way from the quantiser to the code tables, in
+// scanned order: (position << 16) + level symbol, both below 2^15 (a
+// component with larger levels, which only samples far above their depth's
+// range can make, is counted by warp_wide_bits). The two entries before the
+// first hold the state a component starts with (previous run 4, previous
+// level 1), then the last two counted.
+constexpr uint32_t kGroupChunks = 16;  // 32-coefficient chunks quantised before codes are counted
+constexpr uint32_t kNonzeroBuf = 2 + 63 + 32 * kGroupChunks + 3;
+constexpr uint32_t kWeightsAt = kNonzeroBuf, kIdsAt = kNonzeroBuf + 64;
+// Words of shared memory a warp's count takes: its list, then the inverse
+// weights and chunk numbers it works with.
+constexpr uint32_t kCountWords = kIdsAt + 12;
+// |F| from here on may make a level symbol of 2^15: 8 / (W qScale) is at most 4.
+constexpr float kWideCoef = 8191.0f;
+
+// The bits of a run and level (with its sign) past the tables: `n` its entry
+// less the position before it, `k` the same of the non-zero before it.
+__device__ __noinline__ uint32_t long_code_bits(uint32_t e0, uint32_t e1, uint32_t e2) {
+    const uint32_t run = (e0 >> 16) - (e1 >> 16) - 1u;
+    const uint32_t prev_run = ((e1 >> 16) - (e2 >> 16) - 1u) & 0xFFFFu;
+    return cb_len32(run_book(prev_run), run) + cb_len32(level_book(e1 & 0xFFFFu), e0 & 0xFFFFu) + 1u;
+}
+
+// Bits of two neighbouring non-zeros, the entries c = (c.x, c.y) after the
+// two before them, b: each one's run by the run before it, its level by the
+// level before it, and a sign. All contexts are in the four entries, so
+// every pair is counted by its own lane. Run and level go through every
+// step as the two halves of a word: an entry less the position before it
+// and 1, clamped to the tables' last columns or to the contexts' last rows,
+// is one instruction.
+__device__ __forceinline__ uint32_t pair_bits(uint2 b, uint2 c, const CountTables &t, bool second) {
+    constexpr uint32_t kLast = ((kRunLens - 1u) << 16) | (kLevelLens - 1u), kRows = (15u << 16) | 8u;
+    const uint32_t nbx = ~b.x & 0xFFFF0000u, nby = ~b.y & 0xFFFF0000u, ncx = ~c.x & 0xFFFF0000u;
+    const uint32_t i0 = __viaddmin_s16x2(b.y, nbx, kRows) * CountTables::kRow + __viaddmin_s16x2(c.x, nby, kLast);
+    const uint32_t i1 = __viaddmin_s16x2(c.x, nby, kRows) * CountTables::kRow + __viaddmin_s16x2(c.y, ncx, kLast);
+    const uint8_t *run = &t.run[0][0], *level = &t.level[0][0];
+    uint32_t l0 = (uint32_t)run[i0 >> 16] + level[i0 & 0xFFFFu];
+    uint32_t l1 = (uint32_t)run[i1 >> 16] + level[i1 & 0xFFFFu];
+    if ((l0 | l1) >= kLongCode) {
+        if (l0 >= kLongCode) l0 = long_code_bits(c.x, b.y, b.x);
+        if (l1 >= kLongCode && second) l1 = long_code_bits(c.y, c.x, b.y);
     }
+    return second ? l0 + l1 : l0;
 }
 
-// Bits of one quantised component (src/encode.rs:398-409), one lane: the
-// crate's own walk over the scanned positions.
-__device__ uint32_t lane_component_bits(const float *f, const float *cmax, uint32_t n_blocks, const CompQuant &q,
-                                        const LenTables &t) {
-    AcCount c;
-    c.pos = n_blocks;
-    ac_walk_dense(f, cmax, n_blocks, q, [&](float v, float inv, uint32_t p) { count_position(c, v, inv, p, t); });
-    return dc_bits(f, n_blocks, __ldg(q.inv)) + c.bits;
-}
-
-// The same count over the candidates of each chunk only (the writer's
-// walk): the candidate masks cost a compare a coefficient, and only the
-// candidates are quantised and coded. Faster than the position-by-position
-// walk where most coefficients quantise to zero (coarse quantisers), slower
-// where most do not.
-__device__ uint32_t lane_component_bits_sparse(const float *f, const float *cmax, uint32_t n_blocks,
-                                               const CompQuant &q, const LenTables &t) {
-    uint32_t bits = 0;
-    ac_walk_sparse(f, cmax, n_blocks, q, [&](AcWalk &w, uint32_t run, uint32_t level, bool) {
-        bits += t.run_len(w.prev_run, run) + t.level_len(w.prev_level, level) + 1u;
-    });
-    return dc_bits(f, n_blocks, __ldg(q.inv)) + bits;
-}
-
-// Code lengths of a run and of a level by context, from the tables when
-// they hold the symbol (src/vlc.rs:397-415).
-__device__ __forceinline__ uint32_t run_len_of(const LenTables &t, uint32_t ctx, uint32_t r) {
-    return r < 32u ? t.run[ctx][r] : cb_len(run_book(ctx), r);
-}
-__device__ __forceinline__ uint32_t level_len_of(const LenTables &t, uint32_t ctx, uint32_t l) {
-    return l < 32u ? t.level[ctx][l] : cb_len(level_book(ctx), l);
-}
-
-// Bits of one quantised component (src/encode.rs:398-409), split over a
-// group of kSeg lanes, for short launches bound by one lane's walk: lane r
-// walks the r-th run of chunks as if the walk started there (previous run
-// 4, previous level 1, last position its start), which gets every code
-// right but the segment's first (run and level by the previous segment's
-// state) and its second's run (by the first's run). Lanes past the first
-// also find their segment's first two non-zeros, and the group's first
-// lane puts the segments together in order, replacing those codes with the
-// right ones: the sum is the one-lane walk's. Every lane of the warp takes
-// part (the exchange is by shuffles); `active` is false for lanes past the
-// work.
-template <int kSeg>
-__device__ uint32_t group_component_bits(bool active, const float *f, const float *cmax, uint32_t nb,
-                                         const CompQuant &q, const LenTables &t) {
-    const uint32_t lane = threadIdx.x & 31u, r = lane % (uint32_t)kSeg, base = lane - r;
-    const uint32_t chunks = active ? 2u * nb : 0u;
-    const uint32_t c_lo = chunks * r / kSeg, c_hi = chunks * (r + 1) / kSeg;
-    const uint32_t shift = active ? 31u - __clz(nb) : 0u;
-    const uint32_t start = r == 0 ? nb : 32u * c_lo;
-    AcCount c;
-    c.pos = start;
-    for (uint32_t k = c_lo; k < c_hi; k++) {
-        if (chunk_is_zero(cmax, q, k)) continue;
-        const uint32_t c0 = 32u * k;
-        if (nb >= 4) {
-            for (uint32_t p0 = max(c0, nb); p0 < c0 + 32u; p0 += 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(f + p0));
-                const float iv = __ldg(q.inv + (p0 >> shift));
-                count_position(c, v.x, iv, p0, t);
-                count_position(c, v.y, iv, p0 + 1, t);
-                count_position(c, v.z, iv, p0 + 2, t);
-                count_position(c, v.w, iv, p0 + 3, t);
-            }
-        } else {
-            for (uint32_t p0 = c0; p0 < c0 + 32u; p0 += 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(f + p0));
-                const float ia = __ldg(q.inv + (p0 >> 1)), ib = __ldg(q.inv + (p0 >> 1) + 1);
-                if (p0 > 0) {
-                    count_position(c, v.x, ia, p0, t);
-                    count_position(c, v.y, ia, p0 + 1, t);
-                }
-                count_position(c, v.z, ib, p0 + 2, t);
-                count_position(c, v.w, ib, p0 + 3, t);
-            }
-        }
-    }
-    // The segment's first two non-zeros (lanes past the first).
-    uint32_t found = 0, q1 = 0, l1 = 0, q2 = 0;
-    if (r > 0) {
-        for (uint32_t k = c_lo; k < c_hi && found < 2u; k++) {
-            if (chunk_is_zero(cmax, q, k)) continue;
-            for (uint32_t p = 32u * k; p < 32u * k + 32u && found < 2u; p++) {
-                const int32_t m = magnitude(__fmul_rn(__ldg(f + p), __ldg(q.inv + (p >> shift))), kAcRounding);
-                if (m >= 1) {
-                    if (found == 0) {
-                        q1 = p;
-                        l1 = (uint32_t)m - 1u;
-                    } else {
-                        q2 = p;
-                    }
-                    found++;
-                }
-            }
-        }
-    }
-    // Put the segments together on the group's first lane.
-    uint32_t bits = c.bits, pos = c.pos, rctx = c.run_ctx, lctx = c.level_ctx;
-#pragma unroll
-    for (int j = 1; j < kSeg; j++) {
-        const uint32_t src = base + (uint32_t)j;
-        const uint32_t s_bits = __shfl_sync(0xffffffffu, c.bits, src);
-        const uint32_t s_found = __shfl_sync(0xffffffffu, found, src);
-        const uint32_t s_q1 = __shfl_sync(0xffffffffu, q1, src);
-        const uint32_t s_l1 = __shfl_sync(0xffffffffu, l1, src);
-        const uint32_t s_q2 = __shfl_sync(0xffffffffu, q2, src);
-        const uint32_t s_start = __shfl_sync(0xffffffffu, start, src);
-        const uint32_t s_pos = __shfl_sync(0xffffffffu, c.pos, src);
-        const uint32_t s_rctx = __shfl_sync(0xffffffffu, c.run_ctx, src);
-        const uint32_t s_lctx = __shfl_sync(0xffffffffu, c.level_ctx, src);
-        if (r == 0 && s_found > 0) {
-            const uint32_t run1 = s_q1 - pos, run1_seg = s_q1 - s_start;
-            // The first code: right contexts and run, in place of the
-            // segment's own (unsigned arithmetic: the sum comes out right).
-            bits += s_bits + run_len_of(t, rctx, run1) + level_len_of(t, lctx, s_l1) -
-                    run_len_of(t, 4u, run1_seg) - level_len_of(t, 1u, s_l1);
-            if (s_found == 1) {
-                pos = s_q1 + 1u;
-                rctx = min(run1, 15u);
-                lctx = min(s_l1, 8u);
-            } else {
-                // The second code's run by the first's right run.
-                const uint32_t run2 = s_q2 - s_q1 - 1u;
-                bits += run_len_of(t, min(run1, 15u), run2) - run_len_of(t, min(run1_seg, 15u), run2);
-                pos = s_pos;
-                rctx = s_rctx;
-                lctx = s_lctx;
-            }
-        }
-    }
-    return (r == 0 && active) ? dc_bits(f, nb, __ldg(q.inv)) + bits : 0u;
-}
-
-// The same count with a whole warp on one component, for when latency
-// matters more than throughput (few items, or one slice the share-out
-// needs): lane l takes scanned positions 32 k + l; a non-zero's run and its
-// contexts (the previous non-zero's run and level symbol) come from the
-// lanes below it or from what the last step carried.
 // kShared: f and cmax point into shared memory (plain loads); else into
 // global memory (read-only loads).
 template <bool kShared>
@@ -680,55 +522,226 @@ __device__ __forceinline__ float coef_load(const float *f, uint32_t i) {
         return __ldg(f + i);
 }
 
-template <bool kShared = false>
-__device__ uint32_t warp_component_bits(const float *f, const float *cmax, uint32_t n_blocks, const CompQuant &cq,
-                                        const LenTables &t) {
-    const float *inv = cq.inv;
-    const int lane = threadIdx.x & 31;
-    const uint32_t total = 64u * n_blocks;
+// What a component's count starts from, loaded ahead: each lane's two chunk
+// maxima and its DC.
+struct CompHead {
+    float max_lo, max_hi, dc;
+};
+
+template <bool kShared>
+__device__ __forceinline__ CompHead comp_head(const float *f, const float *cmax, uint32_t n_blocks) {
+    const uint32_t lane = threadIdx.x & 31u, chunks = 2u * n_blocks;
+    CompHead h{0.0f, 0.0f, 0.0f};
+    if (lane < chunks) h.max_lo = coef_load<kShared>(cmax, lane);
+    if (lane + 32u < chunks) h.max_hi = coef_load<kShared>(cmax, lane + 32u);
+    if (lane < n_blocks) h.dc = coef_load<kShared>(f, lane);
+    return h;
+}
+
+// A warp's list of non-zeros: filled 32 coefficients at a time, counted 64
+// non-zeros at a time.
+struct NonzeroList {
+    uint32_t *buf;
+    uint32_t first, end;  // shared addresses of buf + 2 and past the last entry
+    uint32_t bits;
+    __device__ __forceinline__ void start(uint32_t *b, uint32_t n_blocks) {
+        buf = b;
+        first = end = (uint32_t)__cvta_generic_to_shared(b + 2);
+        bits = 0;
+        if ((threadIdx.x & 31u) == 0) {
+            b[0] = (n_blocks - 6u) << 16;
+            b[1] = ((n_blocks - 1u) << 16) | 1u;
+        }
+    }
+    // A lane's coefficient of a chunk; tag = (position << 16) - 0x4B000001.
+    // The store is a predicated instruction: as a branch it took about as
+    // many instructions again as all the rest.
+    __device__ __forceinline__ void add(float v, float inv, uint32_t tag, uint32_t below) {
+        // y = |F inv| + 0.42 (src/dsp/scalar.rs:19-39); adding 2^23 rounded
+        // down leaves floor(y) in the low bits.
+        const float y = __fadd_rn(fabsf(__fmul_rn(v, inv)), kAcRounding);
+        const uint32_t b = __ballot_sync(0xffffffffu, y >= 1.0f);
+        const uint32_t at = end + 4u * __popc(b & below);
+        const uint32_t entry = __float_as_uint(__fadd_rd(y, 8388608.0f)) + tag;
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %2, 0f3F800000;\n\t@p st.shared.u32 [%0], %1;\n\t}"
+                     :
+                     : "r"(at), "r"(entry), "f"(y)
+                     : "memory");
+        end += 4u * __popc(b);
+    }
+    // Counts the whole groups of 64; what is left, and the two entries
+    // before it, go to the front.
+    __device__ __forceinline__ void count(const CountTables &t) {
+        const uint32_t lane = threadIdx.x & 31u;
+        __syncwarp();
+        const uint32_t full = ((end - first) >> 2) & ~63u;
+        if (full) {
+            const uint2 *q = reinterpret_cast<const uint2 *>(buf) + lane;
+#pragma unroll 1
+            for (const uint2 *stop = q + full / 2u; q < stop; q += 32) bits += pair_bits(q[0], q[1], t, true);
+            const uint2 keep = q[0];
+            const uint32_t last = buf[full + 64u];
+            __syncwarp();
+            reinterpret_cast<uint2 *>(buf)[lane] = keep;
+            if (lane == 0) buf[64] = last;
+            __syncwarp();
+            end -= 4u * full;
+        }
+    }
+    __device__ __forceinline__ uint32_t finish(const CountTables &t) {
+        const uint32_t lane = threadIdx.x & 31u;
+        const uint2 *q = reinterpret_cast<const uint2 *>(buf) + lane;
+        const int32_t n = (int32_t)((end - first) >> 2) - (int32_t)(2u * lane);
+        if (n > 0) {
+            uint2 c = q[1];
+            if (n == 1) c.y = c.x + (1u << 16);  // no entry there: any valid one, not counted
+            bits += pair_bits(q[0], c, t, n > 1);
+        }
+        return bits;
+    }
+};
+
+// The AC part of warp_component_bits for a component of 2^kLog blocks, every
+// chunk in turn.
+template <int kLog, bool kShared>
+__device__ __forceinline__ uint32_t warp_dense_bits(const float *f, const float *inv, const CountTables &t,
+                                                    uint32_t *buf) {
+    constexpr uint32_t kBlocks = 1u << kLog, kChunks = 2u * kBlocks;
+    constexpr uint32_t kGroup = kChunks < kGroupChunks ? kChunks : kGroupChunks;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t below = (1u << lane) - 1u;
+    // The 64 inverse weights, where every chunk finds its own at a constant
+    // distance: chunk c's scanned position of this lane is 32 c + lane, its
+    // weight's place (32 c >> kLog) + (lane >> kLog).
+    float *w = reinterpret_cast<float *>(buf + kWeightsAt);
+    w[lane] = __ldg(inv + lane);
+    w[lane + 32u] = __ldg(inv + lane + 32u);
+    __syncwarp();
+    w += lane >> kLog;
+    NonzeroList list;
+    list.start(buf, kBlocks);
+    f += lane;
+#pragma unroll 1
+    for (uint32_t g = 0; g < kChunks; g += kGroup) {
+        float v[kGroup], iv[kGroup];
+#pragma unroll
+        for (uint32_t i = 0; i < kGroup; i++) v[i] = coef_load<kShared>(f, 32u * i);
+#pragma unroll
+        for (uint32_t i = 0; i < kGroup; i++) iv[i] = w[(32u * i) >> kLog];
+        if (g == 0 && lane < kBlocks) v[0] = 0.0f;  // position `lane` of chunk 0 is a DC
+        const uint32_t tag = ((32u * g + lane) << 16) - 0x4B000001u;
+#pragma unroll
+        for (uint32_t i = 0; i < kGroup; i++) list.add(v[i], iv[i], tag + (i << 21), below);
+        list.count(t);
+        f += 32u * kGroup;
+        w += (32u * kGroup) >> kLog;
+    }
+    return list.finish(t);
+}
+
+// The same for a component with few chunks that may hold a non-zero, whose
+// numbers are the first `n` bytes of `chunks`: 8 of them in flight at a time.
+template <bool kShared>
+__device__ __forceinline__ uint32_t warp_sparse_bits(const float *f, const float *inv, uint32_t n_blocks,
+                                                     const uint8_t *chunks, uint32_t n, const CountTables &t,
+                                                     uint32_t *buf) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t below = (1u << lane) - 1u;
     const uint32_t shift = 31u - __clz(n_blocks);
-    uint32_t bits = 0;
-    int32_t carry_pos = (int32_t)n_blocks - 1;
-    uint32_t carry_run = 4, carry_level = 1;
-    for (uint32_t base = 0; base < total; base += 32) {
-        // Past the DCs a chunk that quantises to zero changes nothing.
-        if (base > 0 && coef_load<kShared>(cmax, base >> 5) < __ldg(cq.chunk + (base >> 5))) continue;
-        const uint32_t p = base + lane;
-        const uint32_t sidx = p >> shift;
-        const int32_t q = quantise1(coef_load<kShared>(f, p), __ldg(inv + sidx), sidx == 0 ? 0.5f : kAcRounding);
-        if (base == 0) {
-            // The DCs (n_blocks <= 32, all in this step).
-            const int32_t left = __shfl_up_sync(0xffffffffu, q, 1);
-            const int32_t diff = (int32_t)((uint32_t)q - (uint32_t)left);
-            const int32_t prev_diff_raw = __shfl_up_sync(0xffffffffu, diff, 1);
-            if (p < n_blocks) {
-                if (p == 0) {
-                    bits += cb_len(kFirstDcBook, signed_to_symbol(q));
-                } else {
-                    const int32_t prev_diff = p == 1 ? 3 : prev_diff_raw;
-                    bits += cb_len(dc_book(prev_diff), signed_to_symbol(prev_diff < 0 ? -diff : diff));
-                }
+    NonzeroList list;
+    list.start(buf, n_blocks);
+#pragma unroll 1
+    for (uint32_t k = 0; k < n; k += 8) {
+        float v[8], iv[8];
+        uint32_t p[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++) {
+            p[i] = 32u * chunks[k + i] + lane;
+            v[i] = iv[i] = 0.0f;
+            if (k + i < n) {
+                v[i] = coef_load<kShared>(f, p[i]);
+                iv[i] = __ldg(inv + (p[i] >> shift));
             }
         }
-        const bool nz = q != 0 && p >= n_blocks;
-        const uint32_t mask = __ballot_sync(0xffffffffu, nz);
-        if (mask == 0) continue;
-        const uint32_t below = mask & ((1u << lane) - 1u);
-        const int src = below ? 31 - __clz(below) : lane;
-        const int32_t prev_pos = below ? (int32_t)(base + src) : carry_pos;
-        const uint32_t run = nz ? (uint32_t)((int32_t)p - prev_pos - 1) : 0u;
-        const uint32_t level = nz ? (q < 0 ? 0u - (uint32_t)q : (uint32_t)q) - 1u : 0u;
-        const uint32_t src_run = __shfl_sync(0xffffffffu, run, src);
-        const uint32_t src_level = __shfl_sync(0xffffffffu, level, src);
-        if (nz) bits += t.run_len(below ? src_run : carry_run, run) + t.level_len(below ? src_level : carry_level, level) + 1u;
-        const int top = 31 - __clz(mask);
-        carry_pos = (int32_t)(base + top);
-        carry_run = __shfl_sync(0xffffffffu, run, top);
-        carry_level = __shfl_sync(0xffffffffu, level, top);
-    }
+        if (p[0] < n_blocks) v[0] = 0.0f;  // the DCs
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) bits += __shfl_xor_sync(0xffffffffu, bits, o);
+        for (uint32_t i = 0; i < 8; i++)
+            if (k + i < n) list.add(v[i], iv[i], (p[i] << 16) - 0x4B000001u, below);
+        list.count(t);
+    }
+    return list.finish(t);
+}
+
+// The same for levels of any size, by one lane's walk: only a component whose
+// largest |F| reaches kWideCoef comes here.
+template <bool kShared>
+__device__ __noinline__ uint32_t warp_wide_bits(const float *f, const float *inv, uint32_t n_blocks) {
+    uint32_t bits = 0;
+    if ((threadIdx.x & 31u) == 0) {
+        const uint32_t shift = 31u - __clz(n_blocks);
+        uint32_t prev_run = 4, prev_level = 1, pos = n_blocks;
+        for (uint32_t p = n_blocks; p < 64u * n_blocks; p++) {
+            const int32_t m = magnitude(__fmul_rn(coef_load<kShared>(f, p), __ldg(inv + (p >> shift))), kAcRounding);
+            if (m < 1) continue;
+            const uint32_t run = p - pos, level = (uint32_t)m - 1u;
+            bits += cb_len(run_book(prev_run), run) + cb_len(level_book(prev_level), level) + 1u;
+            prev_run = run;
+            prev_level = level;
+            pos = p + 1u;
+        }
+    }
     return bits;
+}
+
+// Bits of one quantised component (src/encode.rs:398-409), the whole warp.
+// Two stages, a group of 16 chunks at a time: the warp quantises a chunk's 32
+// coefficients, one a lane (loads of 128 contiguous bytes, all of a group's
+// in flight at once), and appends the non-zeros to a list in order by ballot
+// and popcount; then each lane takes two neighbouring non-zeros of a full 64
+// and looks their code lengths up. So zeros cost no per-code work, and no
+// code waits for the one before it. Where most chunks quantise to zero only
+// the others are read. Every lane gets the sum.
+template <bool kShared = false>
+__device__ __forceinline__ uint32_t warp_component_bits(const float *f, const CompHead &h, uint32_t n_blocks, const CompQuant &cq,
+                                        const CountTables &t, uint32_t *buf) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t below = (1u << lane) - 1u;
+    const uint32_t chunks = 2u * n_blocks;
+    // The chunks that hold a candidate.
+    const uint32_t live_lo = __ballot_sync(0xffffffffu, lane < chunks && h.max_lo >= __ldg(cq.chunk + lane));
+    uint32_t live_hi = 0;
+    if (n_blocks == 32u) live_hi = __ballot_sync(0xffffffffu, h.max_hi >= __ldg(cq.chunk + lane + 32u));
+    // The DCs (n_blocks <= 32), a lane each: EG5 of the first, then Table 9
+    // by |previous difference|, the sign flipped after a negative one.
+    const int32_t q = quantise1(h.dc, __ldg(cq.inv), 0.5f);
+    const int32_t left = __shfl_up_sync(0xffffffffu, q, 1);
+    const int32_t diff = (int32_t)((uint32_t)q - (uint32_t)left);
+    const int32_t before = __shfl_up_sync(0xffffffffu, diff, 1);
+    const int32_t prev_diff = lane == 1 ? 3 : before;
+    const Codebook book = lane == 0 ? kFirstDcBook : dc_book(prev_diff);
+    const uint32_t symbol = signed_to_symbol(lane == 0 ? q : (prev_diff < 0 ? -diff : diff));
+    uint32_t bits = lane < n_blocks ? cb_len32(book, symbol) : 0u;
+    const uint32_t n_live = __popc(live_lo) + __popc(live_hi);
+    __syncwarp();  // the last component's entries are read
+    if (__any_sync(0xffffffffu, fmaxf(h.max_lo, h.max_hi) >= kWideCoef)) {
+        bits += warp_wide_bits<kShared>(f, cq.inv, n_blocks);
+    } else if (8u * n_live > 5u * chunks) {
+        switch (n_blocks) {
+        case 32: bits += warp_dense_bits<5, kShared>(f, cq.inv, t, buf); break;
+        case 16: bits += warp_dense_bits<4, kShared>(f, cq.inv, t, buf); break;
+        case 8: bits += warp_dense_bits<3, kShared>(f, cq.inv, t, buf); break;
+        case 4: bits += warp_dense_bits<2, kShared>(f, cq.inv, t, buf); break;
+        default: bits += warp_dense_bits<1, kShared>(f, cq.inv, t, buf); break;
+        }
+    } else if (n_live) {
+        // The live chunks' numbers, in order (at most 40, read 8 at a time).
+        uint8_t *ids = reinterpret_cast<uint8_t *>(buf + kIdsAt);
+        if ((live_lo >> lane) & 1u) ids[__popc(live_lo & below)] = (uint8_t)lane;
+        if ((live_hi >> lane) & 1u) ids[__popc(live_lo) + __popc(live_hi & below)] = (uint8_t)(lane + 32u);
+        __syncwarp();
+        bits += warp_sparse_bits<kShared>(f, cq.inv, n_blocks, ids, n_live, t, buf);
+    }
+    return __reduce_add_sync(0xffffffffu, bits);
 }
 
 // The quantiser table of quantization_index qi (layout beside kQuantStride).
@@ -743,83 +756,75 @@ __device__ __forceinline__ void comp_layout(const EncFrameDesc &fd, uint32_t mbs
     offset = comp == 0 ? 0u : 64u * mbs * (4u + (comp - 1u) * cpm);
 }
 
-// From this quantiser index up, a lane costs a component over its chunks'
-// candidates only (measured on UHD 4:2:2 10-bit: 1.5x faster at 56, 1.1x
-// slower at 28).
-constexpr uint32_t kSparseCostQi = 40;
-
-// Bytes of one slice component at quantiser qi (one lane).
-__device__ __forceinline__ uint32_t component_bytes(const EncodeLaunch &e, const EncSliceDesc &sd, const EncPicDesc &pd,
-                                                    const EncFrameDesc &fd, uint32_t comp, uint32_t qi,
-                                                    const LenTables &t) {
-    uint32_t nb, off;
-    comp_layout(fd, sd.mbs, comp, nb, off);
-    const CompQuant q = comp_quant(quant_base(e, pd, qi), comp, nb);
-    const float *f = e.coef + sd.coef + off, *cmax = e.coef_max + ((sd.coef + off) >> 5);
-    const uint32_t bits = qi >= kSparseCostQi ? lane_component_bits_sparse(f, cmax, nb, q, t)
-                                              : lane_component_bits(f, cmax, nb, q, t);
-    return (bits + 7u) / 8u;
-}
-
 // Bytes of one slice component at quantiser qi, the whole warp.
 __device__ __forceinline__ uint32_t warp_component_bytes(const EncodeLaunch &e, const EncSliceDesc &sd,
                                                          const EncPicDesc &pd, const EncFrameDesc &fd, uint32_t comp,
-                                                         uint32_t qi, const LenTables &t) {
+                                                         uint32_t qi, const CountTables &t, uint32_t *buf) {
     uint32_t nb, off;
     comp_layout(fd, sd.mbs, comp, nb, off);
     const CompQuant q = comp_quant(quant_base(e, pd, qi), comp, nb);
-    const uint32_t bits = warp_component_bits(e.coef + sd.coef + off, e.coef_max + ((sd.coef + off) >> 5), nb, q, t);
+    const float *f = e.coef + sd.coef + off;
+    const uint32_t bits =
+        warp_component_bits(f, comp_head<false>(f, e.coef_max + ((sd.coef + off) >> 5), nb), nb, q, t, buf);
     return (bits + 7u) / 8u;
 }
 
 constexpr int kCostThreads = 256;
+constexpr int kCostBlocks = 4;  // CTAs an SM
 
-// Work items are (component, slice), component-major: a warp's lanes take
-// the same component of 32 neighbouring slices, which cost about the same
-// (and whose zero chunks mostly coincide, so the lanes skip them together).
-// Persistent: as many CTAs as are resident, each warp taking 32 items at a
-// time from the probe's counter, so no warp waits for the slowest of its
-// CTA and the last wave is not left part-empty.
-__global__ void __launch_bounds__(kCostThreads, 6) k_cost(EncodeLaunch e, int step) {
-    __shared__ LenTables t;
+// A warp per slice component, (component, slice) component-major. A warp
+// takes `take` neighbouring items (at most 32) from the probe's counter at a
+// time: its lanes look the items' places up side by side, so the chain of
+// descriptor loads is waited for once, and the items are costed in turn.
+__global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost(EncodeLaunch e, int step, uint32_t take) {
+    __shared__ CountTables t;
+    __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     t.fill();
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t items = 3u * e.n_slices;
     for (;;) {
         uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(e.cost_taken + step, 32u);
+        if (lane == 0) base = atomicAdd(e.cost_taken + step, take);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= items) break;
+        // This lane's item: its first coefficient (a multiple of 64), its
+        // quantiser table and component group, its block count (0: none).
         const uint32_t item = base + lane;
-        if (item >= items) continue;
         const uint32_t comp = item / e.n_slices, s = item - comp * e.n_slices;
-        const EncSliceDesc sd = e.slices[s];
-        const int32_t qi = e.state[sd.pic].probe_qi;
-        if (qi == 0) continue;
-        const EncPicDesc &pd = e.pics[sd.pic];
-        const EncFrameDesc &fd = e.frames[pd.frame];
-        e.probe_comp[((uint64_t)step * e.n_slices + s) * 3u + comp] =
-            component_bytes(e, sd, pd, fd, comp, (uint32_t)qi, t);
+        uint32_t my_coef = 0, my_quant = 0, my_blocks = 0, my_bytes = 0;
+        if (lane < take && item < items) {
+            const EncSliceDesc sd = e.slices[s];
+            const int32_t qi = e.state[sd.pic].probe_qi;
+            const EncPicDesc &pd = e.pics[sd.pic];
+            uint32_t off;
+            comp_layout(e.frames[pd.frame], sd.mbs, comp, my_blocks, off);
+            my_coef = (uint32_t)((sd.coef + off) >> 6);
+            my_quant = ((pd.quant * 225u + (uint32_t)qi) << 1) | (comp > 0 ? 1u : 0u);
+            if (qi == 0) my_blocks = 0;
+        }
+        const uint32_t costed = __ballot_sync(0xffffffffu, my_blocks != 0);
+        const auto head = [&](uint32_t j) {
+            const uint64_t coef = (uint64_t)__shfl_sync(0xffffffffu, my_coef, j) << 6;
+            return comp_head<false>(e.coef + coef, e.coef_max + (coef >> 5), __shfl_sync(0xffffffffu, my_blocks, j));
+        };
+        // The next item's maxima and DCs are on their way while one is costed.
+        CompHead next{};
+        if (costed) next = head((uint32_t)__ffs(costed) - 1u);
+        for (uint32_t left = costed; left;) {
+            const uint32_t j = (uint32_t)__ffs(left) - 1u;
+            left &= left - 1u;
+            const CompHead h = next;
+            if (left) next = head((uint32_t)__ffs(left) - 1u);
+            const uint32_t nb = __shfl_sync(0xffffffffu, my_blocks, j);
+            const uint32_t quant = __shfl_sync(0xffffffffu, my_quant, j);
+            const uint64_t coef = (uint64_t)__shfl_sync(0xffffffffu, my_coef, j) << 6;
+            const CompQuant q = comp_quant(e.quant + (uint64_t)(quant >> 1) * kQuantStride, quant & 1u, nb);
+            const uint32_t bits = warp_component_bits(e.coef + coef, h, nb, q, t, buf[threadIdx.x >> 5]);
+            if (lane == j) my_bytes = (bits + 7u) / 8u;
+        }
+        if ((costed >> lane) & 1u) e.probe_comp[((uint64_t)step * e.n_slices + s) * 3u + comp] = my_bytes;
     }
-}
-
-// k_cost with a warp per item, for batches too small to fill the GPU with
-// one lane per item.
-__global__ void __launch_bounds__(kCostThreads) k_cost_warp(EncodeLaunch e, int step) {
-    __shared__ LenTables t;
-    t.fill();
-    __syncthreads();
-    const uint32_t item = blockIdx.x * (kCostThreads / 32) + (threadIdx.x >> 5);
-    if (item >= 3u * e.n_slices) return;
-    const uint32_t s = item / 3u, comp = item - 3u * s;
-    const EncSliceDesc sd = e.slices[s];
-    const int32_t qi = e.state[sd.pic].probe_qi;
-    if (qi == 0) return;
-    const EncPicDesc &pd = e.pics[sd.pic];
-    const EncFrameDesc &fd = e.frames[pd.frame];
-    const uint32_t bytes = warp_component_bytes(e, sd, pd, fd, comp, (uint32_t)qi, t);
-    if ((threadIdx.x & 31) == 0) e.probe_comp[((uint64_t)step * e.n_slices + s) * 3u + comp] = bytes;
 }
 
 // A slice's size from its component bytes, and whether every 16-bit size
@@ -904,46 +909,22 @@ __global__ void __launch_bounds__(kCostThreads) k_window_select(EncodeLaunch e, 
 }
 
 // Costs the listed slices at window level `level` (quantiser uniform - 1 -
-// level): a lane per (component, slice), component-major, or a warp each.
-// Lanes per component in the window levels' lane mode: these launches cover
-// candidate lists, too short to fill the GPU, so a component's walk is
-// split to cut the launch's length.
-constexpr int kWindowSegments = 4;
-
-template <bool kWarp>
-__global__ void __launch_bounds__(kCostThreads) k_cost_window(EncodeLaunch e, int level) {
-    __shared__ LenTables t;
-    const uint32_t n = e.win_count[level];
-    if (blockIdx.x * (kWarp ? kCostThreads / 32 : kCostThreads / kWindowSegments) >= 3u * n) return;  // the whole block
+// level), a warp per (slice, component).
+__global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_window(EncodeLaunch e, int level) {
+    __shared__ CountTables t;
+    __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
+    const uint32_t items = 3u * e.win_count[level], stride = gridDim.x * (kCostThreads / 32);
+    if (blockIdx.x * (kCostThreads / 32) >= items) return;  // the whole block
     t.fill();
     __syncthreads();
-    if (kWarp) {
-        const uint32_t item = blockIdx.x * (kCostThreads / 32) + (threadIdx.x >> 5);
-        if (item >= 3u * n) return;
+    for (uint32_t item = blockIdx.x * (kCostThreads / 32) + (threadIdx.x >> 5); item < items; item += stride) {
         const uint32_t comp = item % 3u, s = e.win_list[item / 3u];
         const EncSliceDesc sd = e.slices[s];
         const uint32_t qi = (uint32_t)(e.state[sd.pic].uniform - 1 - level);
         const EncPicDesc &pd = e.pics[sd.pic];
-        const uint32_t bytes = warp_component_bytes(e, sd, pd, e.frames[pd.frame], comp, qi, t);
+        const uint32_t bytes =
+            warp_component_bytes(e, sd, pd, e.frames[pd.frame], comp, qi, t, buf[threadIdx.x >> 5]);
         if ((threadIdx.x & 31) == 0) e.win_comp[((uint64_t)level * e.n_slices + s) * 3u + comp] = bytes;
-    } else {
-        const uint32_t thread = blockIdx.x * kCostThreads + threadIdx.x;
-        if ((thread & ~31u) / kWindowSegments >= 3u * n) return;  // the whole warp
-        const uint32_t item = thread / kWindowSegments;
-        const bool active = item < 3u * n;
-        const uint32_t comp = active ? item / n : 0u;
-        const uint32_t s = e.win_list[active ? item - comp * n : 0u];
-        const EncSliceDesc sd = e.slices[s];
-        const uint32_t qi = active ? (uint32_t)(e.state[sd.pic].uniform - 1 - level) : 1u;
-        const EncPicDesc &pd = e.pics[sd.pic];
-        const EncFrameDesc &fd = e.frames[pd.frame];
-        uint32_t nb, off;
-        comp_layout(fd, sd.mbs, comp, nb, off);
-        const uint32_t bits = group_component_bits<kWindowSegments>(active, e.coef + sd.coef + off,
-                                                                    e.coef_max + ((sd.coef + off) >> 5), nb,
-                                                                    comp_quant(quant_base(e, pd, qi), comp, nb), t);
-        if (active && thread % kWindowSegments == 0)
-            e.win_comp[((uint64_t)level * e.n_slices + s) * 3u + comp] = (bits + 7u) / 8u;
     }
 }
 
@@ -973,8 +954,9 @@ __global__ void __launch_bounds__(kCostThreads) k_cost_window(EncodeLaunch e, in
 constexpr uint32_t kTailSlices = 16;  // a picture's tail: slices within this many slices' macroblocks of its end
 constexpr uint32_t kTailLevels = 4;
 
-__global__ void __launch_bounds__(kCostThreads) k_cost_deep(EncodeLaunch e) {
-    __shared__ LenTables t;
+__global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_deep(EncodeLaunch e) {
+    __shared__ CountTables t;
+    __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     t.fill();
     __syncthreads();
     const uint32_t s = blockIdx.x * (kCostThreads / 32) + (threadIdx.x >> 5);
@@ -1027,7 +1009,8 @@ __global__ void __launch_bounds__(kCostThreads) k_cost_deep(EncodeLaunch e) {
             const int32_t qi = st.uniform - 1 - kWindow - (int32_t)j;
             if (qi < 1) break;
             uint32_t c3[3];
-            for (uint32_t comp = 0; comp < 3; comp++) c3[comp] = warp_component_bytes(e, sd, pd, fd, comp, (uint32_t)qi, t);
+            for (uint32_t comp = 0; comp < 3; comp++)
+                c3[comp] = warp_component_bytes(e, sd, pd, fd, comp, (uint32_t)qi, t, buf[threadIdx.x >> 5]);
             n = slice_total(hb, c3, alpha, fits);
             if (lane == 0)
                 e.deep[(uint64_t)s * kDeepLevels + j] =
@@ -1273,7 +1256,8 @@ constexpr int kShareWarps = 1;
 constexpr uint32_t kShareLadderBytes = 32u * kDeepLevels * sizeof(uint2) + 32u * (kWindow + kDeepLevels) * sizeof(uint64_t);
 
 __global__ void __launch_bounds__(32 * kShareWarps) k_shareout(EncodeLaunch e) {
-    __shared__ LenTables t;
+    __shared__ CountTables t;
+    __shared__ __align__(8) uint32_t buf[kShareWarps][kCountWords];
     // The slice a deep step costs, copied in once (its coefficients, then
     // its chunk maxima): the warp walks it for every quantiser it tries,
     // and from DRAM each of its chunks waited out a full load.
@@ -1403,7 +1387,8 @@ __global__ void __launch_bounds__(32 * kShareWarps) k_shareout(EncodeLaunch e) {
                         uint32_t nb, off;
                         comp_layout(fd, fsd.mbs, c, nb, off);
                         const CompQuant q = comp_quant(quant_base(e, pd, (uint32_t)(qi - 1)), c, nb);
-                        n3[c] = (warp_component_bits<true>(sf + off, smax + (off >> 5), nb, q, t) + 7u) / 8u;
+                        const CompHead h = comp_head<true>(sf + off, smax + (off >> 5), nb);
+                        n3[c] = (warp_component_bits<true>(sf + off, h, nb, q, t, buf[threadIdx.x >> 5]) + 7u) / 8u;
                     }
                     bool fits;
                     const uint64_t n = slice_total(hb, n3, alpha, fits);
@@ -1742,30 +1727,19 @@ cudaError_t launch_rc_init(const EncodeLaunch &e, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// One lane per item when the batch has enough items to fill the GPU that
-// way (a lane's walk is long, so it needs the whole machine's worth of
-// them); otherwise a warp per item.
-// A lane per slice component needs enough of them to fill the GPU; below
-// that, a warp per component.
-static bool lane_mode(const EncodeLaunch &e) {
-    return 3ull * e.n_slices >= (uint64_t)e.lane_items_per_sm * (uint64_t)e.sm_count;
+// CTAs of a kernel that walks `items` warp items at a stride: all that are
+// resident, or what the items need.
+static uint32_t cost_grid(const EncodeLaunch &e, uint32_t items) {
+    return std::min<uint32_t>((items + kCostThreads / 32 - 1) / (kCostThreads / 32), (uint32_t)(kCostBlocks * e.sm_count));
 }
 
 cudaError_t launch_cost(const EncodeLaunch &e, int step, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
-    const uint32_t items = 3u * e.n_slices;
-    if (lane_mode(e)) {
-        static int per_sm = 0;  // resident CTAs of k_cost per SM (the same for every device of a build)
-        if (per_sm == 0) {
-            int fit = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_cost, kCostThreads, 0);
-            per_sm = fit > 0 ? fit : 1;
-        }
-        const uint32_t need = (items + kCostThreads - 1) / kCostThreads;
-        const uint32_t grid = std::min<uint32_t>(need, (uint32_t)(per_sm * e.sm_count));
-        k_cost<<<grid, kCostThreads, 0, s>>>(e, step);
-    } else
-        k_cost_warp<<<(items + kCostThreads / 32 - 1) / (kCostThreads / 32), kCostThreads, 0, s>>>(e, step);
+    // Items a warp takes at once: enough to share the look-ups, few enough
+    // that every resident warp comes back several times.
+    const uint32_t items = 3u * e.n_slices, warps = (uint32_t)(kCostBlocks * e.sm_count) * (kCostThreads / 32);
+    const uint32_t take = std::max(1u, std::min(32u, items / (4u * warps)));
+    k_cost<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, step, take);
     return cudaGetLastError();
 }
 
@@ -1781,12 +1755,8 @@ cudaError_t launch_cost_window(const EncodeLaunch &e, int level, cudaStream_t s)
     k_window_select<<<(e.n_slices + kCostThreads - 1) / kCostThreads, kCostThreads, 0, s>>>(e, level);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
-    // The grid covers every slice; blocks past the list's end return.
-    if (lane_mode(e))
-        k_cost_window<false><<<(items * kWindowSegments + kCostThreads - 1) / kCostThreads, kCostThreads, 0, s>>>(
-            e, level);
-    else
-        k_cost_window<true><<<(items + kCostThreads / 32 - 1) / (kCostThreads / 32), kCostThreads, 0, s>>>(e, level);
+    // Blocks past the list's end return.
+    k_cost_window<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, level);
     return cudaGetLastError();
 }
 
