@@ -455,17 +455,26 @@ struct CountTables {
     static constexpr uint32_t kRow = 132;
     uint8_t run[16][kRow];
     uint8_t level[9][kRow];
-    __device__ void fill() {
-        for (uint32_t i = threadIdx.x; i < 16 * kRunLens; i += blockDim.x) {
-            const uint32_t c = i / kRunLens, n = i % kRunLens;
-            run[c][n] = (uint8_t)(n + 1u < kRunLens ? cb_len32(run_book(c), n) : kLongCode);
-        }
-        for (uint32_t i = threadIdx.x; i < 9 * kLevelLens; i += blockDim.x) {
-            const uint32_t c = i / kLevelLens, n = i % kLevelLens;
-            level[c][n] = (uint8_t)(n + 1u < kLevelLens ? cb_len32(level_book(c), n) + 1u : kLongCode);
-        }
-    }
+    uint8_t pad[12];  // a whole number of 16-byte words
+    // Copies the device's table (built once, by configure_encode_kernels).
+    __device__ __forceinline__ void fill();
 };
+__device__ uint4 d_count_tables[sizeof(CountTables) / sizeof(uint4)];
+
+__device__ __forceinline__ void CountTables::fill() {
+    for (uint32_t i = threadIdx.x; i < sizeof(CountTables) / sizeof(uint4); i += blockDim.x)
+        reinterpret_cast<uint4 *>(this)[i] = d_count_tables[i];
+}
+
+void build_count_tables(CountTables &t) {
+    t = CountTables{};
+    for (uint32_t c = 0; c < 16; c++)
+        for (uint32_t n = 0; n < kRunLens; n++)
+            t.run[c][n] = (uint8_t)(n + 1u < kRunLens ? cb_len32(run_book(c), n) : kLongCode);
+    for (uint32_t c = 0; c < 9; c++)
+        for (uint32_t n = 0; n < kLevelLens; n++)
+            t.level[c][n] = (uint8_t)(n + 1u < kLevelLens ? cb_len32(level_book(c), n) + 1u : kLongCode);
+}
 
 // A warp's non-zeros on their way from the quantiser to the code tables, in
 // scanned order: (position << 16) + level symbol, both below 2^15 (a
@@ -473,12 +482,18 @@ struct CountTables {
 // range can make, is counted by warp_wide_bits). The two entries before the
 // first hold the state a component starts with (previous run 4, previous
 // level 1), then the last two counted.
-constexpr uint32_t kGroupChunks = 16;  // 32-coefficient chunks quantised before codes are counted
-constexpr uint32_t kNonzeroBuf = 2 + 63 + 32 * kGroupChunks + 3;
+constexpr uint32_t kGroupRuns = 4;  // runs of 128 coefficients quantised before codes are counted
+constexpr uint32_t kNonzeroBuf = 2 + 63 + 128 * kGroupRuns + 3;
 constexpr uint32_t kWeightsAt = kNonzeroBuf, kIdsAt = kNonzeroBuf + 64;
 // Words of shared memory a warp's count takes: its list, then the inverse
 // weights and chunk numbers it works with.
-constexpr uint32_t kCountWords = kIdsAt + 12;
+constexpr uint32_t kCountWords = kIdsAt + 8;
+// Components with more than this many live chunks of every 8 are read whole,
+// the others by the list of their live chunks (30 UHD frames, the probe at
+// quantiser index 56: 372 us at 3, 382 at 2, 415 at 5; 16 4:4:4 12-bit fields
+// 76, 78 and 82).
+constexpr uint32_t kLiveOf8 = 3;
+static_assert(64u * kLiveOf8 / 8u <= 4u * (kCountWords - kIdsAt), "the list holds a 32-block component's live chunks");
 // |F| from here on may make a level symbol of 2^15: 8 / (W qScale) is at most 4.
 constexpr float kWideCoef = 8191.0f;
 
@@ -520,6 +535,17 @@ __device__ __forceinline__ float coef_load(const float *f, uint32_t i) {
         return f[i];
     else
         return __ldg(f + i);
+}
+
+// Length of the code of a DC difference's symbol n by a = min(|previous
+// difference|, 3) (Table 9), and with a = 5 of the first DC's (EG5). EGk is
+// 2 floor(log2(n + 2^k)) - k + 1 bits, and a is k but for a = 2, whose
+// codebook (1, 2, 3) has (n >> 2) + 3 bits below 8 and from there on, as
+// 2^3 is also where its Rice part ends, 2 floor(log2(n)).
+__device__ __forceinline__ uint32_t dc_len(uint32_t a, uint32_t n) {
+    const uint32_t add = a == 2u ? 0u : 1u << a, sub = a == 2u ? 2u : a + 1u;
+    const uint32_t len = 2u * bit_len32(n + add) - sub;
+    return a == 2u && n < 8u ? (n >> 2) + 3u : len;
 }
 
 // What a component's count starts from, loaded ahead: each lane's two chunk
@@ -569,6 +595,37 @@ struct NonzeroList {
                      : "memory");
         end += 4u * __popc(b);
     }
+    // Four coefficients a lane of each of kRuns runs of 128 positions: y the
+    // quantised magnitudes before their floor, `counts` the lane's non-zeros
+    // by run (a byte each), `tag` of the lane's first position.
+    template <uint32_t kRuns>
+    __device__ __forceinline__ void add_runs(const float (&y)[4 * kRuns], uint32_t counts, uint32_t tag) {
+        // Sums over the lanes up to this one; at most 128 a byte.
+        uint32_t sums = counts;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .u32 t;\n\tshfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n\t"
+                         "@p add.u32 %0, %0, t;\n\t}"
+                         : "+r"(sums)
+                         : "r"(o));
+        const uint32_t totals = __shfl_sync(0xffffffffu, sums, 31);
+        const uint32_t before = sums - counts;
+#pragma unroll
+        for (uint32_t r = 0; r < kRuns; r++) {
+            uint32_t at = end + 4u * ((before >> (8 * r)) & 255u);
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++) {
+                // Adding 2^23 rounded down leaves floor(y) in the low bits.
+                const uint32_t entry = __float_as_uint(__fadd_rd(y[4 * r + k], 8388608.0f)) + tag + ((128u * r + k) << 16);
+                asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %2, 0f3F800000;\n\t@p st.shared.u32 [%0], %1;\n\t"
+                             "@p add.u32 %0, %0, 4;\n\t}"
+                             : "+r"(at)
+                             : "r"(entry), "f"(y[4 * r + k])
+                             : "memory");
+            }
+            end += 4u * ((totals >> (8 * r)) & 255u);
+        }
+    }
     // Counts the whole groups of 64; what is left, and the two entries
     // before it, go to the front.
     __device__ __forceinline__ void count(const CountTables &t) {
@@ -601,49 +658,75 @@ struct NonzeroList {
     }
 };
 
+template <bool kShared>
+__device__ __forceinline__ float4 coef_load4(const float *f) {
+    if constexpr (kShared)
+        return *reinterpret_cast<const float4 *>(f);
+    else
+        return __ldg(reinterpret_cast<const float4 *>(f));
+}
+
 // The AC part of warp_component_bits for a component of 2^kLog blocks, every
-// chunk in turn.
+// coefficient in turn. A lane takes four neighbouring positions of each run
+// of 128, four runs at a time; how many non-zeros the lanes below hold in
+// each run comes from one scan of four byte counts.
 template <int kLog, bool kShared>
 __device__ __forceinline__ uint32_t warp_dense_bits(const float *f, const float *inv, const CountTables &t,
                                                     uint32_t *buf) {
-    constexpr uint32_t kBlocks = 1u << kLog, kChunks = 2u * kBlocks;
-    constexpr uint32_t kGroup = kChunks < kGroupChunks ? kChunks : kGroupChunks;
+    constexpr uint32_t kBlocks = 1u << kLog, kRuns = kBlocks / 2u;
+    constexpr uint32_t kGroup = kRuns < kGroupRuns ? kRuns : kGroupRuns;
+    constexpr bool kSplit = kBlocks == 2u;  // a lane's four positions are of two scan positions
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t below = (1u << lane) - 1u;
-    // The 64 inverse weights, where every chunk finds its own at a constant
-    // distance: chunk c's scanned position of this lane is 32 c + lane, its
-    // weight's place (32 c >> kLog) + (lane >> kLog).
+    // The 64 inverse weights, where every run finds its own at a constant
+    // distance: run r's positions of this lane start at 128 r + 4 lane, their
+    // weight's place is (128 r >> kLog) + (4 lane >> kLog).
     float *w = reinterpret_cast<float *>(buf + kWeightsAt);
     w[lane] = __ldg(inv + lane);
     w[lane + 32u] = __ldg(inv + lane + 32u);
     __syncwarp();
-    w += lane >> kLog;
+    w += (4u * lane) >> kLog;
     NonzeroList list;
     list.start(buf, kBlocks);
-    f += lane;
+    f += 4u * lane;
 #pragma unroll 1
-    for (uint32_t g = 0; g < kChunks; g += kGroup) {
-        float v[kGroup], iv[kGroup];
+    for (uint32_t g = 0; g < kRuns; g += kGroup) {
+        float y[4 * kGroup];
 #pragma unroll
-        for (uint32_t i = 0; i < kGroup; i++) v[i] = coef_load<kShared>(f, 32u * i);
+        for (uint32_t r = 0; r < kGroup; r++) {
+            const float4 v = coef_load4<kShared>(f + 128u * r);
+            y[4 * r] = v.x;
+            y[4 * r + 1] = v.y;
+            y[4 * r + 2] = v.z;
+            y[4 * r + 3] = v.w;
+        }
+        if (g == 0 && 4u * lane < kBlocks) {  // the DCs
+            y[0] = y[1] = 0.0f;
+            if (!kSplit) y[2] = y[3] = 0.0f;
+        }
+        uint32_t counts = 0;
 #pragma unroll
-        for (uint32_t i = 0; i < kGroup; i++) iv[i] = w[(32u * i) >> kLog];
-        if (g == 0 && lane < kBlocks) v[0] = 0.0f;  // position `lane` of chunk 0 is a DC
-        const uint32_t tag = ((32u * g + lane) << 16) - 0x4B000001u;
+        for (uint32_t r = 0; r < kGroup; r++) {
+            const float wa = w[(128u * r) >> kLog], wb = kSplit ? w[((128u * r) >> kLog) + 1u] : wa;
 #pragma unroll
-        for (uint32_t i = 0; i < kGroup; i++) list.add(v[i], iv[i], tag + (i << 21), below);
+            for (uint32_t k = 0; k < 4; k++) {
+                // |F inv| + 0.42 (src/dsp/scalar.rs:19-39), a non-zero from 1 up.
+                y[4 * r + k] = __fadd_rn(fabsf(__fmul_rn(y[4 * r + k], k < 2 ? wa : wb)), kAcRounding);
+                if (y[4 * r + k] >= 1.0f) counts += 1u << (8 * r);
+            }
+        }
+        list.add_runs<kGroup>(y, counts, ((128u * g + 4u * lane) << 16) - 0x4B000001u);
         list.count(t);
-        f += 32u * kGroup;
-        w += (32u * kGroup) >> kLog;
+        f += 128u * kGroup;
+        w += (128u * kGroup) >> kLog;
     }
     return list.finish(t);
 }
 
 // The same for a component with few chunks that may hold a non-zero, whose
-// numbers are the first `n` bytes of `chunks`: 8 of them in flight at a time.
+// numbers are the first `n` bytes of `ids`: 8 of them in flight at a time.
 template <bool kShared>
 __device__ __forceinline__ uint32_t warp_sparse_bits(const float *f, const float *inv, uint32_t n_blocks,
-                                                     const uint8_t *chunks, uint32_t n, const CountTables &t,
+                                                     const uint2 *ids, uint32_t n, const CountTables &t,
                                                      uint32_t *buf) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t below = (1u << lane) - 1u;
@@ -652,11 +735,12 @@ __device__ __forceinline__ uint32_t warp_sparse_bits(const float *f, const float
     list.start(buf, n_blocks);
 #pragma unroll 1
     for (uint32_t k = 0; k < n; k += 8) {
+        const uint2 id = ids[k >> 3];
         float v[8], iv[8];
         uint32_t p[8];
 #pragma unroll
         for (uint32_t i = 0; i < 8; i++) {
-            p[i] = 32u * chunks[k + i] + lane;
+            p[i] = 32u * (((i < 4 ? id.x : id.y) >> (8 * (i & 3))) & 255u) + lane;
             v[i] = iv[i] = 0.0f;
             if (k + i < n) {
                 v[i] = coef_load<kShared>(f, p[i]);
@@ -694,13 +778,18 @@ __device__ __noinline__ uint32_t warp_wide_bits(const float *f, const float *inv
 }
 
 // Bits of one quantised component (src/encode.rs:398-409), the whole warp.
-// Two stages, a group of 16 chunks at a time: the warp quantises a chunk's 32
-// coefficients, one a lane (loads of 128 contiguous bytes, all of a group's
-// in flight at once), and appends the non-zeros to a list in order by ballot
-// and popcount; then each lane takes two neighbouring non-zeros of a full 64
-// and looks their code lengths up. So zeros cost no per-code work, and no
-// code waits for the one before it. Where most chunks quantise to zero only
-// the others are read. Every lane gets the sum.
+// Two stages, 512 coefficients at a time: the warp quantises them (16 a lane,
+// their loads all in flight at once) and appends the non-zeros to a list in
+// order; then each lane takes two neighbouring non-zeros of a full 64 and
+// looks their code lengths up. So zeros cost no per-code work, and no code
+// waits for the one before it. Where most chunks quantise to zero only the
+// others are read. Every lane gets the sum.
+//
+// Bound by issue (76-78 % of the slots; 26 warp instructions for 32
+// coefficients at 36 % non-zeros, DRAM at 4.6 TB/s): 30 UHD 4:2:2 frames
+// take 450 us a probe near the answer, where a lane per component walking
+// its codes in order, each look-up waiting for the last, took 800; 30 1080p
+// frames 130 us for 700.
 template <bool kShared = false>
 __device__ __forceinline__ uint32_t warp_component_bits(const float *f, const CompHead &h, uint32_t n_blocks, const CompQuant &cq,
                                         const CountTables &t, uint32_t *buf) {
@@ -717,15 +806,17 @@ __device__ __forceinline__ uint32_t warp_component_bits(const float *f, const Co
     const int32_t left = __shfl_up_sync(0xffffffffu, q, 1);
     const int32_t diff = (int32_t)((uint32_t)q - (uint32_t)left);
     const int32_t before = __shfl_up_sync(0xffffffffu, diff, 1);
-    const int32_t prev_diff = lane == 1 ? 3 : before;
-    const Codebook book = lane == 0 ? kFirstDcBook : dc_book(prev_diff);
-    const uint32_t symbol = signed_to_symbol(lane == 0 ? q : (prev_diff < 0 ? -diff : diff));
-    uint32_t bits = lane < n_blocks ? cb_len32(book, symbol) : 0u;
+    const int32_t prev_diff = lane == 0 ? 5 : (lane == 1 ? 3 : before);
+    const int32_t value = lane == 0 ? q : (prev_diff < 0 ? -diff : diff);
+    // 0, -1, 1, -2, 2, ... -> 0, 1, 2, 3, 4, ...
+    const uint32_t symbol = ((uint32_t)value << 1) ^ (uint32_t)(value >> 31);
+    const uint32_t len = dc_len(min((uint32_t)abs(prev_diff), lane == 0 ? 5u : 3u), symbol);
+    uint32_t bits = lane < n_blocks ? len : 0u;
     const uint32_t n_live = __popc(live_lo) + __popc(live_hi);
     __syncwarp();  // the last component's entries are read
     if (__any_sync(0xffffffffu, fmaxf(h.max_lo, h.max_hi) >= kWideCoef)) {
         bits += warp_wide_bits<kShared>(f, cq.inv, n_blocks);
-    } else if (8u * n_live > 5u * chunks) {
+    } else if (kLiveOf8 * chunks < 8u * n_live) {
         switch (n_blocks) {
         case 32: bits += warp_dense_bits<5, kShared>(f, cq.inv, t, buf); break;
         case 16: bits += warp_dense_bits<4, kShared>(f, cq.inv, t, buf); break;
@@ -734,12 +825,12 @@ __device__ __forceinline__ uint32_t warp_component_bits(const float *f, const Co
         default: bits += warp_dense_bits<1, kShared>(f, cq.inv, t, buf); break;
         }
     } else if (n_live) {
-        // The live chunks' numbers, in order (at most 40, read 8 at a time).
+        // The live chunks' numbers, in order (at most 24).
         uint8_t *ids = reinterpret_cast<uint8_t *>(buf + kIdsAt);
         if ((live_lo >> lane) & 1u) ids[__popc(live_lo & below)] = (uint8_t)lane;
         if ((live_hi >> lane) & 1u) ids[__popc(live_lo) + __popc(live_hi & below)] = (uint8_t)(lane + 32u);
         __syncwarp();
-        bits += warp_sparse_bits<kShared>(f, cq.inv, n_blocks, ids, n_live, t, buf);
+        bits += warp_sparse_bits<kShared>(f, cq.inv, n_blocks, reinterpret_cast<const uint2 *>(ids), n_live, t, buf);
     }
     return __reduce_add_sync(0xffffffffu, bits);
 }
@@ -770,60 +861,66 @@ __device__ __forceinline__ uint32_t warp_component_bytes(const EncodeLaunch &e, 
 }
 
 constexpr int kCostThreads = 256;
-constexpr int kCostBlocks = 4;  // CTAs an SM
+constexpr int kCostBlocks = 4;      // CTAs an SM (5, at 48 registers: 7 % slower)
+constexpr uint32_t kCostTake = 4;   // items a warp of k_cost takes at once, at most (2: 3 % slower; 19, as 4 rounds a warp: 7 %)
 
 // A warp per slice component, (component, slice) component-major. A warp
 // takes `take` neighbouring items (at most 32) from the probe's counter at a
 // time: its lanes look the items' places up side by side, so the chain of
 // descriptor loads is waited for once, and the items are costed in turn.
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost(EncodeLaunch e, int step, uint32_t take) {
-    __shared__ CountTables t;
+    __shared__ __align__(16) CountTables t;
     __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     t.fill();
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t items = 3u * e.n_slices;
+    uint32_t grab = 0;
+    if (lane == 0) grab = atomicAdd(e.cost_taken + step, take);
     for (;;) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(e.cost_taken + step, take);
-        base = __shfl_sync(0xffffffffu, base, 0);
+        const uint32_t base = __shfl_sync(0xffffffffu, grab, 0);
         if (base >= items) break;
+        if (lane == 0) grab = atomicAdd(e.cost_taken + step, take);  // the next one, on its way meanwhile
         // This lane's item: its first coefficient (a multiple of 64), its
         // quantiser table and component group, its block count (0: none).
         const uint32_t item = base + lane;
-        const uint32_t comp = item / e.n_slices, s = item - comp * e.n_slices;
-        uint32_t my_coef = 0, my_quant = 0, my_blocks = 0, my_bytes = 0;
+        uint32_t my_coef = 0, my_quant = 0, my_blocks = 0, my_bytes = 0, out = 0;
         if (lane < take && item < items) {
+            const uint32_t comp = item < e.n_slices ? 0u : (item < 2u * e.n_slices ? 1u : 2u);
+            const uint32_t s = item - comp * e.n_slices;
             const EncSliceDesc sd = e.slices[s];
-            const int32_t qi = e.state[sd.pic].probe_qi;
-            const EncPicDesc &pd = e.pics[sd.pic];
-            uint32_t off;
-            comp_layout(e.frames[pd.frame], sd.mbs, comp, my_blocks, off);
+            const uint32_t qi = (uint32_t)e.state[sd.pic].probe_qi, set = e.state[sd.pic].quant;
+            out = 3u * s + comp;
+            const uint32_t off = comp == 0 ? 0u : 64u * sd.mbs * (4u + (comp - 1u) * sd.cpm);
             my_coef = (uint32_t)((sd.coef + off) >> 6);
-            my_quant = ((pd.quant * 225u + (uint32_t)qi) << 1) | (comp > 0 ? 1u : 0u);
-            if (qi == 0) my_blocks = 0;
+            my_quant = ((set * 225u + qi) << 1) | (comp > 0 ? 1u : 0u);
+            if (qi != 0) my_blocks = (comp == 0 ? 4u : sd.cpm) * sd.mbs;
         }
         const uint32_t costed = __ballot_sync(0xffffffffu, my_blocks != 0);
-        const auto head = [&](uint32_t j) {
-            const uint64_t coef = (uint64_t)__shfl_sync(0xffffffffu, my_coef, j) << 6;
-            return comp_head<false>(e.coef + coef, e.coef_max + (coef >> 5), __shfl_sync(0xffffffffu, my_blocks, j));
-        };
         // The next item's maxima and DCs are on their way while one is costed.
-        CompHead next{};
-        if (costed) next = head((uint32_t)__ffs(costed) - 1u);
+        CompHead next_head{};
+        uint32_t next_blocks = 0;
+        const float *next_f = e.coef;
+        const auto look = [&](uint32_t j) {
+            const uint64_t coef = (uint64_t)__shfl_sync(0xffffffffu, my_coef, j) << 6;
+            next_blocks = __shfl_sync(0xffffffffu, my_blocks, j);
+            next_f = e.coef + coef;
+            next_head = comp_head<false>(next_f, e.coef_max + (coef >> 5), next_blocks);
+        };
+        if (costed) look((uint32_t)__ffs(costed) - 1u);
         for (uint32_t left = costed; left;) {
             const uint32_t j = (uint32_t)__ffs(left) - 1u;
             left &= left - 1u;
-            const CompHead h = next;
-            if (left) next = head((uint32_t)__ffs(left) - 1u);
-            const uint32_t nb = __shfl_sync(0xffffffffu, my_blocks, j);
+            const CompHead h = next_head;
+            const uint32_t nb = next_blocks;
+            const float *f = next_f;
+            if (left) look((uint32_t)__ffs(left) - 1u);
             const uint32_t quant = __shfl_sync(0xffffffffu, my_quant, j);
-            const uint64_t coef = (uint64_t)__shfl_sync(0xffffffffu, my_coef, j) << 6;
             const CompQuant q = comp_quant(e.quant + (uint64_t)(quant >> 1) * kQuantStride, quant & 1u, nb);
-            const uint32_t bits = warp_component_bits(e.coef + coef, h, nb, q, t, buf[threadIdx.x >> 5]);
+            const uint32_t bits = warp_component_bits(f, h, nb, q, t, buf[threadIdx.x >> 5]);
             if (lane == j) my_bytes = (bits + 7u) / 8u;
         }
-        if ((costed >> lane) & 1u) e.probe_comp[((uint64_t)step * e.n_slices + s) * 3u + comp] = my_bytes;
+        if (my_blocks) e.probe_comp[(uint64_t)step * 3u * e.n_slices + out] = my_bytes;
     }
 }
 
@@ -911,7 +1008,7 @@ __global__ void __launch_bounds__(kCostThreads) k_window_select(EncodeLaunch e, 
 // Costs the listed slices at window level `level` (quantiser uniform - 1 -
 // level), a warp per (slice, component).
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_window(EncodeLaunch e, int level) {
-    __shared__ CountTables t;
+    __shared__ __align__(16) CountTables t;
     __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     const uint32_t items = 3u * e.win_count[level], stride = gridDim.x * (kCostThreads / 32);
     if (blockIdx.x * (kCostThreads / 32) >= items) return;  // the whole block
@@ -955,7 +1052,7 @@ constexpr uint32_t kTailSlices = 16;  // a picture's tail: slices within this ma
 constexpr uint32_t kTailLevels = 4;
 
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_deep(EncodeLaunch e) {
-    __shared__ CountTables t;
+    __shared__ __align__(16) CountTables t;
     __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     t.fill();
     __syncthreads();
@@ -1055,6 +1152,7 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_init(EncodeLaunch e) {
         st.lo_probe = -1;
         st.fits_at_all = 0;
         st.uniform = 224;
+        st.quant = pd.quant;
         e.state[blockIdx.x] = st;
         if (blockIdx.x == 0) {
             for (int j = 0; j < kWindow; j++) e.win_count[j] = 0;
@@ -1256,7 +1354,7 @@ constexpr int kShareWarps = 1;
 constexpr uint32_t kShareLadderBytes = 32u * kDeepLevels * sizeof(uint2) + 32u * (kWindow + kDeepLevels) * sizeof(uint64_t);
 
 __global__ void __launch_bounds__(32 * kShareWarps) k_shareout(EncodeLaunch e) {
-    __shared__ CountTables t;
+    __shared__ __align__(16) CountTables t;
     __shared__ __align__(8) uint32_t buf[kShareWarps][kCountWords];
     // The slice a deep step costs, copied in once (its coefficients, then
     // its chunk maxima): the warp walks it for every quantiser it tries,
@@ -1736,9 +1834,10 @@ static uint32_t cost_grid(const EncodeLaunch &e, uint32_t items) {
 cudaError_t launch_cost(const EncodeLaunch &e, int step, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
     // Items a warp takes at once: enough to share the look-ups, few enough
-    // that every resident warp comes back several times.
+    // that the last ones do not hold the launch up (a component takes a warp
+    // about 6 us when all warps are busy).
     const uint32_t items = 3u * e.n_slices, warps = (uint32_t)(kCostBlocks * e.sm_count) * (kCostThreads / 32);
-    const uint32_t take = std::max(1u, std::min(32u, items / (4u * warps)));
+    const uint32_t take = std::max(1u, std::min(kCostTake, items / (8u * warps)));
     k_cost<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, step, take);
     return cudaGetLastError();
 }
@@ -1801,6 +1900,9 @@ cudaError_t configure_encode_kernels() {
     cudaError_t err0 = cudaFuncSetAttribute(k_shareout, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)(kShareWarps * kShareLadderBytes));
     if (err0 != cudaSuccess) return err0;
+    CountTables tables;
+    build_count_tables(tables);
+    if ((err0 = cudaMemcpyToSymbol(d_count_tables, &tables, sizeof tables)) != cudaSuccess) return err0;
     float basis[64];
     dct_basis(basis);
     cudaError_t err = cudaMemcpyToSymbol(c_fdct_basis, basis, sizeof basis);

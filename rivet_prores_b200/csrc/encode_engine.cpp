@@ -245,6 +245,7 @@ Status plan_encode(const prores_config *cfg, const prores_frame *in, int n, Enco
                     s.mb_x = (uint16_t)mx;
                     s.mb_y = (uint16_t)my;
                     s.mbs = w;
+                    s.cpm = cpm;
                     plan->sdesc.push_back(s);
                     mx += w;
                 }

@@ -56,6 +56,7 @@ struct EncSliceDesc {
     uint32_t pic;
     uint16_t mb_x, mb_y;
     uint32_t mbs;
+    uint32_t cpm;  // blocks of each chroma component a macroblock: 2 or 4
 };
 
 // Rate-control state of one picture (src/encode.rs:685-794).
@@ -70,6 +71,7 @@ struct EncPicState {
     int32_t lo_probe;    // the failed probe step at lo - 1, or -1
     int32_t fits_at_all;
     int32_t uniform;
+    uint32_t quant;      // the picture's quantiser table set (beside probe_qi, for k_cost)
     uint8_t step_qi[12];  // the quantiser each probe step costed (0: none)
 };
 
