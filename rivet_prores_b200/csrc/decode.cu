@@ -9,8 +9,8 @@
 //              run/level/sign codes of the interleaved scan (:484-540) as a
 //              list of (position, value) entries, or the alpha
 //              run/difference codes (:570-595) straight into the alpha plane.
-//   k_idct     one CTA per slice: the entries placed in shared memory,
-//              inverse quantisation, the 8x8 IDCT in the crate's exact
+//   k_idct     one warp per 32 blocks, a lane each: the entries dequantised
+//              into shared memory, the 8x8 IDCT in the crate's exact
 //              single-precision order (src/dct.rs:36-66,
 //              src/dsp/scalar.rs:8-12) and the sample conversion, stored as
 //              woven 16-byte rows (src/decode.rs:395-438).
@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "codec_tables.h"
 #include "device_types.h"
@@ -29,7 +30,7 @@
 
 namespace prores {
 
-__constant__ uint8_t c_scan[2][64];
+__device__ uint8_t d_scan[2][64];  // scanned index of each raster position, progressive and interlaced
 __constant__ float c_idct_basis[64];  // T[x][u] (dct_basis)
 
 namespace {
@@ -148,6 +149,7 @@ __device__ __forceinline__ int read_sym(Bits &b, Codebook cb, uint32_t &sym) {
 // and their entry holds -2^20 + k. Half the bytes of (index, value) pairs
 // of 32-bit words, for values of any size.
 constexpr int32_t kListMin = -(1 << 20) + 2048;
+constexpr uint32_t kListBig = 1u << 31;  // in a list's count: it has values at the back of its region
 
 struct CoefList {
     uint32_t *w;
@@ -186,13 +188,6 @@ struct SlotOut {
         }
     }
 };
-
-// An entry's (index, value), reading a large value from the region's back.
-__device__ __forceinline__ void list_entry(const uint32_t *w, uint32_t cap, uint32_t e, uint32_t &n, int32_t &v) {
-    n = e >> 21;
-    v = (int32_t)(e << 11) >> 11;
-    if (v < kListMin) v = (int32_t)__ldg(w + 2u * cap - 1u - (uint32_t)(v + (1 << 20)));
-}
 
 // The read position as a 64-bit window consumed from the top: `cur` holds
 // the bits [pos, pos + avail) MSB first with zeros below, and is refilled
@@ -583,7 +578,7 @@ __device__ void decode_item(const DecodeLaunch &d, uint32_t comp, uint32_t s, co
         const uint64_t base = sd.coef + (comp == 0 ? 0ull : 64ull * sd.mbs * (4u + (comp - 1u) * cpm));
         CoefList list{reinterpret_cast<uint32_t *>(d.coef + base), 64u * n_blocks, 0u, 0u};
         err = decode_component(b, n_blocks, list, run_tab, level_tab);
-        d.coef_count[3ull * s + comp] = list.count;
+        d.coef_count[3ull * s + comp] = list.count | (list.big ? kListBig : 0u);
     }
     *slot = make_int2(err, 0);
 }
@@ -667,6 +662,19 @@ __global__ void __launch_bounds__(kLocateThreads) k_locate(DecodeLaunch d) {
             sd.mbs = mbs;
             sd.coef = p.coef_base + ((uint64_t)row * p.width_in_mb + mb_x) * coef_per_mb;
             d.slices[p.slice_base + k] = sd;
+            // The slice's items for k_idct: its parts, or a group's once (the
+            // fused decode alone has none).
+            const IdctShape shape = idct_shape(fd.chroma, p.log2_slice_mbs);
+            if (!d.idct_items) {
+            } else if (shape.slices > 1u) {
+                if (k % shape.slices == 0)
+                    d.idct_items[p.idct_base + k / shape.slices] =
+                        make_uint4(p.slice_base + k, min(shape.slices, p.n_slices - k) << 8, blockIdx.x, p.frame);
+            } else {
+                for (uint32_t part = 0; part < shape.parts; part++)
+                    d.idct_items[p.idct_base + k * shape.parts + part] =
+                        make_uint4(p.slice_base + k, (1u << 8) | part, blockIdx.x, p.frame);
+            }
         }
         __syncthreads();
         if (threadIdx.x == kLocateThreads - 1) carry += (warp ? warp_sums[warp - 1] : 0u) + incl;
@@ -717,9 +725,6 @@ __global__ void __launch_bounds__(kEntropyMaxThreads) k_entropy(DecodeLaunch d) 
     }
 }
 
-constexpr int kIdctThreads = 256;
-constexpr int kMaxSliceCoefs = 64 * 12 * 8;  // 8 macroblocks of 4:4:4
-
 // Placement of block b of macroblock m (src/decode.rs:395-413).
 __device__ __forceinline__ void block_xy(uint32_t comp, uint32_t chroma, uint32_t mb_x, uint32_t mb_y, uint32_t m,
                                          uint32_t b, uint32_t &bx, uint32_t &by) {
@@ -736,225 +741,286 @@ __device__ __forceinline__ void block_xy(uint32_t comp, uint32_t chroma, uint32_
     }
 }
 
-__global__ void __launch_bounds__(kIdctThreads, 5) k_idct(DecodeLaunch d) {
+// k_idct: a warp takes up to 32 blocks (IdctShape), a lane each for the
+// transform. The warp dequantises the components' lists into its own shared
+// memory, every lane runs its block's rows and then its columns from there
+// with the paired sums of pair_math.h (13 instructions a sample for both
+// passes, from 24 with a product for every term), and stores whole 16-byte
+// rows from registers: neighbouring lanes hold neighbouring blocks, so a
+// store covers 256 contiguous bytes and nothing is staged. No barrier wider
+// than a warp; the next list words are on their way while the last are
+// placed. Bound by issue (66 % of the slots, 37 instructions a sample at 36 %
+// non-zeros) and by the 24 warps an SM that the blocks' 8.7 kB leave room for
+// (20, at 102 registers: 11 % slower; 16: 25 %). 32 UHD 4:2:2 frames take
+// 822 us, where a CTA per slice with index arithmetic for every row and
+// column task and all 64 products took 1990; a mixed batch 430 for 1585.
+constexpr int kIdctWarps = 4;
+// A block's floats in shared memory: 64 and 4 more, so that eight lanes'
+// 16-byte reads of the same place in neighbouring blocks meet no bank twice.
+constexpr uint32_t kBlockStride = 68;
+struct IdctWarp {
+    float f[32 * kBlockStride];
+    // By scanned index, luma then chroma: the weight, which as a float has
+    // its low 16 bits clear, with the raster position's byte offset in them.
+    uint32_t weight[2][64];
+};
+
+// floor(a), floor(b) as integers clamped to [0, 2^16), a in the low half (an
+// infinity clamps, a NaN gives 0, as a maximum with 0 would).
+__device__ __forceinline__ uint32_t floor_pair(float a, float b) {
+    uint32_t r;
+    asm("{\n\t.reg .s32 i, j;\n\tcvt.rmi.s32.f32 i, %1;\n\tcvt.rmi.s32.f32 j, %2;\n\t"
+        "cvt.pack.sat.u16.s32 %0, j, i;\n\t}"
+        : "=r"(r)
+        : "f"(a), "f"(b));
+    return r;
+}
+
+// The column pass of four columns t (in shared memory: t[8 v] is row v's
+// four), rows in order, zero rows (clear in `rows`) skipped, and the
+// conversion floor(v scale + bias) clamped. Stored columns are in the order
+// the row pass leaves them: 0, 1, 3, 2 (kForward) or 7, 6, 4, 5; words kFirst
+// and kFirst + 1 of out[y] get row y's samples in picture order.
+template <int kFirst, bool kForward>
+__device__ __forceinline__ void idct_columns(const float *t, uint32_t rows, float oscale, uint64_t bias2, uint32_t max2,
+                                             uint32_t (&out)[8][4]) {
+    Pairs8 c[4];
+    const auto term = [&](auto v) {
+        constexpr int u = decltype(v)::value;
+        if (u > 0 && !((rows >> u) & 1u)) return;
+        const float4 r = *reinterpret_cast<const float4 *>(t + 8 * u);
+        pairs_term<u, u == 0>(c[0], r.x, c_idct_basis);
+        pairs_term<u, u == 0>(c[1], r.y, c_idct_basis);
+        pairs_term<u, u == 0>(c[2], r.z, c_idct_basis);
+        pairs_term<u, u == 0>(c[3], r.w, c_idct_basis);
+    };
+    term(std::integral_constant<int, 0>{});
+    term(std::integral_constant<int, 1>{});
+    term(std::integral_constant<int, 2>{});
+    term(std::integral_constant<int, 3>{});
+    term(std::integral_constant<int, 4>{});
+    term(std::integral_constant<int, 5>{});
+    term(std::integral_constant<int, 6>{});
+    term(std::integral_constant<int, 7>{});
+    // Two rows, ya and yb, of the pair m of every column.
+    const auto put = [&](uint64_t Pairs8::*m, int ya, int yb) {
+        float lo[4], hi[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float a, b;
+            pair_split(c[k].*m, a, b);
+            pair_split(pair_add(pair_of(__fmul_rn(a, oscale), __fmul_rn(b, oscale)), bias2), lo[k], hi[k]);
+        }
+        if (kForward) {
+            out[ya][kFirst] = __vminu2(floor_pair(lo[0], lo[1]), max2);
+            out[ya][kFirst + 1] = __vminu2(floor_pair(lo[3], lo[2]), max2);
+            out[yb][kFirst] = __vminu2(floor_pair(hi[0], hi[1]), max2);
+            out[yb][kFirst + 1] = __vminu2(floor_pair(hi[3], hi[2]), max2);
+        } else {
+            out[ya][kFirst] = __vminu2(floor_pair(lo[2], lo[3]), max2);
+            out[ya][kFirst + 1] = __vminu2(floor_pair(lo[1], lo[0]), max2);
+            out[yb][kFirst] = __vminu2(floor_pair(hi[2], hi[3]), max2);
+            out[yb][kFirst + 1] = __vminu2(floor_pair(hi[1], hi[0]), max2);
+        }
+    };
+    put(&Pairs8::o01, 0, 1);
+    put(&Pairs8::o32, 3, 2);
+    put(&Pairs8::o45, 4, 5);
+    put(&Pairs8::o76, 7, 6);
+}
+
+__global__ void __launch_bounds__(32 * kIdctWarps, 6) k_idct(DecodeLaunch d) {
     extern __shared__ __align__(16) unsigned char smem[];
-    int32_t *cs = reinterpret_cast<int32_t *>(smem);                   // scanned coefficients
-    float *tmp = reinterpret_cast<float *>(smem);  // row pass, over cs: [v][x][blk] per component
-    uint8_t *nz = smem + 4 * kMaxSliceCoefs;       // non-zero rows, [blk][v]
-    __shared__ float scale[2][64];
-    __shared__ uint8_t scan[64];
-
-    const SliceDesc sd = d.slices[blockIdx.x];
-    const PicDesc &pd = d.pics[sd.pic];
-    if (d.pic_status[sd.pic].locate_slice >= 0) return;
-    const FrameDesc &fd = d.frames[pd.frame];
+    IdctWarp &w = reinterpret_cast<IdctWarp *>(smem)[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t index = blockIdx.x * kIdctWarps + (threadIdx.x >> 5);
+    if (index >= d.n_idct_items) return;
+    // The item names its picture and frame, so every descriptor is fetched at
+    // once, and the first list words once those are there.
+    const uint4 item = d.idct_items[index];
+    const uint32_t first = item.x, n_slices = item.y >> 8, part = item.y & 255u;
+    const PicDesc &pd = d.pics[item.z];
+    const FrameDesc &fd = d.frames[item.w];
+    if (d.pic_status[item.z].locate_slice >= 0) return;
     const uint32_t cpm = fd.chroma == 2 ? 2u : 4u;
-    const uint32_t mbs = sd.mbs;
-    const uint32_t total = 64u * (4u + 2u * cpm) * mbs;
-    const uint32_t tid = threadIdx.x;
+    const IdctShape shape = idct_shape(fd.chroma, pd.log2_slice_mbs);
+    // The components [c0, c1) of the item's slices.
+    const uint32_t c0 = part == 0 ? 0u : (shape.parts == 3u ? part : (cpm == 2u ? 1u : 2u));
+    const uint32_t c1 = part + 1u == shape.parts ? 3u : c0 + (shape.parts == 3u || cpm == 2u ? 1u : 2u);
+    const uint32_t n_lists = n_slices * (c1 - c0);
 
-    // The slice's coefficients: zero the block array, then place each
-    // component's (position, value) entries.
-    int4 *s4 = reinterpret_cast<int4 *>(cs);
-    for (uint32_t i = tid; i < total / 4; i += kIdctThreads) s4[i] = make_int4(0, 0, 0, 0);
-    __syncthreads();
-    for (uint32_t c = 0; c < 3; c++) {
-        const uint32_t cap = 64u * (c == 0 ? 4u : cpm) * mbs;
-        const uint32_t start = c == 0 ? 0u : 64u * mbs * (4u + (c - 1u) * cpm);
-        const uint32_t n = min(d.coef_count[3ull * blockIdx.x + c], cap);
-        const uint32_t *list = reinterpret_cast<const uint32_t *>(d.coef + sd.coef + start);
-        for (uint32_t i = tid; i < n; i += kIdctThreads) {
-            uint32_t pos;
-            int32_t v;
-            list_entry(list, cap, __ldg(list + i), pos, v);
-            if (pos < cap) cs[start + pos] = v;
-        }
+    // Lane l < n_lists looks after list l: slice l / (c1 - c0)'s component.
+    const uint32_t per = c1 - c0;
+    uint32_t list_coef = 0, list_n = 0, list_nb = 1, list_at = 0;  // region / 64, entries, blocks, first lane
+    uint32_t list_xy = 0;                                          // the slice's place in macroblocks
+    float list_q8 = 0.0f;                                          // qScale / 8
+    if (lane < n_lists) {
+        const uint32_t j = per == 1u ? lane : (per == 2u ? lane >> 1 : lane / 3u), c = c0 + lane - j * per;
+        const SliceDesc sd = d.slices[first + j];
+        list_n = d.coef_count[3ull * (first + j) + c];
+        const uint32_t qi = sd.size >= 2 ? d.bits[sd.off + 1] : 1u;
+        list_q8 = (float)qscale(min(max(qi, 1u), 224u)) * 0.125f;
+        list_nb = (c == 0 ? 4u : cpm) * sd.mbs;
+        const uint32_t start = c == 0 ? 0u : sd.mbs * (4u + (c - 1u) * cpm);
+        list_coef = (uint32_t)(sd.coef >> 6) + start;
+        list_at = j * shape.blocks + start - (c0 == 0 ? 0u : sd.mbs * (4u + (c0 - 1u) * cpm));
+        list_xy = sd.mb_x | ((uint32_t)sd.mb_y << 16);
     }
-    uint32_t qi = sd.size >= 2 ? d.bits[sd.off + 1] : 1u;
-    qi = qi < 1u ? 1u : (qi > 224u ? 224u : qi);
-    const uint32_t q = qscale(qi);
-    if (tid < 128) {
-        const uint32_t which = tid >> 6, k = tid & 63;
-        // F = QF * (W * qScale / 8), one factor per raster position (src/decode.rs:356).
-        scale[which][k] = (float)((uint32_t)d.weights[fd.weights * 128u + which * 64u + k] * q) / 8.0f;
-    } else if (tid < 192) {
-        scan[tid - 128] = c_scan[pd.interlaced_scan][tid - 128];
-    }
-    __syncthreads();
+    // This lane's block: its list and component, and its place there.
+    uint32_t my_list = 32, my_comp = 0, my_blk = 0;
 
-    // Row pass: tmp[v][x] = sum_u F[v][u] T[x][u], u in order, from 0
-    // (src/dct.rs:38-53); all-zero rows are skipped, as the crate does.
-    // Blocks of a component and its first coefficient in the slice (by
-    // select, not an indexed array, which would live in local memory).
-    const uint32_t luma_blocks = 4u * mbs, chroma_blocks = cpm * mbs;
-    // Block counts are powers of two: task indices split by shifts, not by
-    // divisions (which run on the conversion pipe this kernel is short of).
-    const uint32_t luma_shift = 31u - __clz(luma_blocks), chroma_shift = 31u - __clz(chroma_blocks);
-    const auto blocks_of = [&](uint32_t c) { return c == 0 ? luma_blocks : chroma_blocks; };
-    const auto shift_of = [&](uint32_t c) { return c == 0 ? luma_shift : chroma_shift; };
-    const auto start_of = [&](uint32_t c) { return c == 0 ? 0u : 64u * (luma_blocks + (c - 1u) * chroma_blocks); };
-    const uint32_t all_blocks = luma_blocks + 2u * chroma_blocks;
-    // The row results are held in registers until every thread has read
-    // its coefficients, then written over them (the two arrays share the
-    // shared memory, so that five CTAs fit on an SM).
-    constexpr int kRowsPerThread = (kMaxSliceCoefs / 8 + kIdctThreads - 1) / kIdctThreads;
-    float held[kRowsPerThread][8];
-    bool held_any[kRowsPerThread];
-#pragma unroll
-    for (int k = 0; k < kRowsPerThread; k++) {
-        const uint32_t t = tid + (uint32_t)k * kIdctThreads;
-        held_any[k] = false;
-        if (t >= all_blocks * 8u) continue;
-        const uint32_t c = t < luma_blocks * 8u ? 0u : (t < (luma_blocks + chroma_blocks) * 8u ? 1u : 2u);
-        const uint32_t tc = t - start_of(c) / 8u;  // 8 row tasks a block
-        const uint32_t nb = blocks_of(c);
-        const uint32_t blk = tc & (nb - 1u), v = tc >> shift_of(c);
-        const int32_t *src = cs + start_of(c);
-        const float *sc = scale[c > 0];
-        float row[8];
-        bool any = false;
-        int32_t q[8];
-        bool wide = false;
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            q[u] = src[nb * scan[8u * v + u] + blk];
-            wide |= (uint32_t)(q[u] + (1 << 22)) >= (1u << 23);
+    // A list's state for the whole warp, and four of its entries from `i` on
+    // (this lane's: i + 4 lane).
+    struct List {
+        const uint32_t *words;
+        uint32_t n, nb, at, shift, comp;
+        bool big;
+        float q8;
+    };
+    const auto open = [&](uint32_t l, uint32_t comp) {
+        List r;
+        r.words = reinterpret_cast<const uint32_t *>(d.coef + ((uint64_t)__shfl_sync(0xffffffffu, list_coef, l) << 6));
+        r.nb = __shfl_sync(0xffffffffu, list_nb, l);
+        r.n = __shfl_sync(0xffffffffu, list_n, l);
+        r.big = (r.n & kListBig) != 0;
+        r.n = min(r.n & ~kListBig, 64u * r.nb);
+        r.at = __shfl_sync(0xffffffffu, list_at, l);
+        r.q8 = __shfl_sync(0xffffffffu, list_q8, l);
+        r.shift = 31u - __clz(r.nb);
+        r.comp = comp;
+        if (lane - r.at < r.nb) {
+            my_list = l;
+            my_comp = comp;
+            my_blk = lane - r.at;
         }
-        // Values below 2^22 in magnitude convert exactly by an add (no
-        // conversion instruction); a wider one, rare, takes the conversion.
-        if (!wide) {
+        return r;
+    };
+    const auto fetch = [&](const List &l, uint32_t i) {
+        i += 4u * lane;
+        return i < l.n ? __ldg(reinterpret_cast<const uint4 *>(l.words + i)) : make_uint4(0, 0, 0, 0);
+    };
+    List list = open(0, c0);
+    uint4 e = fetch(list, 0);
+
+    // Zeros, and the picture's weights in scanned order.
 #pragma unroll
-            for (int u = 0; u < 8; u++) row[u] = __fmul_rn(small_int_to_float(q[u]), sc[8u * v + u]);
+    for (uint32_t i = 0; i < kBlockStride / 4u; i++)
+        reinterpret_cast<float4 *>(w.f)[32u * i + lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+        const uint32_t r = (i & 1u) * 32u + lane;
+        const float weight = (float)d.weights[fd.weights * 128u + 32u * i + lane];
+        w.weight[i >> 1][d_scan[pd.interlaced_scan][r]] = __float_as_uint(weight) | (4u * r);
+    }
+    __syncwarp();
+
+    // The coefficient lists, dequantised (F = QF W qScale / 8,
+    // src/decode.rs:356; W qScale / 8 is exact) into the blocks. Positions
+    // are below the component's end: k_entropy stops at a run that passes it.
+    for (uint32_t l = 0; l < n_lists; l++) {
+        List next = list;
+        uint4 ahead = make_uint4(0, 0, 0, 0);
+        if (l + 1u < n_lists) {
+            next = open(l + 1u, list.comp + 1u == c1 ? c0 : list.comp + 1u);
+            ahead = fetch(next, 0);
+        }
+        const uint32_t *table = w.weight[list.comp > 0 ? 1 : 0];
+        char *blocks = reinterpret_cast<char *>(w.f + list.at * kBlockStride);
+        const auto put = [&](uint32_t x, int32_t v) {
+            const uint32_t pos = x >> 21;
+            const uint32_t t = table[pos >> list.shift];
+            const float scale = __fmul_rn(__uint_as_float(t & 0xFFFF0000u), list.q8);
+            *reinterpret_cast<float *>(blocks + (pos & (list.nb - 1u)) * (4u * kBlockStride) + (t & 0xFFFFu)) =
+                __fmul_rn(__int2float_rn(v), scale);
+        };
+        const auto place = [&](uint32_t x) { put(x, (int32_t)(x << 11) >> 11); };
+        uint32_t i = 0;
+        if (!list.big) {
+            for (; i + 128u <= list.n; i += 128u) {
+                const uint4 x = e;
+                e = fetch(list, i + 128u);
+                place(x.x);
+                place(x.y);
+                place(x.z);
+                place(x.w);
+            }
+            i += 4u * lane;
+            if (i < list.n) place(e.x);
+            if (i + 1u < list.n) place(e.y);
+            if (i + 2u < list.n) place(e.z);
+            if (i + 3u < list.n) place(e.w);
+        } else {
+            for (i = lane; i < list.n; i += 32u) {
+                const uint32_t x = __ldg(list.words + i);
+                int32_t v = (int32_t)(x << 11) >> 11;
+                if (v < kListMin) v = (int32_t)__ldg(list.words + 128u * list.nb - 1u - (uint32_t)(v + (1 << 20)));
+                put(x, v);
+            }
+        }
+        list = next;
+        e = ahead;
+    }
+    __syncwarp();
+
+    // Row pass: tmp[v][x] = sum_u F[v][u] T[x][u], u in order (src/dct.rs:
+    // 38-53), each lane its block's rows over their coefficients, in the
+    // order 0, 1, 3, 2, 7, 6, 4, 5 the sums come in. A row that is zero in
+    // all 32 blocks stays zero.
+    float *blk = w.f + lane * kBlockStride;
+    uint32_t rows = 1u;
+#pragma unroll 1
+    for (uint32_t v = 0; v < 8; v++) {
+        const float4 a = *reinterpret_cast<const float4 *>(blk + 8u * v);
+        const float4 b = *reinterpret_cast<const float4 *>(blk + 8u * v + 4u);
+        const uint32_t any = __float_as_uint(a.x) | __float_as_uint(a.y) | __float_as_uint(a.z) | __float_as_uint(a.w) |
+                             __float_as_uint(b.x) | __float_as_uint(b.y) | __float_as_uint(b.z) | __float_as_uint(b.w);
+        if (!__any_sync(0xffffffffu, any != 0)) continue;
+        rows |= 1u << v;
+        Pairs8 o;
+        pairs_term<0, true>(o, a.x, c_idct_basis);
+        pairs_term<1, false>(o, a.y, c_idct_basis);
+        pairs_term<2, false>(o, a.z, c_idct_basis);
+        pairs_term<3, false>(o, a.w, c_idct_basis);
+        pairs_term<4, false>(o, b.x, c_idct_basis);
+        pairs_term<5, false>(o, b.y, c_idct_basis);
+        pairs_term<6, false>(o, b.z, c_idct_basis);
+        pairs_term<7, false>(o, b.w, c_idct_basis);
+        *reinterpret_cast<ulonglong2 *>(blk + 8u * v) = make_ulonglong2(o.o01, o.o32);
+        *reinterpret_cast<ulonglong2 *>(blk + 8u * v + 4u) = make_ulonglong2(o.o76, o.o45);
+    }
+
+    // Column pass and conversion, half a block's columns at a time.
+    uint32_t px[8][4];
+    {
+        const uint64_t bias2 = pair_of(fd.out_bias, fd.out_bias);
+        const uint32_t max1 = (1u << fd.bit_depth) - 1u, max2 = max1 | (max1 << 16);
+        idct_columns<0, true>(blk, rows, fd.out_scale, bias2, max2, px);
+        idct_columns<2, false>(blk + 4, rows, fd.out_scale, bias2, max2, px);
+    }
+
+    // A 16-byte row of the block at a time: neighbouring lanes' blocks are
+    // neighbours in the picture.
+    const uint32_t xy = __shfl_sync(0xffffffffu, list_xy, my_list);
+    if (my_list == 32u) return;
+    const uint32_t mb_shift = my_comp == 0 || cpm == 4u ? 2u : 1u;
+    uint32_t bx, by;
+    block_xy(my_comp, fd.chroma, xy & 0xFFFFu, xy >> 16, my_blk >> mb_shift, my_blk & ((1u << mb_shift) - 1u), bx, by);
+    const uint32_t pw = fd.plane_w[my_comp];
+    if (bx >= pw || by >= pd.height) return;
+    uint16_t *plane = fd.out_planes ? fd.out_planes + (fd.plane_off[my_comp] - fd.plane_off[0])
+                                    : d.planes + fd.plane_off[my_comp];
+    uint16_t *dst = plane + (uint64_t)(pd.first_row + pd.row_step * by) * pw + bx;
+    const uint64_t pitch = (uint64_t)pd.row_step * pw;
+    const uint32_t cols = min(8u, pw - bx), n_rows = min(8u, pd.height - by);
+#pragma unroll
+    for (uint32_t y = 0; y < 8; y++, dst += pitch) {
+        if (y >= n_rows) break;
+        if (cols == 8u && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0)) {
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(px[y][0], px[y][1], px[y][2], px[y][3]);
         } else {
 #pragma unroll
-            for (int u = 0; u < 8; u++) row[u] = __fmul_rn(__int2float_rn(q[u]), sc[8u * v + u]);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; u++) any |= row[u] != 0.0f;
-        held_any[k] = any;
-        if (any) {
-            // Outputs x = 2 j, 2 j + 1 summed as a pair, each in the same
-            // order; the products stay scalar (see pair_math.h).
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                uint64_t acc = 0;
-#pragma unroll
-                for (int u = 0; u < 8; u++)
-                    acc = pair_add(acc, pair_of(__fmul_rn(row[u], c_idct_basis[8 * (2 * j) + u]),
-                                                __fmul_rn(row[u], c_idct_basis[8 * (2 * j + 1) + u])));
-                pair_split(acc, held[k][2 * j], held[k][2 * j + 1]);
-            }
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kRowsPerThread; k++) {
-        const uint32_t t = tid + (uint32_t)k * kIdctThreads;
-        if (t >= all_blocks * 8u) continue;
-        const uint32_t c = t < luma_blocks * 8u ? 0u : (t < (luma_blocks + chroma_blocks) * 8u ? 1u : 2u);
-        const uint32_t tc = t - start_of(c) / 8u;  // 8 row tasks a block
-        const uint32_t nb = blocks_of(c);
-        const uint32_t blk = tc & (nb - 1u), v = tc >> shift_of(c);
-        nz[(start_of(c) / 64u + blk) * 8u + v] = held_any[k];
-        if (held_any[k]) {
-            float *dst = tmp + start_of(c);
-#pragma unroll
-            for (int x = 0; x < 8; x++) dst[(v * 8u + x) * nb + blk] = held[k][x];
-        }
-    }
-    __syncthreads();
-
-    // Column pass and conversion: out[y][x] = sum_v T[y][v] tmp[v][x] in
-    // order (src/dct.rs:54-64), then floor(v scale + bias) clamped
-    // (src/dsp/scalar.rs:8-12). A task is two neighbouring columns of one
-    // block, so each row result is read once; neighbouring threads take
-    // neighbouring blocks (no bank conflicts). The samples go to shared
-    // memory as pairs, [y][column pair][blk] per component.
-    const float oscale = fd.out_scale, obias = fd.out_bias, omax = fd.out_max;
-    uint32_t *stage = reinterpret_cast<uint32_t *>(smem + 4 * kMaxSliceCoefs + kMaxSliceCoefs / 8);
-    // floor(v) clamped to [0, max] of the converted value v = a scale + bias.
-    const auto convert = [&](float v) { return floor_clamped(v, omax); };
-    for (uint32_t t = tid; t < all_blocks * 4u; t += kIdctThreads) {
-        const uint32_t c = t < luma_blocks * 4u ? 0u : (t < (luma_blocks + chroma_blocks) * 4u ? 1u : 2u);
-        const uint32_t tc = t - start_of(c) / 16u;  // 4 column tasks a block
-        const uint32_t nb = blocks_of(c);
-        const uint32_t blk = tc & (nb - 1u), j = tc >> shift_of(c);
-        const float *src = tmp + start_of(c) + 2u * j * nb + blk;
-        const uint64_t rows = *reinterpret_cast<const uint64_t *>(nz + (start_of(c) / 64u + blk) * 8u);
-        // Outputs y = 2 i, 2 i + 1 of each column a pair.
-        uint64_t a0[4], a1[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) a0[i] = a1[i] = 0;
-#pragma unroll
-        for (int v = 0; v < 8; v++) {
-            if (!((rows >> (8 * v)) & 0xffu)) continue;
-            const float t0 = src[8u * v * nb], t1 = src[8u * v * nb + nb];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float w0 = c_idct_basis[8 * (2 * i) + v], w1 = c_idct_basis[8 * (2 * i + 1) + v];
-                a0[i] = pair_add(a0[i], pair_of(__fmul_rn(w0, t0), __fmul_rn(w1, t0)));
-                a1[i] = pair_add(a1[i], pair_of(__fmul_rn(w0, t1), __fmul_rn(w1, t1)));
-            }
-        }
-        const uint64_t ob2 = pair_of(obias, obias);
-        const auto scaled = [&](uint64_t a) {
-            float lo, hi;
-            pair_split(a, lo, hi);
-            return pair_add(pair_of(__fmul_rn(lo, oscale), __fmul_rn(hi, oscale)), ob2);
-        };
-        uint32_t *dst = stage + start_of(c) / 2u + j * nb + blk;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            float p0, p1, q0, q1;
-            pair_split(scaled(a0[i]), p0, p1);
-            pair_split(scaled(a1[i]), q0, q1);
-            dst[4u * (2 * i) * nb] = convert(p0) | (convert(q0) << 16);
-            dst[4u * (2 * i + 1) * nb] = convert(p1) | (convert(q1) << 16);
-        }
-    }
-    __syncthreads();
-
-    // Stores: a thread writes one 8-sample row of a block; neighbouring
-    // threads write neighbouring row segments of the picture.
-    for (uint32_t c = 0; c < 3; c++) {
-        const uint32_t segs = (c == 0 || cpm == 4) ? 2u * mbs : mbs;
-        const uint32_t per_mb = c == 0 ? 4u : cpm;
-        const uint32_t nb = blocks_of(c);
-        const uint32_t pw = fd.plane_w[c];
-        uint16_t *plane = fd.out_planes ? fd.out_planes + (fd.plane_off[c] - fd.plane_off[0]) : d.planes + fd.plane_off[c];
-        for (uint32_t t = tid; t < 16u * segs; t += kIdctThreads) {
-            const uint32_t r = t >> (31u - __clz(segs)), sx = t & (segs - 1u);
-            uint32_t m, bb;
-            if (c == 0) {
-                m = sx >> 1;
-                bb = ((r >> 3) << 1) | (sx & 1u);
-            } else if (cpm == 2) {
-                m = sx;
-                bb = r >> 3;
-            } else {
-                m = sx >> 1;
-                bb = ((sx & 1u) << 1) | (r >> 3);
-            }
-            const uint32_t blk = m * per_mb + bb, y = r & 7u;
-            uint32_t bx, by;
-            block_xy(c, fd.chroma, sd.mb_x, sd.mb_y, m, bb, bx, by);
-            if (bx >= pw || by + y >= pd.height) continue;
-            const uint32_t *src = stage + start_of(c) / 2u + 4u * y * nb + blk;
-            uint4 v;
-            v.x = src[0];
-            v.y = src[nb];
-            v.z = src[2u * nb];
-            v.w = src[3u * nb];
-            const uint32_t cols = min(8u, pw - bx);
-            uint16_t *dst = plane + (uint64_t)(pd.first_row + pd.row_step * (by + y)) * pw + bx;
-            if (cols == 8u && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0)) {
-                *reinterpret_cast<uint4 *>(dst) = v;
-            } else {
-                for (uint32_t x = 0; x < cols; x++) {
-                    const uint32_t w = x < 2u ? v.x : (x < 4u ? v.y : (x < 6u ? v.z : v.w));
-                    dst[x] = (uint16_t)(w >> (16u * (x & 1u)));
-                }
-            }
+            for (uint32_t x = 0; x < 8; x++)
+                if (x < cols) dst[x] = (uint16_t)(px[y][x / 2u] >> (16u * (x & 1u)));
         }
     }
 }
@@ -1241,7 +1307,7 @@ cudaError_t upload_scans() {
         s[0][i] = kProgressiveScan[i];
         s[1][i] = kInterlacedScan[i];
     }
-    return cudaMemcpyToSymbol(c_scan, s, sizeof s);
+    return cudaMemcpyToSymbol(d_scan, s, sizeof s);
 }
 
 cudaError_t launch_locate(const DecodeLaunch &d, cudaStream_t s) {
@@ -1256,12 +1322,11 @@ cudaError_t launch_entropy(const DecodeLaunch &d, const EntropyShape &shape, cud
     return cudaGetLastError();
 }
 
-// Coefficients (row results over them), non-zero row flags, sample pairs.
-size_t idct_smem_bytes() { return 4 * kMaxSliceCoefs + kMaxSliceCoefs / 8 + 2 * kMaxSliceCoefs; }
+static size_t idct_smem_bytes() { return kIdctWarps * sizeof(IdctWarp); }
 
 cudaError_t launch_idct(const DecodeLaunch &d, cudaStream_t s) {
-    if (d.n_slices == 0) return cudaSuccess;
-    k_idct<<<d.n_slices, kIdctThreads, idct_smem_bytes(), s>>>(d);
+    if (d.n_idct_items == 0) return cudaSuccess;
+    k_idct<<<(d.n_idct_items + kIdctWarps - 1) / kIdctWarps, 32 * kIdctWarps, idct_smem_bytes(), s>>>(d);
     return cudaGetLastError();
 }
 

@@ -41,7 +41,22 @@ struct PicDesc {
     uint32_t frame;
     uint32_t height, first_row, row_step;  // picture rows and where they land in the frame
     uint32_t interlaced_scan;
+    uint32_t idct_base;  // the picture's first item in DecodeLaunch::idct_items
 };
+
+// How k_idct, which takes up to 32 blocks a warp, splits the slices of a
+// picture by their nominal macroblocks: `parts` items a slice (whole
+// components), or one item for `slices` neighbouring slices, the blocks of
+// each at a distance of `blocks` lanes. Row-end slices, which are narrower,
+// leave lanes idle.
+struct IdctShape {
+    uint32_t parts, slices, blocks;
+};
+__host__ __device__ inline IdctShape idct_shape(uint32_t chroma, uint32_t log2_slice_mbs) {
+    const uint32_t blocks = (chroma == 2 ? 8u : 12u) << log2_slice_mbs;
+    if (blocks >= 32u) return IdctShape{(blocks + 31u) / 32u, 1u, blocks};
+    return IdctShape{1u, 32u / blocks, blocks};
+}
 
 // One slice, located (filled on the device from the slice table).
 struct SliceDesc {
@@ -103,7 +118,10 @@ struct DecodeLaunch {
     uint16_t *alpha;
     const uint8_t *weights;  // [set][2][64] raster weights
     unsigned int *work_counter;
-    uint32_t n_frames, n_pics, n_slices;
+    // k_idct's items, written by k_locate: a first slice, the number of
+    // slices << 8 | the part (IdctShape), the picture and the frame.
+    uint4 *idct_items;
+    uint32_t n_frames, n_pics, n_slices, n_idct_items;
     uint32_t entropy_per_lane;  // slice components a lane decodes per grab of the work counter
     // Fused decode: slices a CTA takes at once, and the coefficient
     // positions its shared memory holds for them (group x the most any

@@ -238,7 +238,7 @@ cudaError_t Stager::finish() {
 
 void Workspace::bind_stream(Context *owner) {
     for (DeviceBuf *b : {&bits, &frames, &pics, &slices, &slot_status, &pic_status, &coef, &coef_count, &planes,
-                         &alpha, &weights, &counter, &enc_in, &enc_alpha_in, &enc_coef, &enc_cost, &enc_pic_state,
+                         &alpha, &weights, &counter, &idct_items, &enc_in, &enc_alpha_in, &enc_coef, &enc_cost, &enc_pic_state,
                          &enc_out, &enc_slice_out, &enc_alpha_bits, &enc_alpha_bytes, &enc_frame_out}) {
         b->stream = stream;
         b->wait_ms = wait_ms;
@@ -249,7 +249,7 @@ void Workspace::bind_stream(Context *owner) {
 size_t Workspace::device_bytes() const {
     size_t n = 0;
     for (const DeviceBuf *b : {&bits, &frames, &pics, &slices, &slot_status, &pic_status, &coef, &coef_count, &planes,
-                               &alpha, &weights, &counter, &enc_in, &enc_alpha_in, &enc_coef, &enc_cost,
+                               &alpha, &weights, &counter, &idct_items, &enc_in, &enc_alpha_in, &enc_coef, &enc_cost,
                                &enc_pic_state, &enc_out, &enc_slice_out, &enc_alpha_bits, &enc_alpha_bytes,
                                &enc_frame_out})
         n += b->cap;
@@ -523,6 +523,10 @@ Status plan_decode(const prores_buf *in, int n, uint32_t out_depth, DecodePlan &
             p.interlaced_scan = h.interlace != 0;
             plan.pdesc.push_back(p);
             plan.n_slices += (uint32_t)n_slices;
+            const IdctShape shape = idct_shape((uint32_t)h.chroma, ph.log2_slice_mbs);
+            plan.pdesc.back().idct_base = plan.n_idct_items;
+            plan.n_idct_items += shape.slices > 1 ? (uint32_t)((n_slices + shape.slices - 1) / shape.slices)
+                                                  : (uint32_t)n_slices * shape.parts;
             plan.coef_total += (size_t)width_in_mb * height_in_mb * 64u * (4u + 2u * cpm);
             f.n_pics++;
             pos += ph.picture_size;
@@ -552,6 +556,7 @@ Status upload_decode(Context &ctx, Workspace &ws, const DecodePlan &plan, cudaSt
     PR_CUDA(ws.pics.reserve(sizeof(PicDesc) * (plan.pdesc.size() + 1)), "cudaMalloc");
     PR_CUDA(ws.slices.reserve(sizeof(SliceDesc) * (plan.n_slices + 1)), "cudaMalloc");
     PR_CUDA(ws.slot_status.reserve(sizeof(int2) * 4 * ((size_t)plan.n_slices + 1)), "cudaMalloc");
+    PR_CUDA(ws.idct_items.reserve(sizeof(uint4) * ((size_t)plan.n_idct_items + 1)), "cudaMalloc");
     PR_CUDA(ws.pic_status.reserve(sizeof(PicStatus) * (plan.pdesc.size() + 1)), "cudaMalloc");
     PR_CUDA(ws.planes.reserve(2 * (plan.planes_total + 8)), "cudaMalloc planes");
     PR_CUDA(ws.alpha.reserve(2 * (plan.alpha_total + 8)), "cudaMalloc alpha");
@@ -605,6 +610,8 @@ DecodeLaunch decode_launch_params(Context &ctx, Workspace &ws, const DecodePlan 
     d.n_frames = (uint32_t)plan.fdesc.size();
     d.n_pics = (uint32_t)plan.pdesc.size();
     d.n_slices = plan.n_slices;
+    d.idct_items = ws.idct_items.as<uint4>();
+    d.n_idct_items = plan.n_idct_items;
     const Tuning t = ctx.current_tuning();
     d.entropy_per_lane = (uint32_t)t.entropy_components_per_lane;
     fused_group(plan, (uint32_t)t.decode_slot_positions, d.group, d.group_positions);

@@ -94,7 +94,8 @@ struct Workspace {
     int device = 0;
     uint32_t wait_ms = kDefaultWaitMs;  // the context's bound when the workspace was taken
     cudaStream_t stream = nullptr;
-    DeviceBuf bits, frames, pics, slices, slot_status, pic_status, coef, coef_count, planes, alpha, weights, counter;
+    DeviceBuf bits, frames, pics, slices, slot_status, pic_status, coef, coef_count, planes, alpha, weights, counter,
+        idct_items;
     // encode
     DeviceBuf enc_in, enc_alpha_in, enc_coef, enc_cost, enc_pic_state, enc_out, enc_slice_out, enc_alpha_bits,
         enc_alpha_bytes, enc_frame_out;
@@ -188,7 +189,7 @@ struct DecodePlan {
     std::vector<PicDesc> pdesc;
     std::vector<uint8_t> weights;
     size_t bits_total = 0, planes_total = 0, alpha_total = 0, coef_total = 0;
-    uint32_t n_slices = 0;
+    uint32_t n_slices = 0, n_idct_items = 0;
     struct Copy {
         const uint8_t *src;
         size_t dst, len;
