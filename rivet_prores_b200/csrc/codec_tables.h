@@ -146,15 +146,19 @@ inline void dct_basis(float out[64]) {
 // run codebooks for previousRun 0-1, 2-3, 4, 5-8, 9-14, 15+ (rows 0-5) and
 // Table 11's level codebooks for previousLevelSymbol 0, 1, 2, 3, 4-7, 8+
 // (rows 0-5). For every kBookBits-bit window prefix an entry holds the
-// codeword it starts with when that is kBookBits bits or fewer and its
-// symbol is below 64: its length (4 bits), its symbol (6 bits) and the row
-// the next code of the same kind is read with, the row of the context this
-// symbol makes (3 bits); 0 otherwise (the decoder then reads the codeword
-// by arithmetic). Eleven bits hold all but about 0.1 % of the run and level
-// codewords of UHD 422 HQ frames (nine bits left about 1 %).
+// codeword it starts with when that is kBookBits bits or fewer: its length
+// (bits 0-3; bit 4 is clear, so that a funnel shift, which takes its amount
+// from the low 5 bits, can take the entry itself), its run or its absolute
+// level (bits 5-11) and the row the next code of the same kind is read with,
+// the row of the context this symbol makes (bits 12-14, in place as that
+// row's byte offset); kBookMiss otherwise (the decoder then reads the
+// codeword by arithmetic). Eleven bits hold every run below 124 and level
+// below 125.
 static constexpr uint32_t kBookBits = 11;
 static constexpr uint32_t kBookEntries = 1u << kBookBits;
 static constexpr uint32_t kBookTableWords = 6 * kBookEntries;
+static constexpr uint32_t kBookRowShift = 12;
+static constexpr uint32_t kBookMiss = 16;
 
 PR_HD uint32_t run_book_row(uint32_t prev_run) {
     return (uint32_t)(0x5444444333321100ull >> (4u * (prev_run < 15u ? prev_run : 15u))) & 15u;
@@ -162,23 +166,26 @@ PR_HD uint32_t run_book_row(uint32_t prev_run) {
 PR_HD uint32_t level_book_row(uint32_t prev_level) {
     return (uint32_t)(0x544443210ull >> (4u * (prev_level < 8u ? prev_level : 8u))) & 15u;
 }
+// A row's codebook (that of the first context of the row).
+PR_HD Codebook run_book_of_row(uint32_t row) { return run_book((0xF95420u >> (4u * row)) & 15u); }
+PR_HD Codebook level_book_of_row(uint32_t row) { return level_book((0x843210u >> (4u * row)) & 15u); }
 
 inline void build_book_tables(uint16_t *run, uint16_t *level) {
-    static const uint32_t run_ctx[6] = {0, 2, 4, 5, 9, 15};
-    static const uint32_t level_ctx[6] = {0, 1, 2, 3, 4, 8};
+    static_assert(2u * kBookEntries == 1u << kBookRowShift, "a row's number in place is its byte offset");
     for (int kind = 0; kind < 2; kind++) {
         uint16_t *out = kind == 0 ? run : level;
         for (uint32_t row = 0; row < 6; row++) {
-            const Codebook cb = kind == 0 ? run_book(run_ctx[row]) : level_book(level_ctx[row]);
+            const Codebook cb = kind == 0 ? run_book_of_row(row) : level_book_of_row(row);
             uint16_t *r = out + row * kBookEntries;
-            for (uint32_t i = 0; i < kBookEntries; i++) r[i] = 0;
-            for (uint32_t n = 0; n < 64; n++) {
+            for (uint32_t i = 0; i < kBookEntries; i++) r[i] = (uint16_t)kBookMiss;
+            for (uint32_t n = 0; n < 127; n++) {
                 const uint32_t len = cb_len(cb, n);
                 if (len > kBookBits) continue;
                 const uint32_t next = kind == 0 ? run_book_row(n) : level_book_row(n);
+                const uint32_t value = kind == 0 ? n : n + 1;
                 const uint32_t first = (uint32_t)cb_bits(cb, n) << (kBookBits - len);
                 for (uint32_t p = 0; p < (1u << (kBookBits - len)); p++)
-                    r[first + p] = (uint16_t)(len | (n << 4) | (next << 10));
+                    r[first + p] = (uint16_t)(len | (value << 5) | (next << kBookRowShift));
             }
         }
     }

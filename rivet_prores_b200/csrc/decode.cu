@@ -8,7 +8,8 @@
 //              the slice header (src/decode.rs:301-338), then the DC and
 //              run/level/sign codes of the interleaved scan (:484-540) as a
 //              list of (position, value) entries, or the alpha
-//              run/difference codes (:570-595) straight into the alpha plane.
+//              run/difference codes (:570-595) straight into the alpha plane;
+//              the lanes of a warp step together.
 //   k_idct     one warp per 32 blocks, a lane each: the entries dequantised
 //              into shared memory, the 8x8 IDCT in the crate's exact
 //              single-precision order (src/dct.rs:36-66,
@@ -68,9 +69,13 @@ struct Bits {
 
     __device__ __forceinline__ uint64_t ld(uint64_t i) const { return bswap64(__ldg(w + i)); }
     __device__ __forceinline__ void init(const uint8_t *base, uint64_t byte_off, uint64_t len) {
+        init_at(base, byte_off * 8, (byte_off + len) * 8);
+    }
+    // The same over bits [from, to).
+    __device__ __forceinline__ void init_at(const uint8_t *base, uint64_t from, uint64_t to) {
         w = reinterpret_cast<const uint64_t *>(base);
-        pos = byte_off * 8;
-        end = pos + len * 8;
+        pos = from;
+        end = to;
         idx = pos >> 6;
         w0 = ld(idx);
         w1 = ld(idx + 1);
@@ -103,10 +108,6 @@ struct Bits {
         v = peek() >> (64 - n);
         pos += n;
         return DE_OK;
-    }
-    // RDD 36 endOfData(): 31 or fewer bits remain, all zero (src/bits.rs:98-101).
-    __device__ __forceinline__ bool end_of_data() {
-        return remaining() <= 31 && peek() == 0;
     }
 };
 
@@ -144,24 +145,49 @@ __device__ __forceinline__ int read_sym(Bits &b, Codebook cb, uint32_t &sym) {
 
 // A component's coefficient list, in a region of 2 cap 32-bit words (cap =
 // 64 n_blocks, the component's positions): entries from the front, each
-// (scanned index << 21) | value in 21-bit two's complement. Values outside
-// [kListMin, 2^20) go to the back of the region, the k-th at 2 cap - 1 - k,
-// and their entry holds -2^20 + k. Half the bytes of (index, value) pairs
-// of 32-bit words, for values of any size.
-constexpr int32_t kListMin = -(1 << 20) + 2048;
+// (scanned index << 21) | (magnitude << 5) | sign, in which a table entry's
+// level and 32 times the index are in place. Magnitudes from kListBigMag up go to the back of the region as whole values, the k-th at
+// 2 cap - 1 - k, and their entry holds kListBigMag + k. Half the bytes of
+// (index, value) pairs of 32-bit words, for values of any size.
+constexpr uint32_t kListBigMag = (1u << 16) - 2048u;
 constexpr uint32_t kListBig = 1u << 31;  // in a list's count: it has values at the back of its region
 
 struct CoefList {
     uint32_t *w;
     uint32_t cap, big, count;
+    // The last four entries. They go out 16 bytes at a time: every lane has a
+    // region of its own, so each lane's store takes the memory pipe a cycle,
+    // and one store an entry held up the table reads queued behind it.
+    uint4 last;
+    __device__ __forceinline__ void push(bool ok, uint32_t e) {
+        last.x = ok ? last.y : last.x;
+        last.y = ok ? last.z : last.y;
+        last.z = ok ? last.w : last.z;
+        last.w = ok ? e : last.w;
+        count += ok ? 1u : 0u;
+        if (ok && (count & 3u) == 0) *reinterpret_cast<uint4 *>(w + count - 4u) = last;
+    }
+    __device__ __forceinline__ void finish() {
+        const uint32_t n = count & 3u;
+        if (n > 2u) w[count - 3u] = last.y;
+        if (n > 1u) w[count - 2u] = last.z;
+        if (n > 0u) w[count - 1u] = last.w;
+    }
     __device__ __forceinline__ void put(uint32_t n, int32_t v) {
-        if (v >= kListMin && v < (1 << 20)) {
-            w[count++] = (n << 21) | ((uint32_t)v & 0x1FFFFFu);
-        } else {
+        uint32_t mag = v < 0 ? 0u - (uint32_t)v : (uint32_t)v;
+        uint32_t sign = (uint32_t)(v < 0);
+        if (mag >= kListBigMag) {
             w[2u * cap - 1u - big] = (uint32_t)v;
-            w[count++] = (n << 21) | ((uint32_t)(-(1 << 20) + (int32_t)big) & 0x1FFFFFu);
+            mag = kListBigMag + big;
+            sign = 0;
             big++;
         }
+        push(true, (n << 21) | (mag << 5) | sign);
+    }
+    // If `ok`, the coefficient at n32 / 32 whose level is that of table entry
+    // e2 and whose sign is the top bit of t.
+    __device__ __forceinline__ void put_code(bool ok, uint32_t n32, uint32_t e2, uint32_t t) {
+        push(ok, (n32 << 16) + ((e2 & 0xFE0u) | (t >> 31)));
     }
 };
 
@@ -187,47 +213,9 @@ struct SlotOut {
             wide[n] = v;
         }
     }
-};
-
-// The read position as a 64-bit window consumed from the top: `cur` holds
-// the bits [pos, pos + avail) MSB first with zeros below, and is refilled
-// 32 bits at a time from the words after it, which are fetched two ahead
-// and kept as loaded (byte-swapped only when they enter the window), so a
-// refill never waits for the load it issues. A symbol costs shifts of the
-// window rather than a fresh funnel shift of two words. Reads the same
-// bits as Bits; only used while at least 32 bits of the component remain,
-// so the top 32 bits are always data. The words fetched reach 12 bytes past
-// the component's data at most, inside the bitstream buffer's padding.
-struct Window {
-    const uint32_t *w;
-    uint64_t cur;
-    uint32_t avail, left;  // valid bits in cur (>= 32); bits of the component from pos on
-    uint64_t next;         // index of the word after those in cur
-    uint32_t raw1, raw2;   // words next and next + 1, as loaded
-
-    __device__ __forceinline__ static uint32_t be32(uint32_t v) { return __byte_perm(v, 0, 0x0123); }
-    __device__ __forceinline__ void init(const uint8_t *base, uint64_t pos, uint64_t end) {
-        w = reinterpret_cast<const uint32_t *>(base);
-        const uint64_t i = pos >> 5;
-        const uint32_t skip = (uint32_t)(pos & 31);
-        cur = (((uint64_t)be32(__ldg(w + i)) << 32) | be32(__ldg(w + i + 1))) << skip;
-        avail = 64u - skip;
-        next = i + 2;
-        raw1 = __ldg(w + next);
-        raw2 = __ldg(w + next + 1);
-        left = (uint32_t)(end - pos);
-    }
-    __device__ __forceinline__ uint32_t top() const { return (uint32_t)(cur >> 32); }
-    __device__ __forceinline__ void consume(uint32_t len) {
-        cur <<= len;
-        avail -= len;
-        left -= len;
-        if (avail < 32u) {
-            cur |= (uint64_t)be32(raw1) << (32u - avail);
-            avail += 32u;
-            raw1 = raw2;
-            raw2 = __ldg(w + ++next + 1);
-        }
+    __device__ __forceinline__ void put_code(bool ok, uint32_t n32, uint32_t e2, uint32_t t) {
+        const int32_t level = (int32_t)((e2 >> 5) & 127u);
+        if (ok) slot[n32 >> 5] = (T)((int32_t)t < 0 ? -level : level);
     }
 };
 
@@ -254,257 +242,462 @@ __device__ __forceinline__ bool window_code(uint32_t t, Codebook cb, uint32_t &s
     return true;
 }
 
-// scanned_coefficients() of one component (src/decode.rs:484-540): every
-// coefficient the codes give, in scanned-index order, handed to `out.put`
-// (position, value); the positions not handed over are zero. `run_tab` and
-// `level_tab` are the packed prefix tables of build_book_tables (a row per
-// distinct codebook). While 32 or more bits remain, codes are read from the
-// window: a run, level and sign whose codewords are both in the tables in
-// one go, any other codeword of up to 32 bits by window_code, a symbol at a
-// time (all the bits they take are data, so they come out as the general
-// reader would read them). A longer codeword and the last bits of the data
-// go through the general reader, which also names every failure as the
-// crate does.
-// The DC part of decode_scanned() (src/decode.rs:486-498): the first
-// DC by EG5, each next one as a difference by Table 9 on the previous
-// difference, the sign flipped after a negative one.
-template <class Out>
-__device__ int decode_dc(Bits &b, uint32_t n_blocks, Out &out, Window &win, bool &in_win) {
-    // Each code from the window while 32 or more bits remain (all of them
-    // data, so a codeword of up to 32 bits reads as the general reader
-    // would); otherwise, or for a longer one, the general reader, which
-    // names any failure. The window is left at the first AC code.
-    in_win = b.remaining() >= 32;
-    if (in_win) win.init(reinterpret_cast<const uint8_t *>(b.w), b.pos, b.end);
-    int32_t prev_dc = 0, prev_diff = 3;
-    for (uint32_t i = 0; i < n_blocks; i++) {
-        const Codebook cb = i == 0 ? kFirstDcBook : dc_book(prev_diff);
-        uint32_t sym, len;
-        if (in_win && win.left >= 32u && window_code(win.top(), cb, sym, len)) {
-            win.consume(len);
-        } else {
-            if (in_win) b.pos = b.end - win.left;
-            const int err = read_sym(b, cb, sym);
-            if (err) return err;
-            in_win = b.remaining() >= 32;
-            if (in_win) win.init(reinterpret_cast<const uint8_t *>(b.w), b.pos, b.end);
-        }
-        if (i == 0) {
-            prev_dc = symbol_to_signed(sym);
-            out.put(0, prev_dc);
-            continue;
-        }
-        int32_t n = symbol_to_signed(sym);
-        int32_t diff = prev_diff < 0 ? -n : n;
-        int64_t s = (int64_t)prev_dc + diff;
-        if (s > INT32_MAX || s < INT32_MIN) return DE_DC_OVERFLOW;
-        prev_dc = (int32_t)s;
-        out.put(i, prev_dc);
-        prev_diff = diff;
+// Readers of a component's bits for the lanes of a warp that run together:
+// two 32-bit words, MSB first, a bit offset in the first, and the component's
+// bits from there on. top() is the next 32 bits (those past the component's
+// end are its neighbour's), advance() moves on by up to 32 bits, check() lets
+// the reader fetch ahead; between two checks it moves on by 4 words at most.
+__device__ __forceinline__ uint32_t be32(uint32_t v) { return __byte_perm(v, 0, 0x0123); }
+
+// Words straight from global memory, two of them on their way. A lane that
+// moves on waits for what any lane loaded last: the fused decoder's reader,
+// which has no shared memory to spare.
+struct WordReader {
+    const uint32_t *next;  // the word after the two on their way
+    uint32_t w0, w1, raw1, raw2, pos;
+    int32_t nleft;  // the bits left, negated
+    __device__ __forceinline__ void init(const uint64_t *base, uint64_t from, uint64_t to) {
+        next = reinterpret_cast<const uint32_t *>(base) + (from >> 5);
+        w0 = be32(__ldg(next));
+        w1 = be32(__ldg(next + 1));
+        raw1 = __ldg(next + 2);
+        raw2 = __ldg(next + 3);
+        next += 4;
+        pos = (uint32_t)from & 31u;
+        nleft = -(int32_t)(to - from);
     }
-    if (in_win) b.pos = b.end - win.left;
-    return DE_OK;
+    __device__ __forceinline__ uint32_t left() const { return (uint32_t)-nleft; }
+    __device__ __forceinline__ uint32_t top() const { return __funnelshift_l(w1, w0, pos); }
+    // The 32 bits from `off` (at most 32) bits on.
+    __device__ __forceinline__ uint32_t top_at(uint32_t off) const {
+        const uint32_t p = pos + off;
+        return __funnelshift_l(p < 32u ? w1 : be32(raw1), p < 32u ? w0 : w1, p);
+    }
+    __device__ __forceinline__ void advance(uint32_t len) {
+        pos += len;
+        nleft += (int32_t)len;
+        if (pos >= 32u) {
+            pos -= 32u;
+            w0 = w1;
+            w1 = be32(raw1);
+            raw1 = raw2;
+            raw2 = __ldg(next++);
+        }
+    }
+    __device__ __forceinline__ void check(uint32_t, bool) {}
+};
+
+// Words from a ring of 8 a lane in shared memory, filled 16 bytes at a time
+// at the checks, each from a load made at a check before. A register that any
+// lane has a load in flight to stalls the whole warp when it is next read, so
+// the loads land where only a check reads them: with the words taken from
+// registers as loaded (WordReader) a warp waited out a load nearly every code
+// (11 of 16 stall cycles an instruction). Fetches reach at most 16 words past
+// the read position.
+struct RingReader {
+    uint32_t *ring;    // this lane's word 0; word k is ring[32 (k & 7)]
+    const uint4 *src;  // the block after q
+    uint4 q;           // the ring's next block
+    uint32_t w0, w1, w2, pos;
+    int32_t nleft;
+    uint32_t rd, wr;  // the number of w2, and of the next word the ring gets
+    __device__ __forceinline__ void put(uint4 v) {
+        uint32_t *at = ring + 32u * (wr & 7u);  // wr is a multiple of 4
+        at[0] = be32(v.x);
+        at[32] = be32(v.y);
+        at[64] = be32(v.z);
+        at[96] = be32(v.w);
+        wr += 4;
+    }
+    __device__ __forceinline__ void init(const uint64_t *base, uint64_t from, uint64_t to) {
+        src = reinterpret_cast<const uint4 *>(base) + (from >> 7);
+        const uint4 a = __ldg(src), b = __ldg(src + 1);
+        q = __ldg(src + 2);
+        src += 3;
+        wr = 0;
+        put(a);
+        put(b);
+        rd = (((uint32_t)from >> 5) & 3u) + 2u;
+        w0 = ring[32u * (rd - 2u)];
+        w1 = ring[32u * (rd - 1u)];
+        w2 = ring[32u * rd];
+        pos = (uint32_t)from & 31u;
+        nleft = -(int32_t)(to - from);
+    }
+    __device__ __forceinline__ uint32_t left() const { return (uint32_t)-nleft; }
+    __device__ __forceinline__ uint32_t top() const { return __funnelshift_l(w1, w0, pos); }
+    // The 32 bits from `off` (at most 32) bits on.
+    __device__ __forceinline__ uint32_t top_at(uint32_t off) const {
+        const uint32_t p = pos + off;
+        return __funnelshift_l(p < 32u ? w1 : w2, p < 32u ? w0 : w1, p);
+    }
+    // No branch: a lane that stays within its word loads the same w2 again.
+    __device__ __forceinline__ void advance(uint32_t len) {
+        pos += len;
+        nleft += (int32_t)len;
+        const bool on = pos >= 32u;
+        w0 = on ? w1 : w0;
+        w1 = on ? w2 : w1;
+        rd += on ? 1u : 0u;
+        pos &= 31u;
+        w2 = ring[32u * (rd & 7u)];
+    }
+    __device__ __forceinline__ void check(uint32_t mask, bool live) {
+        do {
+            // Words rd to wr - 1 are still to come; a block fits beside 4.
+            if (live && wr - rd < 5u) {
+                put(q);
+                q = __ldg(src++);
+            }
+        } while (__any_sync(mask, live && wr - rd < 5u));
+    }
+};
+
+// The DC part of scanned_coefficients() (src/decode.rs:486-498): the first
+// DC by EG5, each next one as a difference by Table 9 on the previous
+// difference, the sign flipped after a negative one. The lanes of `mask` run
+// it together, four codes between checks. A code that is 32 bits or fewer and
+// all data is read from top(): with z leading zeros, EGk is 2 z + k + 1 bits,
+// z + k + 1 of them n + 2^k; Table 9's (1, 2, 3) for |difference| 2 is 3 or 4
+// bits with z <= 1, from there on 2 z + 2 bits, z + 2 of them n itself. Any
+// other code waits for the end of the four and goes by the general reader,
+// which names any failure.
+template <class Reader, class Out>
+__device__ __forceinline__ int decode_dc(uint32_t mask, bool live, Reader &r, const Bits &b, uint32_t n_blocks, Out &out) {
+    int err = DE_OK;
+    uint32_t i = 0;
+    int32_t prev_dc = 0, prev_diff = 3;
+    const auto take = [&](uint32_t sym) {
+        const int32_t n = symbol_to_signed(sym);
+        if (i == 0) {
+            prev_dc = n;
+        } else {
+            prev_diff = prev_diff < 0 ? -n : n;
+            const int64_t s = (int64_t)prev_dc + prev_diff;
+            if (s > INT32_MAX || s < INT32_MIN) err = DE_DC_OVERFLOW;
+            prev_dc = (int32_t)s;
+        }
+        if (!err) out.put(i++, prev_dc);
+        live = err == DE_OK;
+    };
+    while (__any_sync(mask, live && i < n_blocks)) {
+        bool stuck = false;
+#pragma unroll 1
+        for (int k = 0; k < 4; k++) {
+            const uint32_t t = r.top(), z = __clz(t);
+            const uint32_t a = i == 0 ? 5u : min((uint32_t)abs(prev_diff), 3u), e = a == 2u ? 1u : a;
+            const bool rice = a == 2u && z <= 1u;
+            const uint32_t len = rice ? z + 3u : 2u * z + e + 1u;
+            const uint32_t sym = rice ? (z << 2) | ((t << (z + 1u)) >> 30)
+                                      : ((t << z) >> ((31u - z - e) & 31u)) - (a == 2u ? 0u : 1u << e);
+            if (live && i < n_blocks) {
+                stuck = r.nleft > -32 || len > 32u;
+                if (!stuck) {
+                    r.advance(len);
+                    take(sym);
+                }
+            }
+        }
+        r.check(mask, live);
+        if (__any_sync(mask, stuck)) {
+            if (stuck) {
+                Bits g;
+                g.init_at(reinterpret_cast<const uint8_t *>(b.w), b.end - r.left(), b.end);
+                uint32_t sym = 0;
+                err = read_sym(g, i == 0 ? kFirstDcBook : dc_book(prev_diff), sym);
+                if (!err) {
+                    r.init(b.w, g.pos, b.end);
+                    take(sym);
+                }
+                live = err == DE_OK;
+            }
+            r.check(mask, live);
+        }
+    }
+    return err;
 }
 
-template <class Out>
-__device__ int decode_component(Bits &b, uint32_t n_blocks, Out &out, const uint16_t *run_tab,
-                                const uint16_t *level_tab) {
-    Window win;
-    bool in_win;
-    int err = decode_dc(b, n_blocks, out, win, in_win);
-    if (err) return err;
-    const uint32_t total = n_blocks * 64;
-    uint32_t n = n_blocks, prev_run = 4, prev_level = 1;
-    // One run, level and sign an iteration: from the window while it holds
-    // the read position and 32 or more bits remain, else by the general
-    // reader (which then hands the position back to a fresh window). A lane
-    // that takes the general reader leaves the others only for that one
-    // iteration.
-    uint32_t rrow = run_book_row(prev_run) * kBookEntries, lrow = level_book_row(prev_level) * kBookEntries;
-    for (;;) {
-        bool level_next = false;  // the run is read; its level and sign are the general reader's
-        if (in_win && win.left >= 32u) {
-            const uint32_t t = win.top();
-            const uint32_t e1 = run_tab[rrow + (t >> (32 - kBookBits))];
-            uint32_t run = 0, l = 0;
-            bool got = true;
-            if (e1) {
-                l = e1 & 15u;
-                run = (e1 >> 4) & 63u;
-                const uint32_t t2 = t << l;
-                const uint32_t e2 = level_tab[lrow + (t2 >> (32 - kBookBits))];
-                if (e2) {
-                    // Run, level and sign in one go.
-                    const uint32_t l2 = e2 & 15u;
-                    prev_run = run;
-                    prev_level = (e2 >> 4) & 63u;
-                    n += run;
-                    if (n >= total) return DE_RUN_PAST_END;
-                    const int32_t level = (int32_t)prev_level + 1;
-                    out.put(n, (t2 << l2) >> 31 ? -level : level);
-                    n += 1;
-                    rrow = (e1 >> 10) * kBookEntries;
-                    lrow = (e2 >> 10) * kBookEntries;
-                    win.consume(l + l2 + 1u);
-                    continue;
-                }
-            } else {
-                got = window_code(t, run_book(prev_run), run, l);
-            }
-            if (got) {
-                prev_run = run;
+// The AC part of scanned_coefficients() (src/decode.rs:499-540): every
+// coefficient the codes give, in scanned-index order, handed to `out`; the
+// positions not handed over are zero. The lanes of `mask` run it together, a
+// component each (`live` false: none). A step reads one run, level and sign
+// from the prefix tables without a branch; a lane whose code is not there, or
+// runs past its data or its positions, stays where it is, and after four
+// steps such lanes leave the others for one code. Bits past the end of the
+// component read as zero, as the crate's reader has them, so the tables serve
+// to the last code. What they do not hold goes by window_code and, for
+// codewords over 32 bits and for naming every failure as the crate does, by
+// read_sym. `r` is at the first AC code; `b` gives the bitstream and the end.
+template <class Reader, class Out>
+__device__ __forceinline__ int decode_ac(uint32_t mask, bool live, Reader &r, const Bits &b, uint32_t n_blocks,
+                                         Out &out, const uint16_t *run_tab, const uint16_t *level_tab) {
+    const char *run_bytes = reinterpret_cast<const char *>(run_tab);
+    const char *level_bytes = reinterpret_cast<const char *>(level_tab);
+    const uint32_t total32 = n_blocks * 64u * 32u;
+    uint32_t n32 = n_blocks * 32u;  // 32 times the position
+    // The rows of previous run 4 and previous level 1.
+    uint32_t rrow = 2u << kBookRowShift, lrow = 1u << kBookRowShift;
+    int err = DE_OK;
+    bool ok = false, done = false;  // of a lane's last step
+    if (!live) r.nleft = 0;         // done from the start
+    const auto step = [&]() {
+        // Zeros past the end: 32 - left bits when that is positive.
+        const uint32_t past = (uint32_t)__viaddmax_s32(r.nleft, 32, 0);
+        const uint32_t t = r.top() & __funnelshift_lc(0u, 0xFFFFFFFFu, past);
+        const uint32_t e1 = *reinterpret_cast<const uint16_t *>(run_bytes + (rrow | ((t >> 20) & 0xFFEu)));
+        const uint32_t t2 = __funnelshift_l(0u, t, e1);
+        const uint32_t e2 = *reinterpret_cast<const uint16_t *>(level_bytes + (lrow | ((t2 >> 20) & 0xFFEu)));
+        const uint32_t t3 = __funnelshift_l(0u, t2, e2);
+        const uint32_t len = (e1 & 15u) + (e2 & 15u) + 1u;  // at most 23
+        const uint32_t at32 = n32 + (e1 & 0xFE0u);
+        // endOfData(): 31 or fewer bits remain, all zero (no run code is).
+        done = past > 0 && t == 0;
+        ok = ((e1 | e2) & kBookMiss) == 0 && r.nleft + (int32_t)len <= 0 && at32 < total32;
+        out.put_code(ok, at32, e2, t3);
+        n32 = ok ? at32 + 32u : n32;
+        rrow = ok ? e1 & (7u << kBookRowShift) : rrow;
+        lrow = ok ? e2 & (7u << kBookRowShift) : lrow;
+        r.advance(ok ? len : 0u);
+    };
+    // One code by any means, at most 65 bits.
+    const auto slow_step = [&]() {
+        const uint32_t total = n_blocks * 64u;
+        uint32_t run = 0, lvl = 0, l = 0, n = n32 >> 5;
+        bool have_run = false, have_level = false, neg = false;
+        if (r.nleft <= -32) {  // all of top() is data
+            have_run = window_code(r.top(), run_book_of_row(rrow >> kBookRowShift), run, l);
+            if (have_run) {
                 n += run;
-                if (n >= total) return DE_RUN_PAST_END;
-                win.consume(l);
-                uint32_t lvl = 0;
-                got = false;
-                if (win.left >= 32u) {
-                    const uint32_t u = win.top();
-                    const uint32_t e2 = level_tab[lrow + (u >> (32 - kBookBits))];
-                    if (e2) {
-                        lvl = (e2 >> 4) & 63u;
-                        l = e2 & 15u;
-                        got = true;
-                    } else {
-                        got = window_code(u, level_book(prev_level), lvl, l);
-                    }
+                if (n >= total) err = DE_RUN_PAST_END;
+                r.advance(l);
+                if (r.nleft <= -32) have_level = window_code(r.top(), level_book_of_row(lrow >> kBookRowShift), lvl, l);
+                if (have_level) {
+                    r.advance(l);
+                    if (r.nleft == 0 && !err) err = DE_PAST_END;
+                    neg = r.top() >> 31;
+                    r.advance(1u);
                 }
-                if (got) {
-                    win.consume(l);
-                    prev_level = lvl;
-                    if (win.left == 0) return DE_PAST_END;
-                    const bool neg = win.top() >> 31;
-                    win.consume(1u);
-                    const int32_t level = (int32_t)lvl + 1;
-                    out.put(n, neg ? -level : level);
-                    n += 1;
-                    rrow = run_book_row(prev_run) * kBookEntries;
-                    lrow = level_book_row(prev_level) * kBookEntries;
-                    continue;
-                }
-                level_next = true;
             }
         }
-        // The general reader, from the window's position.
-        if (in_win) b.pos = b.end - win.left;
-        if (!level_next) {
-            if (b.remaining() <= 31 && b.peek() == 0) break;  // endOfData()
-            uint32_t run;
-            if ((err = read_sym(b, run_book(prev_run), run))) return err;
-            prev_run = run;
-            n += run;
-            if (n >= total) return DE_RUN_PAST_END;
+        if (!have_level && !err) {
+            Bits g;
+            g.init_at(reinterpret_cast<const uint8_t *>(b.w), b.end - r.left(), b.end);
+            if (!have_run) {
+                err = read_sym(g, run_book_of_row(rrow >> kBookRowShift), run);
+                n += run;
+                if (!err && n >= total) err = DE_RUN_PAST_END;
+            }
+            if (!err) err = read_sym(g, level_book_of_row(lrow >> kBookRowShift), lvl);
+            if (!err && g.remaining() < 1) err = DE_PAST_END;
+            if (!err) {
+                neg = g.peek() >> 63;
+                r.init(b.w, g.pos + 1, b.end);
+            }
         }
-        uint32_t lvl;
-        if ((err = read_sym(b, level_book(prev_level), lvl))) return err;
-        prev_level = lvl;
-        if (b.remaining() < 1) return DE_PAST_END;
-        const bool neg = b.peek() >> 63;
-        b.pos += 1;
-        const int32_t level = (int32_t)lvl + 1;
-        out.put(n, neg ? -level : level);
-        n += 1;
-        rrow = run_book_row(prev_run) * kBookEntries;
-        lrow = level_book_row(prev_level) * kBookEntries;
-        in_win = b.remaining() >= 32;
-        if (in_win) win.init(reinterpret_cast<const uint8_t *>(b.w), b.pos, b.end);
+        if (!err) {
+            const int32_t level = (int32_t)lvl + 1;
+            out.put(n, neg ? -level : level);
+            n32 = (n + 1u) * 32u;
+            rrow = run_book_row(run) << kBookRowShift;
+            lrow = level_book_row(lvl) << kBookRowShift;
+        } else {
+            r.nleft = 0;
+        }
+    };
+    for (;;) {
+        step();
+        step();
+        step();
+        step();
+        r.check(mask, !done);
+        const bool stuck = !ok && !done;
+        if (__any_sync(mask, stuck)) {
+            if (stuck) slow_step();
+            r.check(mask, !done && err == DE_OK);
+        } else if (!__any_sync(mask, !done)) {
+            break;
+        }
     }
-    return DE_OK;
+    return err;
 }
 
 __device__ __forceinline__ uint16_t rescale(uint32_t a, uint64_t m, bool identity) {
     return identity ? (uint16_t)a : (uint16_t)(((uint64_t)a * m + (1ull << 39)) >> 40);
 }
 
-// scanned_alpha() (src/decode.rs:570-595) and its placement (:365-389).
-__device__ int decode_alpha(Bits &b, const FrameDesc &fd, const PicDesc &pd, const SliceDesc &sd, uint16_t *alpha) {
-    const uint32_t bits = fd.alpha_bits;
-    const uint32_t cols = 16u * sd.mbs;
-    const uint32_t count = cols * 16u;
-    const uint32_t rows = (uint32_t)sd.mb_y + 1u < pd.height_in_mb ? 16u : pd.height - 16u * (pd.height_in_mb - 1u);
-    const uint32_t needed = cols * rows;
-    const uint32_t width = fd.width;
+// Where a slice's alpha samples go, and how they are coded.
+struct AlphaArea {
+    uint16_t *row;         // the slice's first sample
+    uint64_t pitch;        // samples from a row to the next of the picture
+    uint32_t cols, ncols;  // coded samples a row (16 a macroblock), those inside the picture
+    uint32_t rows;         // rows inside the picture
+    uint32_t bits;
+    uint64_t rescale_m;
+    bool identity;
+};
+
+__device__ __forceinline__ AlphaArea alpha_area(const FrameDesc &fd, const PicDesc &pd, const SliceDesc &sd,
+                                                uint16_t *alpha) {
+    AlphaArea a;
+    a.bits = fd.alpha_bits;
+    a.cols = 16u * sd.mbs;
+    a.rows = (uint32_t)sd.mb_y + 1u < pd.height_in_mb ? 16u : pd.height - 16u * (pd.height_in_mb - 1u);
     const uint32_t x0 = 16u * sd.mb_x;
-    const uint32_t ncols = min(cols, width - x0);
-    const int32_t mask = (int32_t)((1u << bits) - 1u);
-    const uint32_t mag_bits = bits == 8 ? 3u : 6u;
-    uint16_t *plane = fd.out_alpha ? fd.out_alpha : alpha + fd.alpha_off;
-    const uint32_t cshift = (uint32_t)__ffs(cols) - 1u;  // cols is 16 times a power of two
+    a.ncols = min(a.cols, fd.width - x0);
+    a.row = (fd.out_alpha ? fd.out_alpha : alpha + fd.alpha_off) +
+            (uint64_t)(pd.first_row + pd.row_step * (16u * sd.mb_y)) * fd.width + x0;
+    a.pitch = (uint64_t)pd.row_step * fd.width;
+    a.rescale_m = fd.rescale_m;
+    a.identity = fd.rescale_identity != 0;
+    return a;
+}
+
+// scanned_alpha() (src/decode.rs:570-595) and its placement (:365-389). The
+// lanes of `mask` run it together, a slice each. A step reads a difference
+// and its run when the last run is used up, and adds samples of the run to a
+// group of 8, which goes out as one 16-byte store when it is full (a row is a
+// whole number of groups): a lane in a long run and a lane with a code for
+// every sample take the same steps. A code that runs past its data or the
+// slice waits for the end of three steps and goes by the general reader,
+// which names the failure.
+template <class Reader>
+__device__ __forceinline__ int decode_alpha(uint32_t mask, bool live, Reader &r, const Bits &b, AlphaArea a) {
+    const uint32_t count = a.cols * 16u, needed = a.cols * a.rows;
+    const int32_t value_mask = (int32_t)((1u << a.bits) - 1u);
+    const uint32_t mag_bits = a.bits == 8 ? 3u : 6u;
     int32_t prev = -1;
-    uint32_t n = 0;
-    int err;
-    while (n < count) {
-        if (n >= needed && b.end_of_data()) break;
-        uint64_t v;
-        int32_t diff;
-        uint32_t run;
-        if (b.remaining() >= 64) {
-            // A difference and a run take at most 34 bits: both from one
-            // look at the next 64, all of them data.
-            const uint64_t w = b.peek();
-            uint32_t used;
-            if (w >> 63) {
-                diff = (int32_t)((w << 1) >> (64u - bits));
-                used = 1u + bits;
-            } else {
-                const int32_t a = (int32_t)((w << 1) >> (64u - mag_bits)) + 1;
-                diff = ((w << (1u + mag_bits)) >> 63) ? -a : a;
-                used = 2u + mag_bits;
-            }
-            const uint64_t u = w << used;
-            if (u >> 63) {
-                run = 1;
-                used += 1u;
-            } else {
-                const uint32_t r4 = (uint32_t)((u << 1) >> 60);
-                if (r4) {
-                    run = r4 + 1u;
-                    used += 5u;
-                } else {
-                    run = (uint32_t)((u << 5) >> 53) + 1u;
-                    used += 16u;
-                }
-            }
-            b.pos += used;
-        } else {
-            if ((err = b.read(1, v))) return err;
-            if (v == 1) {
-                if ((err = b.read(bits, v))) return err;
-                diff = (int32_t)v;
-            } else {
-                if ((err = b.read(mag_bits, v))) return err;
-                int32_t a = (int32_t)v + 1;
-                if ((err = b.read(1, v))) return err;
-                diff = v ? -a : a;
-            }
-            if ((err = b.read(1, v))) return err;
-            if (v == 1) {
-                run = 1;
-            } else {
-                if ((err = b.read(4, v))) return err;
-                if (v != 0) {
-                    run = (uint32_t)v + 1;
-                } else {
-                    if ((err = b.read(11, v))) return err;
-                    run = (uint32_t)v + 1;
-                }
-            }
-        }
-        int32_t value = (int32_t)((uint32_t)prev + (uint32_t)diff) & mask;
-        prev = value;
-        if (n + run > count) return DE_ALPHA_RUN;
-        uint16_t out = rescale((uint32_t)value, fd.rescale_m, fd.rescale_identity != 0);
-        uint32_t stop = min(n + run, needed);
-        for (uint32_t i = n; i < stop;) {
-            uint32_t r = i >> cshift, c = i & (cols - 1u);
-            uint32_t seg_end = min(stop - i, cols - c);  // samples left in this row of the run
-            uint16_t *row = plane + (uint64_t)(pd.first_row + pd.row_step * (16u * sd.mb_y + r)) * width + x0;
-            for (uint32_t k = c; k < c + seg_end && k < ncols; k++) row[k] = out;
-            i += seg_end;
-        }
+    uint32_t n = 0, run_left = 0;  // samples up to the end of the run, those of it not placed
+    uint32_t pair = 0;             // the run's sample, twice
+    uint32_t fill = 0, col = 0, row = 0;
+    uint4 group = make_uint4(0, 0, 0, 0);
+    int err = DE_OK;
+    bool done = !live, stuck = false;
+    const auto start_run = [&](int32_t diff, uint32_t run) {
+        prev = (int32_t)((uint32_t)prev + (uint32_t)diff) & value_mask;
+        pair = 0x10001u * rescale((uint32_t)prev, a.rescale_m, a.identity);
+        run_left = run;
         n += run;
+    };
+    const auto step = [&]() {
+        const bool need = run_left == 0 && !done;
+        const uint32_t past = (uint32_t)__viaddmax_s32(r.nleft, 32, 0);
+        const uint32_t t = r.top() & __funnelshift_lc(0u, 0xFFFFFFFFu, past);
+        // Tables 13 and 14: `1` and the difference in full, or `0`, magnitude
+        // - 1 and a sign.
+        const bool full = t >> 31;
+        const int32_t mag = (int32_t)((t << 1) >> (32u - mag_bits)) + 1;
+        const bool neg = (t << (1u + mag_bits)) >> 31;
+        const int32_t diff = full ? (int32_t)((t << 1) >> (32u - a.bits)) : (neg ? -mag : mag);
+        const uint32_t dlen = full ? 1u + a.bits : 2u + mag_bits;
+        // Table 12: `1`; `0` and 4 bits of run - 1; or 5 zeros and 11 bits.
+        const uint32_t u = r.top_at(dlen);
+        const uint32_t r4 = (u << 1) >> 28;
+        const uint32_t run = u >> 31 ? 1u : (r4 ? r4 + 1u : ((u << 5) >> 21) + 1u);
+        const uint32_t rlen = u >> 31 ? 1u : (r4 ? 5u : 16u);
+        const bool end = n >= count || (n >= needed && past > 0 && t == 0);
+        const bool ok = need && !end && r.nleft + (int32_t)(dlen + rlen) <= 0 && n + run <= count;
+        done = done || (need && end);
+        stuck = need && !end && !ok;
+        if (ok) start_run(diff, run);
+        r.advance(ok ? dlen : 0u);
+        r.advance(ok ? rlen : 0u);
+        // The samples from `fill` on take the run's value; those past its
+        // end are overwritten later.
+        const uint32_t k = min(run_left, 8u - fill);
+        const auto keep = [&](uint32_t at) {  // of the two samples from `at`, the bits of those before `fill`
+            return ~__funnelshift_lc(0u, 0xFFFFFFFFu, (uint32_t)max(16 * ((int32_t)fill - (int32_t)at), 0));
+        };
+        const auto merge = [&](uint32_t w, uint32_t at) { return (w & keep(at)) | (pair & ~keep(at)); };
+        group.x = merge(group.x, 0);
+        group.y = merge(group.y, 2);
+        group.z = merge(group.z, 4);
+        group.w = merge(group.w, 6);
+        fill += k;
+        run_left -= k;
+        if (fill == 8u) {
+            fill = 0;
+            if (row < a.rows && col < a.ncols) {
+                uint16_t *dst = a.row + col;
+                if (col + 8u <= a.ncols && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+                    *reinterpret_cast<uint4 *>(dst) = group;
+                } else {
+                    const uint32_t words[4] = {group.x, group.y, group.z, group.w};
+#pragma unroll
+                    for (uint32_t x = 0; x < 8; x++)
+                        if (col + x < a.ncols) dst[x] = (uint16_t)(words[x / 2u] >> (16u * (x & 1u)));
+                }
+            }
+            col += 8u;
+            if (col == a.cols) {
+                col = 0;
+                row++;
+                a.row += a.pitch;
+            }
+        }
+    };
+    // A code of the general reader.
+    const auto slow_step = [&]() {
+        Bits g;
+        g.init_at(reinterpret_cast<const uint8_t *>(b.w), b.end - r.left(), b.end);
+        uint64_t v = 0;
+        int32_t diff = 0;
+        uint32_t run = 1;
+        err = g.read(1, v);
+        if (!err && v == 1) {
+            err = g.read(a.bits, v);
+            diff = (int32_t)v;
+        } else if (!err) {
+            err = g.read(mag_bits, v);
+            const int32_t mag = (int32_t)v + 1;
+            if (!err) err = g.read(1, v);
+            diff = v ? -mag : mag;
+        }
+        if (!err) err = g.read(1, v);
+        if (!err && v == 0) {
+            err = g.read(4, v);
+            if (!err && v == 0) err = g.read(11, v);
+            run = (uint32_t)v + 1u;
+        }
+        if (!err && n + run > count) err = DE_ALPHA_RUN;
+        if (!err) {
+            start_run(diff, run);
+            r.init(b.w, g.pos, b.end);
+        } else {
+            done = true;
+        }
+    };
+    for (;;) {
+        step();
+        step();
+        step();
+        r.check(mask, !done);
+        if (__any_sync(mask, stuck)) {
+            if (stuck) slow_step();
+            stuck = false;
+            r.check(mask, !done);
+        } else if (!__any_sync(mask, !done)) {
+            break;
+        }
     }
-    return DE_OK;
+    return err;
+}
+
+// One component by one lane of any warp (the fused decoder).
+template <class Out>
+__device__ int decode_component(Bits &b, uint32_t n_blocks, Out &out, const uint16_t *run_tab,
+                                const uint16_t *level_tab) {
+    const uint32_t mask = __activemask();
+    WordReader r;
+    r.init(b.w, b.pos, b.end);
+    const int err = decode_dc(mask, true, r, b, n_blocks, out);
+    const int ac_err = decode_ac(mask, err == DE_OK, r, b, n_blocks, out, run_tab, level_tab);
+    return err ? err : ac_err;
+}
+
+__device__ int decode_alpha_alone(Bits &b, const AlphaArea &a) {
+    WordReader r;
+    r.init(b.w, b.pos, b.end);
+    return decode_alpha(__activemask(), true, r, b, a);
 }
 
 // The slice header (src/decode.rs:301-338) and where component `comp` (0
@@ -545,42 +738,67 @@ __device__ int2 component_range(const uint8_t *sb, uint32_t size, bool has_alpha
     return make_int2(DE_OK, 0);
 }
 
-// One work item: component `comp` (0 Y', 1 Cb, 2 Cr, 3 alpha) of slice `s`.
-__device__ void decode_item(const DecodeLaunch &d, uint32_t comp, uint32_t s, const uint16_t *run_tab,
-                            const uint16_t *level_tab) {
-    int2 *slot = d.slot_status + 4ull * s + comp;
-    const SliceDesc sd = d.slices[s];
-    const PicDesc &pd = d.pics[sd.pic];
-    if (d.pic_status[sd.pic].locate_slice >= 0) return;  // never read: the picture failed before decoding
-    // Every run writes every count of the slices it decodes (a failing
-    // component's too), so k_idct never reads a stale one.
-    if (comp < 3) d.coef_count[3ull * s + comp] = 0;
-    const FrameDesc &fd = d.frames[pd.frame];
-    const bool has_alpha = fd.alpha_bits != 0;
-    if (comp == 3 && !has_alpha) {
-        *slot = make_int2(DE_OK, 0);
-        return;
+// One work item a lane: component `comp` (0 Y', 1 Cb, 2 Cr, 3 alpha) of slice
+// `s`, or none (`valid` false). All lanes of the warp come here together.
+__device__ __forceinline__ void decode_items(const DecodeLaunch &d, bool valid, uint32_t comp, uint32_t s,
+                                             const uint16_t *run_tab, const uint16_t *level_tab, uint32_t *ring) {
+    Bits b{};
+    CoefList list{};
+    uint32_t n_blocks = 0;
+    bool live = false, live_alpha = false;  // a colour component, an alpha component to decode
+    AlphaArea area{};
+    int2 status = make_int2(DE_OK, 0);
+    if (valid) {
+        const SliceDesc sd = d.slices[s];
+        const PicDesc &pd = d.pics[sd.pic];
+        // A picture that failed before decoding is never read.
+        valid = d.pic_status[sd.pic].locate_slice < 0;
+        const FrameDesc &fd = d.frames[pd.frame];
+        const bool has_alpha = fd.alpha_bits != 0;
+        if (valid && (comp < 3 || has_alpha)) {
+            uint32_t start = 0, len = 0;
+            const int2 hdr_err = component_range(d.bits + sd.off, sd.size, has_alpha, comp, start, len);
+            if (hdr_err.x != DE_OK) {
+                if (comp == 0) status = hdr_err;
+            } else {
+                b.init(d.bits, sd.off + start, len);
+                if (comp == 3) {
+                    area = alpha_area(fd, pd, sd, d.alpha);
+                    live_alpha = true;
+                } else {
+                    const uint32_t cpm = fd.chroma == 2 ? 2u : 4u;
+                    n_blocks = (comp == 0 ? 4u : cpm) * sd.mbs;
+                    const uint64_t base = sd.coef + (comp == 0 ? 0ull : 64ull * sd.mbs * (4u + (comp - 1u) * cpm));
+                    list.w = reinterpret_cast<uint32_t *>(d.coef + base);
+                    list.cap = 64u * n_blocks;
+                    live = true;
+                }
+            }
+        }
     }
-    uint32_t start = 0, len = 0;
-    const int2 hdr_err = component_range(d.bits + sd.off, sd.size, has_alpha, comp, start, len);
-    if (hdr_err.x != DE_OK) {
-        *slot = comp == 0 ? hdr_err : make_int2(DE_OK, 0);
-        return;
+    __syncwarp();
+    RingReader r{};
+    r.ring = ring;
+    if (live || live_alpha) r.init(b.w, b.pos, b.end);
+    r.check(0xffffffffu, live || live_alpha);
+    if (__any_sync(0xffffffffu, live_alpha)) {
+        const int err = decode_alpha(0xffffffffu, live_alpha, r, b, area);
+        if (live_alpha) status.x = err;
     }
-    Bits b;
-    b.init(d.bits, sd.off + start, len);
-    int err;
-    if (comp == 3) {
-        err = decode_alpha(b, fd, pd, sd, d.alpha);
-    } else {
-        const uint32_t cpm = fd.chroma == 2 ? 2u : 4u;
-        const uint32_t n_blocks = (comp == 0 ? 4u : cpm) * sd.mbs;
-        const uint64_t base = sd.coef + (comp == 0 ? 0ull : 64ull * sd.mbs * (4u + (comp - 1u) * cpm));
-        CoefList list{reinterpret_cast<uint32_t *>(d.coef + base), 64u * n_blocks, 0u, 0u};
-        err = decode_component(b, n_blocks, list, run_tab, level_tab);
-        d.coef_count[3ull * s + comp] = list.count | (list.big ? kListBig : 0u);
+    if (__any_sync(0xffffffffu, live)) {
+        const int dc_err = decode_dc(0xffffffffu, live, r, b, n_blocks, list);
+        const int ac_err = decode_ac(0xffffffffu, live && dc_err == DE_OK, r, b, n_blocks, list, run_tab, level_tab);
+        if (live) {
+            status.x = dc_err ? dc_err : ac_err;
+            list.finish();
+        }
     }
-    *slot = make_int2(err, 0);
+    if (valid) {
+        // Every run writes every count of the slices it decodes (a failing
+        // component's too), so k_idct never reads a stale one.
+        if (comp < 3) d.coef_count[3ull * s + comp] = list.count | (list.big ? kListBig : 0u);
+        d.slot_status[4ull * s + comp] = status;
+    }
 }
 
 // ------------------------------------------------------------------ kernels
@@ -695,11 +913,21 @@ constexpr int kEntropyMaxThreads = 512;
 // Persistent: each warp takes 32 x entropy_per_lane slice components per
 // grab of the work counter, a lane each in turn, component-major, until the
 // list runs out. The alpha components come first: where a frame has alpha,
-// its run/difference codes take a lane several times as long as a colour
-// component, and started last they would leave the launch waiting on them.
+// its codes take a lane several times as long as a colour component, and
+// started last they would leave the launch waiting on them.
+//
+// Bound by the length of a component's chain of codes (small batches: a step
+// waits for two table reads one after the other) and by integer issue (full
+// ones: 63 % of the slots, 72 % of the ALU pipe, 22 of 32 lanes at work).
+// 32 UHD 4:2:2 frames take 680 us, one 175, 8 UHD 4:4:4 frames with 16-bit
+// alpha 1030; with a branch for every case, loads and single-entry stores
+// among the steps, 1810, 535 and 2770. 83 registers leave 24 warps an SM;
+// held to 64 for 32 warps the spills cost 14 %.
 __global__ void __launch_bounds__(kEntropyMaxThreads) k_entropy(DecodeLaunch d) {
-    __shared__ uint16_t run_tab[kBookTableWords];
-    __shared__ uint16_t level_tab[kBookTableWords];
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint16_t *run_tab = reinterpret_cast<uint16_t *>(smem), *level_tab = run_tab + kBookTableWords;
+    // Each warp's ring: word k of lane l at [32 k + l].
+    uint32_t *ring = reinterpret_cast<uint32_t *>(level_tab + kBookTableWords) + 8u * (threadIdx.x & ~31u) + (threadIdx.x & 31u);
     for (uint32_t i = threadIdx.x; i < kBookTableWords / 2; i += blockDim.x) {
         reinterpret_cast<uint32_t *>(run_tab)[i] = reinterpret_cast<const uint32_t *>(d.tables.run_books)[i];
         reinterpret_cast<uint32_t *>(level_tab)[i] = reinterpret_cast<const uint32_t *>(d.tables.level_books)[i];
@@ -716,12 +944,9 @@ __global__ void __launch_bounds__(kEntropyMaxThreads) k_entropy(DecodeLaunch d) 
         if (base >= items) break;
         for (uint32_t k = 0; k < per_lane; k++) {
             const uint32_t item = base + 32u * k + lane;
-            if (item < items) {
-                const uint32_t kind = item / d.n_slices, s = item - kind * d.n_slices;
-                decode_item(d, kind == 0 ? 3u : kind - 1u, s, run_tab, level_tab);
-            }
+            const uint32_t kind = item / d.n_slices, s = item - kind * d.n_slices;
+            decode_items(d, item < items, kind == 0 ? 3u : kind - 1u, s, run_tab, level_tab, ring);
         }
-        __syncwarp();
     }
 }
 
@@ -926,14 +1151,17 @@ __global__ void __launch_bounds__(32 * kIdctWarps, 6) k_idct(DecodeLaunch d) {
         }
         const uint32_t *table = w.weight[list.comp > 0 ? 1 : 0];
         char *blocks = reinterpret_cast<char *>(w.f + list.at * kBlockStride);
-        const auto put = [&](uint32_t x, int32_t v) {
+        const auto put = [&](uint32_t x, float v) {
             const uint32_t pos = x >> 21;
             const uint32_t t = table[pos >> list.shift];
             const float scale = __fmul_rn(__uint_as_float(t & 0xFFFF0000u), list.q8);
             *reinterpret_cast<float *>(blocks + (pos & (list.nb - 1u)) * (4u * kBlockStride) + (t & 0xFFFFu)) =
-                __fmul_rn(__int2float_rn(v), scale);
+                __fmul_rn(v, scale);
         };
-        const auto place = [&](uint32_t x) { put(x, (int32_t)(x << 11) >> 11); };
+        const auto small = [](uint32_t x) {
+            return __uint_as_float(__float_as_uint(__uint2float_rn((x >> 5) & 0xFFFFu)) | (x << 31));
+        };
+        const auto place = [&](uint32_t x) { put(x, small(x)); };
         uint32_t i = 0;
         if (!list.big) {
             for (; i + 128u <= list.n; i += 128u) {
@@ -951,10 +1179,9 @@ __global__ void __launch_bounds__(32 * kIdctWarps, 6) k_idct(DecodeLaunch d) {
             if (i + 3u < list.n) place(e.w);
         } else {
             for (i = lane; i < list.n; i += 32u) {
-                const uint32_t x = __ldg(list.words + i);
-                int32_t v = (int32_t)(x << 11) >> 11;
-                if (v < kListMin) v = (int32_t)__ldg(list.words + 128u * list.nb - 1u - (uint32_t)(v + (1 << 20)));
-                put(x, v);
+                const uint32_t x = __ldg(list.words + i), mag = (x >> 5) & 0xFFFFu;
+                put(x, mag < kListBigMag ? small(x)
+                                         : __int2float_rn((int32_t)__ldg(list.words + 128u * list.nb - 1u - (mag - kListBigMag))));
             }
         }
         list = next;
@@ -1223,7 +1450,7 @@ __global__ void __launch_bounds__(kDecodeThreads) k_decode(DecodeLaunch d) {
                 b.init(d.bits, sd.off + start, len);
                 int err;
                 if (c == 3) {
-                    err = decode_alpha(b, fd, pd, sd, d.alpha);
+                    err = decode_alpha_alone(b, alpha_area(fd, pd, sd, d.alpha));
                 } else {
                     const uint32_t nb = c == 0 ? e.nb_y : e.nb_c;
                     const uint32_t off = c == 0 ? 0u : 64u * (e.nb_y + (c - 1u) * e.nb_c);
@@ -1316,9 +1543,13 @@ cudaError_t launch_locate(const DecodeLaunch &d, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// The prefix tables, and 8 words a lane for the rings: CTAs of 8 warps fill an
+// SM's 228 KB four times over to the byte.
+static size_t entropy_smem_bytes(int warps_per_block) { return 2 * 2 * kBookTableWords + 1024u * warps_per_block; }
+
 cudaError_t launch_entropy(const DecodeLaunch &d, const EntropyShape &shape, cudaStream_t s) {
     if (d.n_slices == 0) return cudaSuccess;
-    k_entropy<<<shape.grid, 32 * shape.warps_per_block, 0, s>>>(d);
+    k_entropy<<<shape.grid, 32 * shape.warps_per_block, entropy_smem_bytes(shape.warps_per_block), s>>>(d);
     return cudaGetLastError();
 }
 
@@ -1373,6 +1604,9 @@ cudaError_t launch_decode(const DecodeLaunch &d, int grid, cudaStream_t s) {
 cudaError_t configure_decode_kernels() {
     cudaError_t e = cudaFuncSetAttribute(k_idct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)idct_smem_bytes());
     if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_entropy, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)entropy_smem_bytes(kEntropyMaxThreads / 32));
+    if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_decode<int16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecodeSmemMax);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_decode<int8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecodeSmemMax);
@@ -1386,7 +1620,8 @@ cudaError_t configure_decode_kernels() {
 int entropy_grid(int device, int warps_per_block, int blocks_per_sm) {
     int sms = 0, fit = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_entropy, 32 * warps_per_block, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_entropy, 32 * warps_per_block,
+                                                  entropy_smem_bytes(warps_per_block));
     if (fit < 1) fit = 1;
     const int per_sm = blocks_per_sm > 0 && blocks_per_sm < fit ? blocks_per_sm : fit;
     return sms * per_sm;

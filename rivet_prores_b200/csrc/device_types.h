@@ -98,8 +98,11 @@ struct DeviceTables {
     float *basis;            // T[x][u] at 8x + u, as the crate computes it
 };
 
+// Zero bytes after the bitstreams of a batch.
+constexpr size_t kBitsPadding = 128;
+
 struct DecodeLaunch {
-    const uint8_t *bits;  // bitstream buffer (64 bytes of zero padding after the end)
+    const uint8_t *bits;  // bitstream buffer (kBitsPadding zero bytes after the end; 64 suffice for the fused decode)
     uint64_t bits_len;
     const FrameDesc *frames;
     const PicDesc *pics;
@@ -108,9 +111,9 @@ struct DecodeLaunch {
     PicStatus *pic_status;
     // 8 bytes per coefficient position of every slice component. The
     // two-kernel decode keeps each component's coefficient list there: 32-bit
-    // entries (scanned position << 21 | 21-bit value; larger values at the
-    // region's back, see CoefList in decode.cu) in position order, with
-    // coef_count[3 s + c] entries. The fused decode keeps only values that do
+    // entries (scanned position << 21 | magnitude << 5 | sign; larger values
+    // at the region's back, see CoefList in decode.cu) in position order, with
+    // coef_count[3 s + c] entries (top bit: there are larger values). The fused decode keeps only values that do
     // not fit 16 bits there, as int32 at their position (see SlotOut).
     uint64_t *coef;
     uint32_t *coef_count;

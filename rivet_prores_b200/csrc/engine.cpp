@@ -548,10 +548,10 @@ Status upload_decode_bits(Workspace &ws, const DecodePlan &plan, const prores_bu
 
 Status upload_decode(Context &ctx, Workspace &ws, const DecodePlan &plan, cudaStream_t s) {
     (void)ctx;
-    // 64 bytes of zero padding after the bitstreams: the readers fetch the
-    // aligned word after the one they are in.
-    PR_CUDA(ws.bits.reserve(plan.bits_total + 64), "cudaMalloc bitstream");
-    PR_CUDA(cudaMemsetAsync(ws.bits.as<uint8_t>() + plan.bits_total, 0, 64, s), "memset");
+    // Zero padding after the bitstreams: the readers fetch up to 16 words
+    // past the position they are at.
+    PR_CUDA(ws.bits.reserve(plan.bits_total + kBitsPadding), "cudaMalloc bitstream");
+    PR_CUDA(cudaMemsetAsync(ws.bits.as<uint8_t>() + plan.bits_total, 0, kBitsPadding, s), "memset");
     PR_CUDA(ws.frames.reserve(sizeof(FrameDesc) * (plan.fdesc.size() + 1)), "cudaMalloc");
     PR_CUDA(ws.pics.reserve(sizeof(PicDesc) * (plan.pdesc.size() + 1)), "cudaMalloc");
     PR_CUDA(ws.slices.reserve(sizeof(SliceDesc) * (plan.n_slices + 1)), "cudaMalloc");
