@@ -22,9 +22,10 @@
 //   k_layout / k_frame
 //                 slice offsets (an exclusive scan per picture), picture and
 //                 frame sizes, the frame and picture headers.
-//   k_pack        one CTA per slice: the slice header, the table entry, and
-//                 each component's codes bit-packed straight into the frame
-//                 (src/encode.rs:413-437, :797-829), plus the alpha codes.
+//   k_pack        one warp per slice component: its codes bit-packed into
+//                 shared memory and from there into the frame
+//                 (src/encode.rs:413-437, :797-829); k_pack_headers the slice
+//                 headers and table entries, k_pack_alpha the alpha codes.
 //
 // Output bits are OR-ed into a zeroed buffer as big-endian 32-bit words, so
 // writers that share a word never need to be ordered.
@@ -308,62 +309,7 @@ __global__ void __launch_bounds__(32 * kAlphaWarps) k_alpha_size(EncodeLaunch e)
     if (lane == 0) e.alpha_bytes[s] = (bits + 7u) / 8u;
 }
 
-__device__ void alpha_write(const EncodeLaunch &e, const EncSliceDesc &sd, const EncPicDesc &pd,
-                            const EncFrameDesc &fd, AlphaScratch &sc, uint64_t bitpos) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t n_runs = alpha_runs(e, sd, pd, fd, sc);
-    const uint32_t bits = fd.alpha_bits;
-    const uint32_t max = bits == 8 ? 8u : 64u;
-    uint64_t carry = 0;
-    for (uint32_t base = 0; base < n_runs; base += 32) {
-        const uint32_t j = base + lane;
-        uint32_t dlen = 0, len = 0;
-        if (j < n_runs) len = alpha_run_bits(sc, j, bits, dlen);
-        uint32_t incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (j < n_runs) {
-            const uint64_t at = bitpos + carry + incl - len;
-            const int32_t prev = j ? (int32_t)sc.value[j - 1] : -1;
-            const int32_t diff = (int32_t)sc.value[j] - prev;
-            const uint32_t a = diff < 0 ? 0u - (uint32_t)diff : (uint32_t)diff;
-            // Tables 13/14: `0`, |d| - 1, sign; or `1` and d mod 2^bits.
-            if (a >= 1u && a <= max)
-                put_field(e.out, at, ((uint64_t)(a - 1u) << 1) | (uint64_t)(diff < 0), dlen);
-            else
-                put_field(e.out, at, (1ull << bits) | ((uint32_t)diff & ((1u << bits) - 1u)), dlen);
-            // Table 12: `1`; `0` and 4 bits of run - 1; or 5 zeros and 11 bits.
-            const uint32_t run = (uint32_t)sc.start[j + 1] - sc.start[j];
-            put_field(e.out, at + dlen, run == 1u ? 1u : run - 1u, len - dlen);
-        }
-        carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-}
-
 // ---------------------------------------------------------------- costing
-
-// Codeword lengths of run and level symbols below 32 by context, kept in
-// shared memory by the kernels that count or write codes.
-struct LenTables {
-    uint8_t run[16][32];
-    uint8_t level[9][32];
-    __device__ void fill() {
-        for (uint32_t i = threadIdx.x; i < 16 * 32; i += blockDim.x) run[i >> 5][i & 31] = (uint8_t)cb_len(run_book(i >> 5), i & 31);
-        for (uint32_t i = threadIdx.x; i < 9 * 32; i += blockDim.x)
-            level[i >> 5][i & 31] = (uint8_t)cb_len(level_book(i >> 5), i & 31);
-    }
-    __device__ __forceinline__ uint32_t run_len(uint32_t ctx, uint32_t r) const {
-        const uint32_t c = ctx < 15u ? ctx : 15u;
-        return r < 32u ? run[c][r] : cb_len(run_book(c), r);
-    }
-    __device__ __forceinline__ uint32_t level_len(uint32_t ctx, uint32_t lvl) const {
-        const uint32_t c = ctx < 8u ? ctx : 8u;
-        return lvl < 32u ? level[c][lvl] : cb_len(level_book(c), lvl);
-    }
-};
 
 // One AC position of a lane's walk: x = F inv, m = floor(|x| + 0.42)
 // (src/dsp/scalar.rs:19-39) as an integer; only a non-zero coefficient is
@@ -505,27 +451,32 @@ __device__ __noinline__ uint32_t long_code_bits(uint32_t e0, uint32_t e1, uint32
     return cb_len32(run_book(prev_run), run) + cb_len32(level_book(e1 & 0xFFFFu), e0 & 0xFFFFu) + 1u;
 }
 
-// Bits of two neighbouring non-zeros, the entries c = (c.x, c.y) after the
-// two before them, b: each one's run by the run before it, its level by the
-// level before it, and a sign. All contexts are in the four entries, so
-// every pair is counted by its own lane. Run and level go through every
-// step as the two halves of a word: an entry less the position before it
-// and 1, clamped to the tables' last columns or to the contexts' last rows,
-// is one instruction.
-__device__ __forceinline__ uint32_t pair_bits(uint2 b, uint2 c, const CountTables &t, bool second) {
-    constexpr uint32_t kLast = ((kRunLens - 1u) << 16) | (kLevelLens - 1u), kRows = (15u << 16) | 8u;
-    const uint32_t nbx = ~b.x & 0xFFFF0000u, nby = ~b.y & 0xFFFF0000u, ncx = ~c.x & 0xFFFF0000u;
-    const uint32_t i0 = __viaddmin_s16x2(b.y, nbx, kRows) * CountTables::kRow + __viaddmin_s16x2(c.x, nby, kLast);
-    const uint32_t i1 = __viaddmin_s16x2(c.x, nby, kRows) * CountTables::kRow + __viaddmin_s16x2(c.y, ncx, kLast);
-    const uint8_t *run = &t.run[0][0], *level = &t.level[0][0];
-    uint32_t l0 = (uint32_t)run[i0 >> 16] + level[i0 & 0xFFFFu];
-    uint32_t l1 = (uint32_t)run[i1 >> 16] + level[i1 & 0xFFFFu];
-    if ((l0 | l1) >= kLongCode) {
-        if (l0 >= kLongCode) l0 = long_code_bits(c.x, b.y, b.x);
-        if (l1 >= kLongCode && second) l1 = long_code_bits(c.y, c.x, b.y);
+// Sums the bits of two neighbouring non-zeros a lane, the entries c = (c.x,
+// c.y) after the two before them, b; `n` of them are there (below 1: none).
+// Each one's run is coded by the run before it, its level by the level before
+// it, with a sign. All contexts are in the four entries. Run and level go
+// through every step as the two halves of a word: an entry less the position
+// before it and 1, clamped to the tables' last columns or to the contexts'
+// last rows, is one instruction.
+constexpr uint32_t kCodeCols = ((kRunLens - 1u) << 16) | (kLevelLens - 1u), kCodeRows = (15u << 16) | 8u;
+struct CountSink {
+    static constexpr bool kSign = false;
+    const CountTables &t;
+    uint32_t bits;
+    __device__ __forceinline__ void pairs(uint2 b, uint2 c, int32_t n) {
+        const uint32_t nbx = ~b.x & 0xFFFF0000u, nby = ~b.y & 0xFFFF0000u, ncx = ~c.x & 0xFFFF0000u;
+        const uint32_t i0 = __viaddmin_s16x2(b.y, nbx, kCodeRows) * CountTables::kRow + __viaddmin_s16x2(c.x, nby, kCodeCols);
+        const uint32_t i1 = __viaddmin_s16x2(c.x, nby, kCodeRows) * CountTables::kRow + __viaddmin_s16x2(c.y, ncx, kCodeCols);
+        const uint8_t *run = &t.run[0][0], *level = &t.level[0][0];
+        uint32_t l0 = (uint32_t)run[i0 >> 16] + level[i0 & 0xFFFFu];
+        uint32_t l1 = (uint32_t)run[i1 >> 16] + level[i1 & 0xFFFFu];
+        if ((l0 | l1) >= kLongCode) {
+            if (l0 >= kLongCode) l0 = long_code_bits(c.x, b.y, b.x);
+            if (l1 >= kLongCode && n > 1) l1 = long_code_bits(c.y, c.x, b.y);
+        }
+        bits += (n > 0 ? l0 : 0u) + (n > 1 ? l1 : 0u);
     }
-    return second ? l0 + l1 : l0;
-}
+};
 
 // kShared: f and cmax point into shared memory (plain loads); else into
 // global memory (read-only loads).
@@ -564,16 +515,19 @@ __device__ __forceinline__ CompHead comp_head(const float *f, const float *cmax,
     return h;
 }
 
-// A warp's list of non-zeros: filled 32 coefficients at a time, counted 64
-// non-zeros at a time.
+// A warp's list of non-zeros: filled 32 or 512 coefficients at a time, handed
+// to `sink` 64 non-zeros at a time, two neighbouring ones a lane (see
+// CountSink and PackSink: both get them with the whole warp together). With
+// kSign an entry's bit 15 is the coefficient's sign.
+template <class Sink>
 struct NonzeroList {
+    static constexpr bool kSign = Sink::kSign;
+    Sink &sink;
     uint32_t *buf;
     uint32_t first, end;  // shared addresses of buf + 2 and past the last entry
-    uint32_t bits;
-    __device__ __forceinline__ void start(uint32_t *b, uint32_t n_blocks) {
+    __device__ __forceinline__ NonzeroList(Sink &s, uint32_t *b, uint32_t n_blocks) : sink(s) {
         buf = b;
         first = end = (uint32_t)__cvta_generic_to_shared(b + 2);
-        bits = 0;
         if ((threadIdx.x & 31u) == 0) {
             b[0] = (n_blocks - 6u) << 16;
             b[1] = ((n_blocks - 1u) << 16) | 1u;
@@ -588,7 +542,8 @@ struct NonzeroList {
         const float y = __fadd_rn(fabsf(__fmul_rn(v, inv)), kAcRounding);
         const uint32_t b = __ballot_sync(0xffffffffu, y >= 1.0f);
         const uint32_t at = end + 4u * __popc(b & below);
-        const uint32_t entry = __float_as_uint(__fadd_rd(y, 8388608.0f)) + tag;
+        uint32_t entry = __float_as_uint(__fadd_rd(y, 8388608.0f)) + tag;
+        if (kSign) entry += (__float_as_uint(v) >> 16) & 0x8000u;
         asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %2, 0f3F800000;\n\t@p st.shared.u32 [%0], %1;\n\t}"
                      :
                      : "r"(at), "r"(entry), "f"(y)
@@ -596,7 +551,7 @@ struct NonzeroList {
         end += 4u * __popc(b);
     }
     // Four coefficients a lane of each of kRuns runs of 128 positions: y the
-    // quantised magnitudes before their floor, `counts` the lane's non-zeros
+    // quantised magnitudes before their floor (with kSign, signed), `counts` the lane's non-zeros
     // by run (a byte each), `tag` of the lane's first position.
     template <uint32_t kRuns>
     __device__ __forceinline__ void add_runs(const float (&y)[4 * kRuns], uint32_t counts, uint32_t tag) {
@@ -616,26 +571,28 @@ struct NonzeroList {
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++) {
                 // Adding 2^23 rounded down leaves floor(y) in the low bits.
-                const uint32_t entry = __float_as_uint(__fadd_rd(y[4 * r + k], 8388608.0f)) + tag + ((128u * r + k) << 16);
+                const float m = fabsf(y[4 * r + k]);
+                uint32_t entry = __float_as_uint(__fadd_rd(m, 8388608.0f)) + tag + ((128u * r + k) << 16);
+                if (kSign) entry += (__float_as_uint(y[4 * r + k]) >> 16) & 0x8000u;
                 asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.f32 p, %2, 0f3F800000;\n\t@p st.shared.u32 [%0], %1;\n\t"
                              "@p add.u32 %0, %0, 4;\n\t}"
                              : "+r"(at)
-                             : "r"(entry), "f"(y[4 * r + k])
+                             : "r"(entry), "f"(m)
                              : "memory");
             }
             end += 4u * ((totals >> (8 * r)) & 255u);
         }
     }
-    // Counts the whole groups of 64; what is left, and the two entries
+    // Hands the whole groups of 64 over; what is left, and the two entries
     // before it, go to the front.
-    __device__ __forceinline__ void count(const CountTables &t) {
+    __device__ __forceinline__ void drain() {
         const uint32_t lane = threadIdx.x & 31u;
         __syncwarp();
         const uint32_t full = ((end - first) >> 2) & ~63u;
         if (full) {
             const uint2 *q = reinterpret_cast<const uint2 *>(buf) + lane;
 #pragma unroll 1
-            for (const uint2 *stop = q + full / 2u; q < stop; q += 32) bits += pair_bits(q[0], q[1], t, true);
+            for (const uint2 *stop = q + full / 2u; q < stop; q += 32) sink.pairs(q[0], q[1], 2);
             const uint2 keep = q[0];
             const uint32_t last = buf[full + 64u];
             __syncwarp();
@@ -645,16 +602,15 @@ struct NonzeroList {
             end -= 4u * full;
         }
     }
-    __device__ __forceinline__ uint32_t finish(const CountTables &t) {
+    __device__ __forceinline__ void finish() {
         const uint32_t lane = threadIdx.x & 31u;
         const uint2 *q = reinterpret_cast<const uint2 *>(buf) + lane;
         const int32_t n = (int32_t)((end - first) >> 2) - (int32_t)(2u * lane);
-        if (n > 0) {
-            uint2 c = q[1];
-            if (n == 1) c.y = c.x + (1u << 16);  // no entry there: any valid one, not counted
-            bits += pair_bits(q[0], c, t, n > 1);
-        }
-        return bits;
+        // Where there is no entry, any valid one, not used.
+        uint2 b = q[0], c = q[1];
+        if (n < 1) b = make_uint2(0u, 5u << 16), c.x = 6u << 16;
+        if (n < 2) c.y = (c.x & 0xFFFF0000u) + (1u << 16);
+        if (end != first) sink.pairs(b, c, n);
     }
 };
 
@@ -666,13 +622,11 @@ __device__ __forceinline__ float4 coef_load4(const float *f) {
         return __ldg(reinterpret_cast<const float4 *>(f));
 }
 
-// The AC part of warp_component_bits for a component of 2^kLog blocks, every
-// coefficient in turn. A lane takes four neighbouring positions of each run
+// The AC non-zeros of a component of 2^kLog blocks, every coefficient in turn. A lane takes four neighbouring positions of each run
 // of 128, four runs at a time; how many non-zeros the lanes below hold in
 // each run comes from one scan of four byte counts.
-template <int kLog, bool kShared>
-__device__ __forceinline__ uint32_t warp_dense_bits(const float *f, const float *inv, const CountTables &t,
-                                                    uint32_t *buf) {
+template <int kLog, bool kShared, class Sink>
+__device__ __forceinline__ void warp_dense(const float *f, const float *inv, Sink &sink, uint32_t *buf) {
     constexpr uint32_t kBlocks = 1u << kLog, kRuns = kBlocks / 2u;
     constexpr uint32_t kGroup = kRuns < kGroupRuns ? kRuns : kGroupRuns;
     constexpr bool kSplit = kBlocks == 2u;  // a lane's four positions are of two scan positions
@@ -685,8 +639,7 @@ __device__ __forceinline__ uint32_t warp_dense_bits(const float *f, const float 
     w[lane + 32u] = __ldg(inv + lane + 32u);
     __syncwarp();
     w += (4u * lane) >> kLog;
-    NonzeroList list;
-    list.start(buf, kBlocks);
+    NonzeroList<Sink> list(sink, buf, kBlocks);
     f += 4u * lane;
 #pragma unroll 1
     for (uint32_t g = 0; g < kRuns; g += kGroup) {
@@ -710,29 +663,28 @@ __device__ __forceinline__ uint32_t warp_dense_bits(const float *f, const float 
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++) {
                 // |F inv| + 0.42 (src/dsp/scalar.rs:19-39), a non-zero from 1 up.
-                y[4 * r + k] = __fadd_rn(fabsf(__fmul_rn(y[4 * r + k], k < 2 ? wa : wb)), kAcRounding);
-                if (y[4 * r + k] >= 1.0f) counts += 1u << (8 * r);
+                const float m = __fadd_rn(fabsf(__fmul_rn(y[4 * r + k], k < 2 ? wa : wb)), kAcRounding);
+                y[4 * r + k] = Sink::kSign ? copysignf(m, y[4 * r + k]) : m;
+                if (m >= 1.0f) counts += 1u << (8 * r);
             }
         }
-        list.add_runs<kGroup>(y, counts, ((128u * g + 4u * lane) << 16) - 0x4B000001u);
-        list.count(t);
+        list.template add_runs<kGroup>(y, counts, ((128u * g + 4u * lane) << 16) - 0x4B000001u);
+        list.drain();
         f += 128u * kGroup;
         w += (128u * kGroup) >> kLog;
     }
-    return list.finish(t);
+    list.finish();
 }
 
 // The same for a component with few chunks that may hold a non-zero, whose
 // numbers are the first `n` bytes of `ids`: 8 of them in flight at a time.
-template <bool kShared>
-__device__ __forceinline__ uint32_t warp_sparse_bits(const float *f, const float *inv, uint32_t n_blocks,
-                                                     const uint2 *ids, uint32_t n, const CountTables &t,
-                                                     uint32_t *buf) {
+template <bool kShared, class Sink>
+__device__ __forceinline__ void warp_sparse(const float *f, const float *inv, uint32_t n_blocks, const uint2 *ids,
+                                            uint32_t n, Sink &sink, uint32_t *buf) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t below = (1u << lane) - 1u;
     const uint32_t shift = 31u - __clz(n_blocks);
-    NonzeroList list;
-    list.start(buf, n_blocks);
+    NonzeroList<Sink> list(sink, buf, n_blocks);
 #pragma unroll 1
     for (uint32_t k = 0; k < n; k += 8) {
         const uint2 id = ids[k >> 3];
@@ -751,9 +703,60 @@ __device__ __forceinline__ uint32_t warp_sparse_bits(const float *f, const float
 #pragma unroll
         for (uint32_t i = 0; i < 8; i++)
             if (k + i < n) list.add(v[i], iv[i], (p[i] << 16) - 0x4B000001u, below);
-        list.count(t);
+        list.drain();
     }
-    return list.finish(t);
+    list.finish();
+}
+
+// Every AC non-zero of a component to `sink`: all chunks in turn, or where
+// few are live (the bits of live_hi:live_lo) those by their list.
+template <bool kShared, class Sink>
+__device__ __forceinline__ void warp_nonzeros(const float *f, const float *inv, uint32_t n_blocks, uint32_t live_lo,
+                                              uint32_t live_hi, Sink &sink, uint32_t *buf) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t below = (1u << lane) - 1u;
+    const uint32_t n_live = __popc(live_lo) + __popc(live_hi);
+    if (kLiveOf8 * 2u * n_blocks < 8u * n_live) {
+        switch (n_blocks) {
+        case 32: warp_dense<5, kShared>(f, inv, sink, buf); break;
+        case 16: warp_dense<4, kShared>(f, inv, sink, buf); break;
+        case 8: warp_dense<3, kShared>(f, inv, sink, buf); break;
+        case 4: warp_dense<2, kShared>(f, inv, sink, buf); break;
+        default: warp_dense<1, kShared>(f, inv, sink, buf); break;
+        }
+    } else if (n_live) {
+        // The live chunks' numbers, in order (at most 24).
+        uint8_t *ids = reinterpret_cast<uint8_t *>(buf + kIdsAt);
+        if ((live_lo >> lane) & 1u) ids[__popc(live_lo & below)] = (uint8_t)lane;
+        if ((live_hi >> lane) & 1u) ids[__popc(live_lo) + __popc(live_hi & below)] = (uint8_t)(lane + 32u);
+        __syncwarp();
+        warp_sparse<kShared>(f, inv, n_blocks, reinterpret_cast<const uint2 *>(ids), n_live, sink, buf);
+    }
+}
+
+// The chunks of a component that may hold a non-zero at `cq`'s quantiser.
+__device__ __forceinline__ void live_chunks(const CompHead &h, uint32_t n_blocks, const CompQuant &cq, uint32_t &lo,
+                                            uint32_t &hi) {
+    const uint32_t lane = threadIdx.x & 31u;
+    lo = __ballot_sync(0xffffffffu, lane < 2u * n_blocks && h.max_lo >= __ldg(cq.chunk + lane));
+    hi = 0;
+    if (n_blocks == 32u) hi = __ballot_sync(0xffffffffu, h.max_hi >= __ldg(cq.chunk + lane + 32u));
+}
+
+// A lane's DC (lanes below n_blocks) as its code's symbol and its codebook by
+// `a` (see dc_len): EG5 of the first, then Table 9 by |previous difference|,
+// the sign flipped after a negative one.
+__device__ __forceinline__ uint32_t dc_symbol(float dc, float inv0, uint32_t &a) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const int32_t q = quantise1(dc, inv0, 0.5f);
+    const int32_t left = __shfl_up_sync(0xffffffffu, q, 1);
+    const int32_t diff = (int32_t)((uint32_t)q - (uint32_t)left);
+    const int32_t before = __shfl_up_sync(0xffffffffu, diff, 1);
+    const int32_t prev_diff = lane == 0 ? 5 : (lane == 1 ? 3 : before);
+    const int32_t value = lane == 0 ? q : (prev_diff < 0 ? -diff : diff);
+    a = min((uint32_t)abs(prev_diff), lane == 0 ? 5u : 3u);
+    // 0, -1, 1, -2, 2, ... -> 0, 1, 2, 3, 4, ...
+    return ((uint32_t)value << 1) ^ (uint32_t)(value >> 31);
 }
 
 // The same for levels of any size, by one lane's walk: only a component whose
@@ -793,46 +796,16 @@ __device__ __noinline__ uint32_t warp_wide_bits(const float *f, const float *inv
 template <bool kShared = false>
 __device__ __forceinline__ uint32_t warp_component_bits(const float *f, const CompHead &h, uint32_t n_blocks, const CompQuant &cq,
                                         const CountTables &t, uint32_t *buf) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t below = (1u << lane) - 1u;
-    const uint32_t chunks = 2u * n_blocks;
-    // The chunks that hold a candidate.
-    const uint32_t live_lo = __ballot_sync(0xffffffffu, lane < chunks && h.max_lo >= __ldg(cq.chunk + lane));
-    uint32_t live_hi = 0;
-    if (n_blocks == 32u) live_hi = __ballot_sync(0xffffffffu, h.max_hi >= __ldg(cq.chunk + lane + 32u));
-    // The DCs (n_blocks <= 32), a lane each: EG5 of the first, then Table 9
-    // by |previous difference|, the sign flipped after a negative one.
-    const int32_t q = quantise1(h.dc, __ldg(cq.inv), 0.5f);
-    const int32_t left = __shfl_up_sync(0xffffffffu, q, 1);
-    const int32_t diff = (int32_t)((uint32_t)q - (uint32_t)left);
-    const int32_t before = __shfl_up_sync(0xffffffffu, diff, 1);
-    const int32_t prev_diff = lane == 0 ? 5 : (lane == 1 ? 3 : before);
-    const int32_t value = lane == 0 ? q : (prev_diff < 0 ? -diff : diff);
-    // 0, -1, 1, -2, 2, ... -> 0, 1, 2, 3, 4, ...
-    const uint32_t symbol = ((uint32_t)value << 1) ^ (uint32_t)(value >> 31);
-    const uint32_t len = dc_len(min((uint32_t)abs(prev_diff), lane == 0 ? 5u : 3u), symbol);
-    uint32_t bits = lane < n_blocks ? len : 0u;
-    const uint32_t n_live = __popc(live_lo) + __popc(live_hi);
+    uint32_t live_lo, live_hi, a;
+    live_chunks(h, n_blocks, cq, live_lo, live_hi);
+    const uint32_t symbol = dc_symbol(h.dc, __ldg(cq.inv), a), len = dc_len(a, symbol);
+    CountSink sink{t, (threadIdx.x & 31u) < n_blocks ? len : 0u};
     __syncwarp();  // the last component's entries are read
-    if (__any_sync(0xffffffffu, fmaxf(h.max_lo, h.max_hi) >= kWideCoef)) {
-        bits += warp_wide_bits<kShared>(f, cq.inv, n_blocks);
-    } else if (kLiveOf8 * chunks < 8u * n_live) {
-        switch (n_blocks) {
-        case 32: bits += warp_dense_bits<5, kShared>(f, cq.inv, t, buf); break;
-        case 16: bits += warp_dense_bits<4, kShared>(f, cq.inv, t, buf); break;
-        case 8: bits += warp_dense_bits<3, kShared>(f, cq.inv, t, buf); break;
-        case 4: bits += warp_dense_bits<2, kShared>(f, cq.inv, t, buf); break;
-        default: bits += warp_dense_bits<1, kShared>(f, cq.inv, t, buf); break;
-        }
-    } else if (n_live) {
-        // The live chunks' numbers, in order (at most 24).
-        uint8_t *ids = reinterpret_cast<uint8_t *>(buf + kIdsAt);
-        if ((live_lo >> lane) & 1u) ids[__popc(live_lo & below)] = (uint8_t)lane;
-        if ((live_hi >> lane) & 1u) ids[__popc(live_lo) + __popc(live_hi & below)] = (uint8_t)(lane + 32u);
-        __syncwarp();
-        bits += warp_sparse_bits<kShared>(f, cq.inv, n_blocks, reinterpret_cast<const uint2 *>(ids), n_live, t, buf);
-    }
-    return __reduce_add_sync(0xffffffffu, bits);
+    if (__any_sync(0xffffffffu, fmaxf(h.max_lo, h.max_hi) >= kWideCoef))
+        sink.bits += warp_wide_bits<kShared>(f, cq.inv, n_blocks);
+    else
+        warp_nonzeros<kShared>(f, cq.inv, n_blocks, live_lo, live_hi, sink, buf);
+    return __reduce_add_sync(0xffffffffu, sink.bits);
 }
 
 // The quantiser table of quantization_index qi (layout beside kQuantStride).
@@ -1680,23 +1653,182 @@ struct BitOut {
     }
 };
 
-// The writer's tables: beside the code lengths, the codewords (their
-// significant bits) of run and level symbols below 32 by context.
-struct CodeTables : LenTables {
-    uint32_t run_code[16][32];
-    uint32_t level_code[9][32];
-    __device__ void fill_all() {
-        fill();
-        for (uint32_t i = threadIdx.x; i < 16 * 32; i += blockDim.x)
-            run_code[i >> 5][i & 31] = (uint32_t)cb_bits(run_book(i >> 5), i & 31);
-        for (uint32_t i = threadIdx.x; i < 9 * 32; i += blockDim.x)
-            level_code[i >> 5][i & 31] = (uint32_t)cb_bits(level_book(i >> 5), i & 31);
+// The writer's tables by context: a code's length << 24 | its significant
+// bits, of run symbols below 63 and of level symbols below 127 with room for
+// the sign bit; 0 in the last column, for every symbol past those. Both are
+// indexed by context x kRow + symbol; neighbouring contexts start in
+// different banks.
+struct PackTables {
+    static constexpr uint32_t kRow = kLevelLens + 1;
+    uint32_t run[16][kRow];  // kRunLens used
+    uint32_t level[9][kRow];
+    uint32_t pad[3];  // a whole number of 16-byte words
+    __device__ __forceinline__ void fill();
+};
+__device__ uint4 d_pack_tables[sizeof(PackTables) / sizeof(uint4)];
+
+__device__ __forceinline__ void PackTables::fill() {
+    for (uint32_t i = threadIdx.x; i < sizeof(PackTables) / sizeof(uint4); i += blockDim.x)
+        reinterpret_cast<uint4 *>(this)[i] = d_pack_tables[i];
+}
+
+void build_pack_tables(PackTables &t) {
+    t = PackTables{};
+    for (uint32_t c = 0; c < 16; c++)
+        for (uint32_t n = 0; n + 1 < kRunLens; n++)
+            t.run[c][n] = (cb_len32(run_book(c), n) << 24) | (uint32_t)cb_bits(run_book(c), n);
+    for (uint32_t c = 0; c < 9; c++)
+        for (uint32_t n = 0; n + 1 < kLevelLens; n++)
+            t.level[c][n] = ((cb_len32(level_book(c), n) + 1u) << 24) | ((uint32_t)cb_bits(level_book(c), n) << 1);
+}
+
+// A warp's output bits: fields, a lane each, are placed by a scan of their
+// lengths and OR-ed into words in shared memory, which go out 32 at a time,
+// the first and the last (which neighbours share) by an atomic OR. A batch of
+// fields is at most kBatchBits bits.
+constexpr uint32_t kBatchBits = 64 * 56;
+constexpr uint32_t kPackWords = 32 + kBatchBits / 32 + 4;
+struct WarpBits {
+    uint32_t *buf;    // kPackWords words, zero past `bits`
+    uint32_t base;    // its shared address
+    uint32_t *out;    // where word 0 goes
+    uint32_t bits;    // held, from bit 0 of word 0 on
+    bool shared;      // word 0 is shared with what comes before
+    // Once a warp; finish() leaves the buffer zero again.
+    __device__ __forceinline__ void clear(uint32_t *b) {
+        buf = b;
+        base = (uint32_t)__cvta_generic_to_shared(b);
+        for (uint32_t i = threadIdx.x & 31u; i < kPackWords; i += 32u) buf[i] = 0;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void start(uint32_t *o, uint64_t bitpos) {
+        out = o + (bitpos >> 5);
+        bits = (uint32_t)bitpos & 31u;
+        shared = true;
+    }
+    // Room for the lane's `len` bits, in lane order; returns its place.
+    __device__ __forceinline__ uint32_t place(uint32_t len) {
+        uint32_t sum = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+            asm volatile("{\n\t.reg .pred p;\n\t.reg .u32 t;\n\tshfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n\t"
+                         "@p add.u32 %0, %0, t;\n\t}"
+                         : "+r"(sum)
+                         : "r"(o));
+        const uint32_t at = bits + sum - len;
+        bits += __shfl_sync(0xffffffffu, sum, 31);
+        return at;
+    }
+    // If `n` > 0, ORs `v` into word `w` of the buffer.
+    __device__ __forceinline__ void or_word(uint32_t w, uint32_t v, int32_t n) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %2, 0;\n\t@p red.shared.or.b32 [%0], %1;\n\t}"
+                     :
+                     : "r"(base + 4u * w), "r"(v), "r"(n)
+                     : "memory");
+    }
+    // ORs a field of `len` bits (at most 32; 0: none) in at bit `at`.
+    __device__ __forceinline__ void put32(uint32_t at, uint32_t value, uint32_t len) {
+        const uint32_t v = __funnelshift_lc(0u, value, 32u - len), o = at & 31u, w = at >> 5;
+        or_word(w, v >> o, (int32_t)len);
+        or_word(w + 1u, __funnelshift_r(0u, v, o), (int32_t)(o + len) - 32);
+    }
+    // The same of up to 64 bits.
+    __device__ __forceinline__ void put(uint32_t at, uint64_t value, uint32_t len) {
+        const uint64_t v = len ? value << (64u - len) : 0ull;
+        const uint32_t hi = (uint32_t)(v >> 32), lo = (uint32_t)v, o = at & 31u, w = at >> 5;
+        or_word(w, hi >> o, (int32_t)len);
+        or_word(w + 1u, __funnelshift_r(lo, hi, o), (int32_t)(o + len) - 32);
+        or_word(w + 2u, __funnelshift_r(0u, lo, o), (int32_t)(o + len) - 64);
+    }
+    // The whole words out, once there are 32.
+    __device__ __forceinline__ void drain() {
+        __syncwarp();
+        if (bits >= 32u * 32u) flush(bits >> 5);
+    }
+    __device__ __forceinline__ void flush(uint32_t words) {
+        const uint32_t lane = threadIdx.x & 31u;
+        const uint32_t part = buf[words];
+        __syncwarp();
+        for (uint32_t i = lane; i < words; i += 32u) {
+            const uint32_t v = bswap32(buf[i]);
+            buf[i] = 0;
+            if (i == 0 && shared)
+                atomicOr(out, v);
+            else
+                out[i] = v;
+        }
+        __syncwarp();
+        if (lane == 0) {
+            buf[words] = 0;
+            buf[0] = part;
+        }
+        __syncwarp();
+        out += words;
+        bits &= 31u;
+        shared = shared && words == 0;
+    }
+    // Zero bits to the next byte boundary, then everything out.
+    __device__ __forceinline__ void finish() {
+        __syncwarp();
+        if (bits >= 32u) flush(bits >> 5);
+        if ((threadIdx.x & 31u) == 0 && bits) {
+            atomicOr(out, bswap32(buf[0]));
+            buf[0] = 0;
+        }
+        __syncwarp();
+    }
+};
+
+// Writes the codes of two neighbouring non-zeros a lane (see CountSink).
+struct PackSink {
+    static constexpr bool kSign = true;
+    const PackTables &t;
+    WarpBits &w;
+    // The code of entry e after the entries p and pp, at any length.
+    __device__ __noinline__ static uint64_t long_code(uint32_t e, uint32_t p, uint32_t pp, uint32_t &len) {
+        const uint32_t run = (e >> 16) - (p >> 16) - 1u, prev_run = ((p >> 16) - (pp >> 16) - 1u) & 0xFFFFu;
+        const uint32_t level = e & 0x7FFFu, sign = (e >> 15) & 1u;
+        const Codebook rb = run_book(prev_run), lb = level_book(p & 0x7FFFu);
+        const uint32_t ll = cb_len32(lb, level);
+        len = cb_len32(rb, run) + ll + 1u;
+        return (((cb_bits(rb, run) << ll) | cb_bits(lb, level)) << 1) | sign;
+    }
+    __device__ __forceinline__ void pairs(uint2 b, uint2 c, int32_t n) {
+        constexpr uint32_t kNoSign = 0xFFFF7FFFu;
+        const uint32_t sign0 = (c.x >> 15) & 1u, sign1 = (c.y >> 15) & 1u;
+        const uint32_t nbx = ~b.x & 0xFFFF0000u, nby = ~b.y & 0xFFFF0000u, ncx = ~c.x & 0xFFFF0000u;
+        const uint32_t by = b.y & kNoSign, cx = c.x & kNoSign, cy = c.y & kNoSign;
+        const uint32_t i0 = __viaddmin_s16x2(by, nbx, kCodeRows) * PackTables::kRow + __viaddmin_s16x2(cx, nby, kCodeCols);
+        const uint32_t i1 = __viaddmin_s16x2(cx, nby, kCodeRows) * PackTables::kRow + __viaddmin_s16x2(cy, ncx, kCodeCols);
+        const uint32_t *run = &t.run[0][0], *level = &t.level[0][0];
+        const uint32_t r0 = run[i0 >> 16], l0 = level[i0 & 0xFFFFu];
+        const uint32_t r1 = run[i1 >> 16], l1 = level[i1 & 0xFFFFu];
+        uint32_t len0 = (r0 >> 24) + (l0 >> 24), len1 = (r1 >> 24) + (l1 >> 24);
+        const bool long0 = n > 0 && (r0 == 0 || l0 == 0), long1 = n > 1 && (r1 == 0 || l1 == 0);
+        len0 = n > 0 ? len0 : 0u;
+        len1 = n > 1 ? len1 : 0u;
+        // Codes of the tables: at most 28 bits, and mostly two in 32.
+        const uint32_t v0 = (((r0 & 0xFFFFFFu) << (l0 >> 24)) | (l0 & 0xFFFFFFu)) + sign0;
+        const uint32_t v1 = n > 1 ? (((r1 & 0xFFFFFFu) << (l1 >> 24)) | (l1 & 0xFFFFFFu)) + sign1 : 0u;
+        if (!__any_sync(0xffffffffu, len0 + len1 > 32u || long0 || long1)) {
+            w.put32(w.place(len0 + len1), (v0 << len1) | v1, len0 + len1);
+        } else {
+            uint64_t w0 = v0, w1 = v1;
+            if (long0) w0 = long_code(c.x, b.y, b.x, len0);
+            if (long1) w1 = long_code(c.y, c.x, b.y, len1);
+            const uint32_t at = w.place(len0 + len1);
+            w.put(at, w0, len0);
+            w.put(at + len0, w1, len1);
+        }
+        w.drain();
     }
 };
 
 // One quantised component's codes (src/encode.rs:413-437), one lane.
-__device__ void lane_component_write(BitOut &w, const float *f, const float *cmax, uint32_t n_blocks,
-                                     const CompQuant &q, const CodeTables &t) {
+__device__ __noinline__ void lane_component_write(uint32_t *out, uint64_t at, const float *f, const float *cmax,
+                                                  uint32_t n_blocks, const CompQuant &q) {
+    BitOut w;
+    w.init(out, at);
     const float inv0 = __ldg(q.inv);
     int32_t prev_dc = 0, prev_diff = 3;
     for (uint32_t i = 0; i < n_blocks; i++) {
@@ -1716,51 +1848,129 @@ __device__ void lane_component_write(BitOut &w, const float *f, const float *cma
         prev_dc = q;
     }
     ac_walk_sparse(f, cmax, n_blocks, q, [&](const AcWalk &a, uint32_t run, uint32_t level, bool neg) {
-        // Run, level and sign in one field, from the tables, when they can.
-        if (run < 32u && level < 32u) {
-            const uint32_t rc = min(a.prev_run, 15u), lc = min(a.prev_level, 8u);
-            const uint32_t rl = t.run[rc][run], ll = t.level[lc][level];
-            if (rl + ll + 1u <= 32u) {
-                w.put((((uint64_t)t.run_code[rc][run] << ll | t.level_code[lc][level]) << 1) | (uint64_t)neg,
-                      rl + ll + 1u);
-                return;
-            }
-        }
         const Codebook rb = run_book(a.prev_run), lb = level_book(a.prev_level);
-        const uint32_t rl = t.run_len(a.prev_run, run), ll = t.level_len(a.prev_level, level);
-        // Run, level and sign in one field when they fit.
-        if (rl + ll + 1u <= 32u) {
-            w.put((((cb_bits(rb, run) << ll) | cb_bits(lb, level)) << 1) | (uint64_t)neg, rl + ll + 1u);
-        } else {
-            w.put_long(cb_bits(rb, run), rl);
-            w.put_long(cb_bits(lb, level), ll);
-            w.put((uint64_t)neg, 1);
-        }
+        w.put_long(cb_bits(rb, run), cb_len(rb, run));
+        w.put_long(cb_bits(lb, level), cb_len(lb, level));
+        w.put((uint64_t)neg, 1);
     });
     w.finish();
 }
 
-// Each slice component's codes, one lane per (component, slice).
-__global__ void __launch_bounds__(kCostThreads) k_pack(EncodeLaunch e) {
-    __shared__ CodeTables t;
-    t.fill_all();
+// Each slice component's codes (src/encode.rs:413-437), a warp each, the list
+// walked at the resident grid's stride: the non-zeros are gathered as for
+// counting, and their codes placed 64 at a time. A component with levels too
+// large for the list is written by one lane.
+//
+// Bound by issue (72 % of the slots, 51 warp instructions for 32 coefficients
+// at 36 % non-zeros). A lane per component, writing bit by bit into words it
+// OR-ed to memory, took 1390 us for 30 UHD frames, 636 for 30 1080p and 474
+// for one UHD frame (a lane's walk from end to end): 968, 265 and 50 now. Alpha,
+// whose codes were OR-ed into memory one by one, goes through the same words:
+// 8 UHD 4:4:4 frames with it 1595 -> 814.
+__global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_pack(EncodeLaunch e, uint32_t take) {
+    __shared__ __align__(16) PackTables t;
+    __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
+    __shared__ uint32_t words[kCostThreads / 32][kPackWords];
+    t.fill();
     __syncthreads();
-    const uint32_t item = blockIdx.x * kCostThreads + threadIdx.x;
-    if (item >= 3u * e.n_slices) return;
-    const uint32_t comp = item / e.n_slices, s = item - comp * e.n_slices;
-    const EncSliceDesc sd = e.slices[s];
-    const EncPicDesc &pd = e.pics[sd.pic];
-    if (e.frame_status[pd.frame]) return;
-    const EncFrameDesc &fd = e.frames[pd.frame];
-    const EncPicState &st = e.state[sd.pic];
-    uint64_t at = 8ull * (fd.out_base + st.pic_off + e.slice_off[s] + pd.header_bytes);
-    for (uint32_t c = 0; c < comp; c++) at += 8ull * e.final_comp[3ull * s + c];
-    uint32_t nb, off;
-    comp_layout(fd, sd.mbs, comp, nb, off);
-    BitOut w;
-    w.init(e.out, at);
-    lane_component_write(w, e.coef + sd.coef + off, e.coef_max + ((sd.coef + off) >> 5), nb,
-                         comp_quant(quant_base(e, pd, e.final_qi[s]), comp, nb), t);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t items = 3u * e.n_slices, stride = gridDim.x * (kCostThreads / 32) * take;
+    WarpBits w;
+    w.clear(words[warp]);
+    for (uint32_t base = (blockIdx.x * (kCostThreads / 32) + warp) * take; base < items; base += stride) {
+        // This lane's item, as in k_cost, and the bit its codes start at.
+        const uint32_t item = base + lane;
+        uint32_t my_coef = 0, my_quant = 0, my_blocks = 0;
+        uint64_t my_at = 0;
+        if (lane < take && item < items) {
+            const uint32_t comp = item < e.n_slices ? 0u : (item < 2u * e.n_slices ? 1u : 2u);
+            const uint32_t s = item - comp * e.n_slices;
+            const EncSliceDesc sd = e.slices[s];
+            uint64_t at = e.slice_off[s];
+            for (uint32_t c = 0; c < comp; c++) at += e.final_comp[3ull * s + c];
+            const EncPicDesc &pd = e.pics[sd.pic];
+            at += e.state[sd.pic].pic_off + pd.header_bytes + e.frames[pd.frame].out_base;
+            const uint32_t off = comp == 0 ? 0u : 64u * sd.mbs * (4u + (comp - 1u) * sd.cpm);
+            my_coef = (uint32_t)((sd.coef + off) >> 6);
+            my_quant = ((pd.quant * 225u + e.final_qi[s]) << 1) | (comp > 0 ? 1u : 0u);
+            if (e.frame_status[pd.frame] == 0) my_blocks = (comp == 0 ? 4u : sd.cpm) * sd.mbs;
+            my_at = 8ull * at;
+        }
+        CompHead next_head{};
+        uint32_t next_blocks = 0;
+        uint64_t next_coef = 0;
+        const auto look = [&](uint32_t j) {
+            next_coef = (uint64_t)__shfl_sync(0xffffffffu, my_coef, j) << 6;
+            next_blocks = __shfl_sync(0xffffffffu, my_blocks, j);
+            next_head = comp_head<false>(e.coef + next_coef, e.coef_max + (next_coef >> 5), next_blocks);
+        };
+        uint32_t left = __ballot_sync(0xffffffffu, my_blocks != 0);
+        if (left) look((uint32_t)__ffs(left) - 1u);
+        while (left) {
+            const uint32_t j = (uint32_t)__ffs(left) - 1u;
+            left &= left - 1u;
+            const CompHead h = next_head;
+            const uint32_t nb = next_blocks;
+            const uint64_t coef = next_coef;
+            if (left) look((uint32_t)__ffs(left) - 1u);
+            const uint32_t quant = __shfl_sync(0xffffffffu, my_quant, j);
+            const uint64_t at = __shfl_sync(0xffffffffu, my_at, j);
+            const CompQuant cq = comp_quant(e.quant + (uint64_t)(quant >> 1) * kQuantStride, quant & 1u, nb);
+            const float *f = e.coef + coef;
+            if (__any_sync(0xffffffffu, fmaxf(h.max_lo, h.max_hi) >= kWideCoef)) {
+                if (lane == 0) lane_component_write(e.out, at, f, e.coef_max + (coef >> 5), nb, cq);
+                __syncwarp();
+                continue;
+            }
+            w.start(e.out, at);
+            uint32_t live_lo, live_hi, a;
+            live_chunks(h, nb, cq, live_lo, live_hi);
+            const uint32_t symbol = dc_symbol(h.dc, __ldg(cq.inv), a);
+            const uint32_t len = lane < nb ? dc_len(a, symbol) : 0u;
+            // The code's significant bits: n + 2^k of EGk; the codebook for a
+            // difference of 2 has (n & 3) + 4 below 8, from there on n itself.
+            const uint32_t code = a == 2u ? (symbol < 8u ? (symbol & 3u) + 4u : symbol) : symbol + (1u << a);
+            w.put(w.place(len), code, len);
+            w.drain();
+            PackSink sink{t, w};
+            warp_nonzeros<false>(f, cq.inv, nb, live_lo, live_hi, sink, buf[warp]);
+            w.finish();
+        }
+    }
+}
+
+// A slice's alpha codes, the whole warp, a run and its difference a lane.
+__device__ void alpha_write(const EncodeLaunch &e, const EncSliceDesc &sd, const EncPicDesc &pd,
+                            const EncFrameDesc &fd, AlphaScratch &sc, uint32_t *words, uint64_t bitpos) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t n_runs = alpha_runs(e, sd, pd, fd, sc);
+    const uint32_t bits = fd.alpha_bits;
+    const uint32_t max = bits == 8 ? 8u : 64u;
+    WarpBits w;
+    w.clear(words);
+    w.start(e.out, bitpos);
+    for (uint32_t base = 0; base < n_runs; base += 32) {
+        const uint32_t j = base + lane;
+        uint32_t dlen = 0, len = 0;
+        if (j < n_runs) len = alpha_run_bits(sc, j, bits, dlen);
+        uint64_t field = 0;
+        if (j < n_runs) {
+            const int32_t prev = j ? (int32_t)sc.value[j - 1] : -1;
+            const int32_t diff = (int32_t)sc.value[j] - prev;
+            const uint32_t a = diff < 0 ? 0u - (uint32_t)diff : (uint32_t)diff;
+            // Tables 13/14: `0`, |d| - 1, sign; or `1` and d mod 2^bits.
+            if (a >= 1u && a <= max)
+                field = ((a - 1u) << 1) | (uint32_t)(diff < 0);
+            else
+                field = (1u << bits) | ((uint32_t)diff & ((1u << bits) - 1u));
+            // Table 12: `1`; `0` and 4 bits of run - 1; or 5 zeros and 11 bits.
+            const uint32_t run = (uint32_t)sc.start[j + 1] - sc.start[j];
+            field = (field << (len - dlen)) | (run == 1u ? 1u : run - 1u);
+        }
+        w.put(w.place(len), field, len);
+        w.drain();
+    }
+    w.finish();
 }
 
 // Slice headers and table entries, one thread per slice; alpha codes, one
@@ -1791,6 +2001,7 @@ __global__ void k_pack_headers(EncodeLaunch e) {
 
 __global__ void __launch_bounds__(32 * kAlphaWarps) k_pack_alpha(EncodeLaunch e) {
     __shared__ AlphaScratch scratch[kAlphaWarps];
+    __shared__ uint32_t words[kAlphaWarps][kPackWords];
     const uint32_t s = blockIdx.x * kAlphaWarps + (threadIdx.x >> 5);
     if (s >= e.n_slices) return;
     const EncSliceDesc sd = e.slices[s];
@@ -1800,7 +2011,7 @@ __global__ void __launch_bounds__(32 * kAlphaWarps) k_pack_alpha(EncodeLaunch e)
     const EncPicState &st = e.state[sd.pic];
     const uint32_t *c = e.final_comp + 3ull * s;
     const uint64_t at = 8ull * (fd.out_base + st.pic_off + e.slice_off[s] + pd.header_bytes + c[0] + c[1] + c[2]);
-    alpha_write(e, sd, pd, fd, scratch[threadIdx.x >> 5], at);
+    alpha_write(e, sd, pd, fd, scratch[threadIdx.x >> 5], words[threadIdx.x >> 5], at);
 }
 
 }  // namespace
@@ -1831,14 +2042,18 @@ static uint32_t cost_grid(const EncodeLaunch &e, uint32_t items) {
     return std::min<uint32_t>((items + kCostThreads / 32 - 1) / (kCostThreads / 32), (uint32_t)(kCostBlocks * e.sm_count));
 }
 
+// Items a warp takes at once: enough to share the look-ups, few enough that
+// the last ones do not hold the launch up (a component takes a warp about 6 us
+// when all warps are busy).
+static uint32_t cost_take(const EncodeLaunch &e, uint32_t items) {
+    const uint32_t warps = (uint32_t)(kCostBlocks * e.sm_count) * (kCostThreads / 32);
+    return std::max(1u, std::min(kCostTake, items / (8u * warps)));
+}
+
 cudaError_t launch_cost(const EncodeLaunch &e, int step, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
-    // Items a warp takes at once: enough to share the look-ups, few enough
-    // that the last ones do not hold the launch up (a component takes a warp
-    // about 6 us when all warps are busy).
-    const uint32_t items = 3u * e.n_slices, warps = (uint32_t)(kCostBlocks * e.sm_count) * (kCostThreads / 32);
-    const uint32_t take = std::max(1u, std::min(kCostTake, items / (8u * warps)));
-    k_cost<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, step, take);
+    const uint32_t items = 3u * e.n_slices;
+    k_cost<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, step, cost_take(e, items));
     return cudaGetLastError();
 }
 
@@ -1887,7 +2102,7 @@ cudaError_t launch_layout(const EncodeLaunch &e, cudaStream_t s) {
 cudaError_t launch_pack(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
     const uint32_t items = 3u * e.n_slices;
-    k_pack<<<(items + kCostThreads - 1) / kCostThreads, kCostThreads, 0, s>>>(e);
+    k_pack<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, cost_take(e, items));
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     k_pack_headers<<<(e.n_slices + 255) / 256, 256, 0, s>>>(e);
@@ -1903,6 +2118,9 @@ cudaError_t configure_encode_kernels() {
     CountTables tables;
     build_count_tables(tables);
     if ((err0 = cudaMemcpyToSymbol(d_count_tables, &tables, sizeof tables)) != cudaSuccess) return err0;
+    PackTables codes;
+    build_pack_tables(codes);
+    if ((err0 = cudaMemcpyToSymbol(d_pack_tables, &codes, sizeof codes)) != cudaSuccess) return err0;
     float basis[64];
     dct_basis(basis);
     cudaError_t err = cudaMemcpyToSymbol(c_fdct_basis, basis, sizeof basis);
