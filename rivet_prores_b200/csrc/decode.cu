@@ -1070,8 +1070,8 @@ __global__ void __launch_bounds__(32 * kIdctWarps, 6) k_idct(DecodeLaunch d) {
     const uint32_t cpm = fd.chroma == 2 ? 2u : 4u;
     const IdctShape shape = idct_shape(fd.chroma, pd.log2_slice_mbs);
     // The components [c0, c1) of the item's slices.
-    const uint32_t c0 = part == 0 ? 0u : (shape.parts == 3u ? part : (cpm == 2u ? 1u : 2u));
-    const uint32_t c1 = part + 1u == shape.parts ? 3u : c0 + (shape.parts == 3u || cpm == 2u ? 1u : 2u);
+    uint32_t c0, c1;
+    idct_components(shape, cpm, part, c0, c1);
     const uint32_t n_lists = n_slices * (c1 - c0);
 
     // Lane l < n_lists looks after list l: slice l / (c1 - c0)'s component.

@@ -44,8 +44,8 @@ struct PicDesc {
     uint32_t idct_base;  // the picture's first item in DecodeLaunch::idct_items
 };
 
-// How k_idct, which takes up to 32 blocks a warp, splits the slices of a
-// picture by their nominal macroblocks: `parts` items a slice (whole
+// How k_idct and k_fdct, which take up to 32 blocks a warp, split the slices
+// of a picture by their nominal macroblocks: `parts` items a slice (whole
 // components), or one item for `slices` neighbouring slices, the blocks of
 // each at a distance of `blocks` lanes. Row-end slices, which are narrower,
 // leave lanes idle.
@@ -56,6 +56,19 @@ __host__ __device__ inline IdctShape idct_shape(uint32_t chroma, uint32_t log2_s
     const uint32_t blocks = (chroma == 2 ? 8u : 12u) << log2_slice_mbs;
     if (blocks >= 32u) return IdctShape{(blocks + 31u) / 32u, 1u, blocks};
     return IdctShape{1u, 32u / blocks, blocks};
+}
+
+// The components [c0, c1) of part `part` of a slice with `cpm` blocks of each
+// chroma component a macroblock.
+__host__ __device__ inline void idct_components(const IdctShape &shape, uint32_t cpm, uint32_t part, uint32_t &c0,
+                                                uint32_t &c1) {
+    c0 = part == 0 ? 0u : (shape.parts == 3u ? part : (cpm == 2u ? 1u : 2u));
+    c1 = part + 1u == shape.parts ? 3u : c0 + (shape.parts == 3u || cpm == 2u ? 1u : 2u);
+}
+
+// The items of a picture of `n_slices` slices.
+__host__ __device__ inline uint32_t idct_items(const IdctShape &shape, uint32_t n_slices) {
+    return shape.slices > 1u ? (n_slices + shape.slices - 1u) / shape.slices : n_slices * shape.parts;
 }
 
 // One slice, located (filled on the device from the slice table).

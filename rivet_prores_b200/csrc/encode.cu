@@ -1,9 +1,10 @@
 // encode.cu -- the encoder (the crate's src/encode.rs) as sm_100a kernels.
 //
-//   k_fdct        one CTA per slice: edge-replicated 8x8 gathers, p = s 512/2^b
-//                 - 256 and the FDCT in the crate's exact single-precision
-//                 order (src/encode.rs:488-555, src/dct.rs:70-93), written in
-//                 the slice's scanned order once per frame.
+//   k_fdct        one warp per 32 blocks: edge-replicated 8x8 gathers, p = s
+//                 512/2^b - 256 and the FDCT in the crate's exact
+//                 single-precision order (src/encode.rs:488-555,
+//                 src/dct.rs:70-93), written in the slice's scanned order once
+//                 per frame.
 //   k_alpha_size  one warp per slice: the lossless alpha codes' size
 //                 (src/encode.rs:838-868, :457-470); it does not depend on
 //                 the quantiser.
@@ -85,7 +86,7 @@ __device__ __forceinline__ int32_t quantise1(float f, float inv, float r) {
 
 // ---------------------------------------------------------------- fdct
 
-constexpr int kFdctThreads = 128;
+constexpr int kFdctWarps = 4;
 constexpr int kMaxSliceCoefs = 64 * 12 * 8;
 
 __device__ __forceinline__ void block_xy(uint32_t comp, uint32_t chroma, uint32_t mb_x, uint32_t mb_y, uint32_t m,
@@ -103,116 +104,168 @@ __device__ __forceinline__ void block_xy(uint32_t comp, uint32_t chroma, uint32_
     }
 }
 
-// One warp per slice component, one lane per 8x8 block (a component has
-// at most 32 blocks; lanes past the component's count idle). A lane loads
-// its block's 8 rows, transforms them (rows, then columns, in the crate's
-// order; the row results wait in shared memory, lane-minor, so no bank
-// conflicts) and stores each coefficient at its scanned place
-// n * scan[k] + blk: the lanes of a component store consecutive floats.
-// The basis comes from constant memory, read by every lane at the same
-// address. A chunk of 32 scanned coefficients is one scanned position of a
-// 32-block component, or several positions of a smaller one; its largest
-// |F| is reduced over the lanes as each position is stored and kept in
-// shared memory until the component is done. (Cb and Cr of a 4:2:2 slice
-// in one warp measured slower: fewer warps to hide the loads.)
-__global__ void __launch_bounds__(kFdctThreads) k_fdct(EncodeLaunch e) {
-    __shared__ uint32_t cmax_sh[kFdctThreads / 32][64];
-    __shared__ float tmp_sh[kFdctThreads / 32][64][32];  // the row pass, [y * 8 + u][lane]
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t item = blockIdx.x * (kFdctThreads / 32) + warp;
-    if (item >= 3u * e.n_slices) return;  // the whole warp
-    const uint32_t s = item / 3u, c = item - 3u * s;
-    const EncSliceDesc sd = e.slices[s];
-    const EncPicDesc &pd = e.pics[sd.pic];
+// An 8-point forward transform: o[j] is outputs 2 j and 2 j + 1, each the sum
+// of in[x] T[x][u] with x in order, summed as a pair; the products stay
+// scalar (see pair_math.h), and the first is not added to 0 (which changes
+// only the sign of a zero, and no quantised value).
+__device__ __forceinline__ void fdct8(const float (&in)[8], uint64_t (&o)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+#pragma unroll
+        for (int x = 0; x < 8; x++) {
+            const uint64_t term =
+                pair_of(__fmul_rn(in[x], c_fdct_basis[8 * x + 2 * j]), __fmul_rn(in[x], c_fdct_basis[8 * x + 2 * j + 1]));
+            o[j] = x == 0 ? term : pair_add(o[j], term);
+        }
+    }
+}
+
+// Up to 32 blocks a warp, a lane each (IdctShape: a component of 32 blocks,
+// several of fewer, or several slices). A lane loads its block's 8 rows,
+// transforms them (rows, then columns, in the crate's order) in its own column
+// of shared memory, [position][lane], so nothing is exchanged and no bank is
+// met twice. Then the warp writes the components out in scanned order, 16
+// bytes a lane, with the largest |F| of every 32 coefficients (8 lanes).
+// Bound by issue (74 % of the slots, 49 instructions a sample, of which the
+// sums' terms are 23): 30 UHD 4:2:2 frames take 910 us, 1463 with a warp per
+// component (half the lanes idle in 4:2:2 chroma, more in narrow slices) and a
+// reduction for every position's maximum; a mixed batch 545 for 1796. Rows are
+// loaded two ahead (1022 us without), 24 warps an SM.
+struct FdctWarp {
+    float t[64][32];
+    uint8_t raster[64];  // of each scanned position
+};
+
+__global__ void __launch_bounds__(32 * kFdctWarps, 6) k_fdct(EncodeLaunch e) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    FdctWarp &w = reinterpret_cast<FdctWarp *>(smem)[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t index = blockIdx.x * kFdctWarps + (threadIdx.x >> 5);
+    if (index >= e.n_fdct_items) return;  // the whole warp
+    // The item's picture: the last whose items start at or before it.
+    uint32_t pic = 0;
+    for (uint32_t i = 0; i < e.n_pics; i += 32u) {
+        const uint32_t m = __ballot_sync(0xffffffffu, i + lane < e.n_pics && e.pics[i + lane].fdct_base <= index);
+        if (m) pic = i + 31u - __clz(m);
+        if (m != 0xffffffffu) break;
+    }
+    const EncPicDesc &pd = e.pics[pic];
     const EncFrameDesc &fd = e.frames[pd.frame];
     const uint32_t cpm = fd.chroma == 2 ? 2u : 4u;
-    const uint32_t per_mb = c == 0 ? 4u : cpm;
-    const uint32_t nb = per_mb * sd.mbs;
-    const uint32_t start = c == 0 ? 0u : 64u * sd.mbs * (4u + (c - 1u) * cpm);
-    uint32_t *cm = cmax_sh[warp];
-    cm[lane] = 0;
-    cm[lane + 32] = 0;
-    __syncwarp();
-    if (lane < nb) {
-        const uint8_t *scan = c_enc_scan[pd.interlaced_scan];
-        float (*tmp)[32] = tmp_sh[warp];
-        const uint32_t m = lane / per_mb, b = lane - m * per_mb;
-        uint32_t bx, by;
-        block_xy(c, fd.chroma, sd.mb_x, sd.mb_y, m, b, bx, by);
-        const uint32_t w = fd.plane_w[c];
-        const uint16_t *plane = e.in + fd.in_off[c];
-        const float scale = fd.in_scale;
-        // Rows: tmp[y][u] = sum_x p[y][x] T[x][u], x in order from 0.
+    const IdctShape shape = idct_shape(fd.chroma, pd.log2_slice_mbs);
+    const uint32_t local = index - pd.fdct_base;
+    const uint32_t first = shape.slices > 1u ? local * shape.slices : local / shape.parts;
+    const uint32_t part = shape.slices > 1u ? 0u : local - first * shape.parts;
+    const uint32_t n_slices = min(shape.slices, pd.n_slices - first);
+    uint32_t c0, c1;
+    idct_components(shape, cpm, part, c0, c1);
+    w.raster[c_enc_scan[pd.interlaced_scan][lane]] = (uint8_t)lane;
+    w.raster[c_enc_scan[pd.interlaced_scan][lane + 32u]] = (uint8_t)(lane + 32u);
+
+    // This lane's block.
+    const uint32_t j = lane / shape.blocks;
+    if (j < n_slices) {
+        const EncSliceDesc sd = e.slices[pd.slice_base + first + j];
+        const uint32_t nb_y = c0 == 0 ? 4u * sd.mbs : 0u, nb_c = cpm * sd.mbs;
+        uint32_t b = lane - j * shape.blocks, c = 0;
+        if (b >= nb_y) {
+            b -= nb_y;
+            c = max(c0, 1u);
+            if (b >= nb_c) {
+                b -= nb_c;
+                c++;
+            }
+            if (b >= nb_c) c = 3u;  // past the item's blocks
+        }
+        if (c < c1) {
+            const uint32_t per_shift = c == 0 || cpm == 4u ? 2u : 1u;
+            uint32_t bx, by;
+            block_xy(c, fd.chroma, sd.mb_x, sd.mb_y, b >> per_shift, b & ((1u << per_shift) - 1u), bx, by);
+            const uint32_t pw = fd.plane_w[c];
+            const uint16_t *plane = e.in + fd.in_off[c] + (uint64_t)pd.first_row * pw;
+            const float scale = fd.in_scale;
+            const bool wide = bx + 8u <= pw;
+            // Row y's eight samples; the last picture row and column repeat.
+            const auto load = [&](uint32_t y) {
+                const uint16_t *line = plane + (uint64_t)(pd.row_step * min(by + y, pd.height - 1u)) * pw;
+                if (wide && (reinterpret_cast<uintptr_t>(line + bx) & 15u) == 0)
+                    return __ldg(reinterpret_cast<const uint4 *>(line + bx));
+                uint32_t v[8];
 #pragma unroll
-        for (int y = 0; y < 8; y++) {
-            // Edge replication: the last picture row and column repeat.
-            const uint32_t py = min(by + (uint32_t)y, pd.height - 1u);
-            const uint16_t *line = plane + (uint64_t)(pd.first_row + pd.row_step * py) * w;
-            float p[8];
-            if (bx + 8u <= w && ((reinterpret_cast<uintptr_t>(line + bx) & 15u) == 0)) {
-                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(line + bx));
-                const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+                for (uint32_t x = 0; x < 8; x++) v[x] = __ldg(line + min(bx + x, pw - 1u));  // bx may be past the plane
+                return make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
+            };
+            uint4 row = load(0), next = load(1);
+            // p = s 512 / 2^b - 256: the product is exact, so one rounding
+            // is the crate's two.
+#pragma unroll 1
+            for (uint32_t y = 0; y < 8; y++) {
+                const uint4 after = load(min(y + 2u, 7u));  // two rows ahead
+                const uint32_t words[4] = {row.x, row.y, row.z, row.w};
+                float p[8];
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    p[2 * i] = __fsub_rn(__fmul_rn((float)(words[i] & 0xFFFFu), scale), 256.0f);
-                    p[2 * i + 1] = __fsub_rn(__fmul_rn((float)(words[i] >> 16), scale), 256.0f);
+                    p[2 * i] = __fmaf_rn((float)(words[i] & 0xFFFFu), scale, -256.0f);
+                    p[2 * i + 1] = __fmaf_rn((float)(words[i] >> 16), scale, -256.0f);
                 }
-            } else {
+                row = next;
+                next = after;
+                uint64_t o[4];
+                fdct8(p, o);
 #pragma unroll
-                for (int x = 0; x < 8; x++) {
-                    const uint32_t col = min(bx + (uint32_t)x, w - 1u);
-                    p[x] = __fsub_rn(__fmul_rn((float)__ldg(line + col), scale), 256.0f);
-                }
+                for (int k = 0; k < 4; k++) pair_split(o[k], w.t[8 * y + 2 * k][lane], w.t[8 * y + 2 * k + 1][lane]);
             }
-            // Outputs u = 2 j, 2 j + 1 summed as a pair, each in the same
-            // order; the products stay scalar (see pair_math.h).
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                uint64_t acc = 0;
-#pragma unroll
-                for (int x = 0; x < 8; x++)
-                    acc = pair_add(acc, pair_of(__fmul_rn(p[x], c_fdct_basis[8 * x + 2 * j]),
-                                                __fmul_rn(p[x], c_fdct_basis[8 * x + 2 * j + 1])));
-                pair_split(acc, tmp[8 * y + 2 * j][lane], tmp[8 * y + 2 * j + 1][lane]);
-            }
-        }
-        // Columns: F[v][u] = sum_y T[y][v] tmp[y][u], y in order from 0.
-        float *out = e.coef + sd.coef + start;
-        const uint32_t mask = nb >= 32u ? 0xffffffffu : (1u << nb) - 1u;
+            // Columns: F[v][u] = sum_y T[y][v] tmp[y][u], y in order from 0.
 #pragma unroll 1
-        for (int u = 0; u < 8; u++) {
-            float col[8];
+            for (uint32_t u = 0; u < 8; u++) {
+                float col[8];
 #pragma unroll
-            for (int y = 0; y < 8; y++) col[y] = tmp[8 * y + u][lane];
-            float res[8];
+                for (int y = 0; y < 8; y++) col[y] = w.t[8 * y + u][lane];
+                uint64_t o[4];
+                fdct8(col, o);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                // Outputs v = 2 j, 2 j + 1 summed as a pair.
-                uint64_t acc = 0;
-#pragma unroll
-                for (int y = 0; y < 8; y++)
-                    acc = pair_add(acc, pair_of(__fmul_rn(c_fdct_basis[8 * y + 2 * j], col[y]),
-                                                __fmul_rn(c_fdct_basis[8 * y + 2 * j + 1], col[y])));
-                pair_split(acc, res[2 * j], res[2 * j + 1]);
-            }
-#pragma unroll
-            for (int v = 0; v < 8; v++) {
-                const float acc = res[v];
-                const uint32_t sp = scan[8 * v + u];
-                out[nb * sp + lane] = acc;
-                // Every active lane is at this position, in one chunk.
-                const uint32_t big = __reduce_max_sync(mask, __float_as_uint(fabsf(acc)));
-                if (lane == 0) {
-                    const uint32_t j = (nb * sp) >> 5;
-                    cm[j] = max(cm[j], big);
-                }
+                for (int k = 0; k < 4; k++)
+                    pair_split(o[k], w.t[16 * k + u][lane], w.t[16 * k + 8 + u][lane]);
             }
         }
     }
     __syncwarp();
-    // The component's 2 nb chunk maxima.
-    float *cmax = e.coef_max + ((sd.coef + start) >> 5);
-    for (uint32_t j = lane; j < 2u * nb; j += 32) cmax[j] = __uint_as_float(cm[j]);
+
+    // The components, one after another.
+    for (uint32_t k = 0; k < n_slices; k++) {
+        const EncSliceDesc sd = e.slices[pd.slice_base + first + k];
+        uint32_t at = k * shape.blocks;
+        for (uint32_t c = c0; c < c1; c++) {
+            const uint32_t nb = (c == 0 ? 4u : cpm) * sd.mbs;
+            const uint64_t coef = sd.coef + (c == 0 ? 0u : 64u * sd.mbs * (4u + (c - 1u) * cpm));
+            float *out = e.coef + coef, *cmax = e.coef_max + (coef >> 5);
+            if (nb >= 4u) {
+                const uint32_t shift = 29u - __clz(nb);  // four blocks of a position a lane
+#pragma unroll 4
+                for (uint32_t i = lane; i < 16u * nb; i += 32u) {
+                    const uint32_t r = w.raster[i >> shift], b = 4u * (i & ((1u << shift) - 1u));
+                    const float4 v = *reinterpret_cast<const float4 *>(&w.t[r][at + b]);
+                    reinterpret_cast<float4 *>(out)[i] = v;
+                    float m = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+                    if ((lane & 7u) == 0) cmax[i >> 3] = m;
+                }
+            } else {
+#pragma unroll
+                for (uint32_t i = lane; i < 64u; i += 32u) {  // both blocks of a position
+                    const float2 v = *reinterpret_cast<const float2 *>(&w.t[w.raster[i]][at]);
+                    reinterpret_cast<float2 *>(out)[i] = v;
+                    float m = fmaxf(fabsf(v.x), fabsf(v.y));
+#pragma unroll
+                    for (int o = 1; o < 16; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                    if ((lane & 15u) == 0) cmax[i >> 4] = m;
+                }
+            }
+            at += nb;
+        }
+    }
 }
 
 // ---------------------------------------------------------------- alpha
@@ -2018,8 +2071,7 @@ __global__ void __launch_bounds__(32 * kAlphaWarps) k_pack_alpha(EncodeLaunch e)
 
 cudaError_t launch_fdct(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
-    const uint32_t warps = 3u * e.n_slices, per_block = kFdctThreads / 32;
-    k_fdct<<<(warps + per_block - 1) / per_block, kFdctThreads, 0, s>>>(e);
+    k_fdct<<<(e.n_fdct_items + kFdctWarps - 1) / kFdctWarps, 32 * kFdctWarps, kFdctWarps * sizeof(FdctWarp), s>>>(e);
     return cudaGetLastError();
 }
 
@@ -2112,6 +2164,7 @@ cudaError_t launch_pack(const EncodeLaunch &e, cudaStream_t s) {
 }
 
 cudaError_t configure_encode_kernels() {
+    static_assert(sizeof(FdctWarp) % 16 == 0, "the warps' areas are 16-byte aligned");
     cudaError_t err0 = cudaFuncSetAttribute(k_shareout, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)(kShareWarps * kShareLadderBytes));
     if (err0 != cudaSuccess) return err0;

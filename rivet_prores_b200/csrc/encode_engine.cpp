@@ -44,7 +44,7 @@ struct EncodePlan {
     std::vector<uint8_t> quant_keys;  // 129 bytes per set: weights and scan
     std::vector<uint8_t> headers;
     size_t in_total = 0, alpha_total = 0, coef_total = 0, out_total = 0;
-    uint32_t n_slices = 0;
+    uint32_t n_slices = 0, n_fdct_items = 0;
     bool any_alpha = false;
     std::vector<uint64_t> frame_size;
     std::vector<uint32_t> frame_status;
@@ -235,6 +235,8 @@ Status plan_encode(const prores_config *cfg, const prores_frame *in, int n, Enco
             p.quant = quant;
             p.header_bytes = alpha ? 8u : 6u;
             p.interlaced_scan = h.interlace != 0;
+            p.fdct_base = plan->n_fdct_items;
+            plan->n_fdct_items += idct_items(idct_shape((uint32_t)f.chroma, c.log2_slice_mbs), p.n_slices);
             const uint32_t pic_index = (uint32_t)plan->pdesc.size();
             for (uint32_t my = 0; my < p.height_in_mb; my++) {
                 uint32_t mx = 0;
@@ -323,6 +325,7 @@ static EncodeLaunch encode_params(Context &ctx, Workspace &ws, const EncodePlan 
     e.n_frames = (uint32_t)plan.fdesc.size();
     e.n_pics = (uint32_t)plan.pdesc.size();
     e.n_slices = plan.n_slices;
+    e.n_fdct_items = plan.n_fdct_items;
     e.any_alpha = plan.any_alpha;
     e.sm_count = ctx.sm_count;
     return e;

@@ -5,6 +5,8 @@
 
 #include <cstdint>
 
+#include "device_types.h"
+
 namespace prores {
 
 // Bisection steps after the probe at 224: the interval [1, 224] halves
@@ -49,6 +51,7 @@ struct EncPicDesc {
     uint32_t quant;         // index of the picture's quantiser table set
     uint32_t header_bytes;  // slice header: 6, or 8 with alpha
     uint32_t interlaced_scan;
+    uint32_t fdct_base;     // the picture's first item of k_fdct
 };
 
 struct EncSliceDesc {
@@ -130,7 +133,7 @@ struct EncodeLaunch {
     const uint8_t *headers;  // frame header templates
     uint32_t *frame_status;  // per frame: 0, or 1 when the frame outgrew its region
     uint64_t *frame_size;    // per frame
-    uint32_t n_frames, n_pics, n_slices;
+    uint32_t n_frames, n_pics, n_slices, n_fdct_items;
     int any_alpha;
     int sm_count;
 };

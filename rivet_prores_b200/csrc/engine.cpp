@@ -525,8 +525,7 @@ Status plan_decode(const prores_buf *in, int n, uint32_t out_depth, DecodePlan &
             plan.n_slices += (uint32_t)n_slices;
             const IdctShape shape = idct_shape((uint32_t)h.chroma, ph.log2_slice_mbs);
             plan.pdesc.back().idct_base = plan.n_idct_items;
-            plan.n_idct_items += shape.slices > 1 ? (uint32_t)((n_slices + shape.slices - 1) / shape.slices)
-                                                  : (uint32_t)n_slices * shape.parts;
+            plan.n_idct_items += idct_items(shape, (uint32_t)n_slices);
             plan.coef_total += (size_t)width_in_mb * height_in_mb * 64u * (4u + 2u * cpm);
             f.n_pics++;
             pos += ph.picture_size;
