@@ -362,6 +362,44 @@ __global__ void __launch_bounds__(32 * kAlphaWarps) k_alpha_size(EncodeLaunch e)
     if (lane == 0) e.alpha_bytes[s] = (bits + 7u) / 8u;
 }
 
+// ---------------------------------------------------------------- quantisers
+
+// A lower bound on the |F| that quantise to a non-zero AC level at inverse
+// weight inv. A level is non-zero when fl(fl(|F| inv) + 0.42f) >= 1, which
+// needs the exact sum fl(|F| inv) + 0.42f to reach 1 - 2^-25 (the midpoint
+// below 1), and so |F| inv >= (1 - 2^-25 - 0.42f)(1 - 2^-24). The bound takes
+// a margin of 2^-22 and is rounded down, so every non-zero lies at or above
+// it; the kernels re-quantise each candidate exactly.
+__device__ __forceinline__ float nonzero_bound(float inv) {
+    constexpr double y0 = 1.0 - 1.0 / (1 << 25) - (double)kAcRounding;
+    return __double2float_rd(__ddiv_rn(y0 * (1.0 - 1.0 / (1 << 22)), (double)inv));
+}
+
+// A CTA per quantization_index and set (layout beside kQuantStride): inv[scan[k]] =
+// 8 / (W[k] qScale) in single precision for luma and chroma
+// (src/encode.rs:303-329), the non-zero bound of each, and the least bound
+// over each chunk of 32 scanned coefficients. On the host the 225 quantisers
+// of a set took about half a millisecond of every call.
+__global__ void __launch_bounds__(128) k_quant(float *quant, const uint8_t *keys) {
+    __shared__ float bound[128];
+    const uint32_t qi = blockIdx.x, i = threadIdx.x, k = i & 63u, g = i >> 6;
+    const uint8_t *key = keys + kQuantKey * blockIdx.y;
+    float *t = quant + ((uint64_t)blockIdx.y * 225u + qi) * kQuantStride;
+    const uint32_t at = 64u * g + c_enc_scan[key[128]][k];
+    const float inv = __fdiv_rn(8.0f, (float)((uint32_t)key[i] * qscale(qi < 1u ? 1u : qi)));
+    t[at] = inv;
+    bound[at] = nonzero_bound(inv);
+    t[128u + at] = bound[at];
+    __syncthreads();
+    // Chunk j of a component of n blocks is positions 32 j / n to 32 (j + 1) / n - 1.
+    if (k < 60u) {
+        const uint32_t shift = 31u - __clz((k + 4u) >> 1), n = 1u << shift, j = k - (2u * n - 4u);
+        float m = bound[64u * g + 32u * j / n];
+        for (uint32_t p = 32u * j / n + 1u; p < 32u * (j + 1u) / n; p++) m = fminf(m, bound[64u * g + p]);
+        t[256u + 60u * g + k] = m;
+    }
+}
+
 // ---------------------------------------------------------------- costing
 
 // One AC position of a lane's walk: x = F inv, m = floor(|x| + 0.42)
@@ -1144,7 +1182,7 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_deep(EncodeL
     if (lane == 0) e.deep_count[s] = count;
 }
 
-constexpr int kRcThreads = 256;
+constexpr int kRcThreads = 1024;
 
 __device__ __forceinline__ uint64_t block_sum_u64(uint64_t v, uint64_t *sh) {
 #pragma unroll
@@ -1162,7 +1200,8 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_init(EncodeLaunch e) {
     __shared__ uint64_t sh[kRcThreads / 32];
     const EncPicDesc pd = e.pics[blockIdx.x];
     uint64_t a = 0;
-    for (uint32_t k = threadIdx.x; k < pd.n_slices; k += kRcThreads) a += e.alpha_bytes[pd.slice_base + k];
+    if (e.any_alpha)
+        for (uint32_t k = threadIdx.x; k < pd.n_slices; k += kRcThreads) a += e.alpha_bytes[pd.slice_base + k];
     const uint64_t alpha = block_sum_u64(a, sh);
     if (threadIdx.x == 0) {
         // Alpha is lossless and comes on top of the rate; the picture
@@ -1197,12 +1236,13 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_step(EncodeLaunch e, int step
     __syncthreads();
     uint64_t sum = 0;
     bool fit = true;
+#pragma unroll 4
     for (uint32_t k = threadIdx.x; k < pd.n_slices; k += kRcThreads) {
         const uint32_t s = pd.slice_base + k;
         const uint32_t *c = e.probe_comp + ((uint64_t)step * e.n_slices + s) * 3u;
         const uint32_t cc[3] = {c[0], c[1], c[2]};
         bool f;
-        sum += slice_total(pd.header_bytes, cc, e.alpha_bytes[s], f);
+        sum += slice_total(pd.header_bytes, cc, e.any_alpha ? e.alpha_bytes[s] : 0u, f);
         fit = fit && f;
     }
     if (!fit) all_fit = 0;
@@ -2068,6 +2108,11 @@ __global__ void __launch_bounds__(32 * kAlphaWarps) k_pack_alpha(EncodeLaunch e)
 }
 
 }  // namespace
+
+cudaError_t launch_quant(float *quant, const uint8_t *keys, uint32_t sets, cudaStream_t s) {
+    k_quant<<<dim3(225, sets), 128, 0, s>>>(quant, keys);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_fdct(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;

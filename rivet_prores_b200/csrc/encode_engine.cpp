@@ -40,8 +40,7 @@ struct EncodePlan {
     std::vector<EncFrameDesc> fdesc;
     std::vector<EncPicDesc> pdesc;
     std::vector<EncSliceDesc> sdesc;
-    std::vector<float> quant;
-    std::vector<uint8_t> quant_keys;  // 129 bytes per set: weights and scan
+    std::vector<uint8_t> quant_keys;  // kQuantKey bytes per set: weights and scan
     std::vector<uint8_t> headers;
     size_t in_total = 0, alpha_total = 0, coef_total = 0, out_total = 0;
     uint32_t n_slices = 0, n_fdct_items = 0;
@@ -101,56 +100,18 @@ static Status validate(const prores_config &cfg, const prores_frame &f, int *alp
     return Status();
 }
 
-// A lower bound on the |F| that quantise to a non-zero AC level at inverse
-// weight inv. A level is non-zero when fl(fl(|F| inv) + 0.42f) >= 1, which
-// needs the exact sum fl(|F| inv) + 0.42f to reach 1 - 2^-25 (the midpoint
-// below 1), and so |F| inv >= (1 - 2^-25 - 0.42f)(1 - 2^-24). The bound takes
-// a margin of 2^-22 and is rounded down, so every non-zero lies at or above
-// it; the kernels re-quantise each candidate exactly.
-static float nonzero_bound(float inv) {
-    const double y0 = 1.0 - std::ldexp(1.0, -25) - (double)0.42f;
-    const double t = y0 * (1.0 - std::ldexp(1.0, -22)) / (double)inv;
-    float b = (float)t;
-    if ((double)b > t) b = std::nextafter(b, 0.0f);
-    return b;
-}
-
-// Per quantization_index, kQuantStride floats (the layout is given beside
-// kQuantStride): inv[scan[k]] = 8 / (W[k] qScale) in single precision for
-// luma and chroma (src/encode.rs:303-329), the non-zero bound of each, and
-// the least bound over each chunk of 32 scanned coefficients.
+// The quantiser table set of a frame's weights and scan: its key (both
+// matrices in raster order and the scan), from which k_quant builds the
+// tables on the device.
 static uint32_t add_quant(EncodePlan &plan, const FrameHeader &h) {
-    uint8_t key[129];
+    uint8_t key[kQuantKey];
     h.luma_weights(key);
     h.chroma_weights(key + 64);
     key[128] = h.interlace != 0;
-    for (size_t i = 0; i + 129 <= plan.quant_keys.size(); i += 129)
-        if (memcmp(&plan.quant_keys[i], key, 129) == 0) return (uint32_t)(i / 129);
-    plan.quant_keys.insert(plan.quant_keys.end(), key, key + 129);
-    const uint8_t *scan = h.interlace ? kInterlacedScan : kProgressiveScan;
-    const size_t base = plan.quant.size();
-    plan.quant.resize(base + 225 * kQuantStride);
-    for (uint32_t qi = 0; qi <= 224; qi++) {
-        const uint32_t q = qscale(qi < 1 ? 1 : qi);
-        float *t = &plan.quant[base + qi * kQuantStride];
-        for (int k = 0; k < 64; k++) {
-            t[scan[k]] = 8.0f / (float)((uint32_t)key[k] * q);
-            t[64 + scan[k]] = 8.0f / (float)((uint32_t)key[64 + k] * q);
-        }
-        for (int k = 0; k < 128; k++) t[128 + k] = nonzero_bound(t[k]);
-        for (uint32_t g = 0; g < 2; g++) {
-            const float *bound = t + 128 + 64 * g;
-            for (uint32_t n = 2; n <= 16; n *= 2) {
-                float *chunk = t + 256 + 60 * g + (2 * n - 4);
-                for (uint32_t j = 0; j < 2 * n; j++) {
-                    float m = bound[32 * j / n];
-                    for (uint32_t k = 32 * j / n; k < 32 * (j + 1) / n; k++) m = std::min(m, bound[k]);
-                    chunk[j] = m;
-                }
-            }
-        }
-    }
-    return (uint32_t)(plan.quant_keys.size() / 129 - 1);
+    for (size_t i = 0; i + kQuantKey <= plan.quant_keys.size(); i += kQuantKey)
+        if (memcmp(&plan.quant_keys[i], key, kQuantKey) == 0) return (uint32_t)(i / kQuantKey);
+    plan.quant_keys.insert(plan.quant_keys.end(), key, key + kQuantKey);
+    return (uint32_t)(plan.quant_keys.size() / kQuantKey - 1);
 }
 
 Status plan_encode(const prores_config *cfg, const prores_frame *in, int n, EncodePlanPtr &out) {
@@ -384,7 +345,10 @@ Status upload_encode(Context &ctx, Workspace &ws, EncodePlan &plan, const prores
         PR_CUDA(ws.enc_pic_state.reserve(sizeof(EncPicState) * (plan.pdesc.size() + 1)), "cudaMalloc");
         // The coefficients, then (64 floats on) one chunk maximum per 32.
         PR_CUDA(ws.enc_coef.reserve(4 * (plan.coef_total + plan.coef_total / 32 + 128)), "cudaMalloc coefficients");
-        PR_CUDA(ws.weights.reserve(4 * (plan.quant.size() + 64)), "cudaMalloc");
+        // The quantiser tables, then the keys they are built from.
+        const size_t n_sets = plan.quant_keys.size() / kQuantKey;
+        const size_t quant_bytes = 4 * (n_sets * 225 * kQuantStride + 64);
+        PR_CUDA(ws.weights.reserve(quant_bytes + plan.quant_keys.size() + 64), "cudaMalloc");
         PR_CUDA(ws.enc_cost.reserve(cost_bytes(plan)), "cudaMalloc");
         PR_CUDA(ws.enc_out.reserve(plan.out_total + 64), "cudaMalloc output");
         PR_CUDA(ws.enc_frame_out.reserve(plan.headers.size() + 64), "cudaMalloc");
@@ -399,9 +363,11 @@ Status upload_encode(Context &ctx, Workspace &ws, EncodePlan &plan, const prores
         if (!plan.sdesc.empty())
             PR_CUDA(ws.stager.h2d(ws.slices.p, plan.sdesc.data(), sizeof(EncSliceDesc) * plan.sdesc.size(), s),
                     "upload");
-        if (!plan.quant.empty())
-            PR_CUDA(ws.stager.h2d(ws.weights.p, plan.quant.data(), 4 * plan.quant.size(), s),
-                    "upload");
+        if (n_sets) {
+            uint8_t *keys = ws.weights.as<uint8_t>() + quant_bytes;
+            PR_CUDA(ws.stager.h2d(keys, plan.quant_keys.data(), plan.quant_keys.size(), s), "upload");
+            PR_CUDA(launch_quant(ws.weights.as<float>(), keys, (uint32_t)n_sets, s), "k_quant");
+        }
         if (!plan.headers.empty())
             PR_CUDA(ws.stager.h2d(ws.enc_frame_out.p, plan.headers.data(), plan.headers.size(), s),
                     "upload");

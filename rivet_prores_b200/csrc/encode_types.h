@@ -103,6 +103,9 @@ struct SharePrep {
 //               of n blocks, n = 2, 4, 8, 16 (2n chunks each, at 2n - 4).
 // For n = 32 a chunk is one scanned position, whose bound is in [128, 256).
 constexpr uint32_t kQuantStride = 384;
+// What a set is built from: luma and chroma weights in raster order, and
+// whether the scan is the interlaced one.
+constexpr size_t kQuantKey = 129;
 
 struct EncodeLaunch {
     const uint16_t *in;        // input planes
@@ -138,6 +141,8 @@ struct EncodeLaunch {
     int sm_count;
 };
 
+// Builds `sets` quantiser table sets at `quant` from their keys.
+cudaError_t launch_quant(float *quant, const uint8_t *keys, uint32_t sets, cudaStream_t s);
 cudaError_t launch_fdct(const EncodeLaunch &e, cudaStream_t s);
 cudaError_t launch_alpha_size(const EncodeLaunch &e, cudaStream_t s);
 cudaError_t launch_rc_init(const EncodeLaunch &e, cudaStream_t s);

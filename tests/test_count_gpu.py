@@ -45,3 +45,27 @@ def test_every_way_of_counting_gives_the_oracles_packet(kind):
         k, msg, want = O.encode(cfg, pic)
         assert k == O.OK, msg
         assert not isinstance(g, P.Error) and g == want, (kind, i)
+
+
+@pytest.mark.parametrize("weights", ["least", "most", "mixed"])
+def test_quantiser_tables_of_extreme_weights(weights):
+    """The tables the device builds, over coarse and fine quantisers, both
+    scans and both matrices, sets of different frames side by side."""
+    cases = []
+    for i, (chroma, profile) in enumerate(((2, 3), (3, 4), (2, 1))):
+        rng = np.random.Generator(np.random.PCG64(i))
+        luma, chroma_w = ((bytes([2] * 64), bytes([63] * 64)) if weights == "least" else
+                          (bytes([63] * 64), bytes([2] * 64)) if weights == "most" else
+                          (bytes(int(v) for v in rng.integers(2, 64, 64)), None))
+        for interlace in range(2):
+            for target in (None, 1 << 30, 4000):
+                p = _picture("noise" if target else "strong", chroma, 7 * i + interlace)
+                p.interlace = interlace
+                cases.append((O.Config(profile, log2_slice_mbs=i, luma_matrix=luma, chroma_matrix=chroma_w,
+                                       target_frame_bytes=target), p))
+    got = P.Encoder(to_config(cases[0][0])).encode_batch([to_frame(p) for _, p in cases],
+                                                        [to_config(c) for c, _ in cases])
+    for i, ((cfg, pic), g) in enumerate(zip(cases, got)):
+        k, msg, want = O.encode(cfg, pic)
+        assert k == O.OK, msg
+        assert not isinstance(g, P.Error) and g == want, (weights, i)
