@@ -22,7 +22,6 @@
 
 #include <algorithm>
 #include <cstring>
-#include <map>
 #include <vector>
 
 #include "engine.h"
@@ -90,94 +89,75 @@ Status check_spans(const prores_span *frames, int n, size_t data_len) {
     return Status();
 }
 
-// The header regions plan_decode reads, fetched from device memory in three
-// rounds (frame headers; first picture headers; second picture headers of
-// interlaced frames), each one small copy per frame into pinned memory.
+// The header bytes planning reads of a frame: the frame header, then the
+// header of each picture, side by side (zero where the frame is shorter).
+struct HeadSlot {
+    uint8_t head[kFrameHeadBytes];
+    uint8_t pic[2][kPictureHeaderSize];
+};
+constexpr int kHeadBatch = 64;  // frames a launch, their spans passed as its argument
+struct HeadSpans {
+    prores_span span[kHeadBatch];
+};
+
+// A warp per frame gathers its slot, walking to the picture headers as
+// plan_decode does: the first after the frame header, the second after the
+// first picture. `out` is page-locked host memory, which the warps write
+// themselves: one launch and one wait for what took a copy a frame in each
+// of three rounds (32 frames: about 100 us a round, probing and decoding).
+__global__ void __launch_bounds__(32 * 4) k_gather_heads(const uint8_t *data, HeadSpans spans, int n, HeadSlot *out) {
+    const int i = (int)(blockIdx.x * 4 + (threadIdx.x >> 5));
+    const uint32_t lane = threadIdx.x & 31u;
+    if (i >= n) return;
+    const uint8_t *frame = data + spans.span[i].offset;
+    const uint64_t len = spans.span[i].len;
+    const auto at = [&](uint64_t pos) -> uint32_t { return pos < len ? byte_at(frame, pos) : 0u; };
+    for (uint32_t k = lane; k < kFrameHeadBytes; k += 32u) out[i].head[k] = (uint8_t)at(k);
+    uint64_t pos = 8u + ((at(8) << 8) | at(9));
+    for (int p = 0; p < 2; p++) {
+        if (lane < kPictureHeaderSize) out[i].pic[p][lane] = (uint8_t)at(pos + lane);
+        pos += ((uint64_t)at(pos + 1) << 24) | (at(pos + 2) << 16) | (at(pos + 3) << 8) | at(pos + 4);
+    }
+}
+
+// The header bytes of every frame of a call, fetched from device memory.
 struct DeviceHeads {
-    std::vector<std::vector<uint8_t>> head;
-    std::vector<std::map<size_t, std::vector<uint8_t>>> pics;
+    std::vector<HeadSlot> slots;
+    std::vector<size_t> lens;
 
     Status fetch(Workspace &ws, const uint8_t *d_data, const prores_span *frames, int n, cudaStream_t s) {
-        head.assign(n, {});
-        pics.assign(n, {});
-        std::vector<size_t> want(n);
-        for (int i = 0; i < n; i++) want[i] = std::min(frames[i].len, kFrameHeadBytes);
-        Status st = round(ws, d_data, frames, n, s, [&](int i, size_t &pos, size_t &len) {
-            pos = 0;
-            len = want[i];
-            return true;
-        }, [&](int i, const uint8_t *p, size_t len) { head[i].assign(p, p + len); });
-        if (st) return st;
-        // Where each picture header is, as plan_decode walks to it.
-        std::vector<FrameHeader> hdr(n);
-        std::vector<int> ok(n, 0);
-        for (int i = 0; i < n; i++)
-            ok[i] = !parse_frame_header(head[i].data(), frames[i].len, &hdr[i]) && !check_plausible_size(hdr[i]);
-        std::vector<size_t> pos(n, 0);
-        for (int i = 0; i < n; i++) pos[i] = ok[i] ? 8 + (size_t)hdr[i].header_size : 0;
-        for (uint32_t index = 0; index < 2; index++) {
-            st = round(ws, d_data, frames, n, s, [&](int i, size_t &p, size_t &len) {
-                if (!ok[i] || index >= hdr[i].picture_count() || pos[i] > hdr[i].frame_size) return false;
-                p = pos[i];
-                len = std::min((size_t)hdr[i].frame_size - pos[i], kPictureHeaderSize);
-                return true;
-            }, [&](int i, const uint8_t *p, size_t len) { pics[i][pos[i]].assign(p, p + len); });
-            if (st) return st;
-            for (int i = 0; i < n; i++) {
-                auto it = pics[i].find(pos[i]);
-                if (!ok[i] || it == pics[i].end()) {
-                    ok[i] = 0;
-                    continue;
-                }
-                PictureHeader ph;
-                if (parse_picture_header(it->second.data(), hdr[i].frame_size - pos[i], &ph)) {
-                    ok[i] = 0;
-                    continue;
-                }
-                pos[i] += ph.picture_size;
-            }
+        slots.resize(n);
+        lens.resize(n);
+        if (!n) return Status();
+        PR_CUDA(ws.host_small.reserve(sizeof(HeadSlot) * n), "cudaMallocHost");
+        HeadSlot *host = static_cast<HeadSlot *>(ws.host_small.p);
+        for (int first = 0; first < n; first += kHeadBatch) {
+            const int count = std::min(kHeadBatch, n - first);
+            HeadSpans spans{};
+            std::copy(frames + first, frames + first + count, spans.span);
+            k_gather_heads<<<(count + 3) / 4, 32 * 4, 0, s>>>(d_data, spans, count, host + first);
+            PR_CUDA(cudaGetLastError(), "k_gather_heads");
         }
+        Status w = wait_stream(s, ws.wait_ms, "header fetch");
+        if (w) return w;
+        std::copy(host, host + n, slots.begin());
+        for (int i = 0; i < n; i++) lens[i] = frames[i].len;
         return Status();
     }
 
+    const uint8_t *head(int i) const { return slots[i].head; }
+
+    // Bytes [pos, pos + len) of frame i, if a slot holds them.
     const uint8_t *bytes(int i, size_t pos, size_t len) const {
-        static const uint8_t none = 0;
-        if (len == 0) return &none;
-        if (pos == 0) return len <= head[i].size() ? head[i].data() : nullptr;
-        auto it = pics[i].find(pos);
-        return it != pics[i].end() && len <= it->second.size() ? it->second.data() : nullptr;
-    }
-
-  private:
-    template <class Which, class Keep>
-    Status round(Workspace &ws, const uint8_t *d_data, const prores_span *frames, int n, cudaStream_t s, Which which,
-                 Keep keep) {
-        std::vector<size_t> at(n, SIZE_MAX), len(n, 0);
-        size_t total = 0;
-        for (int i = 0; i < n; i++) {
-            size_t p, l;
-            if (!which(i, p, l)) continue;
-            at[i] = total;
-            len[i] = l;
-            total += (l + 15) & ~(size_t)15;
-            (void)p;
+        const HeadSlot &slot = slots[i];
+        if (pos > lens[i] || len > lens[i] - pos) return nullptr;
+        if (pos == 0 && len <= sizeof slot.head) return slot.head;
+        size_t at = 8 + (((size_t)slot.head[8] << 8) | slot.head[9]);
+        for (const uint8_t *p : {slot.pic[0], slot.pic[1]}) {
+            if (pos == at && len <= kPictureHeaderSize) return p;
+            at += ((size_t)p[1] << 24) | ((size_t)p[2] << 16) | ((size_t)p[3] << 8) | p[4];
         }
-        if (!total) return Status();
-        PR_CUDA(ws.host_small.reserve(total), "cudaMallocHost");
-        uint8_t *host = static_cast<uint8_t *>(ws.host_small.p);
-        for (int i = 0; i < n; i++) {
-            size_t p, l;
-            if (at[i] == SIZE_MAX || !which(i, p, l) || !l) continue;
-            PR_CUDA(cudaMemcpyAsync(host + at[i], d_data + frames[i].offset + p, l, cudaMemcpyDeviceToHost, s),
-                    "header fetch");
-        }
-        {
-            Status w = wait_stream(s, ws.wait_ms, "header fetch");
-            if (w) return w;
-        }
-        for (int i = 0; i < n; i++)
-            if (at[i] != SIZE_MAX) keep(i, host + at[i], len[i]);
-        return Status();
+        return len == 0 ? slot.head : nullptr;
     }
 };
 
@@ -278,9 +258,7 @@ int prores_probe_device(prores_ctx *ctx, const uint8_t *d_data, size_t data_len,
     if (st) return fail_status(st);
     std::vector<Status> errs(n);
     for (int i = 0; i < n; i++) {
-        static const uint8_t none = 0;
-        const uint8_t *h = heads.head[i].empty() ? &none : heads.head[i].data();
-        errs[i] = probe_frame(h, frames[i].len, out_bit_depth, &info[i]);  // reads the frame header only
+        errs[i] = probe_frame(heads.head(i), frames[i].len, out_bit_depth, &info[i]);  // reads the frame header only
         status[i] = errs[i].code;
     }
     set_batch_errors(errs);
