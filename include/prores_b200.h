@@ -256,6 +256,17 @@ int prores_decode_device(prores_ctx *ctx, const uint8_t *d_data, size_t data_len
 int prores_encode_device(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, prores_buf *out,
                          int *status, void *stream);
 
+/* Where a packet of prores_encode_into goes: room for `len` bytes for frame
+ * i's packet, which the call fills before it returns, or NULL to give the
+ * whole call up. Called on the calling thread, once a packet. */
+typedef uint8_t *(*prores_packet_room)(void *user, int i, size_t len);
+
+/* prores_encode_batch (device_frames 0; `stream` NULL) or prores_encode_device
+ * (device_frames 1) with the packets written straight where the caller wants
+ * them: out[i].data is what `room` gave, not library-allocated. */
+int prores_encode_into(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, int device_frames,
+                       prores_packet_room room, void *user, prores_buf *out, int *status, void *stream);
+
 /* ---- decode without device allocation --------------------------------- */
 
 /* Size of the fixed device array prores_decode_noalloc keeps its scratch in.

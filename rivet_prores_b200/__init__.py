@@ -673,11 +673,10 @@ class Encoder:
         for i in range(n):
             cfgs[i] = configs[i]._c()
             ins[i] = _frame_to_c(frames[i], keep)
-        if devices:
-            ctxs = (ctypes.c_void_p * len(devices))(*[context(d).handle for d in devices])
-            code = L.prores_encode_batch_multi(ctxs, len(devices), cfgs, ins, n, outs, status)
-        else:
-            code = L.prores_encode_batch(context(self.device).handle, cfgs, ins, n, outs, status)
+        if not devices:
+            return _encode_into(self.device, cfgs, ins, n, outs, status)
+        ctxs = (ctypes.c_void_p * len(devices))(*[context(d).handle for d in devices])
+        code = L.prores_encode_batch_multi(ctxs, len(devices), cfgs, ins, n, outs, status)
         if code != _abi.OK:
             raise _error(code)
         res: List[Union[bytes, Error]] = []
@@ -694,7 +693,6 @@ class Encoder:
         """encode_batch for frames whose planes lie in device memory
         (DeviceFrame: `data`, `alpha` device buffers with data_ptr() and
         numel(), such as torch tensors); the packets come back to the host."""
-        L = _abi.lib()
         n = len(frames)
         configs = list(configs) if configs is not None else [self._config] * n
         cfgs = (Config_ * max(n, 1))()
@@ -715,17 +713,33 @@ class Encoder:
             if f.alpha is not None:
                 c.alpha = ctypes.cast(_device_ptr(f.alpha), ctypes.POINTER(ctypes.c_uint16))
                 c.alpha_len = int(f.alpha.numel())
-        code = L.prores_encode_device(context(self.device).handle, cfgs, ins, n, outs, status, _stream_ptr(stream))
-        if code != _abi.OK:
-            raise _error(code)
-        res: List[Union[bytes, Error]] = []
-        for i in range(n):
-            if status[i] != _abi.OK:
-                res.append(_error(status[i], _abi.batch_error(i)))
-            else:
-                res.append(ctypes.string_at(outs[i].data, outs[i].len))
-                L.prores_buffer_free(outs[i].data)
-        return res
+        return _encode_into(self.device, cfgs, ins, n, outs, status, True, stream)
+
+
+_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype, _new_bytes.argtypes = ctypes.py_object, [ctypes.c_char_p, ctypes.c_ssize_t]
+_bytes_at = ctypes.pythonapi.PyBytes_AsString
+_bytes_at.restype, _bytes_at.argtypes = ctypes.c_void_p, [ctypes.py_object]
+
+
+def _encode_into(device: int, cfgs, ins, n: int, outs, status, device_frames: bool = False,
+                 stream=None) -> List[Union[bytes, Error]]:
+    """One encode call whose packets the library writes straight into new
+    bytes objects."""
+    res: List[Union[bytes, Error, None]] = [None] * n
+
+    def room(_, i, size):
+        res[i] = _new_bytes(None, size)
+        return _bytes_at(res[i])
+
+    code = _abi.lib().prores_encode_into(context(device).handle, cfgs, ins, n, int(device_frames),
+                                         _abi.PACKET_ROOM(room), None, outs, status, _stream_ptr(stream))
+    if code != _abi.OK:
+        raise _error(code)
+    for i in range(n):
+        if status[i] != _abi.OK:
+            res[i] = _error(status[i], _abi.batch_error(i))
+    return res
 
 
 # ------------------------------------------------------------------ resident jobs

@@ -100,6 +100,9 @@ class Tuning_(ctypes.Structure):
     ]
 
 
+# prores_packet_room
+PACKET_ROOM = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t)
+
 _lib = None
 
 
@@ -162,6 +165,8 @@ def lib():
                                                 P(Frame_), P(ctypes.c_int), vp]),
         "prores_encode_device": (ctypes.c_int, [vp, P(Config_), P(Frame_), ctypes.c_int, P(Buf_), P(ctypes.c_int),
                                                 vp]),
+        "prores_encode_into": (ctypes.c_int, [vp, P(Config_), P(Frame_), ctypes.c_int, ctypes.c_int, PACKET_ROOM, vp,
+                                              P(Buf_), P(ctypes.c_int), vp]),
         "prores_set_tuning": (ctypes.c_int, [vp, P(Tuning_)]),
         "prores_get_tuning": (ctypes.c_int, [vp, P(Tuning_)]),
         "prores_set_timeout": (ctypes.c_int, [vp, ctypes.c_uint32]),

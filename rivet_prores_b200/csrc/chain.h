@@ -1,0 +1,39 @@
+// chain.h -- kernels of one stream launched ahead of their turn.
+//
+// A call's kernels run one after another, three dozen of them for an encode,
+// most of them a few microseconds long for a frame or two. Launched in
+// programmatic stream order a kernel's CTAs take their places, and its
+// prologue runs, while the last CTAs of the kernel before finish. Every
+// kernel launched with launch_chained() calls chain_start() first, does only
+// what no kernel of the chain writes (its tables), and calls chain_wait()
+// before anything else and on every path: it returns when the kernel before
+// has completed, and so, each having waited in turn, all kernels before that.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace prores {
+
+#if defined(__CUDACC__)
+__device__ __forceinline__ void chain_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... Params, class... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(std::forward<Args>(args))...);
+}
+#endif
+
+}  // namespace prores

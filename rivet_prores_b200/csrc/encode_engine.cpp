@@ -508,8 +508,10 @@ static bool profiling_on() {
 
 extern "C" {
 
+// `room` (null: malloc) gives each packet's place.
 static int encode_batch(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, prores_buf *out,
-                        int *status, bool device_frames, void *stream) {
+                        int *status, bool device_frames, void *stream, prores_packet_room room = nullptr,
+                        void *user = nullptr) {
     if (!ctx || n < 0) return efail(make_status(PRORES_CONFIG, "no context"));
     cudaSetDevice(ctx->impl.device);
     EncodePlanPtr plan;
@@ -535,16 +537,17 @@ static int encode_batch(prores_ctx *ctx, const prores_config *cfg, const prores_
     }
     for (int i = 0; i < n; i++) {
         if (status[i] != PRORES_OK) continue;
-        uint8_t *p = static_cast<uint8_t *>(malloc(packets[i].len ? packets[i].len : 1));
+        const size_t len = packets[i].len;
+        uint8_t *p = room ? room(user, i, len) : static_cast<uint8_t *>(malloc(len ? len : 1));
         if (!p) {
-            for (int j = 0; j < i; j++) free(const_cast<uint8_t *>(out[j].data));
+            for (int j = 0; j < i && !room; j++) free(const_cast<uint8_t *>(out[j].data));
             for (int j = 0; j < i; j++) out[j] = prores_buf{nullptr, 0};
             ctx->impl.release(std::move(ws));
             return efail(make_status(PRORES_DEVICE, "host allocation failed"));
         }
-        memcpy(p, packets[i].data, packets[i].len);
+        memcpy(p, packets[i].data, len);
         out[i].data = p;
-        out[i].len = packets[i].len;
+        out[i].len = len;
     }
     ctx->impl.release(std::move(ws));
     if (first) set_last_error(first);
@@ -559,6 +562,12 @@ int prores_encode_batch(prores_ctx *ctx, const prores_config *cfg, const prores_
 int prores_encode_device(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, prores_buf *out,
                          int *status, void *stream) {
     return encode_batch(ctx, cfg, in, n, out, status, true, stream);
+}
+
+int prores_encode_into(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, int device_frames,
+                       prores_packet_room room, void *user, prores_buf *out, int *status, void *stream) {
+    if (!room) return efail(make_status(PRORES_CONFIG, "no room for the packets"));
+    return encode_batch(ctx, cfg, in, n, out, status, device_frames != 0, stream, room, user);
 }
 
 int prores_encode(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, uint8_t **out, size_t *out_len) {

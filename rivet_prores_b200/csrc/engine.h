@@ -50,10 +50,12 @@ struct PinnedBuf {
 // locked memory is copied straight (asynchronously); pageable memory goes
 // through a ring of pinned chunks, because a CUDA copy to or from pageable
 // memory returns only when it is done and holds up other host threads' CUDA
-// calls meanwhile. Chunks read back are copied out by finish().
+// calls meanwhile. Chunks read back are copied out by finish(). Chunks of 2
+// MiB: the bus takes one while the next is filled, and what it has left when
+// the last one is filled is short.
 struct Stager {
-    static constexpr int kSlots = 4;
-    static constexpr size_t kChunk = 8u << 20;
+    static constexpr int kSlots = 16;
+    static constexpr size_t kChunk = 2u << 20;
     PinnedBuf buf;
     cudaEvent_t ev[kSlots] = {};
     uint32_t wait_ms = 0;  // bound on each wait for a chunk (0: none)
