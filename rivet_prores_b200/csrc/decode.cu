@@ -25,6 +25,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "chain.h"
 #include "codec_tables.h"
 #include "device_types.h"
 #include "pair_math.h"
@@ -816,6 +817,8 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
 }
 
 __global__ void __launch_bounds__(kLocateThreads) k_locate(DecodeLaunch d) {
+    chain_start();
+    chain_wait();
     __shared__ uint32_t warp_sums[kLocateThreads / 32];
     __shared__ uint64_t carry;
     __shared__ int first_bad;
@@ -924,6 +927,7 @@ constexpr int kEntropyMaxThreads = 512;
 // among the steps, 1810, 535 and 2770. 83 registers leave 24 warps an SM;
 // held to 64 for 32 warps the spills cost 14 %.
 __global__ void __launch_bounds__(kEntropyMaxThreads) k_entropy(DecodeLaunch d) {
+    chain_start();
     extern __shared__ __align__(16) unsigned char smem[];
     uint16_t *run_tab = reinterpret_cast<uint16_t *>(smem), *level_tab = run_tab + kBookTableWords;
     // Each warp's ring: word k of lane l at [32 k + l].
@@ -932,6 +936,7 @@ __global__ void __launch_bounds__(kEntropyMaxThreads) k_entropy(DecodeLaunch d) 
         reinterpret_cast<uint32_t *>(run_tab)[i] = reinterpret_cast<const uint32_t *>(d.tables.run_books)[i];
         reinterpret_cast<uint32_t *>(level_tab)[i] = reinterpret_cast<const uint32_t *>(d.tables.level_books)[i];
     }
+    chain_wait();
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const uint32_t items = 4u * d.n_slices;
@@ -1055,6 +1060,8 @@ __device__ __forceinline__ void idct_columns(const float *t, uint32_t rows, floa
 }
 
 __global__ void __launch_bounds__(32 * kIdctWarps, 6) k_idct(DecodeLaunch d) {
+    chain_start();
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     IdctWarp &w = reinterpret_cast<IdctWarp *>(smem)[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
@@ -1360,6 +1367,8 @@ __device__ __forceinline__ void idct_block(const T *cs, const int32_t *wide, uin
 
 template <class T>
 __global__ void __launch_bounds__(kDecodeThreads) k_decode(DecodeLaunch d) {
+    chain_start();
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     uint16_t *run_tab = reinterpret_cast<uint16_t *>(smem);
     uint16_t *level_tab = run_tab + kBookTableWords;
@@ -1504,6 +1513,8 @@ __global__ void __launch_bounds__(kDecodeThreads) k_decode(DecodeLaunch d) {
 constexpr int kStatusThreads = 256;
 
 __global__ void __launch_bounds__(kStatusThreads) k_status(DecodeLaunch d) {
+    chain_start();
+    chain_wait();
     __shared__ int best;
     const PicDesc p = d.pics[blockIdx.x];
     if (threadIdx.x == 0) best = INT32_MAX;
@@ -1539,8 +1550,7 @@ cudaError_t upload_scans() {
 
 cudaError_t launch_locate(const DecodeLaunch &d, cudaStream_t s) {
     if (d.n_pics == 0) return cudaSuccess;
-    k_locate<<<d.n_pics, kLocateThreads, 0, s>>>(d);
-    return cudaGetLastError();
+    return launch_chained(k_locate, d.n_pics, kLocateThreads, 0, s, d);
 }
 
 // The prefix tables, and 8 words a lane for the rings: CTAs of 8 warps fill an
@@ -1549,22 +1559,21 @@ static size_t entropy_smem_bytes(int warps_per_block) { return 2 * 2 * kBookTabl
 
 cudaError_t launch_entropy(const DecodeLaunch &d, const EntropyShape &shape, cudaStream_t s) {
     if (d.n_slices == 0) return cudaSuccess;
-    k_entropy<<<shape.grid, 32 * shape.warps_per_block, entropy_smem_bytes(shape.warps_per_block), s>>>(d);
-    return cudaGetLastError();
+    return launch_chained(k_entropy, shape.grid, 32 * shape.warps_per_block, entropy_smem_bytes(shape.warps_per_block),
+                          s, d);
 }
 
 static size_t idct_smem_bytes() { return kIdctWarps * sizeof(IdctWarp); }
 
 cudaError_t launch_idct(const DecodeLaunch &d, cudaStream_t s) {
     if (d.n_idct_items == 0) return cudaSuccess;
-    k_idct<<<(d.n_idct_items + kIdctWarps - 1) / kIdctWarps, 32 * kIdctWarps, idct_smem_bytes(), s>>>(d);
-    return cudaGetLastError();
+    return launch_chained(k_idct, (d.n_idct_items + kIdctWarps - 1) / kIdctWarps, 32 * kIdctWarps, idct_smem_bytes(),
+                          s, d);
 }
 
 cudaError_t launch_status(const DecodeLaunch &d, cudaStream_t s) {
     if (d.n_pics == 0) return cudaSuccess;
-    k_status<<<d.n_pics, kStatusThreads, 0, s>>>(d);
-    return cudaGetLastError();
+    return launch_chained(k_status, d.n_pics, kStatusThreads, 0, s, d);
 }
 
 size_t decode_smem_bytes(uint32_t group, uint32_t group_positions, uint32_t slot_bytes) {
@@ -1594,11 +1603,8 @@ cudaError_t launch_decode(const DecodeLaunch &d, int grid, cudaStream_t s) {
         return cudaErrorInvalidValue;
     const uint32_t groups = (d.n_slices + d.group - 1u) / d.group;
     const int g = grid > 0 && (uint32_t)grid < groups ? grid : (int)groups;
-    if (d.slot_bytes == 1)
-        k_decode<int8_t><<<g, kDecodeThreads, smem, s>>>(d);
-    else
-        k_decode<int16_t><<<g, kDecodeThreads, smem, s>>>(d);
-    return cudaGetLastError();
+    return d.slot_bytes == 1 ? launch_chained(k_decode<int8_t>, g, kDecodeThreads, smem, s, d)
+                             : launch_chained(k_decode<int16_t>, g, kDecodeThreads, smem, s, d);
 }
 
 cudaError_t configure_decode_kernels() {

@@ -35,6 +35,7 @@
 
 #include <cstdint>
 
+#include "chain.h"
 #include "codec_tables.h"
 #include "encode_types.h"
 #include "pair_math.h"
@@ -137,6 +138,8 @@ struct FdctWarp {
 };
 
 __global__ void __launch_bounds__(32 * kFdctWarps, 6) k_fdct(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     FdctWarp &w = reinterpret_cast<FdctWarp *>(smem)[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
@@ -339,6 +342,8 @@ __device__ __forceinline__ uint32_t alpha_run_bits(const AlphaScratch &sc, uint3
 }
 
 __global__ void __launch_bounds__(32 * kAlphaWarps) k_alpha_size(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     __shared__ AlphaScratch scratch[kAlphaWarps];
     const uint32_t s = blockIdx.x * kAlphaWarps + (threadIdx.x >> 5);
     if (s >= e.n_slices) return;
@@ -933,9 +938,11 @@ constexpr uint32_t kCostTake = 4;   // items a warp of k_cost takes at once, at 
 // time: its lanes look the items' places up side by side, so the chain of
 // descriptor loads is waited for once, and the items are costed in turn.
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost(EncodeLaunch e, int step, uint32_t take) {
+    chain_start();
     __shared__ __align__(16) CountTables t;
     __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     t.fill();
+    chain_wait();
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t items = 3u * e.n_slices;
@@ -1030,6 +1037,8 @@ __device__ __forceinline__ const uint32_t *level_comp(const EncodeLaunch &e, con
 // can come to (the crate's prefetch rule, src/encode.rs:741-767). The list
 // order is the atomics' and steers nothing but speed.
 __global__ void __launch_bounds__(kCostThreads) k_window_select(EncodeLaunch e, int level) {
+    chain_start();
+    chain_wait();
     const uint32_t s = blockIdx.x * kCostThreads + threadIdx.x;
     const int lane = threadIdx.x & 31;
     bool take = false;
@@ -1072,6 +1081,8 @@ __global__ void __launch_bounds__(kCostThreads) k_window_select(EncodeLaunch e, 
 // Costs the listed slices at window level `level` (quantiser uniform - 1 -
 // level), a warp per (slice, component).
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_window(EncodeLaunch e, int level) {
+    chain_start();
+    chain_wait();
     __shared__ __align__(16) CountTables t;
     __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     const uint32_t items = 3u * e.win_count[level], stride = gridDim.x * (kCostThreads / 32);
@@ -1116,9 +1127,11 @@ constexpr uint32_t kTailSlices = 16;  // a picture's tail: slices within this ma
 constexpr uint32_t kTailLevels = 4;
 
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_deep(EncodeLaunch e) {
+    chain_start();
     __shared__ __align__(16) CountTables t;
     __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     t.fill();
+    chain_wait();
     __syncthreads();
     const uint32_t s = blockIdx.x * (kCostThreads / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -1197,6 +1210,8 @@ __device__ __forceinline__ uint64_t block_sum_u64(uint64_t v, uint64_t *sh) {
 }
 
 __global__ void __launch_bounds__(kRcThreads) k_rc_init(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     __shared__ uint64_t sh[kRcThreads / 32];
     const EncPicDesc pd = e.pics[blockIdx.x];
     uint64_t a = 0;
@@ -1227,6 +1242,8 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_init(EncodeLaunch e) {
 }
 
 __global__ void __launch_bounds__(kRcThreads) k_rc_step(EncodeLaunch e, int step) {
+    chain_start();
+    chain_wait();
     __shared__ uint64_t sh[kRcThreads / 32];
     __shared__ int all_fit;
     const EncPicDesc pd = e.pics[blockIdx.x];
@@ -1298,6 +1315,8 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_step(EncodeLaunch e, int step
 constexpr uint32_t kDeepFlag = 0x80000000u;  // share_steps: sizes are in final_comp already
 
 __global__ void k_share_prep(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= e.n_slices) return;
     const EncSliceDesc sd = e.slices[s];
@@ -1420,6 +1439,7 @@ constexpr int kShareWarps = 1;
 constexpr uint32_t kShareLadderBytes = 32u * kDeepLevels * sizeof(uint2) + 32u * (kWindow + kDeepLevels) * sizeof(uint64_t);
 
 __global__ void __launch_bounds__(32 * kShareWarps) k_shareout(EncodeLaunch e) {
+    chain_start();
     __shared__ __align__(16) CountTables t;
     __shared__ __align__(8) uint32_t buf[kShareWarps][kCountWords];
     // The slice a deep step costs, copied in once (its coefficients, then
@@ -1436,6 +1456,7 @@ __global__ void __launch_bounds__(32 * kShareWarps) k_shareout(EncodeLaunch e) {
     uint64_t *const tables = reinterpret_cast<uint64_t *>(ladders_all + kShareWarps * 32u * kDeepLevels) +
                              (threadIdx.x >> 5) * (32u * (kWindow + kDeepLevels));
     t.fill();
+    chain_wait();
     __syncthreads();
     const uint32_t p = blockIdx.x * kShareWarps + (threadIdx.x >> 5);
     if (p >= e.n_pics) return;
@@ -1582,6 +1603,8 @@ __global__ void __launch_bounds__(32 * kShareWarps) k_shareout(EncodeLaunch e) {
 }
 
 __global__ void k_share_final(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= e.n_slices) return;
     const EncSliceDesc sd = e.slices[s];
@@ -1623,6 +1646,8 @@ __device__ __forceinline__ uint64_t warp_incl_scan64(uint64_t v) {
 // Slice offsets within the picture (after its header and table) and the
 // picture's size (src/encode.rs:820-829).
 __global__ void __launch_bounds__(kLayoutThreads) k_layout(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     __shared__ uint64_t warp_sums[kLayoutThreads / 32];
     __shared__ uint64_t carry;
     const EncPicDesc pd = e.pics[blockIdx.x];
@@ -1655,6 +1680,8 @@ __global__ void __launch_bounds__(kLayoutThreads) k_layout(EncodeLaunch e) {
 // Picture places and sizes, the frame header and frame_size, the picture
 // headers (src/header.rs:174-199, :292-304). One thread per frame.
 __global__ void k_frame(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= e.n_frames) return;
     const EncFrameDesc fd = e.frames[f];
@@ -1961,10 +1988,12 @@ __device__ __noinline__ void lane_component_write(uint32_t *out, uint64_t at, co
 // whose codes were OR-ed into memory one by one, goes through the same words:
 // 8 UHD 4:4:4 frames with it 1595 -> 814.
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_pack(EncodeLaunch e, uint32_t take) {
+    chain_start();
     __shared__ __align__(16) PackTables t;
     __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
     __shared__ uint32_t words[kCostThreads / 32][kPackWords];
     t.fill();
+    chain_wait();
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t items = 3u * e.n_slices, stride = gridDim.x * (kCostThreads / 32) * take;
@@ -2069,6 +2098,8 @@ __device__ void alpha_write(const EncodeLaunch &e, const EncSliceDesc &sd, const
 // Slice headers and table entries, one thread per slice; alpha codes, one
 // warp per slice.
 __global__ void k_pack_headers(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= e.n_slices) return;
     const EncSliceDesc sd = e.slices[s];
@@ -2093,6 +2124,8 @@ __global__ void k_pack_headers(EncodeLaunch e) {
 }
 
 __global__ void __launch_bounds__(32 * kAlphaWarps) k_pack_alpha(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
     __shared__ AlphaScratch scratch[kAlphaWarps];
     __shared__ uint32_t words[kAlphaWarps][kPackWords];
     const uint32_t s = blockIdx.x * kAlphaWarps + (threadIdx.x >> 5);
@@ -2116,21 +2149,19 @@ cudaError_t launch_quant(float *quant, const uint8_t *keys, uint32_t sets, cudaS
 
 cudaError_t launch_fdct(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
-    k_fdct<<<(e.n_fdct_items + kFdctWarps - 1) / kFdctWarps, 32 * kFdctWarps, kFdctWarps * sizeof(FdctWarp), s>>>(e);
-    return cudaGetLastError();
+    return launch_chained(k_fdct, (e.n_fdct_items + kFdctWarps - 1) / kFdctWarps, 32 * kFdctWarps,
+                          kFdctWarps * sizeof(FdctWarp), s, e);
 }
 
 cudaError_t launch_alpha_size(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
     if (!e.any_alpha) return cudaMemsetAsync(e.alpha_bytes, 0, 4ull * e.n_slices, s);
-    k_alpha_size<<<(e.n_slices + kAlphaWarps - 1) / kAlphaWarps, 32 * kAlphaWarps, 0, s>>>(e);
-    return cudaGetLastError();
+    return launch_chained(k_alpha_size, (e.n_slices + kAlphaWarps - 1) / kAlphaWarps, 32 * kAlphaWarps, 0, s, e);
 }
 
 cudaError_t launch_rc_init(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_pics) return cudaSuccess;
-    k_rc_init<<<e.n_pics, kRcThreads, 0, s>>>(e);
-    return cudaGetLastError();
+    return launch_chained(k_rc_init, e.n_pics, kRcThreads, 0, s, e);
 }
 
 // CTAs of a kernel that walks `items` warp items at a stride: all that are
@@ -2150,62 +2181,54 @@ static uint32_t cost_take(const EncodeLaunch &e, uint32_t items) {
 cudaError_t launch_cost(const EncodeLaunch &e, int step, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
     const uint32_t items = 3u * e.n_slices;
-    k_cost<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, step, cost_take(e, items));
-    return cudaGetLastError();
+    return launch_chained(k_cost, cost_grid(e, items), kCostThreads, 0, s, e, step, cost_take(e, items));
 }
 
 cudaError_t launch_rc_step(const EncodeLaunch &e, int step, cudaStream_t s) {
     if (!e.n_pics) return cudaSuccess;
-    k_rc_step<<<e.n_pics, kRcThreads, 0, s>>>(e, step);
-    return cudaGetLastError();
+    return launch_chained(k_rc_step, e.n_pics, kRcThreads, 0, s, e, step);
 }
 
 cudaError_t launch_cost_window(const EncodeLaunch &e, int level, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
     const uint32_t items = 3u * e.n_slices;
-    k_window_select<<<(e.n_slices + kCostThreads - 1) / kCostThreads, kCostThreads, 0, s>>>(e, level);
-    cudaError_t err = cudaGetLastError();
+    cudaError_t err =
+        launch_chained(k_window_select, (e.n_slices + kCostThreads - 1) / kCostThreads, kCostThreads, 0, s, e, level);
     if (err != cudaSuccess) return err;
     // Blocks past the list's end return.
-    k_cost_window<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, level);
-    return cudaGetLastError();
+    return launch_chained(k_cost_window, cost_grid(e, items), kCostThreads, 0, s, e, level);
 }
 
 cudaError_t launch_cost_deep(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
-    k_cost_deep<<<(e.n_slices + kCostThreads / 32 - 1) / (kCostThreads / 32), kCostThreads, 0, s>>>(e);
-    return cudaGetLastError();
+    return launch_chained(k_cost_deep, (e.n_slices + kCostThreads / 32 - 1) / (kCostThreads / 32), kCostThreads, 0, s,
+                          e);
 }
 
 cudaError_t launch_shareout(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_pics) return cudaSuccess;
-    k_share_prep<<<(e.n_slices + 255) / 256, 256, 0, s>>>(e);
-    cudaError_t err = cudaGetLastError();
+    cudaError_t err = launch_chained(k_share_prep, (e.n_slices + 255) / 256, 256, 0, s, e);
     if (err != cudaSuccess) return err;
-    k_shareout<<<(e.n_pics + kShareWarps - 1) / kShareWarps, 32 * kShareWarps, kShareWarps * kShareLadderBytes, s>>>(e);
-    if ((err = cudaGetLastError()) != cudaSuccess) return err;
-    k_share_final<<<(e.n_slices + 255) / 256, 256, 0, s>>>(e);
-    return cudaGetLastError();
+    err = launch_chained(k_shareout, (e.n_pics + kShareWarps - 1) / kShareWarps, 32 * kShareWarps,
+                         kShareWarps * kShareLadderBytes, s, e);
+    if (err != cudaSuccess) return err;
+    return launch_chained(k_share_final, (e.n_slices + 255) / 256, 256, 0, s, e);
 }
 
 cudaError_t launch_layout(const EncodeLaunch &e, cudaStream_t s) {
-    if (e.n_pics) k_layout<<<e.n_pics, kLayoutThreads, 0, s>>>(e);
-    cudaError_t err = cudaGetLastError();
+    cudaError_t err = e.n_pics ? launch_chained(k_layout, e.n_pics, kLayoutThreads, 0, s, e) : cudaSuccess;
     if (err != cudaSuccess || !e.n_frames) return err;
-    k_frame<<<(e.n_frames + 127) / 128, 128, 0, s>>>(e);
-    return cudaGetLastError();
+    return launch_chained(k_frame, (e.n_frames + 127) / 128, 128, 0, s, e);
 }
 
 cudaError_t launch_pack(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
     const uint32_t items = 3u * e.n_slices;
-    k_pack<<<cost_grid(e, items), kCostThreads, 0, s>>>(e, cost_take(e, items));
-    cudaError_t err = cudaGetLastError();
+    cudaError_t err = launch_chained(k_pack, cost_grid(e, items), kCostThreads, 0, s, e, cost_take(e, items));
     if (err != cudaSuccess) return err;
-    k_pack_headers<<<(e.n_slices + 255) / 256, 256, 0, s>>>(e);
-    if ((err = cudaGetLastError()) != cudaSuccess || !e.any_alpha) return err;
-    k_pack_alpha<<<(e.n_slices + kAlphaWarps - 1) / kAlphaWarps, 32 * kAlphaWarps, 0, s>>>(e);
-    return cudaGetLastError();
+    err = launch_chained(k_pack_headers, (e.n_slices + 255) / 256, 256, 0, s, e);
+    if (err != cudaSuccess || !e.any_alpha) return err;
+    return launch_chained(k_pack_alpha, (e.n_slices + kAlphaWarps - 1) / kAlphaWarps, 32 * kAlphaWarps, 0, s, e);
 }
 
 cudaError_t configure_encode_kernels() {
