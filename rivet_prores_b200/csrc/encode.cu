@@ -1307,10 +1307,9 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_step(EncodeLaunch e, int step
 //                  level, the threshold on D and the size over the base;
 //   k_shareout     one warp per picture, the only serial part: D against
 //                  the thresholds (the window's, then each slice's deep
-//                  ladder from k_cost_deep), 32 slices at a time by ballot,
-//                  each stepping slice settled by its own lane; the warp
-//                  costs a deeper quantiser together when a slice gets past
-//                  all of them;
+//                  ladder from k_cost_deep), 32 slices at a time, their
+//                  thresholds copied ahead; where a slice gets past all of
+//                  them, the block's other warps cost the next quantisers;
 //   k_share_final  every slice in parallel: its quantiser and sizes.
 constexpr uint32_t kDeepFlag = 0x80000000u;  // share_steps: sizes are in final_comp already
 
@@ -1334,81 +1333,62 @@ __global__ void k_share_prep(EncodeLaunch e) {
         pr.base = (uint32_t)base;
         pr.hba = hb + alpha;
         pr.rem = (uint32_t)rem;
-        pr.shift = shift;
-        pr.deep_count = e.deep_count[s];
+        pr.shift = (uint8_t)shift;
+        uint64_t run = 0;
+        uint32_t levels = 0;  // the walk's levels before it stops whatever D is
+        bool stopped = false;
 #pragma unroll
         for (int j = 0; j < kWindow; j++) {
+            const bool more = st.uniform - j > 1;
+            const uint32_t *c = more ? level_comp(e, st, (uint32_t)j, s) : nullptr;
+            const bool known = more && c[0] != kNotCosted;
+            if (!stopped && more && !known) pr.uncosted_at_end = 1;
+            stopped = stopped || !known;
             pr.thr[j] = ~0ull;
-            if (st.uniform - j <= 1) continue;
-            const uint32_t *c = level_comp(e, st, (uint32_t)j, s);
-            if (c[0] == kNotCosted) continue;  // unknown: the walk costs it if reached
+            if (stopped) continue;
             const uint32_t cc[3] = {c[0], c[1], c[2]};
             bool fits;
             const uint64_t n = slice_total(hb, cc, alpha, fits);
-            pr.known |= 1u << j;
+            const uint64_t thr = !fits ? ~0ull : n <= base ? 0ull : ((((n - base) * rem) + sd.mbs - 1) >> shift);
+            run = run > thr ? run : thr;
+            pr.thr[j] = run;
             pr.delta[j] = (int32_t)((int64_t)n - (int64_t)base);
-            if (fits) pr.thr[j] = n <= base ? 0ull : ((((n - base) * rem) + sd.mbs - 1) >> shift);
+            levels++;
         }
+        if (!stopped) {
+            pr.deep_count = (uint8_t)min(e.deep_count[s], (uint32_t)(st.uniform - 1 - kWindow));
+            levels += pr.deep_count;
+            pr.uncosted_at_end = st.uniform - (int32_t)levels > 1;
+        }
+        pr.levels = (uint8_t)levels;
     }
     e.share_prep[s] = pr;
 }
 
 // A level past the window from a slice's deep ladder: its size, and whether
 // it fits.
-__device__ __forceinline__ uint64_t deep_size(const SharePrep &p, uint2 v, bool &fits) {
+__device__ __forceinline__ uint32_t deep_size(const SharePrep &p, uint2 v, bool &fits) {
     fits = (v.y >> 16) != 0;
-    return (uint64_t)p.hba + (v.x & 0xFFFFu) + (v.x >> 16) + (v.y & 0xFFFFu);
+    return p.hba + (v.x & 0xFFFFu) + (v.x >> 16) + (v.y & 0xFFFFu);
 }
 
-// The steps a slice takes at D through its known levels (the walk of
-// src/encode.rs:776-788 while the sizes are known: the window's, then its
-// deep ladder, level j at deep[32 j]), as a table the share-out searches
-// each time it settles the slice: at [32 k] the least D that lets the
-// slice take k + 1 steps given that it took k (~0 where the level does not
-// fit), made non-decreasing (a running maximum), so that the steps at D are
-// the number of entries <= D; `len` is where the walk stops whatever D is,
-// and `deep_at_end` whether it then needs a level nobody costed.
-__device__ __forceinline__ void steps_table(const SharePrep &p, const uint2 *deep, int32_t uniform, uint64_t *tab,
-                                            uint32_t &len, bool &deep_at_end) {
-    uint64_t run = 0;
-    uint32_t k = 0;
-    deep_at_end = false;
-#pragma unroll
-    for (int j = 0; j < kWindow; j++) {
-        // k == j steps so far: the quantiser is uniform - j.
-        if (uniform - j <= 1) {
-            len = k;
-            return;
-        }
-        if (!((p.known >> j) & 1u)) {
-            len = k;
-            deep_at_end = true;
-            return;
-        }
-        run = max(run, p.thr[j]);
-        tab[32u * k] = run;
-        k++;
-    }
+// A slice's deep levels (level j at deep[32 j]) continuing SharePrep::thr:
+// tab[32 j] the least D that lets the slice take kWindow + 1 + j steps.
+__device__ __forceinline__ void deep_table(const SharePrep &p, const uint2 *deep, uint64_t *tab) {
+    uint64_t run = p.thr[kWindow - 1];
+#pragma unroll 4
     for (uint32_t j = 0; j < p.deep_count; j++) {
-        if (uniform - (int32_t)k <= 1) {
-            len = k;
-            return;
-        }
         bool fits;
-        const uint64_t n = deep_size(p, deep[32u * j], fits);
-        const uint64_t thr =
-            !fits ? ~0ull : (n <= p.base ? 0ull : (((n - p.base) * p.rem) + (1u << p.shift) - 1u) >> p.shift);
+        const uint32_t n = deep_size(p, deep[32u * j], fits);
+        const uint64_t over = n <= p.base ? 0u : n - p.base;
+        const uint64_t thr = fits ? (over * p.rem + (1u << p.shift) - 1u) >> p.shift : ~(uint64_t)0;
         run = max(run, thr);
-        tab[32u * k] = run;
-        k++;
+        tab[32u * j] = run;
     }
-    len = k;
-    deep_at_end = uniform - (int32_t)k > 1;
 }
 
-// The steps at D from steps_table(): a binary search.
-__device__ __forceinline__ uint32_t steps_from(const uint64_t *tab, uint32_t len, bool deep_at_end, uint64_t D,
-                                               bool &deep_needed) {
+// The deep levels that D lets the slice take: a binary search.
+__device__ __forceinline__ uint32_t deep_steps(const uint64_t *tab, uint32_t len, uint64_t D) {
     uint32_t lo = 0, hi = len;
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
@@ -1417,189 +1397,286 @@ __device__ __forceinline__ uint32_t steps_from(const uint64_t *tab, uint32_t len
         else
             hi = mid;
     }
-    deep_needed = lo == len && deep_at_end;
     return lo;
 }
 
-// The size over the base after `ks` steps (ks >= 1).
-__device__ __forceinline__ int64_t delta_at(const SharePrep &p, const uint2 *deep, uint32_t ks) {
-    if (ks <= (uint32_t)kWindow) {
-        int32_t d = p.delta[0];
-#pragma unroll
-        for (int j = 1; j < kWindow; j++)
-            if ((uint32_t)j + 1u == ks) d = p.delta[j];
-        return d;
+// Quantisers costed at a time for a slice that needs one nobody costed, and
+// the warps that do, one per component and quantiser (32 frames of mixed
+// sizes: 686, 603 and 551 us with 1, 2 and 4; the others have none).
+constexpr int kShareTries = 4;
+constexpr int kShareHelpers = 3 * kShareTries;
+constexpr int kShareThreads = 32 * (1 + kShareHelpers);
+
+// What k_shareout's first warp asks the others for, and their answer.
+struct ShareJob {
+    uint64_t D;
+    uint32_t slice;  // ~0: no more
+    uint32_t steps;  // taken so far; with kDeepFlag once sizes are in final_comp
+    int32_t delta;   // the size over the base after them
+    uint32_t base;
+};
+
+struct ShareShared {
+    CountTables t;
+    // The slice being costed, copied in once (its coefficients, then its
+    // chunk maxima): the warps walk it for every quantiser they try.
+    __align__(16) float stage[kMaxSliceCoefs + kMaxSliceCoefs / 32];
+    __align__(8) uint32_t buf[kShareHelpers][kCountWords];
+    uint32_t sizes[2][kShareTries][3];
+    ShareJob job;
+    // Per lane, of the 32 slices being settled and of the next ones: their
+    // thresholds (16-byte words, of two chunks ahead), their ladders (of one
+    // ahead), and the deep levels' table.
+    uint4 prep[3][sizeof(SharePrep) / sizeof(uint4)][32];
+    uint2 ladder[2][kDeepLevels][32];
+    uint64_t table[kDeepLevels][32];
+};
+
+__device__ __forceinline__ void copy8_async(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy16_async(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Barriers of k_shareout: a job is posted / its answer is (all threads); the
+// helpers among themselves.
+__device__ __forceinline__ void share_barrier(int id, int threads) {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+constexpr int kJobPosted = 1, kJobDone = 2, kHelpersOnly = 3;
+
+// A helper warp: costs one component of the slice at one of the kShareTries
+// next finer quantisers, until the slice no longer fits its allowance (fixed
+// during the slice's walk).
+__device__ void share_help(const EncodeLaunch &e, const EncPicDesc &pd, int32_t uniform, ShareShared &sh) {
+    const uint32_t h = (threadIdx.x >> 5) - 1u, lane = threadIdx.x & 31u;
+    const uint32_t c = h % 3u, ahead = h / 3u, tid = threadIdx.x - 32u;
+    const EncFrameDesc &fd = e.frames[pd.frame];
+    for (;;) {
+        share_barrier(kJobPosted, kShareThreads);
+        const ShareJob job = sh.job;
+        if (job.slice == ~0u) return;
+        const uint32_t s = job.slice;
+        const EncSliceDesc sd = e.slices[s];
+        const uint32_t alpha = e.alpha_bytes[s];
+        const uint32_t cpm = fd.chroma == 2 ? 2u : 4u;
+        const uint32_t total = 64u * (4u + 2u * cpm) * sd.mbs;
+        float *const smax = sh.stage + kMaxSliceCoefs;
+        for (uint32_t i = tid; i < total / 4u; i += 32u * kShareHelpers)
+            copy16_async(sh.stage + 4u * i, e.coef + sd.coef + 4u * i);
+        const float *msrc = e.coef_max + (sd.coef >> 5);
+        for (uint32_t i = tid; i < total / 32u; i += 32u * kShareHelpers) smax[i] = __ldg(msrc + i);
+        const uint64_t allowed = job.base + job.D * sd.mbs / mbs_from(pd, sd);
+        copies_wait();
+        share_barrier(kHelpersOnly, 32 * kShareHelpers);
+        uint32_t nb, off;
+        comp_layout(fd, sd.mbs, c, nb, off);
+        const float *f = sh.stage + off;
+        const CompHead head = comp_head<true>(f, smax + (off >> 5), nb);
+        uint32_t steps = job.steps, c3[3] = {0, 0, 0};
+        int32_t delta = job.delta, qi = uniform - (int32_t)job.steps;
+        bool any = false, more = qi > 1;
+        for (uint32_t turn = 0; more; turn ^= 1u) {
+            const int32_t mine = qi - 1 - (int32_t)ahead;
+            if (mine >= 1) {
+                const CompQuant q = comp_quant(quant_base(e, pd, (uint32_t)mine), c, nb);
+                const uint32_t bits = warp_component_bits<true>(f, head, nb, q, sh.t, sh.buf[h]);
+                if (lane == 0) sh.sizes[turn][ahead][c] = (bits + 7u) / 8u;
+            }
+            share_barrier(kHelpersOnly, 32 * kShareHelpers);
+            for (int a = 0; more && a < kShareTries; a++) {
+                const uint32_t n3[3] = {sh.sizes[turn][a][0], sh.sizes[turn][a][1], sh.sizes[turn][a][2]};
+                bool fits;
+                const uint64_t n = slice_total(pd.header_bytes, n3, alpha, fits);
+                if (!(fits && n <= allowed)) {
+                    more = false;
+                    break;
+                }
+                qi -= 1;
+                steps++;
+                delta = (int32_t)n - (int32_t)job.base;
+                c3[0] = n3[0];
+                c3[1] = n3[1];
+                c3[2] = n3[2];
+                any = true;
+                more = qi > 1;
+            }
+        }
+        if (tid == 0) {
+            if (any) {
+                e.final_comp[3ull * s] = c3[0];
+                e.final_comp[3ull * s + 1] = c3[1];
+                e.final_comp[3ull * s + 2] = c3[2];
+                steps |= kDeepFlag;
+            }
+            sh.job.steps = steps;
+            sh.job.delta = delta;
+        }
+        share_barrier(kJobDone, kShareThreads);
     }
-    bool fits;
-    return (int64_t)deep_size(p, deep[32u * (ks - 1u - kWindow)], fits) - (int64_t)p.base;
 }
 
-constexpr int kShareWarps = 1;
-// A warp's staged ladders and steps tables.
-constexpr uint32_t kShareLadderBytes = 32u * kDeepLevels * sizeof(uint2) + 32u * (kWindow + kDeepLevels) * sizeof(uint64_t);
-
-__global__ void __launch_bounds__(32 * kShareWarps) k_shareout(EncodeLaunch e) {
-    chain_start();
-    __shared__ __align__(16) CountTables t;
-    __shared__ __align__(8) uint32_t buf[kShareWarps][kCountWords];
-    // The slice a deep step costs, copied in once (its coefficients, then
-    // its chunk maxima): the warp walks it for every quantiser it tries,
-    // and from DRAM each of its chunks waited out a full load.
-    __shared__ __align__(16) float stage[kShareWarps][kMaxSliceCoefs + kMaxSliceCoefs / 32];
-    // The ladders of the 32 slices a warp settles, level j of lane l at
-    // [32 j + l] (dynamic shared memory, kShareLadderBytes a warp): the
-    // settling rounds walk them again and again, and from global memory
-    // every level of the walk was a dependent load.
-    extern __shared__ uint2 ladders_all[];
-    uint2 *const ladders = ladders_all + (threadIdx.x >> 5) * (32u * kDeepLevels);
-    // Each lane's steps_table(), [32 k + lane], after all warps' ladders.
-    uint64_t *const tables = reinterpret_cast<uint64_t *>(ladders_all + kShareWarps * 32u * kDeepLevels) +
-                             (threadIdx.x >> 5) * (32u * (kWindow + kDeepLevels));
-    t.fill();
-    chain_wait();
-    __syncthreads();
-    const uint32_t p = blockIdx.x * kShareWarps + (threadIdx.x >> 5);
-    if (p >= e.n_pics) return;
+// The settling warp: 32 slices at a time.
+__device__ void share_settle(const EncodeLaunch &e, const EncPicDesc &pd, uint64_t D, ShareShared &sh) {
     const int lane = threadIdx.x & 31;
-    const EncPicDesc pd = e.pics[p];
-    const EncPicState st = e.state[p];
-    const bool refine = st.uniform > 1 && st.fits_at_all;
-    if (!refine) {
-        for (uint32_t k = lane; k < pd.n_slices; k += 32) e.share_steps[pd.slice_base + k] = 0;
-        return;
-    }
-    const EncFrameDesc &fd = e.frames[pd.frame];
-    const uint32_t hb = pd.header_bytes;
-    uint64_t D = st.budget - st.hi_total;
-    SharePrep next{};
-    if ((uint32_t)lane < pd.n_slices) next = e.share_prep[pd.slice_base + lane];
+    constexpr uint32_t kPrepWords = sizeof(SharePrep) / sizeof(uint4);
+    // What the next chunks need is copied to shared memory while one is
+    // settled, a lane's slice by the lane, which alone reads it.
+    const auto fetch_prep = [&](uint32_t k0, uint32_t slot) {
+        if (k0 + lane >= pd.n_slices) return;
+        const uint4 *src = reinterpret_cast<const uint4 *>(e.share_prep + pd.slice_base + k0 + lane);
+#pragma unroll
+        for (uint32_t w = 0; w < kPrepWords; w++) copy16_async(&sh.prep[slot][w][lane], src + w);
+    };
+    const auto load_prep = [&](uint32_t slot) {
+        union {
+            SharePrep p;
+            uint4 w[kPrepWords];
+        } u;
+#pragma unroll
+        for (uint32_t w = 0; w < kPrepWords; w++) u.w[w] = sh.prep[slot][w][lane];
+        return u.p;
+    };
+    const auto fetch_ladder = [&](uint32_t k0, uint32_t slot, uint32_t half) {
+        if (k0 + lane >= pd.n_slices) return;
+        const uint32_t count = load_prep(slot).deep_count;
+        const uint2 *src = e.deep + (uint64_t)(pd.slice_base + k0 + lane) * kDeepLevels;
+#pragma unroll 4
+        for (uint32_t j = 0; j < count; j++) copy8_async(&sh.ladder[half][j][lane], src + j);
+    };
+    fetch_prep(0, 0);
+    copies_wait();
+    fetch_prep(32, 1);
+    fetch_ladder(0, 0, 0);
+    uint32_t slot = 0, half = 0;
     for (uint32_t k0 = 0; k0 < pd.n_slices; k0 += 32) {
-        const SharePrep mine = next;
         const uint32_t k = k0 + lane;
         const bool live = k < pd.n_slices;
-        uint2 *my_deep = ladders + lane;
-        __syncwarp();  // the last chunk's walks are over
+        copies_wait();
+        const uint32_t slot1 = slot == 2u ? 0u : slot + 1u, slot2 = slot1 == 2u ? 0u : slot1 + 1u;
+        fetch_prep(k0 + 64, slot2);
+        fetch_ladder(k0 + 32, slot1, half ^ 1u);
+        // Past the picture's end: no level, at any D.
+        SharePrep mine{};
         if (live) {
-            const uint2 *src = e.deep + (uint64_t)(pd.slice_base + k) * kDeepLevels;
-#pragma unroll 4
-            for (uint32_t j = 0; j < mine.deep_count; j++) my_deep[32u * j] = src[j];
+            mine = load_prep(slot);
+        } else {
+#pragma unroll
+            for (int j = 0; j < kWindow; j++) mine.thr[j] = ~0ull;
         }
-        uint32_t my_len = 0;
-        bool my_deep_at_end = false;
-        if (live) steps_table(mine, my_deep, st.uniform, tables + lane, my_len, my_deep_at_end);
-        __syncwarp();
-        // The next chunk's thresholds, fetched while this chunk is walked.
-        if (k + 32 < pd.n_slices) next = e.share_prep[pd.slice_base + k + 32];
+        const uint2 *my_deep = &sh.ladder[half][0][lane];
+        uint64_t *my_table = &sh.table[0][lane];
+        bool table_built = false;
         uint32_t my_steps = 0;
         uint32_t done = 0;  // lanes below are settled
         while (done < 32u) {
             // The walk is sequential: a slice's slack D is what the slices
-            // before it left. Each lane guesses its D, takes its steps there,
-            // and the guesses are redone from the exclusive sum of the steps'
-            // size changes until none moves. A lane's D depends only on the
-            // lanes before it, so after t rounds the first t lanes are exact
-            // and the fixed point reached (at most 33 rounds) is the
-            // sequential walk's. Lanes from the first one that needs a level
-            // nobody costed (`deep`) on wait for the warp to cost it.
+            // before it left. Each lane guesses its D and takes its steps
+            // there; the guesses are redone from the exclusive sum of the
+            // steps' size changes until no lane's steps change. A lane's D
+            // depends only on the lanes before it, so after t rounds the
+            // first t lanes are exact and the fixed point reached (at most 33
+            // rounds) is the sequential walk's. The first lane that needs a
+            // level nobody costed, and those after it, wait for the helpers
+            // to cost it.
             uint64_t myD = D;
-            uint32_t ks = 0;
-            int64_t dl = 0;
-            uint32_t first_deep = 32;
+            uint32_t ks = 0, guessed = 0;           // the steps at myD, and those it came from
+            int32_t mine_dl = 0, before = 0;        // a size that fits is below 2^16
+            uint32_t upto_deep = 0;                 // the lanes up to the first deep one; 0: none is
             for (int round = 0; round < 34; round++) {
-                bool deep = false;
-                ks = live && (uint32_t)lane >= done ? steps_from(tables + lane, my_len, my_deep_at_end, myD, deep) : 0u;
-                const uint32_t deep_mask = __ballot_sync(0xffffffffu, live && (uint32_t)lane >= done && deep);
-                const uint32_t fd_lane = deep_mask ? (uint32_t)__ffs(deep_mask) - 1u : 32u;
-                const int64_t mine_dl = ks ? delta_at(mine, my_deep, ks) : 0;
-                dl = (uint32_t)lane < fd_lane ? mine_dl : 0;
-                // Inclusive sum of dl over the lanes.
-                int64_t incl = dl;
+                ks = 0;
+                mine_dl = 0;
+                if ((uint32_t)lane >= done) {
+#pragma unroll
+                    for (int j = 0; j < kWindow; j++) {
+                        const bool taken = mine.thr[j] <= myD;
+                        ks += taken;
+                        mine_dl = taken ? mine.delta[j] : mine_dl;
+                    }
+                }
+                const bool past = ks == (uint32_t)kWindow && mine.deep_count > 0;
+                if (__any_sync(0xffffffffu, past)) {
+                    if (!table_built) deep_table(mine, my_deep, my_table);
+                    table_built = true;
+                    const uint32_t j = past ? deep_steps(my_table, mine.deep_count, myD) : 0u;
+                    if (j) {
+                        bool fits;
+                        ks += j;
+                        mine_dl = (int32_t)(deep_size(mine, my_deep[32u * (j - 1u)], fits) - mine.base);
+                    }
+                }
+                const uint32_t deep_mask =
+                    __ballot_sync(0xffffffffu, (uint32_t)lane >= done && mine.uncosted_at_end && ks == mine.levels);
+                const uint32_t moved = __ballot_sync(0xffffffffu, ks != guessed);
+                upto_deep = deep_mask ? deep_mask ^ (deep_mask - 1u) : 0u;
+                if (!(moved & (upto_deep ? upto_deep : ~0u))) break;
+                guessed = ks;
+                // Inclusive sum over the lanes.
+                int32_t incl = mine_dl;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
-                    const int64_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                    const int32_t v = __shfl_up_sync(0xffffffffu, incl, o);
                     if (lane >= o) incl += v;
                 }
-                const uint64_t newD = (uint64_t)((int64_t)D - (incl - dl));
-                const bool moved = (uint32_t)lane >= done && (uint32_t)lane <= fd_lane && newD != myD;
-                myD = newD;
-                const bool again = __any_sync(0xffffffffu, moved) || fd_lane != first_deep;
-                first_deep = fd_lane;
-                if (!again) break;
+                before = incl - mine_dl;
+                myD = (uint64_t)((int64_t)D - before);
             }
-            // Lanes done .. first_deep - 1 are settled at myD with ks steps.
-            if ((uint32_t)lane >= done && (uint32_t)lane < first_deep) my_steps = ks;
-            const int64_t settled = __shfl_sync(0xffffffffu, (int64_t)D - (int64_t)myD, first_deep < 32u ? first_deep : 31u);
-            if (first_deep >= 32u) {
+            const uint32_t f = upto_deep ? 31u - (uint32_t)__clz(upto_deep) : 32u;
+            // Lanes done .. f - 1 are settled at myD with ks steps.
+            if ((uint32_t)lane >= done && (uint32_t)lane < f) my_steps = ks;
+            if (f == 32u) {
                 // Every lane settled: D after the chunk.
-                const int64_t total = __shfl_sync(0xffffffffu, (int64_t)D - (int64_t)myD + dl, 31);
-                D = (uint64_t)((int64_t)D - total);
+                D = (uint64_t)((int64_t)D - __shfl_sync(0xffffffffu, before + mine_dl, 31));
                 break;
             }
-            // The deep lane, at its exact D: the warp costs quantiser qi - 1
-            // and the slice steps while it fits its allowance (fixed during
-            // the slice's walk).
-            D = (uint64_t)((int64_t)D - settled);
-            const uint32_t f = first_deep;
-            const uint32_t fk = __shfl_sync(0xffffffffu, ks, f);
-            const int64_t my_delta = ks ? delta_at(mine, my_deep, ks) : 0;
-            int64_t delta = __shfl_sync(0xffffffffu, my_delta, f);
-            uint32_t steps = fk;
-            {
-                const uint32_t s = pd.slice_base + k0 + f;
-                const EncSliceDesc fsd = e.slices[s];
-                const uint32_t fbase = __shfl_sync(0xffffffffu, mine.base, f);
-                const uint32_t alpha = e.alpha_bytes[s];
-                const uint64_t allowed = fbase + D * fsd.mbs / mbs_from(pd, fsd);
-                uint32_t c3[3] = {0, 0, 0};
-                int32_t qi = st.uniform - (int32_t)fk;
-                bool any = false;
-                float *sf = stage[threadIdx.x >> 5], *smax = sf + kMaxSliceCoefs;
-                const uint32_t cpm = fd.chroma == 2 ? 2u : 4u;
-                const uint32_t total = 64u * (4u + 2u * cpm) * fsd.mbs;
-                if (qi > 1) {
-                    __syncwarp();  // the last deep slice's walks are over
-                    const float4 *src = reinterpret_cast<const float4 *>(e.coef + fsd.coef);
-#pragma unroll 4
-                    for (uint32_t i = (uint32_t)lane; i < total / 4u; i += 32u)
-                        reinterpret_cast<float4 *>(sf)[i] = __ldg(src + i);
-                    const float *msrc = e.coef_max + (fsd.coef >> 5);
-                    for (uint32_t i = (uint32_t)lane; i < total / 32u; i += 32u) smax[i] = __ldg(msrc + i);
-                    __syncwarp();
-                }
-                while (qi > 1) {
-                    uint32_t n3[3];
-                    for (uint32_t c = 0; c < 3; c++) {
-                        uint32_t nb, off;
-                        comp_layout(fd, fsd.mbs, c, nb, off);
-                        const CompQuant q = comp_quant(quant_base(e, pd, (uint32_t)(qi - 1)), c, nb);
-                        const CompHead h = comp_head<true>(sf + off, smax + (off >> 5), nb);
-                        n3[c] = (warp_component_bits<true>(sf + off, h, nb, q, t, buf[threadIdx.x >> 5]) + 7u) / 8u;
-                    }
-                    bool fits;
-                    const uint64_t n = slice_total(hb, n3, alpha, fits);
-                    if (!(fits && n <= allowed)) break;
-                    qi -= 1;
-                    steps++;
-                    delta = (int64_t)n - (int64_t)fbase;
-                    c3[0] = n3[0];
-                    c3[1] = n3[1];
-                    c3[2] = n3[2];
-                    any = true;
-                }
-                if (any && lane == 0) {
-                    e.final_comp[3ull * s] = c3[0];
-                    e.final_comp[3ull * s + 1] = c3[1];
-                    e.final_comp[3ull * s + 2] = c3[2];
-                    steps |= kDeepFlag;
-                }
-                steps = __shfl_sync(0xffffffffu, steps, 0);
-            }
-            if (lane == (int)f) my_steps = steps;
-            D = (uint64_t)((int64_t)D - delta);
+            // The deep lane, at its exact D.
+            D = (uint64_t)((int64_t)D - __shfl_sync(0xffffffffu, before, f));
+            if (lane == (int)f) sh.job = ShareJob{D, pd.slice_base + k, ks, mine_dl, mine.base};
+            share_barrier(kJobPosted, kShareThreads);
+            share_barrier(kJobDone, kShareThreads);
+            if (lane == (int)f) my_steps = sh.job.steps;
+            D = (uint64_t)((int64_t)D - sh.job.delta);
             done = f + 1;
         }
         if (live) e.share_steps[pd.slice_base + k] = my_steps;
+        slot = slot1;
+        half ^= 1u;
     }
+    if (lane == 0) sh.job.slice = ~0u;
+    share_barrier(kJobPosted, kShareThreads);
+}
+
+// A block per picture: a warp that settles its slices, and helpers. Bound by
+// the settling warp's chain: about 1170 cycles a chunk of 32 UHD slices, of
+// them 700 in its two rounds (thresholds against D, the votes, a scan), 200 to
+// start the next chunks' copies. One UHD frame 122 -> 73 us, 30 of them 152 ->
+// 85, and 32 frames of mixed sizes, whose slices often get past their ladders,
+// 1243 -> 516. Before, each round ended with a scan, also to find that nothing
+// had moved; each chunk built its lanes' whole tables first (10,000 cycles
+// where the ladders are long); and the one warp copied a slice past its ladder
+// in and costed it alone (24,000 cycles a slice, 7,000 now).
+__global__ void __launch_bounds__(kShareThreads) k_shareout(EncodeLaunch e) {
+    chain_start();
+    extern __shared__ __align__(16) uint8_t share_smem[];
+    ShareShared &sh = *reinterpret_cast<ShareShared *>(share_smem);
+    sh.t.fill();
+    chain_wait();
+    __syncthreads();
+    const EncPicDesc pd = e.pics[blockIdx.x];
+    const EncPicState st = e.state[blockIdx.x];
+    if (!(st.uniform > 1 && st.fits_at_all)) {
+        for (uint32_t k = threadIdx.x; k < pd.n_slices; k += kShareThreads) e.share_steps[pd.slice_base + k] = 0;
+        return;
+    }
+    if (threadIdx.x < 32u)
+        share_settle(e, pd, st.budget - st.hi_total, sh);
+    else
+        share_help(e, pd, st.uniform, sh);
 }
 
 __global__ void k_share_final(EncodeLaunch e) {
@@ -2209,8 +2286,7 @@ cudaError_t launch_shareout(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_pics) return cudaSuccess;
     cudaError_t err = launch_chained(k_share_prep, (e.n_slices + 255) / 256, 256, 0, s, e);
     if (err != cudaSuccess) return err;
-    err = launch_chained(k_shareout, (e.n_pics + kShareWarps - 1) / kShareWarps, 32 * kShareWarps,
-                         kShareWarps * kShareLadderBytes, s, e);
+    err = launch_chained(k_shareout, e.n_pics, kShareThreads, sizeof(ShareShared), s, e);
     if (err != cudaSuccess) return err;
     return launch_chained(k_share_final, (e.n_slices + 255) / 256, 256, 0, s, e);
 }
@@ -2234,7 +2310,7 @@ cudaError_t launch_pack(const EncodeLaunch &e, cudaStream_t s) {
 cudaError_t configure_encode_kernels() {
     static_assert(sizeof(FdctWarp) % 16 == 0, "the warps' areas are 16-byte aligned");
     cudaError_t err0 = cudaFuncSetAttribute(k_shareout, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)(kShareWarps * kShareLadderBytes));
+                                            (int)sizeof(ShareShared));
     if (err0 != cudaSuccess) return err0;
     CountTables tables;
     build_count_tables(tables);

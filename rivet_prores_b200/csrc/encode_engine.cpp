@@ -265,6 +265,7 @@ static EncodeLaunch encode_params(Context &ctx, Workspace &ws, const EncodePlan 
     o = (o + 15) & ~(size_t)15;
     e.slice_off = reinterpret_cast<uint64_t *>(base + o);
     o += 8 * ns;
+    o = (o + 15) & ~(size_t)15;
     e.share_prep = reinterpret_cast<SharePrep *>(base + o);
     o += sizeof(SharePrep) * ns;
     e.share_steps = reinterpret_cast<uint32_t *>(base + o);

@@ -82,18 +82,23 @@ struct EncPicState {
 constexpr uint32_t kNotCosted = 0xFFFFFFFFu;
 
 // A slice's share-out inputs: its size at the uniform quantiser, and per
-// window level (bit j of `known` when costed) the smallest D that lets it
-// step there (~0 when the size does not fit) and the size over the base.
-struct SharePrep {
+// window level the least D that lets the slice step that far (the running
+// maximum of the levels' own thresholds; ~0 when one does not fit, or the
+// walk stops before) and the size over the base.
+struct alignas(16) SharePrep {
     uint64_t thr[kWindow];
     int32_t delta[kWindow];
     uint32_t base;
-    uint32_t known;
-    // For the levels past the window (deep_count of them, in `deep`): the
-    // slice header and alpha bytes, the macroblocks from the slice to the
-    // end of the picture, and log2 of the slice's macroblocks.
-    uint32_t hba, rem, shift, deep_count;
+    // Levels the walk knows (the window's, then `deep_count` in `deep`),
+    // whether it would need one that nobody costed after them, and log2 of
+    // the slice's macroblocks.
+    uint8_t levels, deep_count, uncosted_at_end, shift;
+    // For the levels past the window: the slice header and alpha bytes, the
+    // macroblocks from the slice to the end of the picture.
+    uint32_t hba, rem;
 };
+static_assert(sizeof(SharePrep) == 64, "copied 16 bytes at a time");
+static_assert(kWindow + kDeepLevels < 256, "levels counted in a byte");
 
 // Per quantiser set and quantization_index, kQuantStride floats:
 //   [0, 128)    8 / (W qScale) at the scanned positions, luma then chroma;
