@@ -1100,8 +1100,8 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_window(Encod
     }
 }
 
-// The levels past the window, costed ahead of the share-out, a warp per
-// slice, every slice at once: a slice whose last window level fits and is
+// The levels past the window, costed ahead of the share-out, every slice at
+// once: a slice whose last window level fits and is
 // within its likely allowance goes on to the next finer quantiser, and so
 // on while the size it just found fits and stays within that allowance,
 // for up to kDeepLevels levels. A slice's ladder depends on nothing but its
@@ -1126,73 +1126,125 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_window(Encod
 constexpr uint32_t kTailSlices = 16;  // a picture's tail: slices within this many slices' macroblocks of its end
 constexpr uint32_t kTailLevels = 4;
 
-__global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost_deep(EncodeLaunch e) {
+// The slices with a ladder, listed (in the atomics' order, which steers
+// nothing but speed).
+__global__ void __launch_bounds__(kCostThreads) k_deep_select(EncodeLaunch e) {
+    chain_start();
+    chain_wait();
+    const uint32_t s = blockIdx.x * kCostThreads + threadIdx.x;
+    DeepItem item{};
+    if (s < e.n_slices) {
+        const EncSliceDesc sd = e.slices[s];
+        const EncPicState st = e.state[sd.pic];
+        e.deep_count[s] = 0;
+        if (st.fits_at_all && st.uniform - kWindow > 1) {
+            const EncPicDesc &pd = e.pics[sd.pic];
+            const uint32_t hb = pd.header_bytes, alpha = e.alpha_bytes[s];
+            const uint32_t *u = e.probe_comp + ((uint64_t)st.hi_probe * e.n_slices + s) * 3u;
+            const uint32_t uc[3] = {u[0], u[1], u[2]};
+            bool f0;
+            const uint64_t used = slice_total(hb, uc, alpha, f0);
+            const uint64_t slack = st.budget - st.hi_total;
+            const uint64_t most = used + slack * sd.mbs / mbs_from(pd, sd);
+            const uint64_t share = slack * sd.mbs / ((uint64_t)pd.width_in_mb * pd.height_in_mb);
+            const uint32_t *c = level_comp(e, st, kWindow - 1, s);
+            bool fits = false;
+            uint64_t n = ~0ull;
+            if (c[0] != kNotCosted) {
+                const uint32_t cc[3] = {c[0], c[1], c[2]};
+                n = slice_total(hb, cc, alpha, fits);
+            }
+            // The slice's step: its size change a finer quantiser, the larger
+            // of the first step and the mean of the window's next three (the
+            // first can be far larger than the rest: above quantiser index
+            // 128 a step of the index is 4 of qScale, below it 1).
+            const uint32_t *c1 = level_comp(e, st, 0, s);
+            uint64_t step = 0, n1 = 0;
+            if (c1[0] != kNotCosted) {
+                const uint32_t cc[3] = {c1[0], c1[1], c1[2]};
+                bool f1;
+                n1 = slice_total(hb, cc, alpha, f1);
+                step = n1 > used ? n1 - used : 0u;
+                if (c[0] != kNotCosted) step = min(step, n > n1 ? (n - n1) / (uint64_t)(kWindow - 1) : 0u);
+            }
+            // A slice whose step is small beside its share (a coarse
+            // quantiser, where a step often changes no size) walks many
+            // levels wherever its allowance lands: its ladder goes to the
+            // most. So do the last slices of a picture, where what the slices
+            // before left gathers, for at most kTailLevels levels.
+            const bool coarse = 4u * step <= share;
+            const bool tail = mbs_from(pd, sd) <= (uint64_t)kTailSlices * sd.mbs;
+            const uint64_t likely = coarse || tail ? most : min(most, used + share + share / 4u + step);
+            const uint32_t levels = coarse ? (uint32_t)kDeepLevels : (tail ? kTailLevels : (uint32_t)kDeepLevels);
+            if (fits && n <= likely)
+                item = DeepItem{likely, s, min(levels, (uint32_t)(st.uniform - 1 - kWindow)), hb + alpha};
+        }
+    }
+    const uint32_t m = __ballot_sync(0xffffffffu, item.levels != 0);
+    if (m) {
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t at = 0;
+        if (lane == (uint32_t)__ffs(m) - 1u) at = atomicAdd(e.deep_listed, (uint32_t)__popc(m));
+        at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
+        if (item.levels) e.deep_list[at + __popc(m & ((1u << lane) - 1u))] = item;
+    }
+}
+
+// Blocks take the listed slices, with a warp for each component and each of
+// the next kDeepTries levels. Bound by the longest ladders, whose levels
+// follow one another: a warp a slice, component after component and level
+// after level, took one UHD frame 44 us, 30 of them 128 and 32 frames of mixed
+// sizes 394; this takes 13, 25 and 76 with both its kernels. In smaller teams,
+// four times 3 warps a block for a level at a time: 29, 33 and 181; twice 6
+// warps: 18, 21 and 107; the same with a list of each block's own 32 slices
+// instead of the one of all: 77, 126 and 378 (neighbours' ladders are long
+// together).
+constexpr uint32_t kDeepTries = 4;
+constexpr uint32_t kDeepThreads = 32 * 3 * kDeepTries;
+constexpr int kDeepBlocks = 2;
+
+__global__ void __launch_bounds__(kDeepThreads, kDeepBlocks) k_cost_deep(EncodeLaunch e) {
     chain_start();
     __shared__ __align__(16) CountTables t;
-    __shared__ __align__(8) uint32_t buf[kCostThreads / 32][kCountWords];
+    __shared__ __align__(8) uint32_t buf[kDeepThreads / 32][kCountWords];
+    __shared__ uint32_t now, sizes[2][kDeepTries][3];
     t.fill();
     chain_wait();
     __syncthreads();
-    const uint32_t s = blockIdx.x * (kCostThreads / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (s >= e.n_slices) return;
-    const EncSliceDesc sd = e.slices[s];
-    const EncPicState st = e.state[sd.pic];
-    uint32_t count = 0;
-    if (st.fits_at_all && st.uniform - kWindow > 1) {
+    const uint32_t listed = e.deep_listed[0];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t comp = warp % 3u, ahead = warp / 3u;
+    for (;;) {
+        if (threadIdx.x == 0) now = atomicAdd(e.deep_listed + 1, 1u);
+        __syncthreads();
+        if (now >= listed) return;
+        const DeepItem item = e.deep_list[now];
+        const EncSliceDesc sd = e.slices[item.s];
         const EncPicDesc &pd = e.pics[sd.pic];
         const EncFrameDesc &fd = e.frames[pd.frame];
-        const uint32_t hb = pd.header_bytes, alpha = e.alpha_bytes[s];
-        const uint32_t *u = e.probe_comp + ((uint64_t)st.hi_probe * e.n_slices + s) * 3u;
-        const uint32_t uc[3] = {u[0], u[1], u[2]};
-        bool f0;
-        const uint64_t used = slice_total(hb, uc, alpha, f0);
-        const uint64_t slack = st.budget - st.hi_total;
-        const uint64_t most = used + slack * sd.mbs / mbs_from(pd, sd);
-        const uint64_t share = slack * sd.mbs / ((uint64_t)pd.width_in_mb * pd.height_in_mb);
-        const uint32_t *c = level_comp(e, st, kWindow - 1, s);
-        bool fits = false;
-        uint64_t n = ~0ull;
-        if (c[0] != kNotCosted) {
-            const uint32_t cc[3] = {c[0], c[1], c[2]};
-            n = slice_total(hb, cc, alpha, fits);
+        // Level j is quantiser finest - j, which item.levels keeps above 0.
+        const uint32_t finest = (uint32_t)(e.state[sd.pic].uniform - 1 - kWindow);
+        uint32_t j = 0;
+        bool more = true;
+        for (uint32_t turn = 0; more; turn ^= 1u) {
+            if (j + ahead < item.levels) {
+                const uint32_t bytes = warp_component_bytes(e, sd, pd, fd, comp, finest - j - ahead, t, buf[warp]);
+                if (lane == 0) sizes[turn][ahead][comp] = bytes;
+            }
+            __syncthreads();
+            for (uint32_t a = 0; more && a < kDeepTries; a++) {
+                const uint32_t c3[3] = {sizes[turn][a][0], sizes[turn][a][1], sizes[turn][a][2]};
+                bool fits;
+                const uint64_t n = slice_total(item.hba, c3, 0, fits);
+                if (threadIdx.x == 0)
+                    e.deep[(uint64_t)item.s * kDeepLevels + j] = make_uint2(
+                        min(c3[0], 65535u) | (min(c3[1], 65535u) << 16), min(c3[2], 65535u) | ((fits ? 1u : 0u) << 16));
+                j++;
+                more = fits && n <= item.likely && j < item.levels;
+            }
         }
-        // The slice's step: its size change a finer quantiser, the larger of
-        // the first step and the mean of the window's next three (the first
-        // can be far larger than the rest: above quantiser index 128 a step
-        // of the index is 4 of qScale, below it 1).
-        const uint32_t *c1 = level_comp(e, st, 0, s);
-        uint64_t step = 0, n1 = 0;
-        if (c1[0] != kNotCosted) {
-            const uint32_t cc[3] = {c1[0], c1[1], c1[2]};
-            bool f1;
-            n1 = slice_total(hb, cc, alpha, f1);
-            step = n1 > used ? n1 - used : 0u;
-            if (c[0] != kNotCosted) step = min(step, n > n1 ? (n - n1) / (uint64_t)(kWindow - 1) : 0u);
-        }
-        // A slice whose step is small beside its share (a coarse quantiser,
-        // where a step often changes no size) walks many levels wherever its
-        // allowance lands: its ladder goes to the most. So do the last slices
-        // of a picture, where what the slices before left gathers, for at
-        // most kTailLevels levels.
-        const bool coarse = 4u * step <= share;
-        const bool tail = mbs_from(pd, sd) <= (uint64_t)kTailSlices * sd.mbs;
-        const uint64_t likely = coarse || tail ? most : min(most, used + share + share / 4u + step);
-        const uint32_t levels = coarse ? (uint32_t)kDeepLevels : (tail ? kTailLevels : (uint32_t)kDeepLevels);
-        for (uint32_t j = 0; fits && n <= likely && j < levels; j++) {
-            const int32_t qi = st.uniform - 1 - kWindow - (int32_t)j;
-            if (qi < 1) break;
-            uint32_t c3[3];
-            for (uint32_t comp = 0; comp < 3; comp++)
-                c3[comp] = warp_component_bytes(e, sd, pd, fd, comp, (uint32_t)qi, t, buf[threadIdx.x >> 5]);
-            n = slice_total(hb, c3, alpha, fits);
-            if (lane == 0)
-                e.deep[(uint64_t)s * kDeepLevels + j] =
-                    make_uint2(min(c3[0], 65535u) | (min(c3[1], 65535u) << 16), min(c3[2], 65535u) | ((fits ? 1u : 0u) << 16));
-            count = j + 1;
-        }
+        if (threadIdx.x == 0) e.deep_count[item.s] = j;
     }
-    if (lane == 0) e.deep_count[s] = count;
 }
 
 constexpr int kRcThreads = 1024;
@@ -1237,6 +1289,7 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_init(EncodeLaunch e) {
         if (blockIdx.x == 0) {
             for (int j = 0; j < kWindow; j++) e.win_count[j] = 0;
             for (int j = 0; j < kProbeSteps; j++) e.cost_taken[j] = 0;
+            e.deep_listed[0] = e.deep_listed[1] = 0;
         }
     }
 }
@@ -2278,8 +2331,9 @@ cudaError_t launch_cost_window(const EncodeLaunch &e, int level, cudaStream_t s)
 
 cudaError_t launch_cost_deep(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
-    return launch_chained(k_cost_deep, (e.n_slices + kCostThreads / 32 - 1) / (kCostThreads / 32), kCostThreads, 0, s,
-                          e);
+    cudaError_t err = launch_chained(k_deep_select, (e.n_slices + kCostThreads - 1) / kCostThreads, kCostThreads, 0, s, e);
+    if (err != cudaSuccess) return err;
+    return launch_chained(k_cost_deep, (uint32_t)(kDeepBlocks * e.sm_count), kDeepThreads, 0, s, e);
 }
 
 cudaError_t launch_shareout(const EncodeLaunch &e, cudaStream_t s) {

@@ -112,6 +112,13 @@ constexpr uint32_t kQuantStride = 384;
 // whether the scan is the interlaced one.
 constexpr size_t kQuantKey = 129;
 
+// A slice whose deep ladder is to be costed: it goes on to the next level
+// while its size (hba: its header and alpha bytes) is at most `likely`.
+struct DeepItem {
+    uint64_t likely;
+    uint32_t s, levels, hba;
+};
+
 struct EncodeLaunch {
     const uint16_t *in;        // input planes
     const uint16_t *alpha_in;  // input alpha planes
@@ -137,6 +144,8 @@ struct EncodeLaunch {
     uint2 *deep;           // [slice][kDeepLevels] component bytes past the window: x = Y' | Cb << 16,
                            //   y = Cr | fits << 16 (sizes saturate at 65535, which never fits)
     uint32_t *deep_count;  // [slice] levels in deep
+    DeepItem *deep_list;   // [slice] the slices with a ladder
+    uint32_t *deep_listed; // [2] how many, and how many k_cost_deep has taken
     uint32_t *out;         // output buffer (zeroed before packing), big-endian bit order
     const uint8_t *headers;  // frame header templates
     uint32_t *frame_status;  // per frame: 0, or 1 when the frame outgrew its region
