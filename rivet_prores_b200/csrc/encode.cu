@@ -932,11 +932,20 @@ __device__ __forceinline__ uint32_t warp_component_bytes(const EncodeLaunch &e, 
 constexpr int kCostThreads = 256;
 constexpr int kCostBlocks = 4;      // CTAs an SM (5, at 48 registers: 7 % slower)
 constexpr uint32_t kCostTake = 4;   // items a warp of k_cost takes at once, at most (2: 3 % slower; 19, as 4 rounds a warp: 7 %)
+// Above this many items a warp its next ones are taken before it costs those
+// it has: the counter's answer, about 1 us, is then waited for beside them. A
+// warp that holds items it has not begun leaves others idle at the end, so
+// with fewer they are taken when it is done (one UHD frame, 3 items a warp:
+// 27 -> 25 us a probe; 30 1080p frames, 19 a warp, are better off ahead).
+constexpr uint32_t kGrabAhead = 8;
 
-// A warp per slice component, (component, slice) component-major. A warp
-// takes `take` neighbouring items (at most 32) from the probe's counter at a
-// time: its lanes look the items' places up side by side, so the chain of
-// descriptor loads is waited for once, and the items are costed in turn.
+// A warp per slice component, (component, slice) component-major. Its first
+// items go by its place, so that a batch with an item a warp has each warp at
+// work (all from the counter, 16-20 us a probe of one 1080p frame, now 13-15).
+// From then on a warp takes `take` neighbouring items (at most 32) from the
+// probe's counter at a time: its lanes look the items' places up side by side,
+// so the chain of descriptor loads is waited for once, and the items are
+// costed in turn.
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost(EncodeLaunch e, int step, uint32_t take) {
     chain_start();
     __shared__ __align__(16) CountTables t;
@@ -946,12 +955,13 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost(EncodeLaunch
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t items = 3u * e.n_slices;
-    uint32_t grab = 0;
-    if (lane == 0) grab = atomicAdd(e.cost_taken + step, take);
+    const uint32_t warps = gridDim.x * (kCostThreads / 32);
+    const bool ahead = items > kGrabAhead * warps;
+    uint32_t grab = (blockIdx.x * (kCostThreads / 32) + (threadIdx.x >> 5)) * take;
     for (;;) {
         const uint32_t base = __shfl_sync(0xffffffffu, grab, 0);
         if (base >= items) break;
-        if (lane == 0) grab = atomicAdd(e.cost_taken + step, take);  // the next one, on its way meanwhile
+        if (ahead && lane == 0) grab = warps * take + atomicAdd(e.cost_taken + step, take);
         // This lane's item: its first coefficient (a multiple of 64), its
         // quantiser table and component group, its block count (0: none).
         const uint32_t item = base + lane;
@@ -992,6 +1002,7 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost(EncodeLaunch
             if (lane == j) my_bytes = (bits + 7u) / 8u;
         }
         if (my_blocks) e.probe_comp[(uint64_t)step * 3u * e.n_slices + out] = my_bytes;
+        if (!ahead && lane == 0) grab = warps * take + atomicAdd(e.cost_taken + step, take);
     }
 }
 
@@ -1783,6 +1794,7 @@ __global__ void __launch_bounds__(kLayoutThreads) k_layout(EncodeLaunch e) {
     const EncPicDesc pd = e.pics[blockIdx.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) carry = 8u + 2ull * pd.n_slices;
+    if (threadIdx.x == 0 && blockIdx.x == 0) *e.pack_taken = 0;
     __syncthreads();
     for (uint32_t chunk = 0; chunk < pd.n_slices; chunk += kLayoutThreads) {
         const uint32_t k = chunk + threadIdx.x;
@@ -2106,17 +2118,18 @@ __device__ __noinline__ void lane_component_write(uint32_t *out, uint64_t at, co
     w.finish();
 }
 
-// Each slice component's codes (src/encode.rs:413-437), a warp each, the list
-// walked at the resident grid's stride: the non-zeros are gathered as for
-// counting, and their codes placed 64 at a time. A component with levels too
-// large for the list is written by one lane.
+// Each slice component's codes (src/encode.rs:413-437), a warp each, taken as
+// by k_cost: the non-zeros are gathered as for counting, and their codes
+// placed 64 at a time. A component with levels too large for the list is
+// written by one lane.
 //
 // Bound by issue (72 % of the slots, 51 warp instructions for 32 coefficients
 // at 36 % non-zeros). A lane per component, writing bit by bit into words it
 // OR-ed to memory, took 1390 us for 30 UHD frames, 636 for 30 1080p and 474
-// for one UHD frame (a lane's walk from end to end): 968, 265 and 50 now. Alpha,
-// whose codes were OR-ed into memory one by one, goes through the same words:
-// 8 UHD 4:4:4 frames with it 1595 -> 814.
+// for one UHD frame (a lane's walk from end to end): 968, 265 and 50, and from a
+// counter instead of the grid's stride 865, 245 and 50. Alpha, whose codes were
+// OR-ed into memory one by one, goes through the same words: 8 UHD 4:4:4 frames
+// with it 1595 -> 779.
 __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_pack(EncodeLaunch e, uint32_t take) {
     chain_start();
     __shared__ __align__(16) PackTables t;
@@ -2126,10 +2139,16 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_pack(EncodeLaunch
     chain_wait();
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t items = 3u * e.n_slices, stride = gridDim.x * (kCostThreads / 32) * take;
+    const uint32_t items = 3u * e.n_slices;
     WarpBits w;
     w.clear(words[warp]);
-    for (uint32_t base = (blockIdx.x * (kCostThreads / 32) + warp) * take; base < items; base += stride) {
+    const uint32_t warps = gridDim.x * (kCostThreads / 32);
+    const bool ahead = items > kGrabAhead * warps;
+    uint32_t grab = (blockIdx.x * (kCostThreads / 32) + (threadIdx.x >> 5)) * take;
+    for (;;) {
+        const uint32_t base = __shfl_sync(0xffffffffu, grab, 0);
+        if (base >= items) break;
+        if (ahead && lane == 0) grab = warps * take + atomicAdd(e.pack_taken, take);
         // This lane's item, as in k_cost, and the bit its codes start at.
         const uint32_t item = base + lane;
         uint32_t my_coef = 0, my_quant = 0, my_blocks = 0;
@@ -2188,6 +2207,7 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_pack(EncodeLaunch
             warp_nonzeros<false>(f, cq.inv, nb, live_lo, live_hi, sink, buf[warp]);
             w.finish();
         }
+        if (!ahead && lane == 0) grab = warps * take + atomicAdd(e.pack_taken, take);
     }
 }
 
