@@ -981,10 +981,11 @@ __device__ __forceinline__ void block_xy(uint32_t comp, uint32_t chroma, uint32_
 // than a warp; the next list words are on their way while the last are
 // placed. Bound by issue (66 % of the slots, 37 instructions a sample at 36 %
 // non-zeros) and by the 24 warps an SM that the blocks' 8.7 kB leave room for
-// (20, at 102 registers: 11 % slower; 16: 25 %). 32 UHD 4:2:2 frames take
-// 822 us, where a CTA per slice with index arithmetic for every row and
-// column task and all 64 products took 1990; a mixed batch 430 for 1585.
-constexpr int kIdctWarps = 4;
+// (20, at 102 registers: 11 % slower; 16: 25 %), in CTAs of 2, whose place is
+// free sooner than one of 4 (813 us). 32 UHD 4:2:2 frames take 801 us, where a
+// CTA per slice with index arithmetic for every row and column task and all 64
+// products took 1990; a mixed batch 424 for 1585.
+constexpr int kIdctWarps = 2;
 // A block's floats in shared memory: 64 and 4 more, so that eight lanes'
 // 16-byte reads of the same place in neighbouring blocks meet no bank twice.
 constexpr uint32_t kBlockStride = 68;
@@ -1059,7 +1060,7 @@ __device__ __forceinline__ void idct_columns(const float *t, uint32_t rows, floa
     put(&Pairs8::o76, 7, 6);
 }
 
-__global__ void __launch_bounds__(32 * kIdctWarps, 6) k_idct(DecodeLaunch d) {
+__global__ void __launch_bounds__(32 * kIdctWarps, 12) k_idct(DecodeLaunch d) {
     chain_start();
     chain_wait();
     extern __shared__ __align__(16) unsigned char smem[];

@@ -87,7 +87,7 @@ __device__ __forceinline__ int32_t quantise1(float f, float inv, float r) {
 
 // ---------------------------------------------------------------- fdct
 
-constexpr int kFdctWarps = 4;
+constexpr int kFdctWarps = 3;
 constexpr int kMaxSliceCoefs = 64 * 12 * 8;
 
 __device__ __forceinline__ void block_xy(uint32_t comp, uint32_t chroma, uint32_t mb_x, uint32_t mb_y, uint32_t m,
@@ -128,16 +128,18 @@ __device__ __forceinline__ void fdct8(const float (&in)[8], uint64_t (&o)[4]) {
 // met twice. Then the warp writes the components out in scanned order, 16
 // bytes a lane, with the largest |F| of every 32 coefficients (8 lanes).
 // Bound by issue (74 % of the slots, 49 instructions a sample, of which the
-// sums' terms are 23): 30 UHD 4:2:2 frames take 910 us, 1463 with a warp per
+// sums' terms are 23): 30 UHD 4:2:2 frames take 852 us, 1463 with a warp per
 // component (half the lanes idle in 4:2:2 chroma, more in narrow slices) and a
-// reduction for every position's maximum; a mixed batch 545 for 1796. Rows are
-// loaded two ahead (1022 us without), 24 warps an SM.
+// reduction for every position's maximum; a mixed batch 515 for 1796. Rows are
+// loaded two ahead (12 % slower without). 27 warps fill an SM's shared memory,
+// in blocks of 3, since a block's place is free only when its last warp is
+// done (24 warps, in blocks of 4: 915 us; of 2: 878; of 1: 892).
 struct FdctWarp {
     float t[64][32];
     uint8_t raster[64];  // of each scanned position
 };
 
-__global__ void __launch_bounds__(32 * kFdctWarps, 6) k_fdct(EncodeLaunch e) {
+__global__ void __launch_bounds__(32 * kFdctWarps, 9) k_fdct(EncodeLaunch e) {
     chain_start();
     chain_wait();
     extern __shared__ __align__(16) unsigned char smem[];
