@@ -140,7 +140,6 @@ struct FdctWarp {
 };
 
 __global__ void __launch_bounds__(32 * kFdctWarps, 9) k_fdct(EncodeLaunch e) {
-    chain_start();
     chain_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     FdctWarp &w = reinterpret_cast<FdctWarp *>(smem)[threadIdx.x >> 5];
@@ -344,7 +343,6 @@ __device__ __forceinline__ uint32_t alpha_run_bits(const AlphaScratch &sc, uint3
 }
 
 __global__ void __launch_bounds__(32 * kAlphaWarps) k_alpha_size(EncodeLaunch e) {
-    chain_start();
     chain_wait();
     __shared__ AlphaScratch scratch[kAlphaWarps];
     const uint32_t s = blockIdx.x * kAlphaWarps + (threadIdx.x >> 5);
@@ -2307,7 +2305,7 @@ cudaError_t launch_fdct(const EncodeLaunch &e, cudaStream_t s) {
 
 cudaError_t launch_alpha_size(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_slices) return cudaSuccess;
-    if (!e.any_alpha) return cudaMemsetAsync(e.alpha_bytes, 0, 4ull * e.n_slices, s);
+    if (!e.any_alpha) return cudaSuccess;  // alpha_bytes is zeroed beforehand
     return launch_chained(k_alpha_size, (e.n_slices + kAlphaWarps - 1) / kAlphaWarps, 32 * kAlphaWarps, 0, s, e);
 }
 

@@ -383,7 +383,6 @@ Status upload_encode(Context &ctx, Workspace &ws, EncodePlan &plan, const prores
 static Status enqueue_tail(Context &ctx, Workspace &ws, EncodePlan &plan, cudaStream_t s, KernelTimes *kt) {
     const EncodeLaunch e = encode_params(ctx, ws, plan);
     Status st;
-    PR_CUDA(cudaMemsetAsync(ws.enc_out.p, 0, plan.out_total + 64, s), "memset output");
     PR_CUDA(launch_layout(e, s), "k_layout");
     if ((st = record_kernel(kt, "k_layout", s))) return st;
     PR_CUDA(launch_pack(e, s), "k_pack");
@@ -395,6 +394,10 @@ Status enqueue_encode(Context &ctx, Workspace &ws, EncodePlan &plan, cudaStream_
     const EncodeLaunch e = encode_params(ctx, ws, plan);
     Status st;
     if ((st = record_kernel(kt, "start", s))) return st;
+    // Ahead of the kernels, which start in programmatic order: each memset
+    // among them held its successor back until its predecessor was done.
+    PR_CUDA(cudaMemsetAsync(ws.enc_out.p, 0, plan.out_total + 64, s), "memset output");
+    if (!e.any_alpha && e.n_slices) PR_CUDA(cudaMemsetAsync(e.alpha_bytes, 0, 4ull * e.n_slices, s), "memset sizes");
     PR_CUDA(launch_fdct(e, s), "k_fdct");
     if ((st = record_kernel(kt, "k_fdct", s))) return st;
     PR_CUDA(launch_alpha_size(e, s), "k_alpha_size");
@@ -456,6 +459,7 @@ Status fetch_encode(Context &ctx, Workspace &ws, EncodePlan &plan, cudaStream_t 
             cudaGraphExecDestroy(plan.graph);
             plan.graph = nullptr;
         }
+        PR_CUDA(cudaMemsetAsync(ws.enc_out.p, 0, plan.out_total + 64, s), "memset output");
         Status st = enqueue_tail(ctx, ws, plan, s, nullptr);
         if (st) return st;
     }
