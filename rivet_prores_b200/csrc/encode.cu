@@ -407,27 +407,6 @@ __global__ void __launch_bounds__(128) k_quant(float *quant, const uint8_t *keys
 
 // ---------------------------------------------------------------- costing
 
-// One AC position of a lane's walk: x = F inv, m = floor(|x| + 0.42)
-// (src/dsp/scalar.rs:19-39) as an integer; only a non-zero coefficient is
-// coded (its run from the last one, its level, both by context).
-struct AcWalk {
-    uint32_t prev_run = 4, prev_level = 1, pos = 0;
-};
-
-template <class Emit>
-__device__ __forceinline__ void ac_position(AcWalk &w, float f, float inv, uint32_t p, Emit emit) {
-    const float x = __fmul_rn(f, inv);
-    const int32_t m = magnitude(x, kAcRounding);
-    if (m >= 1) {
-        const uint32_t run = p - w.pos;
-        const uint32_t level = (uint32_t)m - 1u;
-        emit(w, run, level, x < 0.0f);
-        w.prev_run = run;
-        w.prev_level = level;
-        w.pos = p + 1;
-    }
-}
-
 // One component's view of a quantiser table (layout beside kQuantStride):
 // inverse weights and non-zero bounds by scanned position, and the bound of
 // each 32-coefficient chunk of a component of its block count.
@@ -442,48 +421,6 @@ __device__ __forceinline__ CompQuant comp_quant(const float *qb, uint32_t comp, 
     c.bound = qb + 128u + 64u * g;
     c.chunk = n_blocks >= 32u ? c.bound : qb + 256u + 60u * g + (2u * n_blocks - 4u);
     return c;
-}
-
-// Whether chunk j holds no coefficient that quantises to a non-zero: its
-// largest |F| is below the least non-zero bound of its positions.
-__device__ __forceinline__ bool chunk_is_zero(const float *cmax, const CompQuant &q, uint32_t j) {
-    return __ldg(cmax + j) < __ldg(q.chunk + j);
-}
-
-// Walks the candidates of a component's AC positions (n_blocks onwards) in
-// order: chunks that quantise to zero are skipped, a chunk's candidate mask takes one
-// compare per coefficient against the non-zero bound of its position (so
-// it holds every non-zero, and each candidate is re-quantised exactly),
-// and the lane then visits the candidates alone. Suited to heavy per-code
-// work (the writer), where a position-by-position walk would make every
-// lane wait out every other lane's codes.
-template <class Emit>
-__device__ __forceinline__ void ac_walk_sparse(const float *f, const float *cmax, uint32_t n_blocks,
-                                               const CompQuant &q, Emit emit) {
-    const uint32_t total = 64u * n_blocks;
-    const uint32_t shift = 31u - __clz(n_blocks);
-    AcWalk w;
-    w.pos = n_blocks;
-    for (uint32_t c0 = n_blocks & ~31u; c0 < total; c0 += 32) {
-        if (chunk_is_zero(cmax, q, c0 >> 5)) continue;
-        uint32_t mask = 0;
-#pragma unroll
-        for (uint32_t i = 0; i < 8; i++) {
-            const uint32_t e0 = c0 + 4u * i;
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(f + e0));
-            // With two blocks a load spans scan positions e0 / 2 and e0 / 2 + 1.
-            const float ta = __ldg(q.bound + (e0 >> shift)), tb = __ldg(q.bound + ((e0 + 3u) >> shift));
-            const uint32_t nib = (fabsf(v.x) >= ta ? 1u : 0u) | (fabsf(v.y) >= ta ? 2u : 0u) |
-                                 (fabsf(v.z) >= tb ? 4u : 0u) | (fabsf(v.w) >= tb ? 8u : 0u);
-            mask |= nib << (4u * i);
-        }
-        if (c0 == 0) mask &= ~0u << n_blocks;  // the DCs
-        while (mask) {
-            const uint32_t p = c0 + (uint32_t)__ffs(mask) - 1u;
-            mask &= mask - 1u;
-            ac_position(w, __ldg(f + p), __ldg(q.inv + (p >> shift)), p, emit);
-        }
-    }
 }
 
 // Code lengths by context for the warps that count bits: of run symbols
@@ -855,24 +792,42 @@ __device__ __forceinline__ uint32_t dc_symbol(float dc, float inv0, uint32_t &a)
     return ((uint32_t)value << 1) ^ (uint32_t)(value >> 31);
 }
 
-// The same for levels of any size, by one lane's walk: only a component whose
-// largest |F| reaches kWideCoef comes here.
+// The AC codes of a component with levels of any size (its largest |F| reaches
+// kWideCoef), the whole warp, 32 positions at a time: a lane with a non-zero
+// finds the one before it in the lanes' vote, and that one's run and level,
+// its contexts, by shuffles (one lane walking alone held its whole warp: 4
+// 1080p frames of samples past their depth's range took 1430 us, now 274).
+// emit(coded, run, level, negative, previous run,
+// previous level), every lane each time.
+template <bool kShared, class Emit>
+__device__ __forceinline__ void warp_wide_codes(const float *f, const float *inv, uint32_t n_blocks, Emit emit) {
+    const uint32_t lane = threadIdx.x & 31u, shift = 31u - __clz(n_blocks);
+    uint32_t last_run = 4, last_level = 1, next = n_blocks;  // of the last code, and the position after it
+    for (uint32_t p0 = n_blocks; p0 < 64u * n_blocks; p0 += 32u) {
+        const uint32_t p = p0 + lane;
+        float x = 0.0f;
+        if (p < 64u * n_blocks) x = __fmul_rn(coef_load<kShared>(f, p), __ldg(inv + (p >> shift)));
+        const int32_t m = magnitude(x, kAcRounding);
+        const uint32_t coded = __ballot_sync(0xffffffffu, m >= 1);
+        if (!coded) continue;
+        const uint32_t before = coded & ((1u << lane) - 1u), from = 31u - __clz(before);
+        const uint32_t run = p - (before ? p0 + from + 1u : next), level = (uint32_t)m - 1u;
+        const uint32_t run_before = __shfl_sync(0xffffffffu, run, from), level_before = __shfl_sync(0xffffffffu, level, from);
+        emit(m >= 1, run, level, x < 0.0f, before ? run_before : last_run, before ? level_before : last_level);
+        const uint32_t top = 31u - __clz(coded);
+        last_run = __shfl_sync(0xffffffffu, run, top);
+        last_level = __shfl_sync(0xffffffffu, level, top);
+        next = p0 + top + 1u;
+    }
+}
+
 template <bool kShared>
 __device__ __noinline__ uint32_t warp_wide_bits(const float *f, const float *inv, uint32_t n_blocks) {
     uint32_t bits = 0;
-    if ((threadIdx.x & 31u) == 0) {
-        const uint32_t shift = 31u - __clz(n_blocks);
-        uint32_t prev_run = 4, prev_level = 1, pos = n_blocks;
-        for (uint32_t p = n_blocks; p < 64u * n_blocks; p++) {
-            const int32_t m = magnitude(__fmul_rn(coef_load<kShared>(f, p), __ldg(inv + (p >> shift))), kAcRounding);
-            if (m < 1) continue;
-            const uint32_t run = p - pos, level = (uint32_t)m - 1u;
-            bits += cb_len(run_book(prev_run), run) + cb_len(level_book(prev_level), level) + 1u;
-            prev_run = run;
-            prev_level = level;
-            pos = p + 1u;
-        }
-    }
+    warp_wide_codes<kShared>(f, inv, n_blocks, [&](bool coded, uint32_t run, uint32_t level, bool, uint32_t prev_run,
+                                                   uint32_t prev_level) {
+        if (coded) bits += cb_len32(run_book(prev_run), run) + cb_len32(level_book(prev_level), level) + 1u;
+    });
     return bits;
 }
 
@@ -1853,68 +1808,6 @@ __global__ void k_frame(EncodeLaunch e) {
 
 // ---------------------------------------------------------------- packing
 
-// An MSB-first writer into the big-endian output words from an absolute
-// bit position. Words wholly inside the writer's bytes are stored; the
-// partial words at either end, which a neighbour shares, are OR-ed.
-struct BitOut {
-    uint32_t *out;
-    uint64_t cur;  // absolute position of the first bit held
-    uint64_t acc;
-    uint32_t nacc;
-    __device__ __forceinline__ void init(uint32_t *o, uint64_t bitpos) {
-        out = o;
-        cur = bitpos;
-        acc = 0;
-        nacc = 0;
-    }
-    __device__ __forceinline__ void emit() {
-        for (;;) {
-            const uint32_t room = 32u - (uint32_t)(cur & 31u);
-            if (nacc < room) return;
-            const uint32_t chunk = (uint32_t)(acc >> (nacc - room)) & (room == 32u ? 0xFFFFFFFFu : ((1u << room) - 1u));
-            uint32_t *w = out + (cur >> 5);
-            if (room == 32u)
-                *w = bswap32(chunk);
-            else
-                atomicOr(w, bswap32(chunk));
-            nacc -= room;
-            cur += room;
-        }
-    }
-    // A field of n <= 32 bits holding v.
-    __device__ __forceinline__ void put(uint64_t v, uint32_t n) {
-        if (n == 0) return;
-        acc = (acc << n) | v;
-        nacc += n;
-        emit();
-    }
-    // A field of any width holding v (its leading zeros included).
-    __device__ __forceinline__ void put_long(uint64_t v, uint32_t n) {
-        if (n > 64) {
-            put(0, n - 64);
-            n = 64;
-        }
-        if (n > 32) {
-            put(v >> 32, n - 32);
-            v &= 0xFFFFFFFFull;
-            n = 32;
-        }
-        put(v, n);
-    }
-    // Zero bits to the next byte boundary, then the last partial word.
-    __device__ __forceinline__ void finish() {
-        const uint32_t pad = (uint32_t)((8u - ((cur + nacc) & 7u)) & 7u);
-        put(0, pad);
-        if (nacc) {
-            const uint32_t room = 32u - (uint32_t)(cur & 31u);
-            const uint32_t chunk = (uint32_t)(acc & ((1ull << nacc) - 1)) << (room - nacc);
-            atomicOr(out + (cur >> 5), bswap32(chunk));
-            cur += nacc;
-            nacc = 0;
-        }
-    }
-};
-
 // The writer's tables by context: a code's length << 24 | its significant
 // bits, of run symbols below 63 and of level symbols below 127 with room for
 // the sign bit; 0 in the last column, for every symbol past those. Both are
@@ -2086,42 +1979,24 @@ struct PackSink {
     }
 };
 
-// One quantised component's codes (src/encode.rs:413-437), one lane.
-__device__ __noinline__ void lane_component_write(uint32_t *out, uint64_t at, const float *f, const float *cmax,
-                                                  uint32_t n_blocks, const CompQuant &q) {
-    BitOut w;
-    w.init(out, at);
-    const float inv0 = __ldg(q.inv);
-    int32_t prev_dc = 0, prev_diff = 3;
-    for (uint32_t i = 0; i < n_blocks; i++) {
-        const int32_t q = quantise1(__ldg(f + i), inv0, 0.5f);
-        Codebook cb;
-        uint32_t sym;
-        if (i == 0) {
-            cb = kFirstDcBook;
-            sym = signed_to_symbol(q);
-        } else {
-            const int32_t diff = (int32_t)((uint32_t)q - (uint32_t)prev_dc);
-            cb = dc_book(prev_diff);
-            sym = signed_to_symbol(prev_diff < 0 ? -diff : diff);
-            prev_diff = diff;
-        }
-        w.put_long(cb_bits(cb, sym), cb_len(cb, sym));
-        prev_dc = q;
-    }
-    ac_walk_sparse(f, cmax, n_blocks, q, [&](const AcWalk &a, uint32_t run, uint32_t level, bool neg) {
-        const Codebook rb = run_book(a.prev_run), lb = level_book(a.prev_level);
-        w.put_long(cb_bits(rb, run), cb_len(rb, run));
-        w.put_long(cb_bits(lb, level), cb_len(lb, level));
-        w.put((uint64_t)neg, 1);
+// The AC codes of a component with levels of any size. A level's code and sign
+// are at most 64 bits, |F| of 16-bit samples staying below 2^21.
+__device__ __noinline__ WarpBits warp_wide_write(WarpBits w, const float *f, const float *inv, uint32_t n_blocks) {
+    warp_wide_codes<false>(f, inv, n_blocks, [&](bool coded, uint32_t run, uint32_t level, bool neg, uint32_t prev_run,
+                                                 uint32_t prev_level) {
+        const Codebook rb = run_book(prev_run), lb = level_book(prev_level);
+        const uint32_t rlen = coded ? cb_len32(rb, run) : 0u, llen = coded ? cb_len32(lb, level) + 1u : 0u;
+        const uint32_t at = w.place(rlen + llen);
+        w.put(at, coded ? cb_bits(rb, run) : 0u, rlen);
+        w.put(at + rlen, coded ? (cb_bits(lb, level) << 1) | (uint64_t)neg : 0u, llen);
+        w.drain();
     });
-    w.finish();
+    return w;
 }
 
 // Each slice component's codes (src/encode.rs:413-437), a warp each, taken as
 // by k_cost: the non-zeros are gathered as for counting, and their codes
-// placed 64 at a time. A component with levels too large for the list is
-// written by one lane.
+// placed 64 at a time.
 //
 // Bound by issue (72 % of the slots, 51 warp instructions for 32 coefficients
 // at 36 % non-zeros). A lane per component, writing bit by bit into words it
@@ -2188,11 +2063,6 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_pack(EncodeLaunch
             const uint64_t at = __shfl_sync(0xffffffffu, my_at, j);
             const CompQuant cq = comp_quant(e.quant + (uint64_t)(quant >> 1) * kQuantStride, quant & 1u, nb);
             const float *f = e.coef + coef;
-            if (__any_sync(0xffffffffu, fmaxf(h.max_lo, h.max_hi) >= kWideCoef)) {
-                if (lane == 0) lane_component_write(e.out, at, f, e.coef_max + (coef >> 5), nb, cq);
-                __syncwarp();
-                continue;
-            }
             w.start(e.out, at);
             uint32_t live_lo, live_hi, a;
             live_chunks(h, nb, cq, live_lo, live_hi);
@@ -2203,8 +2073,12 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_pack(EncodeLaunch
             const uint32_t code = a == 2u ? (symbol < 8u ? (symbol & 3u) + 4u : symbol) : symbol + (1u << a);
             w.put(w.place(len), code, len);
             w.drain();
-            PackSink sink{t, w};
-            warp_nonzeros<false>(f, cq.inv, nb, live_lo, live_hi, sink, buf[warp]);
+            if (__any_sync(0xffffffffu, fmaxf(h.max_lo, h.max_hi) >= kWideCoef)) {
+                w = warp_wide_write(w, f, cq.inv, nb);
+            } else {
+                PackSink sink{t, w};
+                warp_nonzeros<false>(f, cq.inv, nb, live_lo, live_hi, sink, buf[warp]);
+            }
             w.finish();
         }
         if (!ahead && lane == 0) grab = warps * take + atomicAdd(e.pack_taken, take);
