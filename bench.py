@@ -64,9 +64,9 @@ PUBLISHED_CRATE = ("the crate's README: 1920x1080 422 HQ at 296 encode / 907 dec
 # Figures from ncu captures of these kernels, not measured by this run: the
 # capture's DRAM bytes (read + write) per frame and launch, and issue-slot use.
 CAPTURED = {
-    "k_cost": {"dram_bytes_per_frame": 70.96e6, "issue_active_pct": "41.5",
-               "thread_instructions_per_coefficient": 26.7,
-               "capture": "ncu --set full on an 8-frame UHD 422 HQ encode, its fifth k_cost launch (a dense probe, "
+    "k_cost": {"dram_bytes_per_frame": 69.33e6, "issue_active_pct": "78.5",
+               "thread_instructions_per_coefficient": 29.0,
+               "capture": "ncu on an 8-frame UHD 422 HQ encode, its fifth k_cost launch (a dense probe, "
                           "which reads every coefficient: the heaviest of the nine)"},
 }
 # What limits each kernel, from the ncu captures summarised under profiles/.
@@ -74,13 +74,13 @@ CAPTURED = {
 # bandwidth: the work is byte and integer work, no tensor-core math); none of
 # these kernels reaches it, and "limiter" names what holds it back instead.
 LIMITER = {
-    "k_cost": "latency: 41.5 % of issue slots active, a quarter to two fifths of the warp slots busy",
-    "k_cost_window": "latency, as k_cost; it costs a list of slices that changes with the pictures (level 0 "
+    "k_cost": "instruction issue (79 % of issue slots active), and at the dense probes DRAM at 4.8 TB/s",
+    "k_cost_window": "instruction issue, as k_cost; it costs a list of slices that changes with the pictures (level 0 "
                      "copies from a probe at the same quantiser where there is one), so it has no fixed byte basis",
-    "k_fdct": "instruction issue (83 % of issue slots active)",
-    "k_pack": "latency: half of each warp's lanes active",
-    "k_entropy": "latency: a warp waits for its longest component",
-    "k_idct": "instruction issue (about 108 instructions per sample)",
+    "k_fdct": "instruction issue (76 % of issue slots active)",
+    "k_pack": "instruction issue (76 % of issue slots active)",
+    "k_entropy": "instruction issue (60 % of issue slots active, the ALU pipe 68 %); few frames: the longest component",
+    "k_idct": "instruction issue (68 % of issue slots active, about 35 instructions per sample)",
     "k_decode": "latency: too few components in flight per SM for the entropy step",
 }
 

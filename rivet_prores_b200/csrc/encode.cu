@@ -17,9 +17,13 @@
 //                 src/dsp/scalar.rs:19-39, src/encode.rs:398-409); k_rc_step
 //                 sums a picture's slices and moves its interval.
 //   k_cost_window the next kWindow finer quantisers below the uniform one.
-//   k_shareout    one warp per picture: the sequential share-out of the slack
-//                 (src/encode.rs:769-793), costing any deeper quantiser it
-//                 needs itself.
+//   k_deep_select / k_cost_deep
+//                 the quantisers below those, for the slices likely to need
+//                 them.
+//   k_share_prep / k_shareout / k_share_final
+//                 the sequential share-out of the slack
+//                 (src/encode.rs:769-793), a warp per picture; its block's
+//                 other warps cost any deeper quantiser it needs.
 //   k_layout / k_frame
 //                 slice offsets (an exclusive scan per picture), picture and
 //                 frame sizes, the frame and picture headers.
@@ -839,11 +843,10 @@ __device__ __noinline__ uint32_t warp_wide_bits(const float *f, const float *inv
 // waits for the one before it. Where most chunks quantise to zero only the
 // others are read. Every lane gets the sum.
 //
-// Bound by issue (76-78 % of the slots; 26 warp instructions for 32
-// coefficients at 36 % non-zeros, DRAM at 4.6 TB/s): 30 UHD 4:2:2 frames
-// take 450 us a probe near the answer, where a lane per component walking
-// its codes in order, each look-up waiting for the last, took 800; 30 1080p
-// frames 130 us for 700.
+// Bound by issue (79 % of the slots; 29 thread instructions a coefficient at
+// 36 % non-zeros, DRAM at 4.6 TB/s): 30 UHD 4:2:2 frames take 430 us a probe
+// near the answer, where a lane per component walking its codes in order, each
+// look-up waiting for the last, took 800; 30 1080p frames 123 us for 700.
 template <bool kShared = false>
 __device__ __forceinline__ uint32_t warp_component_bits(const float *f, const CompHead &h, uint32_t n_blocks, const CompQuant &cq,
                                         const CountTables &t, uint32_t *buf) {
