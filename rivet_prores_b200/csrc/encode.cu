@@ -1145,8 +1145,17 @@ __global__ void __launch_bounds__(kCostThreads) k_deep_select(EncodeLaunch e) {
             const bool tail = mbs_from(pd, sd) <= (uint64_t)kTailSlices * sd.mbs;
             const uint64_t likely = coarse || tail ? most : min(most, used + share + share / 4u + step);
             const uint32_t levels = coarse ? (uint32_t)kDeepLevels : (tail ? kTailLevels : (uint32_t)kDeepLevels);
+            uint32_t peak = 0;
+#pragma unroll
+            for (int j = 0; j < kWindow; j++) {
+                const uint32_t *cj = level_comp(e, st, (uint32_t)j, s);
+                const uint32_t cc[3] = {cj[0], cj[1], cj[2]};
+                bool fj;
+                const uint64_t nj = cj[0] == kNotCosted ? 0u : slice_total(hb, cc, alpha, fj);
+                peak = max(peak, cj[0] == kNotCosted || !fj ? ~0u : (uint32_t)nj);
+            }
             if (fits && n <= likely)
-                item = DeepItem{likely, s, min(levels, (uint32_t)(st.uniform - 1 - kWindow)), hb + alpha};
+                item = DeepItem{likely, s, min(levels, (uint32_t)(st.uniform - 1 - kWindow)), hb + alpha, peak};
         }
     }
     const uint32_t m = __ballot_sync(0xffffffffu, item.levels != 0);
@@ -1193,7 +1202,7 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocks) k_cost_deep(EncodeL
         const EncFrameDesc &fd = e.frames[pd.frame];
         // Level j is quantiser finest - j, which item.levels keeps above 0.
         const uint32_t finest = (uint32_t)(e.state[sd.pic].uniform - 1 - kWindow);
-        uint32_t j = 0;
+        uint32_t j = 0, peak = item.peak;
         bool more = true;
         for (uint32_t turn = 0; more; turn ^= 1u) {
             if (j + ahead < item.levels) {
@@ -1205,9 +1214,11 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocks) k_cost_deep(EncodeL
                 const uint32_t c3[3] = {sizes[turn][a][0], sizes[turn][a][1], sizes[turn][a][2]};
                 bool fits;
                 const uint64_t n = slice_total(item.hba, c3, 0, fits);
+                peak = max(peak, fits ? (uint32_t)n : ~0u);
                 if (threadIdx.x == 0)
-                    e.deep[(uint64_t)item.s * kDeepLevels + j] = make_uint2(
-                        min(c3[0], 65535u) | (min(c3[1], 65535u) << 16), min(c3[2], 65535u) | ((fits ? 1u : 0u) << 16));
+                    e.deep[(uint64_t)item.s * kDeepLevels + j] =
+                        make_uint2(min(c3[0], 65535u) | (min(c3[1], 65535u) << 16),
+                                   min(c3[2], 65535u) | ((peak <= 65535u ? peak : 0u) << 16));
                 j++;
                 more = fits && n <= item.likely && j < item.levels;
             }
@@ -1387,34 +1398,33 @@ __global__ void k_share_prep(EncodeLaunch e) {
     e.share_prep[s] = pr;
 }
 
-// A level past the window from a slice's deep ladder: its size, and whether
-// it fits.
-__device__ __forceinline__ uint32_t deep_size(const SharePrep &p, uint2 v, bool &fits) {
-    fits = (v.y >> 16) != 0;
+// The size at a level past the window, from a slice's deep ladder (a level that
+// fits).
+__device__ __forceinline__ uint32_t deep_size(const SharePrep &p, uint2 v) {
     return p.hba + (v.x & 0xFFFFu) + (v.x >> 16) + (v.y & 0xFFFFu);
 }
 
-// A slice's deep levels (level j at deep[32 j]) continuing SharePrep::thr:
-// tab[32 j] the least D that lets the slice take kWindow + 1 + j steps.
-__device__ __forceinline__ void deep_table(const SharePrep &p, const uint2 *deep, uint64_t *tab) {
-    uint64_t run = p.thr[kWindow - 1];
-#pragma unroll 4
-    for (uint32_t j = 0; j < p.deep_count; j++) {
-        bool fits;
-        const uint32_t n = deep_size(p, deep[32u * j], fits);
-        const uint64_t over = n <= p.base ? 0u : n - p.base;
-        const uint64_t thr = fits ? (over * p.rem + (1u << p.shift) - 1u) >> p.shift : ~(uint64_t)0;
-        run = max(run, thr);
-        tab[32u * j] = run;
-    }
-}
-
-// The deep levels that D lets the slice take: a binary search.
-__device__ __forceinline__ uint32_t deep_steps(const uint64_t *tab, uint32_t len, uint64_t D) {
-    uint32_t lo = 0, hi = len;
+// The deep levels (level j at deep[32 j]) that D lets the slice take, all of
+// the window's taken. A level's threshold on D grows with its size, so the
+// running maximum of the thresholds is at most D where the ladder's peak is
+// within the allowance that D gives: a binary search of the peaks, which only
+// grow, from the levels taken at the last D (`last`) on. (A table of 64-bit
+// thresholds for each chunk of 32 slices took 6,500 cycles to build where the
+// ladders are long: 96 frames of mixed sizes 3.43 -> 2.66 ms without it.)
+__device__ __forceinline__ uint32_t deep_steps(const SharePrep &p, const uint2 *deep, uint32_t last, uint64_t D) {
+    const uint64_t allowed = p.base + (D << p.shift) / p.rem;
+    const uint32_t limit = (uint32_t)min(allowed, (uint64_t)65535u);
+    const auto taken = [&](uint32_t j) { return (deep[32u * j].y >> 16) - 1u < limit; };
+    uint32_t lo = 0, hi = p.deep_count;
+    if (last > 0 && !taken(last - 1u))
+        hi = last - 1u;
+    else if (last < hi && !taken(last))
+        lo = hi = last;
+    else
+        lo = last;
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (tab[32u * mid] <= D)
+        if (taken(mid))
             lo = mid + 1u;
         else
             hi = mid;
@@ -1447,11 +1457,10 @@ struct ShareShared {
     uint32_t sizes[2][kShareTries][3];
     ShareJob job;
     // Per lane, of the 32 slices being settled and of the next ones: their
-    // thresholds (16-byte words, of two chunks ahead), their ladders (of one
-    // ahead), and the deep levels' table.
+    // thresholds (16-byte words, of two chunks ahead) and their ladders (of one
+    // ahead).
     uint4 prep[3][sizeof(SharePrep) / sizeof(uint4)][32];
     uint2 ladder[2][kDeepLevels][32];
-    uint64_t table[kDeepLevels][32];
 };
 
 __device__ __forceinline__ void copy8_async(void *dst, const void *src) {
@@ -1592,8 +1601,7 @@ __device__ void share_settle(const EncodeLaunch &e, const EncPicDesc &pd, uint64
             for (int j = 0; j < kWindow; j++) mine.thr[j] = ~0ull;
         }
         const uint2 *my_deep = &sh.ladder[half][0][lane];
-        uint64_t *my_table = &sh.table[0][lane];
-        bool table_built = false;
+        uint32_t last_deep = 0;  // deep levels taken at the last D
         uint32_t my_steps = 0;
         uint32_t done = 0;  // lanes below are settled
         while (done < 32u) {
@@ -1623,13 +1631,10 @@ __device__ void share_settle(const EncodeLaunch &e, const EncPicDesc &pd, uint64
                 }
                 const bool past = ks == (uint32_t)kWindow && mine.deep_count > 0;
                 if (__any_sync(0xffffffffu, past)) {
-                    if (!table_built) deep_table(mine, my_deep, my_table);
-                    table_built = true;
-                    const uint32_t j = past ? deep_steps(my_table, mine.deep_count, myD) : 0u;
-                    if (j) {
-                        bool fits;
-                        ks += j;
-                        mine_dl = (int32_t)(deep_size(mine, my_deep[32u * (j - 1u)], fits) - mine.base);
+                    if (past) last_deep = deep_steps(mine, my_deep, last_deep, myD);
+                    if (past && last_deep) {
+                        ks += last_deep;
+                        mine_dl = (int32_t)(deep_size(mine, my_deep[32u * (last_deep - 1u)]) - mine.base);
                     }
                 }
                 const uint32_t deep_mask =
@@ -1678,8 +1683,8 @@ __device__ void share_settle(const EncodeLaunch &e, const EncPicDesc &pd, uint64
 // them 700 in its two rounds (thresholds against D, the votes, a scan), 200 to
 // start the next chunks' copies. One UHD frame 122 -> 73 us, 30 of them 152 ->
 // 85, and 32 frames of mixed sizes, whose slices often get past their ladders,
-// 1243 -> 516. Before, each round ended with a scan, also to find that nothing
-// had moved; each chunk built its lanes' whole tables first (10,000 cycles
+// 1243 -> 503. Before, each round ended with a scan, also to find that nothing
+// had moved; each chunk built tables of its lanes' thresholds first (10,000 cycles
 // where the ladders are long); and the one warp copied a slice past its ladder
 // in and costed it alone (24,000 cycles a slice, 7,000 now).
 __global__ void __launch_bounds__(kShareThreads) k_shareout(EncodeLaunch e) {

@@ -117,6 +117,7 @@ constexpr size_t kQuantKey = 129;
 struct DeepItem {
     uint64_t likely;
     uint32_t s, levels, hba;
+    uint32_t peak;  // the largest size of its window levels (~0: one unknown)
 };
 
 struct EncodeLaunch {
@@ -142,7 +143,8 @@ struct EncodeLaunch {
     SharePrep *share_prep; // [slice]
     uint32_t *share_steps; // [slice] finer steps taken (top bit: sizes already in final_comp)
     uint2 *deep;           // [slice][kDeepLevels] component bytes past the window: x = Y' | Cb << 16,
-                           //   y = Cr | fits << 16 (sizes saturate at 65535, which never fits)
+                           //   y = Cr | peak << 16: the largest slice size down to that level, the
+                           //   window's included; 0: one did not fit (the bytes saturate at 65535)
     uint32_t *deep_count;  // [slice] levels in deep
     DeepItem *deep_list;   // [slice] the slices with a ladder
     uint32_t *deep_listed; // [2] how many, and how many k_cost_deep has taken
