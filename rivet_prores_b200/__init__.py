@@ -716,9 +716,12 @@ class Encoder:
         return _encode_into(self.device, cfgs, ins, n, outs, status, True, stream)
 
 
-_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
+# Handles of this module's own: the prototypes set on ctypes.pythonapi's
+# functions hold for every user of them in the process.
+_python = ctypes.PyDLL(None)
+_new_bytes = _python.PyBytes_FromStringAndSize
 _new_bytes.restype, _new_bytes.argtypes = ctypes.py_object, [ctypes.c_char_p, ctypes.c_ssize_t]
-_bytes_at = ctypes.pythonapi.PyBytes_AsString
+_bytes_at = _python.PyBytes_AsString
 _bytes_at.restype, _bytes_at.argtypes = ctypes.c_void_p, [ctypes.py_object]
 
 
