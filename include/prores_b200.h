@@ -256,9 +256,24 @@ int prores_decode_device(prores_ctx *ctx, const uint8_t *d_data, size_t data_len
 int prores_encode_device(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, prores_buf *out,
                          int *status, void *stream);
 
+/* The packets of a prores_encode_hold call, where the library keeps them. */
+typedef struct prores_packets prores_packets;
+
+/* prores_encode_batch (device_frames 0; `stream` NULL) or prores_encode_device
+ * (device_frames 1) with the packets left where they arrive: out[i].data
+ * points into the library's page-locked memory until the caller gives *held
+ * (NULL unless PRORES_OK) to prores_packets_free, before prores_destroy. A
+ * caller copies each packet once, at a time of its own, and may give up in
+ * between. Until then the call's workspace, its device buffers included,
+ * serves no other call. */
+int prores_encode_hold(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, int device_frames,
+                       prores_buf *out, int *status, void *stream, prores_packets **held);
+void prores_packets_free(prores_packets *held);
+
 /* Where a packet of prores_encode_into goes: room for `len` bytes for frame
  * i's packet, which the call fills before it returns, or NULL to give the
- * whole call up. Called on the calling thread, once a packet. */
+ * whole call up. Called on the calling thread, once a packet; it has to
+ * return (an exception or a longjmp must not leave through the library). */
 typedef uint8_t *(*prores_packet_room)(void *user, int i, size_t len);
 
 /* prores_encode_batch (device_frames 0; `stream` NULL) or prores_encode_device

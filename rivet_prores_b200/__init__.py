@@ -674,7 +674,7 @@ class Encoder:
             cfgs[i] = configs[i]._c()
             ins[i] = _frame_to_c(frames[i], keep)
         if not devices:
-            return _encode_into(self.device, cfgs, ins, n, outs, status)
+            return _encode_once(self.device, cfgs, ins, n, outs, status)
         ctxs = (ctypes.c_void_p * len(devices))(*[context(d).handle for d in devices])
         code = L.prores_encode_batch_multi(ctxs, len(devices), cfgs, ins, n, outs, status)
         if code != _abi.OK:
@@ -713,7 +713,7 @@ class Encoder:
             if f.alpha is not None:
                 c.alpha = ctypes.cast(_device_ptr(f.alpha), ctypes.POINTER(ctypes.c_uint16))
                 c.alpha_len = int(f.alpha.numel())
-        return _encode_into(self.device, cfgs, ins, n, outs, status, True, stream)
+        return _encode_once(self.device, cfgs, ins, n, outs, status, True, stream)
 
 
 # Handles of this module's own: the prototypes set on ctypes.pythonapi's
@@ -725,23 +725,29 @@ _bytes_at = _python.PyBytes_AsString
 _bytes_at.restype, _bytes_at.argtypes = ctypes.c_void_p, [ctypes.py_object]
 
 
-def _encode_into(device: int, cfgs, ins, n: int, outs, status, device_frames: bool = False,
+def _encode_once(device: int, cfgs, ins, n: int, outs, status, device_frames: bool = False,
                  stream=None) -> List[Union[bytes, Error]]:
-    """One encode call whose packets the library writes straight into new
-    bytes objects."""
-    res: List[Union[bytes, Error, None]] = [None] * n
-
-    def room(_, i, size):
-        res[i] = _new_bytes(None, size)
-        return _bytes_at(res[i])
-
-    code = _abi.lib().prores_encode_into(context(device).handle, cfgs, ins, n, int(device_frames),
-                                         _abi.PACKET_ROOM(room), None, outs, status, _stream_ptr(stream))
-    if code != _abi.OK:
-        raise _error(code)
-    for i in range(n):
-        if status[i] != _abi.OK:
-            res[i] = _error(status[i], _abi.batch_error(i))
+    """One encode call whose packets are copied once, from where they arrive
+    into new bytes objects. No Python code runs inside the library's call: an
+    exception there (a signal's handler may raise one anywhere) could not
+    leave it."""
+    L = _abi.lib()
+    held = ctypes.c_void_p()
+    res: List[Union[bytes, Error]] = []
+    try:
+        code = L.prores_encode_hold(context(device).handle, cfgs, ins, n, int(device_frames), outs, status,
+                                    _stream_ptr(stream), ctypes.byref(held))
+        if code != _abi.OK:
+            raise _error(code)
+        for i in range(n):
+            if status[i] != _abi.OK:
+                res.append(_error(status[i], _abi.batch_error(i)))
+            else:
+                packet = _new_bytes(None, outs[i].len)
+                ctypes.memmove(_bytes_at(packet), outs[i].data, outs[i].len)
+                res.append(packet)
+    finally:
+        L.prores_packets_free(held)
     return res
 
 

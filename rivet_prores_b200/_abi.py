@@ -167,6 +167,9 @@ def lib():
                                                 vp]),
         "prores_encode_into": (ctypes.c_int, [vp, P(Config_), P(Frame_), ctypes.c_int, ctypes.c_int, PACKET_ROOM, vp,
                                               P(Buf_), P(ctypes.c_int), vp]),
+        "prores_encode_hold": (ctypes.c_int, [vp, P(Config_), P(Frame_), ctypes.c_int, ctypes.c_int, P(Buf_),
+                                              P(ctypes.c_int), vp, P(vp)]),
+        "prores_packets_free": (None, [vp]),
         "prores_set_tuning": (ctypes.c_int, [vp, P(Tuning_)]),
         "prores_get_tuning": (ctypes.c_int, [vp, P(Tuning_)]),
         "prores_set_timeout": (ctypes.c_int, [vp, ctypes.c_uint32]),

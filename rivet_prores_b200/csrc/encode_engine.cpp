@@ -517,29 +517,39 @@ static bool profiling_on() {
 
 extern "C" {
 
-// `room` (null: malloc) gives each packet's place.
-static int encode_batch(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, prores_buf *out,
-                        int *status, bool device_frames, void *stream, prores_packet_room room = nullptr,
-                        void *user = nullptr) {
+// Encodes the batch; `packets` then lie in the staging buffer of `ws`.
+static int encode_staged(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, int *status,
+                         bool device_frames, void *stream, std::unique_ptr<Workspace> &ws,
+                         std::vector<prores_buf> &packets) {
     if (!ctx || n < 0) return efail(make_status(PRORES_CONFIG, "no context"));
     cudaSetDevice(ctx->impl.device);
     EncodePlanPtr plan;
     Status st = plan_encode(cfg, in, n, plan);
     if (st) return efail(st);
-    auto ws = ctx->impl.acquire();
+    ws = ctx->impl.acquire();
     if (!ws) return efail(make_status(PRORES_DEVICE, "no stream"));
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ws->stream;
     st = upload_encode(ctx->impl, *ws, *plan, in, s, true, device_frames);
     if (!st) st = enqueue_encode(ctx->impl, *ws, *plan, s, nullptr);
-    std::vector<prores_buf> packets;
     Status first;
     if (!st) st = fetch_encode(ctx->impl, *ws, *plan, s, packets, status, &first);
     if (st) {
         ctx->impl.release_or_retire(std::move(ws));
         return efail(st);
     }
-    // The packets lie in the workspace's staging buffer: copied out before
-    // the workspace goes back to the pool.
+    if (first) set_last_error(first);
+    return PRORES_OK;
+}
+
+// `room` (null: malloc) gives each packet's place.
+static int encode_batch(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, prores_buf *out,
+                        int *status, bool device_frames, void *stream, prores_packet_room room = nullptr,
+                        void *user = nullptr) {
+    std::unique_ptr<Workspace> ws;
+    std::vector<prores_buf> packets;
+    const int code = encode_staged(ctx, cfg, in, n, status, device_frames, stream, ws, packets);
+    if (code != PRORES_OK) return code;
+    // The packets are copied out before the workspace goes back to the pool.
     for (int i = 0; i < n; i++) {
         out[i].data = nullptr;
         out[i].len = 0;
@@ -559,7 +569,6 @@ static int encode_batch(prores_ctx *ctx, const prores_config *cfg, const prores_
         out[i].len = len;
     }
     ctx->impl.release(std::move(ws));
-    if (first) set_last_error(first);
     return PRORES_OK;
 }
 
@@ -577,6 +586,25 @@ int prores_encode_into(prores_ctx *ctx, const prores_config *cfg, const prores_f
                        prores_packet_room room, void *user, prores_buf *out, int *status, void *stream) {
     if (!room) return efail(make_status(PRORES_CONFIG, "no room for the packets"));
     return encode_batch(ctx, cfg, in, n, out, status, device_frames != 0, stream, room, user);
+}
+
+int prores_encode_hold(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, int n, int device_frames,
+                       prores_buf *out, int *status, void *stream, prores_packets **held) {
+    if (!held) return efail(make_status(PRORES_CONFIG, "nowhere to keep the packets"));
+    *held = nullptr;
+    std::unique_ptr<Workspace> ws;
+    std::vector<prores_buf> packets;
+    const int code = encode_staged(ctx, cfg, in, n, status, device_frames != 0, stream, ws, packets);
+    if (code != PRORES_OK) return code;
+    std::copy(packets.begin(), packets.end(), out);
+    *held = new prores_packets{ctx, std::move(ws)};
+    return PRORES_OK;
+}
+
+void prores_packets_free(prores_packets *held) {
+    if (!held) return;
+    held->ctx->impl.release(std::move(held->ws));
+    delete held;
 }
 
 int prores_encode(prores_ctx *ctx, const prores_config *cfg, const prores_frame *in, uint8_t **out, size_t *out_len) {

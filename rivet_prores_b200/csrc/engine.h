@@ -259,6 +259,11 @@ struct prores_decode_job {
     prores::KernelTimes kt;
 };
 
+struct prores_packets {
+    prores_ctx *ctx;
+    std::unique_ptr<prores::Workspace> ws;  // its staging buffer holds them
+};
+
 struct prores_encode_job {
     prores_ctx *ctx = nullptr;
     std::unique_ptr<prores::Workspace> ws;
