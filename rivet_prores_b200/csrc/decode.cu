@@ -1130,7 +1130,7 @@ __global__ void __launch_bounds__(32 * kIdctWarps, 12) k_idct(DecodeLaunch d) {
     };
     const auto fetch = [&](const List &l, uint32_t i) {
         i += 4u * lane;
-        return i < l.n ? __ldg(reinterpret_cast<const uint4 *>(l.words + i)) : make_uint4(0, 0, 0, 0);
+        return i < l.n ? *reinterpret_cast<const uint4 *>(l.words + i) : make_uint4(0, 0, 0, 0);
     };
     List list = open(0, c0);
     uint4 e = fetch(list, 0);
@@ -1187,9 +1187,9 @@ __global__ void __launch_bounds__(32 * kIdctWarps, 12) k_idct(DecodeLaunch d) {
             if (i + 3u < list.n) place(e.w);
         } else {
             for (i = lane; i < list.n; i += 32u) {
-                const uint32_t x = __ldg(list.words + i), mag = (x >> 5) & 0xFFFFu;
+                const uint32_t x = list.words[i], mag = (x >> 5) & 0xFFFFu;
                 put(x, mag < kListBigMag ? small(x)
-                                         : __int2float_rn((int32_t)__ldg(list.words + 128u * list.nb - 1u - (mag - kListBigMag))));
+                                         : __int2float_rn((int32_t)list.words[128u * list.nb - 1u - (mag - kListBigMag)]));
             }
         }
         list = next;

@@ -515,14 +515,12 @@ struct CountSink {
     }
 };
 
-// kShared: f and cmax point into shared memory (plain loads); else into
-// global memory (read-only loads).
+// kShared: f and cmax point into shared memory; else into global memory. Plain
+// loads there too, since a kernel of the chain writes them (chain.h).
 template <bool kShared>
 __device__ __forceinline__ float coef_load(const float *f, uint32_t i) {
-    if constexpr (kShared)
-        return f[i];
-    else
-        return __ldg(f + i);
+    if constexpr (!kShared) __builtin_assume(__isGlobal(f));
+    return f[i];
 }
 
 // Length of the code of a DC difference's symbol n by a = min(|previous
@@ -653,10 +651,8 @@ struct NonzeroList {
 
 template <bool kShared>
 __device__ __forceinline__ float4 coef_load4(const float *f) {
-    if constexpr (kShared)
-        return *reinterpret_cast<const float4 *>(f);
-    else
-        return __ldg(reinterpret_cast<const float4 *>(f));
+    if constexpr (!kShared) __builtin_assume(__isGlobal(f));
+    return *reinterpret_cast<const float4 *>(f);
 }
 
 // The AC non-zeros of a component of 2^kLog blocks, every coefficient in turn. A lane takes four neighbouring positions of each run
@@ -1501,7 +1497,7 @@ __device__ void share_help(const EncodeLaunch &e, const EncPicDesc &pd, int32_t 
         for (uint32_t i = tid; i < total / 4u; i += 32u * kShareHelpers)
             copy16_async(sh.stage + 4u * i, e.coef + sd.coef + 4u * i);
         const float *msrc = e.coef_max + (sd.coef >> 5);
-        for (uint32_t i = tid; i < total / 32u; i += 32u * kShareHelpers) smax[i] = __ldg(msrc + i);
+        for (uint32_t i = tid; i < total / 32u; i += 32u * kShareHelpers) smax[i] = msrc[i];
         const uint64_t allowed = job.base + job.D * sd.mbs / mbs_from(pd, sd);
         copies_wait();
         share_barrier(kHelpersOnly, 32 * kShareHelpers);
