@@ -384,16 +384,18 @@ __device__ __forceinline__ float nonzero_bound(float inv) {
     return __double2float_rd(__ddiv_rn(y0 * (1.0 - 1.0 / (1 << 22)), (double)inv));
 }
 
-// A CTA per quantization_index and set (layout beside kQuantStride): inv[scan[k]] =
-// 8 / (W[k] qScale) in single precision for luma and chroma
+// A CTA per set and quantization_index, one after another in the grid's x
+// (y and z end at 65535): inv[scan[k]] = 8 / (W[k] qScale), laid out as beside
+// kQuantStride, in single precision for luma and chroma
 // (src/encode.rs:303-329), the non-zero bound of each, and the least bound
 // over each chunk of 32 scanned coefficients. On the host the 225 quantisers
 // of a set took about half a millisecond of every call.
 __global__ void __launch_bounds__(128) k_quant(float *quant, const uint8_t *keys) {
     __shared__ float bound[128];
-    const uint32_t qi = blockIdx.x, i = threadIdx.x, k = i & 63u, g = i >> 6;
-    const uint8_t *key = keys + kQuantKey * blockIdx.y;
-    float *t = quant + ((uint64_t)blockIdx.y * 225u + qi) * kQuantStride;
+    const uint32_t set = blockIdx.x / 225u, qi = blockIdx.x - 225u * set;
+    const uint32_t i = threadIdx.x, k = i & 63u, g = i >> 6;
+    const uint8_t *key = keys + kQuantKey * set;
+    float *t = quant + (uint64_t)blockIdx.x * kQuantStride;
     const uint32_t at = 64u * g + c_enc_scan[key[128]][k];
     const float inv = __fdiv_rn(8.0f, (float)((uint32_t)key[i] * qscale(qi < 1u ? 1u : qi)));
     t[at] = inv;
@@ -2171,7 +2173,7 @@ __global__ void __launch_bounds__(32 * kAlphaWarps) k_pack_alpha(EncodeLaunch e)
 }  // namespace
 
 cudaError_t launch_quant(float *quant, const uint8_t *keys, uint32_t sets, cudaStream_t s) {
-    k_quant<<<dim3(225, sets), 128, 0, s>>>(quant, keys);
+    k_quant<<<225u * sets, 128, 0, s>>>(quant, keys);
     return cudaGetLastError();
 }
 
