@@ -1228,7 +1228,8 @@ __global__ void __launch_bounds__(kDeepThreads, kDeepBlocks) k_cost_deep(EncodeL
     }
 }
 
-constexpr int kRcThreads = 1024;
+// Threads a picture of k_rc_init and k_rc_step, at most and at least (rc_threads).
+constexpr int kRcThreads = 1024, kRcThreadsMin = 64;
 
 __device__ __forceinline__ uint64_t block_sum_u64(uint64_t v, uint64_t *sh) {
 #pragma unroll
@@ -1249,7 +1250,7 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_init(EncodeLaunch e) {
     const EncPicDesc pd = e.pics[blockIdx.x];
     uint64_t a = 0;
     if (e.any_alpha)
-        for (uint32_t k = threadIdx.x; k < pd.n_slices; k += kRcThreads) a += e.alpha_bytes[pd.slice_base + k];
+        for (uint32_t k = threadIdx.x; k < pd.n_slices; k += blockDim.x) a += e.alpha_bytes[pd.slice_base + k];
     const uint64_t alpha = block_sum_u64(a, sh);
     if (threadIdx.x == 0) {
         // Alpha is lossless and comes on top of the rate; the picture
@@ -1288,7 +1289,7 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_step(EncodeLaunch e, int step
     uint64_t sum = 0;
     bool fit = true;
 #pragma unroll 4
-    for (uint32_t k = threadIdx.x; k < pd.n_slices; k += kRcThreads) {
+    for (uint32_t k = threadIdx.x; k < pd.n_slices; k += blockDim.x) {
         const uint32_t s = pd.slice_base + k;
         const uint32_t *c = e.probe_comp + ((uint64_t)step * e.n_slices + s) * 3u;
         const uint32_t cc[3] = {c[0], c[1], c[2]};
@@ -2192,9 +2193,20 @@ cudaError_t launch_alpha_size(const EncodeLaunch &e, cudaStream_t s) {
     return launch_chained(k_alpha_size, (e.n_slices + kAlphaWarps - 1) / kAlphaWarps, 32 * kAlphaWarps, 0, s, e);
 }
 
+// A picture's threads in the bisection step: as many as leave every picture's
+// block a place (2048 threads an SM), since more go through its slices sooner
+// (9 steps of 30 UHD frames 162 us with 256, 107 with 1024) and blocks that wait
+// for a place cost all of them a round (4,096 frames of 16x16 72 us a step with
+// 1024 threads each, 10 with 128; 131,072 of them 2230 and, with 64, 141).
+static uint32_t rc_threads(const EncodeLaunch &e) {
+    uint32_t threads = kRcThreads;
+    while (threads > kRcThreadsMin && (uint64_t)threads * e.n_pics > 2048ull * (uint32_t)e.sm_count) threads /= 2;
+    return threads;
+}
+
 cudaError_t launch_rc_init(const EncodeLaunch &e, cudaStream_t s) {
     if (!e.n_pics) return cudaSuccess;
-    return launch_chained(k_rc_init, e.n_pics, kRcThreads, 0, s, e);
+    return launch_chained(k_rc_init, e.n_pics, rc_threads(e), 0, s, e);
 }
 
 // CTAs of a kernel that walks `items` warp items at a stride: all that are
@@ -2219,7 +2231,7 @@ cudaError_t launch_cost(const EncodeLaunch &e, int step, cudaStream_t s) {
 
 cudaError_t launch_rc_step(const EncodeLaunch &e, int step, cudaStream_t s) {
     if (!e.n_pics) return cudaSuccess;
-    return launch_chained(k_rc_step, e.n_pics, kRcThreads, 0, s, e, step);
+    return launch_chained(k_rc_step, e.n_pics, rc_threads(e), 0, s, e, step);
 }
 
 cudaError_t launch_cost_window(const EncodeLaunch &e, int level, cudaStream_t s) {
