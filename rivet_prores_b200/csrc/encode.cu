@@ -937,6 +937,11 @@ __global__ void __launch_bounds__(kCostThreads, kCostBlocks) k_cost(EncodeLaunch
             if (qi != 0) my_blocks = (comp == 0 ? 4u : sd.cpm) * sd.mbs;
         }
         const uint32_t costed = __ballot_sync(0xffffffffu, my_blocks != 0);
+        // With no picture left to cost (each is down to one quantiser, or the
+        // coarsest did not fit its target) the other items are not looked at:
+        // 4 UHD frames 10 us for such a probe, 39 with them. Asked only by a warp
+        // whose items are all settled, so it costs the other probes nothing.
+        if (!costed && step > 0 && e.searching[step] == 0) break;
         // The next item's maxima and DCs are on their way while one is costed.
         CompHead next_head{};
         uint32_t next_blocks = 0;
@@ -1270,7 +1275,7 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_init(EncodeLaunch e) {
         e.state[blockIdx.x] = st;
         if (blockIdx.x == 0) {
             for (int j = 0; j < kWindow; j++) e.win_count[j] = 0;
-            for (int j = 0; j < kProbeSteps; j++) e.cost_taken[j] = 0;
+            for (int j = 0; j < kProbeSteps; j++) e.cost_taken[j] = e.searching[j] = 0;
             e.deep_listed[0] = e.deep_listed[1] = 0;
         }
     }
@@ -1330,6 +1335,7 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_step(EncodeLaunch e, int step
             }
         }
         e.state[blockIdx.x] = st;
+        if (st.probe_qi != 0 && step + 1 < kProbeSteps) atomicAdd(e.searching + step + 1, 1u);
     }
 }
 
@@ -2197,7 +2203,7 @@ cudaError_t launch_alpha_size(const EncodeLaunch &e, cudaStream_t s) {
 // block a place (2048 threads an SM), since more go through its slices sooner
 // (9 steps of 30 UHD frames 162 us with 256, 107 with 1024) and blocks that wait
 // for a place cost all of them a round (4,096 frames of 16x16 72 us a step with
-// 1024 threads each, 10 with 128; 131,072 of them 2230 and, with 64, 141).
+// 1024 threads each, 10 with 64; 131,072 of them 2230 and 141).
 static uint32_t rc_threads(const EncodeLaunch &e) {
     uint32_t threads = kRcThreads;
     while (threads > kRcThreadsMin && (uint64_t)threads * e.n_pics > 2048ull * (uint32_t)e.sm_count) threads /= 2;

@@ -284,6 +284,7 @@ static EncodeLaunch encode_params(Context &ctx, Workspace &ws, const EncodePlan 
     e.cost_taken = reinterpret_cast<uint32_t *>(base + o);
     e.deep_listed = e.cost_taken + kProbeSteps;
     e.pack_taken = e.deep_listed + 2;
+    e.searching = e.pack_taken + 1;
     e.out = ws.enc_out.as<uint32_t>();
     e.headers = ws.enc_frame_out.as<uint8_t>();
     e.frame_status = ws.enc_alpha_bits.as<uint32_t>();
@@ -300,7 +301,7 @@ static EncodeLaunch encode_params(Context &ctx, Workspace &ws, const EncodePlan 
 static size_t cost_bytes(const EncodePlan &plan) {
     const size_t ns = plan.n_slices + 1;
     return 4 * ns * (1 + 3 * kProbeSteps + 3 * kWindow + 3 + 1) + 8 * ns + sizeof(SharePrep) * ns + 4 * ns + 4 * ns +
-           4 * ns + (sizeof(uint2) * kDeepLevels + sizeof(DeepItem)) * ns + 4 * kWindow + 4 * (kProbeSteps + 3) + 256;
+           4 * ns + (sizeof(uint2) * kDeepLevels + sizeof(DeepItem)) * ns + 4 * kWindow + 4 * (2 * kProbeSteps + 3) + 256;
 }
 
 static Status upload_frames(Workspace &ws, const EncodePlan &plan, const prores_frame *in, cudaStream_t s,

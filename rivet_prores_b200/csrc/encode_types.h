@@ -149,6 +149,7 @@ struct EncodeLaunch {
     DeepItem *deep_list;   // [slice] the slices with a ladder
     uint32_t *deep_listed; // [2] how many, and how many k_cost_deep has taken
     uint32_t *pack_taken;  // items the warps of k_pack have taken
+    uint32_t *searching;   // [kProbeSteps] pictures the probe is to cost (from the second on)
     uint32_t *out;         // output buffer (zeroed before packing), big-endian bit order
     const uint8_t *headers;  // frame header templates
     uint32_t *frame_status;  // per frame: 0, or 1 when the frame outgrew its region
