@@ -520,12 +520,14 @@ struct CountSink {
     }
 };
 
-// kShared: f and cmax point into shared memory; else into global memory. Plain
-// loads there too, since a kernel of the chain writes them (chain.h).
+// kShared: f and cmax point into shared memory; else into global memory, where
+// a kernel of the chain wrote them.
 template <bool kShared>
 __device__ __forceinline__ float coef_load(const float *f, uint32_t i) {
-    if constexpr (!kShared) __builtin_assume(__isGlobal(f));
-    return f[i];
+    if constexpr (kShared)
+        return f[i];
+    else
+        return chain_load(f + i);
 }
 
 // Length of the code of a DC difference's symbol n by a = min(|previous
@@ -656,8 +658,10 @@ struct NonzeroList {
 
 template <bool kShared>
 __device__ __forceinline__ float4 coef_load4(const float *f) {
-    if constexpr (!kShared) __builtin_assume(__isGlobal(f));
-    return *reinterpret_cast<const float4 *>(f);
+    if constexpr (kShared)
+        return *reinterpret_cast<const float4 *>(f);
+    else
+        return chain_load4(f);
 }
 
 // The AC non-zeros of a component of 2^kLog blocks, every coefficient in turn. A lane takes four neighbouring positions of each run
