@@ -142,6 +142,21 @@ inline void dct_basis(float out[64]) {
         }
 }
 
+// Whether T has the cosine's symmetries bit for bit, as the decoder's paired
+// sums need them (pair_math.h): T[7 - x][u] = (-1)^u T[x][u], and for even u
+// T[3 - x][u] = T[x][u] (u = 0, 4) or -T[x][u] (u = 2, 6). Rounding a cosine
+// once keeps them, but only if the math library's own result has them.
+inline bool dct_basis_mirrors(const float T[64]) {
+    bool ok = true;
+    for (int x = 0; x < 4; x++)
+        for (int u = 0; u < 8; u++) {
+            const float t = T[8 * x + u];
+            ok = ok && T[8 * (7 - x) + u] == (u % 2 == 0 ? t : -t);
+            if (u % 2 == 0) ok = ok && T[8 * (3 - x) + u] == (u % 4 == 0 ? t : -t);
+        }
+    return ok;
+}
+
 // Prefix tables for the decoder, one row per distinct codebook: Table 10's
 // run codebooks for previousRun 0-1, 2-3, 4, 5-8, 9-14, 15+ (rows 0-5) and
 // Table 11's level codebooks for previousLevelSymbol 0, 1, 2, 3, 4-7, 8+

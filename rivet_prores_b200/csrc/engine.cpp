@@ -751,6 +751,9 @@ static Status make_tables(Context &c) {
     PR_CUDA(cudaMemcpy(c.tables.level_books, level6.data(), level6.size() * 2, cudaMemcpyHostToDevice), "upload");
     float basis[64];
     dct_basis(basis);
+    if (!dct_basis_mirrors(basis))
+        return make_status(PRORES_DEVICE, "the math library's cosines are not symmetric to the last bit, "
+                                          "which the inverse transform relies on");
     PR_CUDA(cudaMalloc(&c.tables.basis, sizeof basis), "cudaMalloc");
     PR_CUDA(cudaMemcpy(c.tables.basis, basis, sizeof basis, cudaMemcpyHostToDevice), "upload");
     return Status();

@@ -42,13 +42,13 @@ __device__ __forceinline__ uint64_t pair_sub(uint64_t a, uint64_t b) {
 }
 
 // The 8-point basis T[x][u] (dct_basis) in single precision has the cosine's
-// symmetries bit for bit: T[7 - x][u] = (-1)^u T[x][u], and for even u
-// T[3 - x][u] = T[x][u] (u = 0, 4) or -T[x][u] (u = 2, 6). So in
-// out[x] = sum_u F[u] T[x][u] the eight products of one u are two (u even) or
-// four (u odd) products and their exact negatives, and with the outputs
-// paired as (0, 1), (7, 6), (3, 2), (4, 5) every pair adds or subtracts one
-// of two product pairs: 24 products and 32 paired sums for 8 outputs, each
-// output's terms in the same order and rounded alike.
+// symmetries bit for bit (every context checks it: dct_basis_mirrors):
+// T[7 - x][u] = (-1)^u T[x][u], and for even u T[3 - x][u] = T[x][u] (u = 0, 4)
+// or -T[x][u] (u = 2, 6). So in out[x] = sum_u F[u] T[x][u] the eight products
+// of one u are two (u even) or four (u odd) products and their exact negatives,
+// and with the outputs paired as (0, 1), (7, 6), (3, 2), (4, 5) every pair adds
+// or subtracts one of two product pairs: 24 products and 32 paired sums for 8
+// outputs, each output's terms in the same order and rounded alike.
 struct Pairs8 {
     uint64_t o01, o76, o32, o45;
 };
