@@ -74,7 +74,7 @@ CAPTURED = {
 # bandwidth: the work is byte and integer work, no tensor-core math); none of
 # these kernels reaches it, and "limiter" names what holds it back instead.
 LIMITER = {
-    "k_cost": "instruction issue (79 % of issue slots active), and at the dense probes DRAM at 4.8 TB/s",
+    "k_cost": "instruction issue (79 % of issue slots active), with DRAM at 3.7 TB/s beside it (8 frames, a dense probe)",
     "k_cost_window": "instruction issue, as k_cost; it costs a list of slices that changes with the pictures (level 0 "
                      "copies from a probe at the same quantiser where there is one), so it has no fixed byte basis",
     "k_fdct": "instruction issue (76 % of issue slots active)",

@@ -167,8 +167,8 @@ inline bool dct_basis_mirrors(const float T[64]) {
 // level (bits 5-11) and the row the next code of the same kind is read with,
 // the row of the context this symbol makes (bits 12-14, in place as that
 // row's byte offset); kBookMiss otherwise (the decoder then reads the
-// codeword by arithmetic). Eleven bits hold every run below 124 and level
-// below 125.
+// codeword by arithmetic). Eleven bits hold every run and level up to 31 in any
+// context, and up to 123 and 124 in the last ones.
 static constexpr uint32_t kBookBits = 11;
 static constexpr uint32_t kBookEntries = 1u << kBookBits;
 static constexpr uint32_t kBookTableWords = 6 * kBookEntries;

@@ -920,12 +920,12 @@ constexpr int kEntropyMaxThreads = 512;
 // started last they would leave the launch waiting on them.
 //
 // Bound by the length of a component's chain of codes (small batches: a step
-// waits for two table reads one after the other) and by integer issue (full
-// ones: 63 % of the slots, 72 % of the ALU pipe, 22 of 32 lanes at work).
+// waits for two table reads one after the other) and by integer issue (8 UHD
+// frames: 60 % of the slots, 68 % of the ALU pipe, 29 of 32 lanes at work).
 // 32 UHD 4:2:2 frames take 680 us, one 175, 8 UHD 4:4:4 frames with 16-bit
 // alpha 1030; with a branch for every case, loads and single-entry stores
-// among the steps, 1810, 535 and 2770. 83 registers leave 24 warps an SM;
-// held to 64 for 32 warps the spills cost 14 %.
+// among the steps, 1810, 535 and 2770. 83 registers, given out as 88, leave
+// two CTAs of 8 warps an SM; held to 64, for four, the spills cost 14 %.
 __global__ void __launch_bounds__(kEntropyMaxThreads) k_entropy(DecodeLaunch d) {
     chain_start();
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1554,8 +1554,8 @@ cudaError_t launch_locate(const DecodeLaunch &d, cudaStream_t s) {
     return launch_chained(k_locate, d.n_pics, kLocateThreads, 0, s, d);
 }
 
-// The prefix tables, and 8 words a lane for the rings: CTAs of 8 warps fill an
-// SM's 228 KB four times over to the byte.
+// The prefix tables, and 8 words a lane for the rings: 56 KB for 8 warps, of
+// which an SM would hold four (its registers hold two).
 static size_t entropy_smem_bytes(int warps_per_block) { return 2 * 2 * kBookTableWords + 1024u * warps_per_block; }
 
 cudaError_t launch_entropy(const DecodeLaunch &d, const EntropyShape &shape, cudaStream_t s) {

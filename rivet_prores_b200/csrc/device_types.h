@@ -106,9 +106,8 @@ struct PicStatus {
 
 // Constant tables the kernels read (built once per device).
 struct DeviceTables {
-    uint16_t *run_books;     // 6 x 512 packed prefix entries: a row per distinct run codebook (Table 10)
-    uint16_t *level_books;   // 6 x 512: a row per distinct level codebook (Table 11)
-    float *basis;            // T[x][u] at 8x + u, as the crate computes it
+    uint16_t *run_books;     // 6 x kBookEntries prefix entries: a row per distinct run codebook (Table 10)
+    uint16_t *level_books;   // 6 x kBookEntries: a row per distinct level codebook (Table 11)
 };
 
 // Zero bytes after the bitstreams of a batch.

@@ -849,7 +849,7 @@ __device__ __noinline__ uint32_t warp_wide_bits(const float *f, const float *inv
 // others are read. Every lane gets the sum.
 //
 // Bound by issue (79 % of the slots; 29 thread instructions a coefficient at
-// 36 % non-zeros, DRAM at 4.6 TB/s): 30 UHD 4:2:2 frames take 430 us a probe
+// 36 % non-zeros, DRAM at 4.8 TB/s): 30 UHD 4:2:2 frames take 430 us a probe
 // near the answer, where a lane per component walking its codes in order, each
 // look-up waiting for the last, took 800; 30 1080p frames 123 us for 700.
 template <bool kShared = false>
@@ -1272,7 +1272,6 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_init(EncodeLaunch e) {
         st.hi = 224;
         st.probe_qi = 224;
         st.hi_probe = 0;
-        st.lo_probe = -1;
         st.fits_at_all = 0;
         st.uniform = 224;
         st.quant = pd.quant;
@@ -1328,7 +1327,6 @@ __global__ void __launch_bounds__(kRcThreads) k_rc_step(EncodeLaunch e, int step
             st.hi_total = total;
         } else {
             st.lo = st.probe_qi + 1;
-            st.lo_probe = step;
         }
         if (st.fits_at_all) {
             if (st.lo < st.hi) {

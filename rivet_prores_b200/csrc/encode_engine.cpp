@@ -249,7 +249,6 @@ static EncodeLaunch encode_params(Context &ctx, Workspace &ws, const EncodePlan 
     e.coef = ws.enc_coef.as<float>();
     e.coef_max = e.coef + plan.coef_total + 64;
     e.quant = ws.weights.as<float>();
-    e.basis = ctx.tables.basis;
     // The per-slice tables share one allocation.
     size_t o = 0;
     e.alpha_bytes = reinterpret_cast<uint32_t *>(base + o);

@@ -71,7 +71,6 @@ struct EncPicState {
     int32_t lo, hi;      // bisection interval
     int32_t probe_qi;    // quantiser of the pass in flight (0: none)
     int32_t hi_probe;    // the probe step whose sizes are at `hi`
-    int32_t lo_probe;    // the failed probe step at lo - 1, or -1
     int32_t fits_at_all;
     int32_t uniform;
     uint32_t quant;      // the picture's quantiser table set (beside probe_qi, for k_cost)
@@ -130,7 +129,6 @@ struct EncodeLaunch {
     float *coef;           // transformed slices, scanned order
     float *coef_max;       // [coef / 32] the largest |F| of each 32 scanned coefficients (a chunk)
     const float *quant;    // [set][225 qi][kQuantStride], see quant_base
-    const float *basis;    // T[x][u]
     uint32_t *alpha_bytes; // per slice
     uint32_t *probe_comp;  // [kProbeSteps][slice][3] component bytes
     uint32_t *win_comp;    // [kWindow][slice][3]

@@ -370,7 +370,6 @@ Context::~Context() {
     retired.clear();
     if (tables.run_books) cudaFree(tables.run_books);
     if (tables.level_books) cudaFree(tables.level_books);
-    if (tables.basis) cudaFree(tables.basis);
 }
 
 Status record_kernel(KernelTimes *kt, const char *name, cudaStream_t s) {
@@ -754,8 +753,6 @@ static Status make_tables(Context &c) {
     if (!dct_basis_mirrors(basis))
         return make_status(PRORES_DEVICE, "the math library's cosines are not symmetric to the last bit, "
                                           "which the inverse transform relies on");
-    PR_CUDA(cudaMalloc(&c.tables.basis, sizeof basis), "cudaMalloc");
-    PR_CUDA(cudaMemcpy(c.tables.basis, basis, sizeof basis, cudaMemcpyHostToDevice), "upload");
     return Status();
 }
 
