@@ -9,16 +9,16 @@
 // before anything else and on every path: it returns when the kernel before
 // has completed, and so, each having waited in turn, all kernels before that.
 //
+// The exceptions are k_fdct and k_alpha_size, which the counting kernels
+// follow: they leave chain_start() to the end of their CTAs. With it, the next
+// kernels' large CTAs took places on the SMs that their own still had use for
+// (30 UHD frames 5.46 -> 5.63 ms, a batch of mixed sizes 5.06 -> 5.16).
+//
 // What a kernel of the chain writes is read with ordinary loads, never with
 // __ldg(): its non-coherent load wants memory that is read-only for the whole
 // life of the reading kernel, and that life begins while the writer may still
 // run. The bitstreams, the input planes, the code and quantiser tables are in
 // place before the chain and may be read either way.
-//
-// The exceptions are k_fdct and k_alpha_size, which the counting kernels
-// follow: they leave chain_start() to the end of their CTAs. With it, the next
-// kernels' large CTAs took places on the SMs that their own still had use for
-// (30 UHD frames 5.46 -> 5.63 ms, a batch of mixed sizes 5.06 -> 5.16).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -35,7 +35,8 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 // that the reading kernel does not write itself. Its address has to come from
 // something read after chain_wait(), which keeps the load behind the wait.
 // (As plain C++ loads, which stay between the stores and shuffles around them,
-// the counting kernels took 0.5 to 1.3 % longer.)
+// k_cost took 0.6 % longer: 30 UHD frames 3388 us for 3367, the mixed batch 2590
+// for 2574. With __ldg they were 3370 and 2567.)
 __device__ __forceinline__ float chain_load(const float *p) {
     float v;
     asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
